@@ -52,7 +52,7 @@ int check_device_error(Ctx* c) {
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
   if (h == 0) return 0;
   SBDX_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-  c->err = "device watchdog: a bulk-copy completion wait timed out in the alpha-beta sigma kernel (code " +
+  c->err = "device watchdog: a wait timed out in the alpha-beta sigma kernel (code " +
            std::to_string(h) + ")";
   return SBDX_ERR_CUDA;
 }
@@ -75,6 +75,7 @@ void free_vector_state(Ctx* c) {
   cudaFree(c->d_xp); c->d_xp = nullptr;
   cudaFree(c->d_y); c->d_y = nullptr;
   cudaFree(c->d_yt); c->d_yt = nullptr;
+  cudaFree(c->d_yab); c->d_yab = nullptr;
   cudaFree(c->d_io_in); c->d_io_in = nullptr;
   cudaFree(c->d_io_out); c->d_io_out = nullptr;
   cudaFree(c->d_wf); c->d_wf = nullptr; c->wf_roots = 0; c->wf_cap = 0;
@@ -178,6 +179,10 @@ int sbdx_ctx_destroy(sbdx_ctx* ctx) {
   cudaFree(c->d_a); cudaFree(c->d_b); cudaFree(c->d_red);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
+  for (auto& e : {c->fork, c->join[0], c->join[1]})
+    if (e) cudaEventDestroy(e);
+  for (auto& x : c->side)
+    if (x) cudaStreamDestroy(x);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   if (c->own_pool && c->pool) cudaMemPoolDestroy(c->pool);
   delete ctx;

@@ -45,16 +45,6 @@ constexpr uint32_t kInfoSingle = 1u << 30;
 // bit 41 set.
 struct SellPanel {
   uint64_t* sell = nullptr;        // [soff[nslice]]
-  // the same records in 32 bits (bits 0-15 position of the ket in the staged
-  // rows, Conn::kpos, relative to the panel's first ket; 16-27 pair index,
-  // 28 sign, 29 padding, 30 integral
-  // copy), read by the packed alpha-beta kernel in blocks of 4 per lane (a
-  // padding record repeats the addresses of a real record of its step):
-  // record m of lane l of slice s at sell32[soff4[s] + 128*(m/4) + 4*l + m%4],
-  // slen4[s] = slen[s] rounded up to a multiple of 4 (padding records)
-  uint32_t* sell32 = nullptr;      // [soff4[nslice]]
-  uint64_t* soff4 = nullptr;       // [nslice + 1]
-  uint32_t* slen4 = nullptr;       // [nslice]
   uint64_t* soff = nullptr;        // [nslice + 1]
   uint32_t* slen = nullptr;        // [nslice]
   uint32_t* vrow = nullptr;        // [nv]
@@ -64,41 +54,65 @@ struct SellPanel {
   size_t nslice = 0, nv = 0;
   int nsplit = 0, nslot = 0, cap = 0;
   int slices_per_warp = 8;         // 8, 12 or 16: virtual rows per CTA = 1024 * this
-  uint32_t jb0 = 0, jb1 = 0;
 };
 
-// Bra strings per block of the blocked same-spin kernel, and the determinant
-// counts from which the default launch codes use it (FP64, FP32 storage).
-constexpr int kBlkRows = 4;
+// Schedule of the packed alpha-beta kernel (built by ab_plan.cu). A record is
+// one beta single: bits 0-11 pair index, 12-27 y slot, 31 same-spin sign,
+// kAbPad: no single. Record m of thread t of batch b sits at
+// rec[4 * (boff[b] + (m / 4) * threads + t) + m % 4].
+constexpr uint32_t kAbPad = 1u << 30;
+struct AbPanel {
+  uint32_t* rec = nullptr;
+  uint64_t* boff = nullptr;     // [nbatch], in blocks of four records
+  uint32_t* bsteps = nullptr;   // [nbatch] steps
+  uint32_t* wsteps = nullptr;   // [nbatch][threads / 32] steps after which a warp is idle
+  uint32_t* ex_row = nullptr;   // [nex] bra strings (local) with extra y slots ...
+  uint32_t* ex_off = nullptr;   // [nex + 1] ... nmain + ex_off[e] .. nmain + ex_off[e + 1]
+  int nmain = 0, nex = 0, ny = 0;  // strings of the panel, strings with extras, y slots
+};
+struct AbPlan {
+  uint32_t* vket = nullptr;  // [xs] ket string of each lane
+  size_t xs = 0;             // nbatch * threads: row stride of Ctx::d_xk
+  int threads = 0, nbatch = 0, np = 0;
+  uint32_t vstr = 0;         // packs per staged integral row (pairs padded to 8)
+  std::vector<AbPanel> panels;
+};
+
+// Bra strings per block of the blocked same-spin kernels, and the determinant
+// counts from which the default launch codes use them (FP64, FP32 storage).
+constexpr int kBlkRows64 = 8, kBlkRows32 = 4;
 constexpr size_t kBlkMinDets64 = 2000000, kBlkMinDets32 = 1000000;
 constexpr uint32_t kNoRow = 0xffffffffu;
 
-// Blocks of the blocked same-spin kernel over the bra strings [row0, row1)
+// Blocks of the blocked same-spin kernels over the bra strings [row0, row1)
 // of one spin. The strings are ordered by their bit-reversed words (strings
 // with the same low-orbital holes and different high-orbital particles side
-// by side: their double excitations reach largely the same ket strings; at
-// 8000 sampled strings per spin the union of four neighbours' double lists
-// holds 0.44 of their entries, against 0.74 in ascending order) and cut into
-// blocks of kBlkRows. Per block the union of its strings' double-excitation
-// kets, ascending, with one signed same-spin value per string of the block
-// (zero where that string does not connect). Singles stay in the CSR.
+// by side: their excitations reach largely the same ket strings; at 8000
+// sampled strings per spin the union of eight neighbours' lists holds 0.31 of
+// their entries, of four 0.43) and cut into blocks of `width` (eight for the
+// FP64 kernel, four for the FP32 one). Per block the union of its strings' single- and double-excitation kets, ascending, padded
+// to a multiple of 8 entries with zero values, with one signed same-spin value
+// per string of the block (zero where that string does not connect).
+// Values: [entry][string].
 // Work items {block, first union entry, one past the last, 1 + partial slot
 // or 0}, longest first; a block with more union entries than the cap is
-// split, its first item also does the diagonal and the singles, and the
-// parts' kBlkRows partial rows (ypart[(slot * kBlkRows + r) * ldx ..]) are
-// summed in slot order by a fix-up kernel.
+// split, and the last of its CTAs to finish sums the parts' partial rows
+// (ypart[(slot * width + r) * pad8(ncol) ..]) in slot order.
 struct SameBlocks {
+  int width = 0;
   size_t nblk = 0, nu = 0;
-  uint4* rows = nullptr;     // [nblk] bra strings (kNoRow: none)
+  uint32_t* rows = nullptr;  // [nblk * width] bra strings (kNoRow: none)
   uint64_t* uoff = nullptr;  // [nblk + 1]
   uint32_t* uket = nullptr;  // [nu]
-  double* uval = nullptr;    // [nu * kBlkRows]
-  float* uval32 = nullptr;   // [nu * kBlkRows]
+  double* uval = nullptr;    // [nu * width] (width 8)
+  float* uval32 = nullptr;   // [nu * width] (width 4)
   uint4* item = nullptr;     // [n_item]
   size_t n_item = 0;
   uint4* split = nullptr;    // [n_split]: {block, first slot, parts, 0}
+  uint32_t* slot = nullptr;  // [n_part]: entry of split
+  uint32_t* done = nullptr;  // [n_split * strips]: items finished (zero between launches)
   int n_split = 0, n_part = 0, cap = 0;
-  double* ypart = nullptr;   // [n_part * kBlkRows * pad8(ncol)]
+  double* ypart = nullptr;   // [n_part * width * pad8(ncol)]
 };
 
 struct Conn {
@@ -130,41 +144,39 @@ struct Conn {
   uint64_t* soff = nullptr;   // [nslice + 1]
   uint32_t* slen = nullptr;   // [nslice] records per lane of each slice
   size_t nslice = 0;
-  // balanced SELL-32 panels of the single-excitation records (beta spin only),
-  // read by the alpha-first alpha-beta kernels: `bal` covers all ket indices;
-  // `panels` (empty unless the packed kernel cannot stage a whole ket row in
-  // shared memory) split the ket range into slices that it can.
+  // balanced SELL-32 of the single-excitation records (beta spin only), read
+  // by the alpha-first kernel with unpacked rows
   SellPanel bal;
-  std::vector<SellPanel> panels;
-  // (beta spin only) position of ket string k in the packed alpha-beta
-  // kernel's staged ket rows: a permutation within aligned groups of 8 chosen
-  // to spread every bra string's singles over the shared-memory bank slots;
-  // the 32-bit records (SellPanel::sell32) hold positions, the 64-bit ones
-  // ket indices
-  uint32_t* kpos = nullptr;   // [n]
   // work items of the packed alpha-beta kernel (alpha spin only), one CTA
   // each, longest first: {bra alpha string, first single, one past the last
-  // single, 1 + partial-row slot or 0}. A string with more singles than the
-  // cap is split into items of at most `item_cap` singles (a multiple of 4)
-  // whose partial rows (ypart[slot * nb ..], FP64) are added to the output in
-  // slot order by a fix-up kernel; the others write the output directly.
+  // single, 1 + partial-row slot or 0}, where the index after a string's last
+  // single stands for the string itself (see sigma_ab_kernel), so every
+  // string has an item. A string with more singles than the
+  // cap is split into items of at most `item_cap` singles whose partial rows
+  // (ypart[slot * pad8(nb) ..], FP64) the last of its CTAs to finish adds to
+  // up into the output in slot order; the others write the output directly.
   uint4* ab_item = nullptr;    // [n_item]
   size_t n_item = 0;
   uint4* ab_split = nullptr;   // [n_split]: {string, first slot, parts, 0}
+  uint32_t* ab_slot = nullptr; // [n_part]: entry of ab_split
+  uint32_t* ab_done = nullptr; // [n_split]: items finished (zero between launches)
   int n_split = 0, n_part = 0, item_cap = 0;
   double* ypart = nullptr;     // [n_part * pad8(nb)]
   // work items of the alpha-first same-spin kernel (either spin), the same
   // scheme over the row's entries (singles then doubles): {bra string, first
   // entry, one past the last entry, 1 + partial-row slot or 0}. Partial rows
   // are [n_same_part * pad8(ncol)] (ncol = the other spin's string count);
-  // every part writes all its columns, and the fix-up assigns their sum.
+  // every part writes all its columns, and the last part to finish assigns
+  // their sum in slot order.
   uint4* same_item = nullptr;
   size_t n_same_item = 0;
   uint4* same_split = nullptr;
+  uint32_t* same_slot = nullptr;  // [n_same_part]: entry of same_split
+  uint32_t* same_done = nullptr;  // [n_same_split * strips]: items finished (zero between launches)
   int n_same_split = 0, n_same_part = 0, same_cap = 0;
   double* same_ypart = nullptr;
-  // blocks of the blocked same-spin kernel over the same rows as same_item
-  SameBlocks blk;
+  // blocks of the blocked same-spin kernels (FP64, FP32) over the same rows as same_item
+  SameBlocks blk[2];
 };
 
 // Largest number of partial-sum slots of split rows (shared memory of the
@@ -174,13 +186,11 @@ constexpr int kMaxSplitSlots = 2048;
 constexpr size_t kAbSmemBudget = 227 * 1024 - 1024;
 // n rounded up to a multiple of 8 (row strides of padded vectors and tables).
 constexpr size_t pad8(size_t n) { return (n + 7) / 8 * 8; }
-// The packed alpha-beta kernel stages its integral row twice: copy 0 at pack
-// index pq, copy 1 at ab7_epad(npair) + pq with ab7_epad = 4 (mod 8), i.e.
-// four 16-byte bank slots further on, so that a record can read whichever
-// copy collides less with the other lanes of its quarter-warp (bit 30 of
-// the 32-bit record). Packs of both copies: ab7_er_packs.
-constexpr size_t ab7_epad(size_t npair) { return (npair + 3) / 8 * 8 + 4; }
-constexpr size_t ab7_er_packs(size_t npair) { return ab7_epad(npair) + npair; }
+// The packed alpha-beta kernel's 16-byte packs per pair and group of alpha
+// singles (5 packs: 10 singles in FP64, 20 with FP32 storage) and the static
+// shared memory beside the dynamic part.
+constexpr int kAbPacks = 5;
+constexpr size_t kAbStaticSmem = 512;
 
 // Stored Hamiltonian (the reference's method 1): off-diagonal elements in CSR
 // over determinant rows, basis phases folded into the values (stored.cu).
@@ -229,6 +239,8 @@ struct Ctx {
   bool have_strings = false;
   // connectivity (0 = alpha, 1 = beta)
   Conn conn[2];
+  AbPlan ab;                // schedule of the packed alpha-beta kernel over the beta singles
+  bool have_sell = false;   // the SELL layouts of the other alpha-beta kernels (built on their first use)
   bool have_conn = false;   // the full connectivity (everything the sigma reads)
   bool have_lists = false;  // at least the excitation lists (Conn CSR and per-entry data)
   // a shard of the alpha strings: the work items (same-spin and alpha-beta
@@ -246,9 +258,15 @@ struct Ctx {
   // sigma: Db[pq * db_stride + ib] = sum_{q in beta(ib)} (pq|qq) (alpha
   // singles), Da[pq * da_stride + ia] = sum_{p in alpha(ia)} (pq|pp) (beta
   // singles); FP64 and FP32 copies; built with the connectivity
+  // (Da is read by the stored Hamiltonian and beside the unpacked alpha-beta
+  // kernels, and built on its first use)
   double *d_Da = nullptr, *d_Db = nullptr;
   float *d_Da32 = nullptr, *d_Db32 = nullptr;
   size_t da_stride = 0, db_stride = 0;
+  // the beta singles' term in the packed alpha-beta kernel: Da by string,
+  // [na x vstride] (FP32: [na x vstride32])
+  double* d_Dr = nullptr;
+  float* d_Dr32 = nullptr;
   // sigma scratch (sized for D): transposed input, FP64 partial outputs
   // The alpha-first sigma keeps its vectors with row strides padded to 8
   // elements (xsa >= nb for the alpha-major ones, xsb >= na for the
@@ -256,9 +274,15 @@ struct Ctx {
   // kernels load whole vectors of columns whatever na and nb are.
   void* d_xt = nullptr;     // nb x xsb elements of the widest type used (8 B)
   void* d_xp = nullptr;     // na x xsa elements (8 B): phi o C, the input in the alpha-first basis
-  double* d_y = nullptr;    // na x xsa FP64: alpha-major partial sigma
-  double* d_yt = nullptr;   // nb x xsb FP64: beta-major partial sigma
+  void* d_xk = nullptr;     // na x ab.xs elements (8 B): phi o C with its columns in the lane order of `ab`
+  double* d_y = nullptr;    // na x xsa FP64: alpha same-spin part of sigma
+  double* d_yab = nullptr;  // na x xsa FP64: opposite-spin part (packed alpha-beta kernel)
+  double* d_yt = nullptr;   // nb x xsb FP64: beta same-spin part, beta-major
   size_t xsa = 0, xsb = 0;
+  // the three independent products of one sigma run side by side: the packed
+  // alpha-beta one on the context stream, the same-spin ones on these
+  cudaStream_t side[2] = {};
+  cudaEvent_t fork = nullptr, join[2] = {};
   void* d_io_in = nullptr;  // D FP64 staging for host-buffer entry points
   // the host-buffer sigma's pipeline: alpha-row chunks whose host<->device
   // copies run on io_copy beside the chunks' kernels on the context stream
@@ -409,6 +433,14 @@ __host__ __device__ __forceinline__ uint64_t other_range(int spin, int x, int y)
 }
 
 // ---- internal entry points shared between translation units ------------------
+// The schedule of the packed alpha-beta kernel, and the SELL layouts of the
+// other alpha-beta kernels (built when a launch code first asks for them).
+int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::vector<uint64_t>& off,
+                  const std::vector<uint64_t>& rec, uint64_t alpha_singles);
+void free_ab_plan(AbPlan& P);
+int ensure_sell(Ctx* c);
+int ensure_coulomb_a(Ctx* c);
+int build_coulomb_tables(Ctx* c);
 // full = false builds the excitation lists only (what the RDM and adjoint
 // kernels read); the sigma entry points need (and rebuild) the full form.
 int build_connectivity(Ctx* c, bool full = true);
@@ -430,7 +462,6 @@ int sigma_rows_device(Ctx* c, int precision, const void* X, void* S, size_t a0, 
 int project_device(Ctx* c, int precision, const void* V, size_t ldv, int m, const void* X, size_t ldx, int nx,
                    size_t D, double* P);
 int build_g_table(Ctx* c);
-int build_coulomb_tables(Ctx* c);
 int diag_terms(Ctx* c);
 // sigma: X (na x nb, type by precision: 0 = FP64, 1 = FP32) -> S (same type)
 int sigma_device(Ctx* c, int precision, const void* X, void* S);
@@ -458,6 +489,6 @@ int davidson_roots(Ctx* c, const sbdx_davidson_params& p, int k, double* dW, dou
 int lowest_diagonal(Ctx* c, int k, std::vector<size_t>& idx);
 
 // Device error codes written to Ctx::d_err.
-constexpr int kErrWatchdogAb = 1;  // alpha-beta kernel: TMA completion wait timed out
+constexpr int kErrWatchdogAb = 1;  // alpha-beta kernels: a wait (TMA completion, step order) timed out
 
 }  // namespace sbdx

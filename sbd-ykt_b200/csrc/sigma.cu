@@ -1007,19 +1007,32 @@ int run_ab(Ctx* c, const T* X) {
 // opposite-spin parity per pair, and the alpha-beta sign is the product of the
 // two same-spin signs stored with the connectivity. The opposite-spin Coulomb
 // term of a single excitation, sum_{q in other} (pq|qq), is read from the
-// per-string Coulomb tables (Ctx::d_Da / d_Db) instead of being summed per pair.
-//   0. Xp = phi o X and Xpt = (phi o X)^T            (phase_split_kernel)
-//   1. alpha same-spin + diagonal on Xp -> Y          (sigma_same_v6_kernel)
-//   2. beta same-spin on Xpt -> Yt                    (sigma_same_v6_kernel)
-//   3. alpha single x beta single on Xp -> Y +=       (sigma_ab_v6_kernel)
-//   4. S = phi o (Y + Yt^T)                           (combine_phase_kernel)
+// per-string Coulomb tables (Ctx::d_Db, d_Dr, d_Da) instead of being summed per pair.
+//   0. Xp = phi o X, Xpt = (phi o X)^T, Xk = Xp in lane order (phase_split_kernel)
+//   1. alpha same-spin on Xp -> Y                     (sigma_same_*_kernel)
+//   2. beta same-spin on Xpt -> Yt                    (sigma_same_*_kernel)
+//   3. alpha x beta on Xk -> Yab                      (sigma_ab_kernel)
+//   4. S = phi o (Y + Yab + Yt^T) + hii o X           (combine_phase_kernel)
+// Step 1 includes the Coulomb terms of the alpha singles with the beta string,
+// step 3 those of the beta singles with the alpha string (one more integral
+// row per alpha string), so step 2 is a product with a constant sparse matrix.
+// The unpacked alpha-beta kernels (codes 61-64) evaluate the pairs only, add
+// them to Y, and leave both Coulomb terms and the diagonal to the same-spin
+// kernels (Dt, hii).
 
+// Blocks ibx < ntx split one 32 x 32 tile; the further ones write 256 columns
+// of 32 rows of Xk, phi o X with its columns in the lane order of the packed
+// alpha-beta kernel (vket: the ket string of each lane), so that kernel's
+// loads are coalesced: one gather per element here instead of one per alpha
+// single there.
 template <typename T>
 __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb, const uint64_t* __restrict__ astr,
                                    const uint64_t* __restrict__ bstr, T* __restrict__ Xp, T* __restrict__ Xpt,
-                                   size_t xsa, size_t xsb) {
+                                   size_t xsa, size_t xsb, const uint32_t* __restrict__ vket, T* __restrict__ Xk,
+                                   size_t xs) {
   __shared__ T tile[32][33];
   __shared__ uint64_t s_pa[32], s_b[32];
+  const size_t ntx = (nb + 31) / 32;
   const size_t ib0 = (size_t)blockIdx.x * 32, ia0 = (size_t)blockIdx.y * 32;
   const int tx = threadIdx.x;
   if (threadIdx.y == 0) {
@@ -1027,6 +1040,21 @@ __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb
     s_b[tx] = ib0 + tx < nb ? bstr[ib0 + tx] : 0ull;
   }
   __syncthreads();
+  if (blockIdx.x >= ntx) {
+    const size_t v = (blockIdx.x - ntx) * 256 + threadIdx.y * 32 + tx;
+    if (v >= xs) return;
+    const size_t ib = vket[v];
+    const uint64_t beta = bstr[ib];
+    const int rows = (int)min((size_t)32, na - ia0);
+    const T* x = X + ia0 * nb + ib;
+    T* o = Xk + ia0 * xs + v;
+#pragma unroll 8
+    for (int k = 0; k < rows; ++k) {
+      const T w = x[(size_t)k * nb];
+      o[(size_t)k * xs] = basis_phase(s_pa[k], beta) ? -w : w;
+    }
+    return;
+  }
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const size_t ia = ia0 + k, ib = ib0 + tx;
     if (ia < na && ib < nb) {
@@ -1043,12 +1071,14 @@ __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb
   }
 }
 
-// S[ia, ib] = phi(ia, ib) (Y[ia, ib] + Yt[ib, ia]), stored in T; Y and Yt
-// have row strides xsa and xsb.
+// S[ia, ib] = phi(ia, ib) (Y[ia, ib] + Yab[ia, ib] + Yt[ib, ia]) + hii[ia, ib]
+// X[ia, ib], stored in T; Y, Yab and Yt have row strides xsa, xsa and xsb.
+// With Yab null: S = phi o (Y + Yt^T).
 template <typename T>
-__global__ void combine_phase_kernel(const double* __restrict__ Y, const double* __restrict__ Yt, size_t na,
-                                     size_t nb, const uint64_t* __restrict__ astr, const uint64_t* __restrict__ bstr,
-                                     T* __restrict__ S, size_t xsa, size_t xsb) {
+__global__ void combine_phase_kernel(const double* __restrict__ Y, const double* __restrict__ Yab,
+                                     const double* __restrict__ Yt, const double* __restrict__ hii,
+                                     const T* __restrict__ X, size_t na, size_t nb, const uint64_t* __restrict__ astr,
+                                     const uint64_t* __restrict__ bstr, T* __restrict__ S, size_t xsa, size_t xsb) {
   __shared__ double tile[32][33];
   __shared__ uint64_t s_pa[32], s_b[32];
   const size_t ib0 = (size_t)blockIdx.x * 32, ia0 = (size_t)blockIdx.y * 32;
@@ -1057,16 +1087,22 @@ __global__ void combine_phase_kernel(const double* __restrict__ Y, const double*
     s_pa[tx] = ia0 + tx < na ? prefix_parity(astr[ia0 + tx]) : 0ull;
     s_b[tx] = ib0 + tx < nb ? bstr[ib0 + tx] : 0ull;
   }
+#pragma unroll 4
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const size_t ib = ib0 + k, ia = ia0 + tx;
     if (ib < nb && ia < na) tile[tx][k] = Yt[ib * xsb + ia];
   }
   __syncthreads();
+#pragma unroll 4
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const size_t ia = ia0 + k, ib = ib0 + tx;
     if (ia < na && ib < nb) {
-      const double y = Y[ia * xsa + ib] + tile[k][tx];
-      S[ia * nb + ib] = (T)(basis_phase(s_pa[k], s_b[tx]) ? -y : y);
+      double y = Y[ia * xsa + ib] + tile[k][tx], d = 0.0;
+      if (Yab != nullptr) {
+        y += Yab[ia * xsa + ib];
+        d = hii[ia * nb + ib] * (double)X[ia * nb + ib];
+      }
+      S[ia * nb + ib] = (T)(basis_phase(s_pa[k], s_b[tx]) ? d - y : d + y);
     }
   }
 }
@@ -1089,12 +1125,66 @@ __global__ void coulomb_table_kernel(const double* __restrict__ G, int L, const 
   D32[pq * stride + k] = (float)v;
 }
 
+// The table by string: row k = sum over the orbitals p of string k of the
+// integral row (pp|..).
+__global__ void coulomb_row_sum_kernel(const double* __restrict__ V, size_t npair, size_t vs, size_t vs32, int L,
+                                       const uint64_t* __restrict__ s, double* __restrict__ D,
+                                       float* __restrict__ D32) {
+  const size_t k = blockIdx.x;
+  const uint64_t bits = s[k] & range_mask(0, L);
+  for (size_t t = threadIdx.x; t < npair; t += blockDim.x) {
+    double v = 0.0;
+    for (uint64_t m = bits; m; m &= m - 1) {
+      const size_t p = (size_t)(__ffsll((long long)m) - 1);
+      v += V[(p * (p + 1) / 2 + p) * vs + t];
+    }
+    D[k * vs + t] = v;
+    D32[k * vs32 + t] = (float)v;
+  }
+}
+
+// True in every thread of the last CTA to arrive for split entry q: the
+// parts' partial rows are then visible to it. The counter returns to zero for
+// the next launch.
+__device__ __forceinline__ bool last_part(uint32_t* done, size_t q, uint32_t parts) {
+  __shared__ int s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(done + q, 1u) + 1 == parts;
+    if (s_last) done[q] = 0;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last != 0;
+}
+
+// Row `row` of Y in columns c0 .. c0 + VEC - 1 as the sum of a split row's
+// partial rows in slot order, by the last part to finish a strip. Partial row
+// k of slot q is ypart row (first slot + q) * stride + k.
+template <int VEC>
+__device__ __forceinline__ void same_split_sum(const uint4* split, const uint32_t* slot_split, uint32_t* done,
+                                               uint32_t slot, int k_rows, const double* ypart, size_t ldx, size_t c0,
+                                               bool active, double* Y, size_t row) {
+  const uint32_t q = slot_split[slot];
+  const uint4 sp = split[q];
+  if (!last_part(done, (size_t)q * gridDim.y + blockIdx.y, sp.z) || !active) return;
+  double t[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) t[v] = 0.0;
+  for (uint32_t p = 0; p < sp.z; ++p)
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) t[v] += __ldcg(ypart + (size_t)(sp.y + p) * k_rows * ldx + c0 + v);
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) Y[row * ldx + c0 + v] = t[v];
+}
+
 // Same-spin excitations in the alpha-first basis, VEC consecutive columns per
 // thread; grid x = bra row (fastest: the resident CTAs share one column strip
 // of the ket rows, which stays in L2), y = column strip. A CTA stages the
 // entries of its row (ket, signed value, signed pair index) in shared memory;
-// per pair a double costs one FMA and a single one add (the Coulomb table
-// element of its column) and one FMA. X and Y rows have stride ldx, a multiple
+// per pair a double costs one FMA and a single, when Dt is given, one add (the
+// Coulomb table element of its column) and one FMA. X and Y rows have stride ldx, a multiple
 // of VEC (padding columns up to ldx are computed and never read); hii has
 // stride ncol.
 template <typename T, int VEC>
@@ -1103,8 +1193,9 @@ sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uin
                      const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
                      const typename Prec<T>::V* __restrict__ val, const uint32_t* __restrict__ info,
                      const typename Prec<T>::V* __restrict__ Dt, size_t dstride, const double* __restrict__ hii,
-                     const uint4* __restrict__ items, double* __restrict__ ypart, double* __restrict__ Y,
-                     int accumulate) {
+                     const uint4* __restrict__ items, const uint4* __restrict__ split,
+                     const uint32_t* __restrict__ slot_split, uint32_t* __restrict__ done, double* __restrict__ ypart,
+                     double* __restrict__ Y) {
   __shared__ uint32_t s_ket[kSameThreads], s_pq[kSameThreads];
   __shared__ double s_val[kSameThreads];
   const uint4 item = items[blockIdx.x];  // bra string, entry range, output row
@@ -1125,7 +1216,7 @@ sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uin
   const unsigned t = threadIdx.x;
   for (uint64_t base = beg; base < end; base += kSameThreads) {
     const int cnt = (int)min((uint64_t)kSameThreads, end - base);
-    const int nsb = send > base ? (int)min((uint64_t)cnt, send - base) : 0;
+    const int nsb = Dt != nullptr && send > base ? (int)min((uint64_t)cnt, send - base) : 0;
     __syncthreads();
     if ((int)t < cnt) {
       const uint64_t e = base + t;
@@ -1156,14 +1247,10 @@ sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uin
     }
   }
   if (active) {
-    if (accumulate && item.w == 0) {  // add to the row (a partial row of a split string is always written)
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) Yrow[c0 + v] += acc[v];
-    } else {
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) Yrow[c0 + v] = acc[v];
-    }
+    for (int v = 0; v < VEC; ++v) Yrow[c0 + v] = acc[v];
   }
+  if (item.w) same_split_sum<VEC>(split, slot_split, done, item.w - 1, 1, ypart, ldx, c0, active, Y, r);
 }
 
 // FP32-storage variant of sigma_same_v6_kernel: products and short runs of up
@@ -1201,7 +1288,8 @@ sigma_same_v6f_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, cons
                       const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
                       const float* __restrict__ val, const uint32_t* __restrict__ info, const float* __restrict__ Dt,
                       size_t dstride, const double* __restrict__ hii, const uint4* __restrict__ items,
-                      double* __restrict__ ypart, double* __restrict__ Y, int accumulate) {
+                      const uint4* __restrict__ split, const uint32_t* __restrict__ slot_split,
+                      uint32_t* __restrict__ done, double* __restrict__ ypart, double* __restrict__ Y) {
   __shared__ uint32_t s_ket[kSameThreads], s_pq[kSameThreads];
   __shared__ float s_val[kSameThreads];
   const uint4 item = items[blockIdx.x];  // bra string, entry range, output row
@@ -1222,7 +1310,7 @@ sigma_same_v6f_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, cons
   const unsigned t = threadIdx.x;
   for (uint64_t base = beg; base < end; base += kSameThreads) {
     const int cnt = (int)min((uint64_t)kSameThreads, end - base);
-    const int nsb = send > base ? (int)min((uint64_t)cnt, send - base) : 0;
+    const int nsb = Dt != nullptr && send > base ? (int)min((uint64_t)cnt, send - base) : 0;
     __syncthreads();
     if ((int)t < cnt) {
       const uint64_t e = base + t;
@@ -1269,212 +1357,259 @@ sigma_same_v6f_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, cons
     }
   }
   if (active) {
-    if (accumulate && item.w == 0) {
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) Yrow[c0 + v] += acc[v];
-    } else {
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) Yrow[c0 + v] = acc[v];
-    }
+    for (int v = 0; v < VEC; ++v) Yrow[c0 + v] = acc[v];
   }
+  if (item.w) same_split_sum<VEC>(split, slot_split, done, item.w - 1, 1, ypart, ldx, c0, active, Y, r);
 }
 
-// VEC consecutive elements in the storage type.
-template <typename T, int VEC> struct LoadT;
-template <int VEC> struct LoadT<double, VEC> {
-  static __device__ __forceinline__ void load(const double* p, double* o) { VecIO<double, VEC>::load(p, o); }
-};
-template <int VEC> struct LoadT<float, VEC> {
-  static __device__ __forceinline__ void load(const float* p, float* o) { VecF<VEC>::load(p, o); }
-};
+// Blocked same-spin products: CTA = (work item of SameBlocks, strip of
+// columns). Every ket row strip of the block's union is loaded once and
+// applied to all bra strings of the block with their signed values (zero
+// where a string does not connect). With Dt, a block's first item adds the
+// Coulomb terms of its strings' singles (the constant part of a single is in
+// the union).
 
-// Signed same-spin values of one union entry of the blocked kernel, one per
-// bra string of the block (kBlkRows = 4).
-template <typename V> struct Vals4;
-template <> struct Vals4<double> { using P = double4; };
-template <> struct Vals4<float> { using P = float4; };
+// Stages up to kSameThreads union entries (kets and values).
+template <int ROWS, typename V>
+__device__ __forceinline__ void stage_union(uint32_t* s_ket, V* s_val, const uint32_t* __restrict__ uket,
+                                            const V* __restrict__ uval, uint64_t base, int cnt) {
+  constexpr int kPer = 16 / sizeof(V);
+  __syncthreads();
+  if ((int)threadIdx.x < cnt) s_ket[threadIdx.x] = uket[base + threadIdx.x];
+  const uint4* src = reinterpret_cast<const uint4*>(uval + base * ROWS);
+  uint4* dst = reinterpret_cast<uint4*>(s_val);
+  for (int i = threadIdx.x; i < cnt * ROWS / kPer; i += kSameThreads) dst[i] = src[i];
+  __syncthreads();
+}
 
-// Resident CTAs per SM the blocked kernel is compiled for (0: no bound; FP32
-// storage: three, which caps its registers at 80 with the deeper unroll of
-// its union loop), and the union entries summed in FP32 before the FP64 row
-// accumulation. Measured at 8000 x 8000 strings: FP64 runs fastest with the
-// union loop unrolled 4 deep and no bound (52 registers, 4 CTAs per SM; an
-// explicit bound of 1 let it take 96 registers and ran 19% slower), FP32 with
-// 8 union entries' ket loads issued ahead.
-template <typename T> struct BlkShape { static constexpr int kMinBlocks = 0; };
-template <> struct BlkShape<float> { static constexpr int kMinBlocks = 3; };
-constexpr int kBlkRun = kRun;
-
-// Blocked same-spin product (codes 31/32/34/38 = columns per thread): one CTA
-// per (work item of SameBlocks, strip of kSameThreads*VEC columns). The first
-// item of a block adds the diagonal and the singles of its kBlkRows bra
-// strings, one string at a time, as sigma_same_v6_kernel does; every item then
-// walks its range of the block's union of double-excitation kets: each ket
-// row strip is loaded once and applied to all strings of the block with their
-// signed values (zero where a string does not connect), so a ket shared by
-// several strings of the block costs one load instead of one per string.
-// FP32 storage (T = float): products summed in FP32 over runs of kBlkRun union
-// entries (or of kRun singles), each run's sum added to the FP64 row
-// accumulator.
-template <typename T, int VEC>
-__global__ void __launch_bounds__(kSameThreads, BlkShape<T>::kMinBlocks)
-sigma_same_blk_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
+// FP64, eight strings per block. A thread owns P pairs of columns, pair p at
+// 64 p + 2 (lane) of its warp's 64 P columns, so every 16-byte load of a warp
+// covers 512 contiguous bytes (a quarter-warp that reads several lines pays a
+// wavefront for each). Loads run kAhead entries ahead of the products.
+template <int P>
+__global__ void __launch_bounds__(kSameThreads, 2)
+sigma_same_blk_kernel(const double* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
                       const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
-                      const T* __restrict__ val, const uint32_t* __restrict__ info, const T* __restrict__ Dt,
-                      size_t dstride, const double* __restrict__ hii, const uint4* __restrict__ brows,
-                      const uint64_t* __restrict__ uoff, const uint32_t* __restrict__ uket,
-                      const typename Vals4<T>::P* __restrict__ uval, const uint4* __restrict__ items,
-                      double* __restrict__ ypart, double* __restrict__ Y, int accumulate) {
-  using P4 = typename Vals4<T>::P;
-  constexpr bool kF32 = std::is_same<T, float>::value;
-  __shared__ uint32_t s_ket[kSameThreads], s_pq[kSameThreads];
-  __shared__ P4 s_val4[kSameThreads];
-  __shared__ T s_val[kSameThreads];
+                      const uint32_t* __restrict__ info, const double* __restrict__ Dt, size_t dstride,
+                      const uint32_t* __restrict__ brows, const uint64_t* __restrict__ uoff,
+                      const uint32_t* __restrict__ uket, const double* __restrict__ uval,
+                      const uint4* __restrict__ items, const uint4* __restrict__ split,
+                      const uint32_t* __restrict__ slot_split, uint32_t* __restrict__ done,
+                      double* __restrict__ ypart, double* __restrict__ Y) {
+  constexpr int ROWS = kBlkRows64, kAhead = 8 / P;
+  __shared__ uint32_t s_ket[kSameThreads + 8];
+  __shared__ __align__(16) double s_val[kSameThreads * ROWS];
   const uint4 item = items[blockIdx.x];  // block, union range, partial slot
-  const uint4 rw = brows[item.x];
-  const uint32_t rows[kBlkRows] = {rw.x, rw.y, rw.z, rw.w};
-  const size_t c0 = ((size_t)blockIdx.y * kSameThreads + threadIdx.x) * VEC;
-  const bool active = c0 < ncol;
-  const unsigned t = threadIdx.x;
-  double acc[kBlkRows][VEC];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const size_t c0 = ((size_t)blockIdx.y * (kSameThreads / 32) + warp) * (64 * P) + 2 * lane;
+  // columns up to ncol rounded up to 8: the rows' padding, never another range's columns
+  const size_t lim = (ncol + 7) & ~(size_t)7;
+  const bool active = c0 - 2 * lane < ncol;  // warp-uniform
+  bool in[P];
 #pragma unroll
-  for (int k = 0; k < kBlkRows; ++k)
+  for (int p = 0; p < P; ++p) in[p] = c0 + 64 * p < lim;
+  const double* xc = X + c0;
+  double acc[ROWS][P][2];
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) acc[k][v] = 0.0;
-  if (item.y == 0) {  // the block's first item: diagonal and singles, string by string
+  for (int k = 0; k < ROWS; ++k)
 #pragma unroll
-    for (int k = 0; k < kBlkRows; ++k) {
-      const uint32_t r = rows[k];
-      if (r == kNoRow) continue;
-      if (hii != nullptr && active) {
-        T x[VEC];
-        LoadT<T, VEC>::load(X + (size_t)r * ldx + c0, x);
+    for (int p = 0; p < P; ++p) acc[k][p][0] = acc[k][p][1] = 0.0;
+  auto load = [&](uint32_t kt, double2 (&o)[P]) {
+    const double* x = xc + (size_t)kt * ldx;
 #pragma unroll
-        for (int v = 0; v < VEC; ++v) acc[k][v] = c0 + v < ncol ? hii[(size_t)r * ncol + c0 + v] * (double)x[v] : 0.0;
-      }
-      const uint64_t beg = off[r], end = beg + nsing[r];
-      for (uint64_t base = beg; base < end; base += kSameThreads) {
-        const int cnt = (int)min((uint64_t)kSameThreads, end - base);
-        __syncthreads();
-        if ((int)t < cnt) {
-          const uint64_t e = base + t;
-          const uint32_t inf = info[e];
-          const T v = val[e];
-          s_ket[t] = ket[e];
-          s_val[t] = (inf >> 31) ? -v : v;
-          s_pq[t] = ((inf >> 12) & 0xfffu) | (inf & kInfoNeg);
-        }
-        __syncthreads();
-        if (!active) continue;
-        for (int e0 = 0; e0 < cnt; e0 += kRun) {
-          const int e1 = min(e0 + kRun, cnt);
-          T pf[VEC];
-#pragma unroll
-          for (int v = 0; v < VEC; ++v) pf[v] = (T)0;
-          for (int e = e0; e < e1; ++e) {
-            const uint32_t pqs = s_pq[e];
-            const T hv = s_val[e];
-            T x[VEC], d[VEC];
-            LoadT<T, VEC>::load(X + (size_t)s_ket[e] * ldx + c0, x);
-            LoadT<T, VEC>::load(Dt + (size_t)(pqs & 0xfffu) * dstride + c0, d);
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) {
-              const T dv = (pqs >> 31) ? -d[v] : d[v];
-              if constexpr (kF32) pf[v] = fmaf(hv + dv, x[v], pf[v]);
-              else acc[k][v] = fma(hv + dv, x[v], acc[k][v]);
-            }
-          }
-          if constexpr (kF32) {
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) acc[k][v] += (double)pf[v];
-          }
-        }
-      }
-    }
-  }
-  // doubles: the block's union entries [u0, u1)
+    for (int p = 0; p < P; ++p)
+      o[p] = in[p] ? __ldg(reinterpret_cast<const double2*>(x + 64 * p)) : make_double2(0.0, 0.0);
+  };
   const uint64_t ub = uoff[item.x];
   const uint64_t beg = ub + item.y, end = ub + item.z;
   for (uint64_t base = beg; base < end; base += kSameThreads) {
-    const int cnt = (int)min((uint64_t)kSameThreads, end - base);
-    __syncthreads();
-    if ((int)t < cnt) {
-      s_ket[t] = uket[base + t];
-      s_val4[t] = uval[base + t];
-    }
-    __syncthreads();
+    const int cnt = (int)min((uint64_t)kSameThreads, end - base);  // a multiple of 8
+    stage_union<ROWS>(s_ket, s_val, uket, uval, base, cnt);
     if (!active) continue;
-    for (int e0 = 0; e0 < cnt; e0 += kBlkRun) {
-      const int e1 = min(e0 + kBlkRun, cnt);
-      T pf[kBlkRows][VEC];
+    double2 x[kAhead][P];
 #pragma unroll
-      for (int k = 0; k < kBlkRows; ++k)
+    for (int u = 0; u < kAhead; ++u) load(s_ket[u], x[u]);
+#pragma unroll 1
+    for (int e0 = 0; e0 < cnt; e0 += 8) {
 #pragma unroll
-        for (int v = 0; v < VEC; ++v) pf[k][v] = (T)0;
-      if constexpr (kF32) {
-#pragma unroll 8
-        for (int e = e0; e < e1; ++e) {
-          T x[VEC];
-          LoadT<T, VEC>::load(X + (size_t)s_ket[e] * ldx + c0, x);
-          const P4 w = s_val4[e];
-          const T wv[kBlkRows] = {w.x, w.y, w.z, w.w};
+      for (int u = 0; u < 8; ++u) {
+        const int e = e0 + u;
+        const double* w = s_val + e * ROWS;
 #pragma unroll
-          for (int k = 0; k < kBlkRows; ++k)
+        for (int k = 0; k < ROWS; k += 2) {
+          const double2 wk = *reinterpret_cast<const double2*>(w + k);
 #pragma unroll
-            for (int v = 0; v < VEC; ++v) pf[k][v] = fmaf(wv[k], x[v], pf[k][v]);
+          for (int p = 0; p < P; ++p) {
+            acc[k][p][0] = fma(wk.x, x[u % kAhead][p].x, acc[k][p][0]);
+            acc[k][p][1] = fma(wk.x, x[u % kAhead][p].y, acc[k][p][1]);
+            acc[k + 1][p][0] = fma(wk.y, x[u % kAhead][p].x, acc[k + 1][p][0]);
+            acc[k + 1][p][1] = fma(wk.y, x[u % kAhead][p].y, acc[k + 1][p][1]);
+          }
         }
+        load(s_ket[min(e + kAhead, cnt - 1)], x[u % kAhead]);
+      }
+    }
+  }
+  if (Dt != nullptr && item.y == 0 && active) {
 #pragma unroll
-        for (int k = 0; k < kBlkRows; ++k)
-#pragma unroll
-          for (int v = 0; v < VEC; ++v) acc[k][v] += (double)pf[k][v];
-      } else {
+    for (int k = 0; k < ROWS; ++k) {
+      const uint32_t r = brows[item.x * ROWS + k];
+      if (r == kNoRow) continue;
+      const uint64_t e0 = off[r];
+      const int ns = (int)nsing[r];
 #pragma unroll 4
-        for (int e = e0; e < e1; ++e) {
-          T x[VEC];
-          LoadT<T, VEC>::load(X + (size_t)s_ket[e] * ldx + c0, x);
-          const P4 w = s_val4[e];
-          const T wv[kBlkRows] = {w.x, w.y, w.z, w.w};
+      for (int s = 0; s < ns; ++s) {
+        const uint32_t inf = __ldg(info + e0 + s);
+        const double* d = Dt + (size_t)((inf >> 12) & 0xfffu) * dstride + c0;
+        double2 x[P];
+        load(__ldg(ket + e0 + s), x);
 #pragma unroll
-          for (int k = 0; k < kBlkRows; ++k)
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) acc[k][v] = fma(wv[k], x[v], acc[k][v]);
+        for (int p = 0; p < P; ++p) {
+          const double2 dv = in[p] ? __ldg(reinterpret_cast<const double2*>(d + 64 * p)) : make_double2(0.0, 0.0);
+          acc[k][p][0] = fma(flip_sign(dv.x, inf >> 31), x[p].x, acc[k][p][0]);
+          acc[k][p][1] = fma(flip_sign(dv.y, inf >> 31), x[p].y, acc[k][p][1]);
         }
       }
     }
   }
-  if (!active) return;
+  if (active) {
 #pragma unroll
-  for (int k = 0; k < kBlkRows; ++k) {
-    const uint32_t r = rows[k];
+    for (int k = 0; k < ROWS; ++k) {
+      const uint32_t r = brows[item.x * ROWS + k];
+      if (item.w == 0 && r == kNoRow) continue;
+      double* y = (item.w ? ypart + ((size_t)(item.w - 1) * ROWS + k) * ldx : Y + (size_t)r * ldx) + c0;
+#pragma unroll
+      for (int p = 0; p < P; ++p)
+        if (in[p]) *reinterpret_cast<double2*>(y + 64 * p) = make_double2(acc[k][p][0], acc[k][p][1]);
+    }
+  }
+  if (item.w == 0) return;
+  const uint32_t sq = slot_split[item.w - 1];
+  const uint4 sp = split[sq];
+  if (!last_part(done, (size_t)sq * gridDim.y + blockIdx.y, sp.z) || !active) return;
+  for (int k = 0; k < ROWS; ++k) {
+    const uint32_t r = brows[item.x * ROWS + k];
     if (r == kNoRow) continue;
-    if (item.w) {  // a part of a split block: its partial row
-      double* y = ypart + ((size_t)(item.w - 1) * kBlkRows + k) * ldx + c0;
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) y[v] = acc[k][v];
-    } else {
-      double* y = Y + (size_t)r * ldx + c0;
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) y[v] = accumulate ? y[v] + acc[k][v] : acc[k][v];
+    for (int p = 0; p < P; ++p) {
+      if (c0 + 64 * p >= lim) continue;
+      double2 t = make_double2(0.0, 0.0);
+      for (uint32_t z = 0; z < sp.z; ++z) {
+        const double2 u = __ldcg(reinterpret_cast<const double2*>(ypart + ((size_t)(sp.y + z) * ROWS + k) * ldx + c0 + 64 * p));
+        t.x += u.x;
+        t.y += u.y;
+      }
+      *reinterpret_cast<double2*>(Y + (size_t)r * ldx + c0 + 64 * p) = t;
     }
   }
 }
 
-// Assigns (or, with accumulate, adds) the sums of the partial rows of the
-// blocks split over several items of the blocked same-spin kernel, parts in
-// slot order; blockIdx.z = string of the block.
-__global__ void same_blk_fixup_kernel(const uint4* __restrict__ split, const uint4* __restrict__ brows,
-                                      const double* __restrict__ ypart, size_t ncol, size_t ldx,
-                                      double* __restrict__ Y, int accumulate) {
-  const uint4 sp = split[blockIdx.y];
-  const uint4 rw = brows[sp.x];
-  const int k = blockIdx.z;
-  const uint32_t r = k == 0 ? rw.x : k == 1 ? rw.y : k == 2 ? rw.z : rw.w;
-  if (r == kNoRow) return;
-  for (size_t col = (size_t)blockIdx.x * blockDim.x + threadIdx.x; col < ncol; col += (size_t)gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (uint32_t q = 0; q < sp.z; ++q) t += ypart[((size_t)(sp.y + q) * kBlkRows + k) * ldx + col];
-    double* y = Y + (size_t)r * ldx + col;
-    *y = accumulate ? *y + t : t;
+// FP32 storage, VEC columns per thread: products summed in FP32 over runs of
+// kRun union entries (or of kRun singles), each run's sum added to the FP64
+// row accumulator. The unions are padded to whole runs, so the run's ket
+// strips are all loaded before the first product and no product is guarded.
+template <int VEC>
+__global__ void __launch_bounds__(kSameThreads, 3)
+sigma_same_blkf_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
+                       const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
+                       const uint32_t* __restrict__ info, const float* __restrict__ Dt, size_t dstride,
+                       const uint32_t* __restrict__ brows,
+                       const uint64_t* __restrict__ uoff, const uint32_t* __restrict__ uket,
+                       const float* __restrict__ uval, const uint4* __restrict__ items,
+                       const uint4* __restrict__ split, const uint32_t* __restrict__ slot_split,
+                       uint32_t* __restrict__ done, double* __restrict__ ypart, double* __restrict__ Y) {
+  constexpr int ROWS = kBlkRows32;
+  static_assert(kRun == 8 && ROWS == 4, "the unions are padded to runs of 8 entries of 4 values");
+  __shared__ __align__(16) uint32_t s_ket[kSameThreads];
+  __shared__ __align__(16) float s_val[kSameThreads * ROWS];
+  const uint4 item = items[blockIdx.x];  // block, union range, partial slot
+  const size_t c0 = ((size_t)blockIdx.y * kSameThreads + threadIdx.x) * VEC;
+  const bool active = c0 < ncol;
+  double acc[ROWS][VEC];
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k)
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) acc[k][v] = 0.0;
+  const uint64_t ub = uoff[item.x];
+  const uint64_t beg = ub + item.y, end = ub + item.z;
+  const float* xc = X + c0;
+  for (uint64_t base = beg; base < end; base += kSameThreads) {
+    const int cnt = (int)min((uint64_t)kSameThreads, end - base);
+    stage_union<ROWS>(s_ket, s_val, uket, uval, base, cnt);
+    if (!active) continue;
+#pragma unroll 1
+    for (int e0 = 0; e0 < cnt; e0 += kRun) {
+      float pf[ROWS][VEC], x[kRun][VEC];
+      const uint4 k0 = *reinterpret_cast<const uint4*>(s_ket + e0), k1 = *reinterpret_cast<const uint4*>(s_ket + e0 + 4);
+      const uint32_t kt[kRun] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+      for (int u = 0; u < kRun; ++u) VecF<VEC>::load(xc + (size_t)kt[u] * ldx, x[u]);
+#pragma unroll
+      for (int u = 0; u < kRun; ++u) {
+        const float4 w4 = *reinterpret_cast<const float4*>(s_val + (e0 + u) * ROWS);
+        const float w[ROWS] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k)
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) pf[k][v] = u == 0 ? w[k] * x[u][v] : fmaf(w[k], x[u][v], pf[k][v]);
+      }
+#pragma unroll
+      for (int k = 0; k < ROWS; ++k)
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) acc[k][v] += (double)pf[k][v];
+    }
+  }
+  if (Dt != nullptr && item.y == 0 && active) {
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const uint32_t r = brows[item.x * ROWS + k];
+      if (r == kNoRow) continue;
+      const uint64_t e0 = off[r];
+      const int ns = (int)nsing[r];
+      for (int s0 = 0; s0 < ns; s0 += kRun) {
+        const int s1 = min(s0 + kRun, ns);
+        float pf[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) pf[v] = 0.f;
+#pragma unroll 4
+        for (int s = s0; s < s1; ++s) {
+          const uint32_t inf = __ldg(info + e0 + s);
+          float x[VEC], d[VEC];
+          VecF<VEC>::load(xc + (size_t)__ldg(ket + e0 + s) * ldx, x);
+          VecF<VEC>::load(Dt + (size_t)((inf >> 12) & 0xfffu) * dstride + c0, d);
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) pf[v] = fmaf((inf >> 31) ? -d[v] : d[v], x[v], pf[v]);
+        }
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) acc[k][v] += (double)pf[v];
+      }
+    }
+  }
+  if (active) {
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const uint32_t r = brows[item.x * ROWS + k];
+      if (item.w == 0 && r == kNoRow) continue;
+      double* y = item.w ? ypart + ((size_t)(item.w - 1) * ROWS + k) * ldx + c0 : Y + (size_t)r * ldx + c0;
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) y[v] = acc[k][v];
+    }
+  }
+  if (item.w == 0) return;
+  const uint32_t sq = slot_split[item.w - 1];
+  const uint4 sp = split[sq];
+  if (!last_part(done, (size_t)sq * gridDim.y + blockIdx.y, sp.z) || !active) return;
+  for (int k = 0; k < ROWS; ++k) {
+    const uint32_t r = brows[item.x * ROWS + k];
+    if (r == kNoRow) continue;
+    double t[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) t[v] = 0.0;
+    for (uint32_t p = 0; p < sp.z; ++p)
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) t[v] += __ldcg(ypart + ((size_t)(sp.y + p) * ROWS + k) * ldx + c0 + v);
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) Y[(size_t)r * ldx + c0 + v] = t[v];
   }
 }
 
@@ -1584,15 +1719,18 @@ sigma_ab_v6_kernel(const T* __restrict__ Xp, size_t nb, size_t ldx, const uint64
   }
 }
 
-// 16-byte packs of the staged rows of the alpha-beta kernel v7: element e of
-// the pack of ket index jb is C'[ja_e, jb] (and of pair index pq, the signed
-// integral s_alpha(ja_e) (a_e i_e|pq)).
+// 16-byte packs of the packed alpha-beta kernel: element e of pack h of pair
+// index pq is the signed integral s_alpha(ja) (a i|pq) of alpha single
+// h * kRows + e of the group.
 template <typename T> struct RowPack;
 template <> struct RowPack<double> {
   using P = double2;
   static constexpr int kRows = 2;
   static __device__ __forceinline__ void set(P& p, int e, double v) { if (e == 0) p.x = v; else p.y = v; }
-  static __device__ __forceinline__ double dot(const P& a, const P& b) { return fma(a.x, b.x, a.y * b.y); }
+  static __device__ __forceinline__ void dot(const P& a, const double* c, double (&t)[2]) {
+    t[0] = fma(a.x, c[0], t[0]);
+    t[1] = fma(a.y, c[1], t[1]);
+  }
 };
 template <> struct RowPack<float> {
   using P = float4;
@@ -1600,314 +1738,360 @@ template <> struct RowPack<float> {
   static __device__ __forceinline__ void set(P& p, int e, float v) {
     if (e == 0) p.x = v; else if (e == 1) p.y = v; else if (e == 2) p.z = v; else p.w = v;
   }
-  // the 4-term dot of one record in FP32, added to the FP64 row sum by the caller
-  static __device__ __forceinline__ double dot(const P& a, const P& b) {
-    return (double)fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w)));
+  // 4-term dots in FP32, summed in FP64
+  static __device__ __forceinline__ void dot(const P& a, const float* c, double (&t)[2]) {
+    const float u = fmaf(a.x, c[0], a.y * c[1]), v = fmaf(a.z, c[2], a.w * c[3]);
+    t[0] += (double)(u + v);
   }
 };
 
-// Alpha single x beta single, v7: as v6 (balanced SELL-32, alpha-first signs,
-// split beta rows), with the staged rows interleaved into 16-byte packs (2
-// FP64 or 4 FP32 rows per group): a record costs two 128-bit shared loads (ket
-// pack, integral pack) for all rows of the group, and the alpha sign is
-// applied to the integrals when they are staged, so the per-record sign is
-// the beta one only. One CTA per (alpha work item, chunk of beta slices): an
-// item is a bra alpha string or, for strings with many singles, a range of
-// them whose partial row goes to its own slot (Conn::ab_item).
-template <typename T, int KS>
-__global__ void __launch_bounds__(kAb6Threads, 1)
-sigma_ab_v7_kernel(const T* __restrict__ Xp, size_t ldx, const uint64_t* __restrict__ a_off,
-                   const uint32_t* __restrict__ a_ket,
-                   const uint32_t* __restrict__ a_info, const uint32_t* __restrict__ sell,
-                   const uint64_t* __restrict__ soff4, const uint32_t* __restrict__ slen4, size_t nslice,
-                   const uint32_t* __restrict__ vrow, const uint32_t* __restrict__ vslot, size_t nv,
-                   const uint32_t* __restrict__ split_row, const uint32_t* __restrict__ split_slot, int nsplit,
-                   const T* __restrict__ Vt, size_t vstride,
-                   int npair, uint32_t epad, uint32_t jb0, size_t nbp, const uint32_t* __restrict__ kpos,
-                   const uint4* __restrict__ items, double* __restrict__ ypart, double* __restrict__ Y) {
+// Arguments of the packed alpha-beta kernel on one panel of bra strings.
+template <typename T>
+struct AbArgs {
+  const T* Xk;       // na x xs: phi o C, columns in lane order
+  size_t xs, ldx;    // ldx: row stride of Y and the partial rows
+  const uint64_t* a_off;
+  const uint32_t *a_ns, *a_ket, *a_info;
+  const T* Vt;       // unpacked integrals, row stride vstride
+  const T* Dr;       // [na] rows of the integral row of the alpha string itself, row stride vstride
+  size_t vstride;
+  int npair;
+  uint32_t vstr;     // packs per staged integral row
+  int max_packs, nbatch, np, panel, nmain, nex, ny;
+  const uint4* rec;
+  const uint64_t* boff;
+  const uint32_t *bsteps, *wsteps, *ex_row, *ex_off;
+  const uint4 *items, *split;
+  const uint32_t* slot_split;
+  uint32_t* done;
+  double *ypart, *Y;
+  int* err;
+};
+
+// Step order of the updates of y: one arrival per warp and step on an
+// mbarrier. A warp waits for step s - 1 before it updates y in step s, so the
+// integral gathers of step s run while slower warps finish step s - 1; with a
+// full barrier per step the shared-memory pipe drains at each one. Phases end
+// by arrivals of this CTA's own warps alone; the wait is bounded all the same.
+__device__ __forceinline__ void step_init(uint32_t bar, uint32_t warps) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(warps) : "memory");
+}
+__device__ __forceinline__ void step_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void step_wait(uint32_t bar, uint32_t ph, int* err) {
+  if (ph == 0) return;
+  const uint32_t parity = (ph - 1) & 1u;
+  for (int it = 0; it < (1 << 20); ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return;
+  }
+  atomicExch(err, kErrWatchdogAb);  // gives up: the result is flagged, nothing waits for it
+}
+
+// All batches of one group of nr alpha singles held in NH packs.
+template <typename T, int NT, int NH>
+__device__ __forceinline__ void ab_sweep(const AbArgs<T>& a, const typename RowPack<T>::P* __restrict__ vs,
+                                         double* __restrict__ y, const uint32_t* s_ket, int nr, uint32_t bar,
+                                         uint32_t& ph) {
+  using RP = RowPack<T>;
+  constexpr int VR = RP::kRows, R = NH * VR;
+  const int warp = threadIdx.x >> 5;
+  for (int b = 0; b < a.nbatch; ++b) {
+    const int steps = (int)a.bsteps[b];
+    const int wst = (int)a.wsteps[b * (NT / 32) + warp];
+    T c[R];
+    const T* xb = a.Xk + (size_t)b * NT + threadIdx.x;
+#pragma unroll
+    for (int r = 0; r < R; ++r) c[r] = (r < nr && wst > 0) ? __ldg(xb + (size_t)s_ket[r] * a.xs) : (T)0;
+    const uint4* rp = a.rec + a.boff[b] + threadIdx.x;
+    uint4 cur = steps > 0 ? __ldg(rp) : make_uint4(kAbPad, kAbPad, kAbPad, kAbPad);
+    for (int m0 = 0; m0 < steps; m0 += 4) {
+      const uint4 nxt = m0 + 4 < wst ? __ldg(rp + (size_t)(m0 / 4 + 1) * NT) : cur;
+      const uint32_t recs[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (m0 + q >= steps) break;
+        const uint32_t rec = recs[q];
+        const bool live = m0 + q < wst;  // warp-uniform
+        double t[2] = {0.0, 0.0};
+        if (live) {
+          const typename RP::P* v = vs + (rec & 0xfffu);
+#pragma unroll
+          for (int h = 0; h < NH; ++h) RP::dot(v[(size_t)h * a.vstr], c + h * VR, t);
+        }
+        step_wait(bar, ph, a.err);  // the previous step's updates of y are done
+        if (live && !(rec & kAbPad)) {
+          double* yp = y + ((rec >> 12) & 0xffffu);
+          *yp += flip_sign(t[0] + t[1], rec >> 31);
+        }
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) step_arrive(bar);
+        ++ph;
+      }
+      cur = nxt;
+    }
+  }
+}
+
+// Alpha single x beta single in the alpha-first basis. One CTA per work item:
+// a bra alpha string, or a range of the singles of a long one (Conn::ab_item).
+// Per group of up to kAbPacks * kRows alpha singles (ja_r, pq_r, s_r) of the
+// item, the signed integral rows s_r (pq_r|..) are staged in shared memory as
+// 16-byte packs; a thread owns one ket string jb at a time, with C'[ja_r, jb]
+// of the whole group in registers, and walks jb's singles (ib <- jb, rs, s):
+// y[ib] += s * sum_r s_r (pq_r|rs) C'[ja_r, jb], y in shared memory. The
+// Coulomb terms of the beta singles with the alpha string ride along as one
+// more "single" ja = ia whose integral row is Dr. The
+// schedule (AbPlan) never lets two threads of a step update the same slot, so
+// a barrier per step orders the updates: no atomics, one summation order.
+//
+// Bound: the shared-memory pipe. Staging integrals instead of ket rows lets a
+// group hold 10 (FP64) or 20 (FP32) alpha singles instead of the 2 or 4 whose
+// ket rows of 8000 strings fit, and replaces the ket gather of every pair by
+// registers: per record of a group one 16-byte gather per pack and one
+// read-add-write of y, against two 16-byte gathers per pack.
+template <typename T, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
   using RP = RowPack<T>;
   using P = typename RP::P;
   constexpr int VR = RP::kRows;
-  constexpr int kWarps = kAb6Threads / 32;
   extern __shared__ __align__(16) unsigned char smem[];
-  P* xs = reinterpret_cast<P*>(smem);   // [nbp]: ket jb at kpos[jb] - jb0 (jb in jb0 .. jb0 + nbp - 1)
-  P* er = xs + nbp;                     // [epad + npair]: copy 0 at pq, copy 1 at epad + pq
-  double* part = reinterpret_cast<double*>(er + epad + npair);
-  // work item: bra alpha string, range of its singles, output row
-  const uint4 item = items[blockIdx.x];
+  __shared__ uint32_t s_ket[kAbPacks * 4], s_pq[kAbPacks * 4];
+  __shared__ __align__(8) uint64_t s_bar;
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
+  uint32_t ph = 0;  // steps finished by this warp
+  if (threadIdx.x == 0) step_init(bar, NT / 32);
+  const uint4 item = a.items[blockIdx.x];
   const size_t ia = item.x;
-  const int kend = (int)item.z;
-  double* __restrict__ Yrow = item.w ? ypart + (size_t)(item.w - 1) * ldx : Y + ia * ldx;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t slice0 = (size_t)blockIdx.y * kWarps * KS;
-  auto slice_of = [&](int k) -> size_t {
-    return slice0 + (size_t)k * kWarps + ((k & 1) ? (kWarps - 1 - warp) : warp);
-  };
-  double acc[KS];
-#pragma unroll
-  for (int k = 0; k < KS; ++k) acc[k] = 0.0;
-  const uint64_t e0 = a_off[ia];
-  for (int k0 = (int)item.y; k0 < kend; k0 += VR) {
-    const int nr = min(VR, kend - k0);
-    const T* xrow[VR];
-    const T* vrow_p[VR];
-    bool neg[VR];
-#pragma unroll
-    for (int e = 0; e < VR; ++e) {
-      const uint64_t ent = e0 + k0 + (e < nr ? e : 0);
-      const uint32_t inf = a_info[ent];
-      xrow[e] = Xp + (size_t)a_ket[ent] * ldx + jb0;
-      vrow_p[e] = Vt + (size_t)((inf >> 12) & 0xfffu) * vstride;
-      neg[e] = (inf >> 31) != 0;
+  double* y = reinterpret_cast<double*>(smem);                        // [ny]
+  P* vs = reinterpret_cast<P*>(smem + (((size_t)a.ny * 8 + 15) & ~(size_t)15));  // [packs][vstr]
+  for (int i = threadIdx.x; i < a.ny; i += NT) y[i] = 0.0;
+  const uint64_t e0 = a.a_off[ia];
+  const int n = (int)(item.z - item.y), ns = (int)a.a_ns[ia];
+  const int rmax = a.max_packs * VR;
+  const int ng = (n + rmax - 1) / rmax;
+  const int per = ng > 0 ? ((n + ng - 1) / ng + VR - 1) / VR * VR : VR;  // balanced groups of whole packs
+  for (int k0 = 0; k0 < n; k0 += per) {
+    const int nr = min(per, n - k0), nh = (nr + VR - 1) / VR;
+    const int nd = min(nr, ns - (int)item.y - k0);  // the rest (at most one) is the string itself
+    __syncthreads();  // the integrals of the group before are no longer read
+    if ((int)threadIdx.x < nh * VR) {
+      uint32_t ket = (uint32_t)ia, pqs = 0;
+      if ((int)threadIdx.x < nd) {
+        const uint64_t ent = e0 + item.y + k0 + threadIdx.x;
+        const uint32_t inf = a.a_info[ent];
+        ket = a.a_ket[ent];
+        pqs = ((inf >> 12) & 0xfffu) | (inf & kInfoNeg);
+      }
+      s_ket[threadIdx.x] = ket;
+      s_pq[threadIdx.x] = pqs;
     }
     __syncthreads();
-    // ket jb goes to position kpos[jb] - jb0, a permutation within aligned
-    // groups of 8: the 8 lanes of a quarter-warp store to 8 different slots.
-    // Each thread loads kStage packs before it stores them, so as many loads
-    // of the ket rows are in flight.
-    constexpr int kStage = 4;
-    for (size_t t0 = threadIdx.x; t0 < nbp; t0 += (size_t)kStage * kAb6Threads) {
-      P p[kStage];
-      uint32_t at[kStage];
+    for (int t = threadIdx.x; t < a.npair; t += NT) {
 #pragma unroll
-      for (int u = 0; u < kStage; ++u) {
-        const size_t t = t0 + (size_t)u * kAb6Threads;
-        at[u] = t < nbp ? __ldg(kpos + jb0 + t) - jb0 : 0u;
+      for (int h = 0; h < kAbPacks; ++h) {
+        if (h >= nh) break;
+        P p;
 #pragma unroll
-        for (int e = 0; e < VR; ++e) RP::set(p[u], e, (e < nr && t < nbp) ? __ldg(xrow[e] + t) : (T)0);
-      }
-#pragma unroll
-      for (int u = 0; u < kStage; ++u)
-        if (t0 + (size_t)u * kAb6Threads < nbp) xs[at[u]] = p[u];
-    }
-    for (int t = threadIdx.x; t < npair; t += kAb6Threads) {
-      P p;
-#pragma unroll
-      for (int e = 0; e < VR; ++e) {
-        const T v = e < nr ? __ldg(vrow_p[e] + t) : (T)0;
-        RP::set(p, e, neg[e] ? -v : v);
-      }
-      er[t] = p;
-      er[epad + t] = p;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < KS; ++k) {
-      const size_t sl = slice_of(k);
-      if (sl >= nslice) continue;
-      // 32-bit records (bits 0-15 staged ket position, 16-27 pair, 28 sign, 29 pad, 30 integral
-      // copy), four per lane per 16-byte load, the next block in flight
-      const uint32_t nblk = slen4[sl] >> 2;
-      const uint4* rp = reinterpret_cast<const uint4*>(sell + soff4[sl]) + lane;
-      double s = acc[k];
-      uint4 cur = nblk ? __ldg(rp) : make_uint4(0u, 0u, 0u, 0u);
-      for (uint32_t bk = 0; bk < nblk; ++bk) {
-        const uint4 nxt = bk + 1 < nblk ? __ldg(rp + 32ull * (bk + 1)) : cur;
-        const uint32_t recs[4] = {cur.x, cur.y, cur.z, cur.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const uint32_t rec = recs[q];
-          const P x = xs[rec & 0xffffu];  // panel-relative position; pad records repeat a real record's addresses
-          const P ev = er[((rec >> 16) & 0xfffu) + ((rec >> 30) & 1u) * epad];
-          double d = RP::dot(ev, x);
-          d = ((rec >> 29) & 1u) ? 0.0 : d;
-          s += flip_sign(d, (rec >> 28) & 1u);
+        for (int e = 0; e < VR; ++e) {
+          const int r = h * VR + e;
+          const uint32_t pqs = s_pq[r];
+          const T* row = r < nd ? a.Vt + (size_t)(pqs & 0xfffu) * a.vstride : a.Dr + ia * a.vstride;
+          const T v = r < nr ? __ldg(row + t) : (T)0;
+          RP::set(p, e, (pqs >> 31) ? -v : v);
         }
-        cur = nxt;
+        vs[(size_t)h * a.vstr + t] = p;
       }
-      acc[k] = s;
     }
-  }
-#pragma unroll
-  for (int k = 0; k < KS; ++k) {
-    const size_t sl = slice_of(k);
-    const size_t pos = sl * 32 + lane;
-    if (sl < nslice && pos < nv) {
-      const uint32_t slot1 = vslot[pos];
-      if (slot1 == 0) Yrow[vrow[pos]] += acc[k];
-      else part[slot1 - 1] = acc[k];
-    }
-  }
-  if (blockIdx.y == 0 && nsplit > 0) {
     __syncthreads();
-    for (int s = threadIdx.x; s < nsplit; s += kAb6Threads) {
-      double t = 0.0;
-      for (uint32_t j = split_slot[s]; j < split_slot[s + 1]; ++j) t += part[j];
-      Yrow[split_row[s]] += t;
+    switch (nh) {
+      case 1: ab_sweep<T, NT, 1>(a, vs, y, s_ket, nr, bar, ph); break;
+      case 2: ab_sweep<T, NT, 2>(a, vs, y, s_ket, nr, bar, ph); break;
+      case 3: ab_sweep<T, NT, 3>(a, vs, y, s_ket, nr, bar, ph); break;
+      case 4: ab_sweep<T, NT, 4>(a, vs, y, s_ket, nr, bar, ph); break;
+      default: ab_sweep<T, NT, 5>(a, vs, y, s_ket, nr, bar, ph); break;
     }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < a.nex; e += NT) {  // extra slots of crowded strings, in slot order
+    double t = y[a.ex_row[e]];
+    for (uint32_t j = a.ex_off[e]; j < a.ex_off[e + 1]; ++j) t += y[a.nmain + j];
+    y[a.ex_row[e]] = t;
+  }
+  if (a.nex > 0) __syncthreads();
+  auto col = [&](int i) -> size_t { return a.np == 1 ? (size_t)i : (size_t)(i / 4) * 4 * a.np + 4 * a.panel + i % 4; };
+  double* __restrict__ Yrow = a.Y + ia * a.ldx;
+  if (item.w == 0) {
+    for (int i = threadIdx.x; i < a.nmain; i += NT) Yrow[col(i)] = y[i];
+    return;
+  }
+  // a part of a split string: its partial row; the last part to finish adds all in slot order
+  double* mine = a.ypart + (size_t)(item.w - 1) * a.ldx;
+  for (int i = threadIdx.x; i < a.nmain; i += NT) mine[col(i)] = y[i];
+  const uint32_t sp = a.slot_split[item.w - 1];
+  const uint4 s = a.split[sp];
+  if (!last_part(a.done, sp, s.z)) return;
+  const double* part = a.ypart + (size_t)s.y * a.ldx;
+  for (int i = threadIdx.x; i < a.nmain; i += NT) {
+    const size_t k = col(i);
+    double t = 0.0;
+    for (uint32_t q = 0; q < s.z; ++q) t += __ldcg(part + (size_t)q * a.ldx + k);
+    Yrow[k] = t;
   }
 }
 
-// Shared memory of v7 on one panel: its ket range, the two copies of the
-// integral row (ab7_er_packs 16-byte packs) and its split slots. (The kernels' dynamic shared-memory limit is always set
-// to the full budget: the attribute is global per kernel, and contexts on
-// other host threads launch the same kernel with other sizes.)
-size_t ab7_smem_bytes(const Ctx* c, const SellPanel& p) {
-  return 16 * ((size_t)(p.jb1 - p.jb0) + ab7_er_packs(c->npair)) + sizeof(double) * (size_t)p.nslot;
+// Packs of a group that fit beside a panel's y slots.
+int ab_packs(const Ctx* c, const AbPanel& p) {
+  int k = kAbPacks;
+  while (k > 1 && 16 * (size_t)k * c->ab.vstr + sizeof(double) * (size_t)p.ny + kAbStaticSmem > kAbSmemBudget) --k;
+  return k;
 }
 
-// The panels v7 runs on: the whole ket range, or the ket-range slices.
-const std::vector<SellPanel>* ab7_panels(const Ctx* c, std::vector<SellPanel>& one) {
-  const Conn& cb = c->conn[1];
-  if (!cb.panels.empty()) return &cb.panels;
-  one.assign(1, cb.bal);
-  return &one;
-}
-
-bool ab7_fits(const Ctx* c) {
-  std::vector<SellPanel> one;
-  for (const SellPanel& p : *ab7_panels(c, one))
-    if (ab7_smem_bytes(c, p) > kAbSmemBudget) return false;
-  return true;
-}
-
-// `it` supplies the work items: the alpha connectivity itself, or the items
-// of a row range (Ctx::range_conn).
-template <typename T, int KS>
-int launch_ab_v7(Ctx* c, const T* Xp, const SellPanel& bp, const Conn& it) {
-  const Conn& ca = c->conn[0];
-  const bool f64 = std::is_same<T, double>::value;
-  const T* Vt = f64 ? (const T*)c->d_V : (const T*)c->d_V32;
-  const size_t vs = f64 ? c->vstride : c->vstride32;
-  const size_t smem = ab7_smem_bytes(c, bp);
-  SBDX_CUDA(c, cudaFuncSetAttribute(sigma_ab_v7_kernel<T, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+template <typename T, int NT, int MINB>
+int launch_ab(Ctx* c, const AbArgs<T>& args, size_t n_item, size_t smem) {
+  SBDX_CUDA(c, cudaFuncSetAttribute(sigma_ab_kernel<T, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kAbSmemBudget));
-  const size_t per_cta = (size_t)(kAb6Threads / 32) * KS;
-  dim3 grid((unsigned)it.n_item, (unsigned)((bp.nslice + per_cta - 1) / per_cta));
-  if (grid.y == 0) grid.y = 1;
-  sigma_ab_v7_kernel<T, KS><<<grid, kAb6Threads, smem, c->stream>>>(
-      Xp, c->xsa, ca.off, ca.ket, ca.info, bp.sell32, bp.soff4, bp.slen4, bp.nslice, bp.vrow, bp.vslot, bp.nv,
-      bp.split_row, bp.split_slot, bp.nsplit, Vt, vs, (int)c->npair, (uint32_t)ab7_epad(c->npair), bp.jb0,
-      (size_t)(bp.jb1 - bp.jb0), c->conn[1].kpos, it.ab_item, it.ypart, c->d_y);
+  sigma_ab_kernel<T, NT, MINB><<<(unsigned)n_item, NT, smem, c->stream>>>(args);
   SBDX_LAUNCHED(c);
   return 0;
 }
 
-// Adds the partial rows of the alpha strings split over several work items to
-// the output, parts in slot order (one fixed summation order).
-__global__ void ab_split_fixup_kernel(const uint4* __restrict__ split, const double* __restrict__ ypart, size_t nb,
-                                      size_t ldx, double* __restrict__ Y) {
-  const uint4 sp = split[blockIdx.y];
-  const double* part = ypart + (size_t)sp.y * ldx;
-  for (size_t ib = (size_t)blockIdx.x * blockDim.x + threadIdx.x; ib < nb; ib += (size_t)gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (uint32_t q = 0; q < sp.z; ++q) t += part[(size_t)q * ldx + ib];
-    Y[(size_t)sp.x * ldx + ib] += t;
-  }
-}
-
+// Yab = the alpha-beta product on Xk (Ctx::d_xk) over the rows of the work
+// items: the alpha connectivity's, or those of a row range (Ctx::range_conn).
 template <typename T>
-int run_ab_v7(Ctx* c, const T* Xp, const Conn* items = nullptr) {
-  const Conn& ca = items ? *items : c->conn[0];
-  if (ca.n_item == 0) return 0;  // no alpha string has a single excitation
-  if (ca.n_part > 0)
-    SBDX_CUDA(c, cudaMemsetAsync(ca.ypart, 0, sizeof(double) * (size_t)ca.n_part * c->xsa, c->stream));
-  std::vector<SellPanel> one;
-  for (const SellPanel& bp : *ab7_panels(c, one)) {
+int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
+  const Conn& ca = c->conn[0];
+  const Conn& it = items ? *items : ca;
+  if (it.n_item == 0) return 0;
+  const bool f64 = std::is_same<T, double>::value;
+  const AbPlan& P = c->ab;
+  for (size_t q = 0; q < P.panels.size(); ++q) {
+    const AbPanel& p = P.panels[q];
+    AbArgs<T> a{};
+    a.Xk = reinterpret_cast<const T*>(c->d_xk);
+    a.xs = P.xs;
+    a.ldx = c->xsa;
+    a.a_off = ca.off;
+    a.a_ns = ca.nsing;
+    a.a_ket = ca.ket;
+    a.a_info = ca.info;
+    a.Dr = f64 ? (const T*)c->d_Dr : (const T*)c->d_Dr32;
+    a.Vt = f64 ? (const T*)c->d_V : (const T*)c->d_V32;
+    a.vstride = f64 ? c->vstride : c->vstride32;
+    a.npair = (int)c->npair;
+    a.vstr = P.vstr;
+    a.max_packs = ab_packs(c, p);
+    a.nbatch = P.nbatch;
+    a.np = P.np;
+    a.panel = (int)q;
+    a.nmain = p.nmain;
+    a.nex = p.nex;
+    a.ny = p.ny;
+    a.rec = reinterpret_cast<const uint4*>(p.rec);
+    a.boff = p.boff;
+    a.bsteps = p.bsteps;
+    a.wsteps = p.wsteps;
+    a.ex_row = p.ex_row;
+    a.ex_off = p.ex_off;
+    a.items = it.ab_item;
+    a.split = it.ab_split;
+    a.slot_split = it.ab_slot;
+    a.done = it.ab_done;
+    a.ypart = it.ypart;
+    a.Y = c->d_yab;
+    a.err = c->d_err;
+    const size_t smem = (((size_t)p.ny * 8 + 15) & ~(size_t)15) + 16 * (size_t)a.max_packs * P.vstr;
     int rc;
-    if (bp.slices_per_warp >= 16) rc = launch_ab_v7<T, 16>(c, Xp, bp, ca);
-    else if (bp.slices_per_warp >= 12) rc = launch_ab_v7<T, 12>(c, Xp, bp, ca);
-    else rc = launch_ab_v7<T, 8>(c, Xp, bp, ca);
+    if (P.threads == 256) rc = launch_ab<T, 256, 4>(c, a, it.n_item, smem);
+    else if (P.threads == 512) rc = launch_ab<T, 512, 2>(c, a, it.n_item, smem);
+    else rc = launch_ab<T, 1024, 1>(c, a, it.n_item, smem);
     if (rc) return rc;
   }
-  if (ca.n_split > 0) {
-    const unsigned bx = (unsigned)std::min<size_t>((c->nb + 255) / 256, 64);
-    ab_split_fixup_kernel<<<dim3(bx, (unsigned)ca.n_split), 256, 0, c->stream>>>(ca.ab_split, ca.ypart, c->nb,
-                                                                                  c->xsa, c->d_y);
-    SBDX_LAUNCHED(c);
-  }
-  return 0;
-}
-
-// Assigns (or, with accumulate, adds) the sum of the partial rows of the bra
-// strings split over several same-spin work items, parts in slot order.
-__global__ void same_split_fixup_kernel(const uint4* __restrict__ split, const double* __restrict__ ypart,
-                                        size_t ncol, size_t ldx, double* __restrict__ Y, int accumulate) {
-  const uint4 sp = split[blockIdx.y];
-  const double* part = ypart + (size_t)sp.y * ldx;
-  for (size_t col = (size_t)blockIdx.x * blockDim.x + threadIdx.x; col < ncol; col += (size_t)gridDim.x * blockDim.x) {
-    double t = 0.0;
-    for (uint32_t q = 0; q < sp.z; ++q) t += part[(size_t)q * ldx + col];
-    double* y = Y + (size_t)sp.x * ldx + col;
-    *y = accumulate ? *y + t : t;
-  }
-}
-
-template <typename T, int VEC>
-int launch_same_v6(Ctx* c, const T* X, size_t nrow, size_t ncol, size_t ldx, const Conn& cn,
-                   const typename Prec<T>::V* val, const typename Prec<T>::V* Dt, size_t dstride, const double* hii,
-                   double* Y, int accumulate) {
-  (void)nrow;
-  if (cn.n_same_item > 0) {
-    dim3 grid((unsigned)cn.n_same_item,
-              (unsigned)((ncol + (size_t)kSameThreads * VEC - 1) / ((size_t)kSameThreads * VEC)));
-    if constexpr (std::is_same<T, float>::value) {
-      sigma_same_v6f_kernel<VEC><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, cn.off, cn.nsing, cn.ket, val,
-                                                                        cn.info, Dt, dstride, hii, cn.same_item,
-                                                                        cn.same_ypart, Y, accumulate);
-    } else {
-      sigma_same_v6_kernel<T, VEC><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, cn.off, cn.nsing, cn.ket, val,
-                                                                         cn.info, Dt, dstride, hii, cn.same_item,
-                                                                         cn.same_ypart, Y, accumulate);
-    }
-    SBDX_LAUNCHED(c);
-  }
-  if (cn.n_same_split > 0) {
-    const unsigned bx = (unsigned)std::min<size_t>((ncol + 255) / 256, 64);
-    same_split_fixup_kernel<<<dim3(bx, (unsigned)cn.n_same_split), 256, 0, c->stream>>>(
-        cn.same_split, cn.same_ypart, ncol, ldx, Y, accumulate);
-    SBDX_LAUNCHED(c);
-  }
   return 0;
 }
 
 template <typename T, int VEC>
-int launch_same_blk(Ctx* c, const T* X, size_t ncol, size_t ldx, const Conn& cn, const T* val, const T* Dt,
-                    size_t dstride, const double* hii, double* Y, int accumulate) {
-  const SameBlocks& B = cn.blk;
-  using P4 = typename Vals4<T>::P;
-  const P4* uval = reinterpret_cast<const P4*>(std::is_same<T, double>::value ? (const void*)B.uval
-                                                                              : (const void*)B.uval32);
-  if (B.n_item > 0) {
-    dim3 grid((unsigned)B.n_item, (unsigned)((ncol + (size_t)kSameThreads * VEC - 1) / ((size_t)kSameThreads * VEC)));
-    sigma_same_blk_kernel<T, VEC><<<grid, kSameThreads, 0, c->stream>>>(
-        X, ncol, ldx, cn.off, cn.nsing, cn.ket, val, cn.info, Dt, dstride, hii, B.rows, B.uoff, B.uket, uval, B.item,
-        B.ypart, Y, accumulate);
-    SBDX_LAUNCHED(c);
+int launch_same_v6(Ctx* c, const T* X, size_t ncol, size_t ldx, const Conn& cn, const typename Prec<T>::V* val,
+                   const typename Prec<T>::V* Dt, size_t dstride, const double* hii, double* Y) {
+  if (cn.n_same_item == 0) return 0;
+  dim3 grid((unsigned)cn.n_same_item,
+            (unsigned)((ncol + (size_t)kSameThreads * VEC - 1) / ((size_t)kSameThreads * VEC)));
+  if constexpr (std::is_same<T, float>::value) {
+    sigma_same_v6f_kernel<VEC><<<grid, kSameThreads, 0, c->stream>>>(
+        X, ncol, ldx, cn.off, cn.nsing, cn.ket, val, cn.info, Dt, dstride, hii, cn.same_item, cn.same_split,
+        cn.same_slot, cn.same_done, cn.same_ypart, Y);
+  } else {
+    sigma_same_v6_kernel<T, VEC><<<grid, kSameThreads, 0, c->stream>>>(
+        X, ncol, ldx, cn.off, cn.nsing, cn.ket, val, cn.info, Dt, dstride, hii, cn.same_item, cn.same_split,
+        cn.same_slot, cn.same_done, cn.same_ypart, Y);
   }
-  if (B.n_split > 0) {
-    const unsigned bx = (unsigned)std::min<size_t>((ncol + 255) / 256, 64);
-    same_blk_fixup_kernel<<<dim3(bx, (unsigned)B.n_split, kBlkRows), 256, 0, c->stream>>>(B.split, B.rows, B.ypart,
-                                                                                         ncol, ldx, Y, accumulate);
-    SBDX_LAUNCHED(c);
-  }
+  SBDX_LAUNCHED(c);
   return 0;
 }
 
-// v6 same-spin codes: 21, 22, 24, 28 = 1, 2, 4, 8 columns per thread, narrowed
-// to the widest vector that divides the row stride and keeps 16-byte
-// alignment (the internal vectors have strides padded to 8 elements, so only
-// a misaligned base narrows).
-// Codes 31, 32, 34, 38: the blocked kernel with as many columns per thread.
-// accumulate: add to Y's rows instead of writing them (the pipelined
-// host-buffer sigma runs the alpha-beta kernel first).
+template <int P>
+int launch_same_blkd(Ctx* c, const double* X, size_t ncol, size_t ldx, const Conn& cn, const double* Dt, size_t dstride,
+                     double* Y) {
+  const SameBlocks& B = cn.blk[0];
+  constexpr size_t cols = (size_t)kSameThreads * 2 * P;
+  const dim3 grid((unsigned)B.n_item, (unsigned)((ncol + cols - 1) / cols));
+  sigma_same_blk_kernel<P><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, cn.off, cn.nsing, cn.ket, cn.info, Dt,
+                                                                 dstride, B.rows, B.uoff, B.uket, B.uval, B.item, B.split,
+                                                                 B.slot, B.done, B.ypart, Y);
+  SBDX_LAUNCHED(c);
+  return 0;
+}
+
+int launch_same_blk(Ctx* c, int vec, const double* X, size_t ncol, size_t ldx, const Conn& cn, const double* Dt,
+                    size_t dstride, double* Y) {
+  if (vec >= 4) return launch_same_blkd<2>(c, X, ncol, ldx, cn, Dt, dstride, Y);
+  return launch_same_blkd<1>(c, X, ncol, ldx, cn, Dt, dstride, Y);
+}
+
+template <int VEC>
+int launch_same_blkf(Ctx* c, const float* X, size_t ncol, size_t ldx, const Conn& cn, const float* Dt, size_t dstride,
+                     double* Y) {
+  const SameBlocks& B = cn.blk[1];
+  const dim3 grid((unsigned)B.n_item, (unsigned)((ncol + (size_t)kSameThreads * VEC - 1) / ((size_t)kSameThreads * VEC)));
+  sigma_same_blkf_kernel<VEC><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, cn.off, cn.nsing, cn.ket, cn.info, Dt,
+                                                                    dstride, B.rows, B.uoff, B.uket, B.uval32, B.item,
+                                                                    B.split, B.slot, B.done, B.ypart, Y);
+  SBDX_LAUNCHED(c);
+  return 0;
+}
+
+int launch_same_blk(Ctx* c, int vec, const float* X, size_t ncol, size_t ldx, const Conn& cn, const float* Dt,
+                    size_t dstride, double* Y) {
+  if (vec >= 4) return launch_same_blkf<4>(c, X, ncol, ldx, cn, Dt, dstride, Y);
+  if (vec == 2) return launch_same_blkf<2>(c, X, ncol, ldx, cn, Dt, dstride, Y);
+  return launch_same_blkf<1>(c, X, ncol, ldx, cn, Dt, dstride, Y);
+}
+
+// Same-spin codes: 21, 22, 24, 28 = 1, 2, 4, 8 columns per thread of the
+// one-string kernels, narrowed to the widest vector that divides the row
+// stride and keeps 16-byte alignment (the internal vectors have strides
+// padded to 8 elements, so only a misaligned base narrows). 31, 32, 34, 38:
+// the blocked kernels with 2 or 4 (FP64), 1, 2 or 4 (FP32) columns per thread;
+// they leave the diagonal out, so with hii (an unpacked alpha-beta code) the one-string kernels run.
 template <typename T>
-int run_same_v6(Ctx* c, int code, const T* X, size_t nrow, size_t ncol, size_t ldx, const Conn& cn,
+int run_same_v6(Ctx* c, int code, const T* X, size_t ncol, size_t ldx, const Conn& cn,
                 const typename Prec<T>::V* val, const typename Prec<T>::V* Dt, size_t dstride, const double* hii,
-                double* Y, int accumulate = 0) {
+                double* Y) {
   int vec = code % 10;
   const bool aligned = (reinterpret_cast<uintptr_t>(X) % 16) == 0;
-  while (vec > 1 && (!aligned || ldx % vec != 0 || dstride % vec != 0)) vec >>= 1;
-  if (code / 10 == 3 && cn.blk.nblk > 0) {  // blocked kernel (31, 32, 34, 38)
-    if (vec >= 8) return launch_same_blk<T, 8>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
-    if (vec >= 4) return launch_same_blk<T, 4>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
-    if (vec == 2) return launch_same_blk<T, 2>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
-    return launch_same_blk<T, 1>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
-  }
-  if (vec >= 8) return launch_same_v6<T, 8>(c, X, nrow, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
-  if (vec >= 4) return launch_same_v6<T, 4>(c, X, nrow, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
-  if (vec == 2) return launch_same_v6<T, 2>(c, X, nrow, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
-  return launch_same_v6<T, 1>(c, X, nrow, ncol, ldx, cn, val, Dt, dstride, hii, Y, accumulate);
+  while (vec > 1 && (!aligned || ldx % vec != 0 || (Dt != nullptr && dstride % vec != 0))) vec >>= 1;
+  if (code / 10 == 3 && cn.blk[0].nblk > 0 && hii == nullptr && aligned)
+    return launch_same_blk(c, vec, X, ncol, ldx, cn, Dt, dstride, Y);
+  if (vec >= 8) return launch_same_v6<T, 8>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
+  if (vec >= 4) return launch_same_v6<T, 4>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
+  if (vec == 2) return launch_same_v6<T, 2>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
+  return launch_same_v6<T, 1>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
 }
 
 template <typename T, int R, int KS>
@@ -1945,10 +2129,7 @@ int launch_ab_v6_ks(Ctx* c, const T* Xp, size_t smem, size_t xstride) {
 template <typename T>
 int run_ab_v6(Ctx* c, int code, const T* Xp) {
   using V = typename Prec<T>::V;
-  if (code / 10 == 7) {  // 71: packed rows, on ket-range panels when a whole row does not fit
-    if (ab7_fits(c)) return run_ab_v7<T>(c, Xp);
-    code = std::is_same<T, double>::value ? 62 : 64;
-  }
+  if (code / 10 == 7) return run_ab_packed<T>(c);  // 71
   const bool f64 = std::is_same<T, double>::value;
   const size_t vs = f64 ? c->vstride : c->vstride32;
   const size_t per = 16 / sizeof(T);
@@ -1971,11 +2152,64 @@ int run_ab_v6(Ctx* c, int code, const T* Xp) {
   return launch_ab_v6_ks<T, 1>(c, Xp, smem, xstride);
 }
 
+// Phase split of the rows [a0, a0 + nr) (X: the whole input), with their
+// lane-order copy when the packed alpha-beta kernel follows.
+template <typename T>
+int launch_split(Ctx* c, const T* X, size_t a0, size_t nr, T* xp, T* xpt, bool lanes) {
+  const size_t nb = c->nb, xs = lanes ? c->ab.xs : 0;
+  const dim3 grid((unsigned)((nb + 31) / 32 + (xs + 255) / 256), (unsigned)((nr + 31) / 32));
+  phase_split_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(
+      X + a0 * nb, nr, nb, c->d_a + a0, c->d_b, xp + a0 * c->xsa, xpt + a0, c->xsa, c->xsb, c->ab.vket,
+      reinterpret_cast<T*>(c->d_xk) + a0 * xs, xs);
+  SBDX_LAUNCHED(c);
+  return 0;
+}
+
+// S (row 0 = alpha string a0) of the rows [a0, a0 + nr); X: the whole input.
+template <typename T>
+int launch_combine(Ctx* c, const T* X, size_t a0, size_t nr, T* S, bool packed) {
+  const size_t nb = c->nb;
+  const dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((nr + 31) / 32));
+  combine_phase_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(
+      c->d_y + a0 * c->xsa, packed ? c->d_yab + a0 * c->xsa : nullptr, c->d_yt + a0, c->d_hii + a0 * nb, X + a0 * nb, nr,
+      nb, c->d_a + a0, c->d_b, S, c->xsa, c->xsb);
+  SBDX_LAUNCHED(c);
+  return 0;
+}
+
 bool same_alpha_first(int code) { return (code > 20 && code < 30) || (code > 30 && code < 40); }
 
 bool is_v6(const Tune& t) {
   return same_alpha_first(t.same_code) && ((t.ab_code > 60 && t.ab_code < 70) || t.ab_code == 71);
 }
+
+// Runs launches of the context on its side streams, so that a small problem's
+// three products, none of which fills the GPU, overlap (FP64 275 x 275 strings:
+// 72.5 us per sigma one after another, 49.5 us side by side; 2000 x 2000: 1324
+// and 1210 us; 8000 x 8000 unchanged within 1%): fork() makes both follow
+// the context stream, on(k) directs the next launches to side stream k, main()
+// back, join() makes the context stream follow both.
+struct SideBySide {
+  Ctx* c;
+  cudaStream_t home;
+  explicit SideBySide(Ctx* ctx) : c(ctx), home(ctx->stream) {}
+  ~SideBySide() { c->stream = home; }
+  int fork() {
+    SBDX_CUDA(c, cudaEventRecord(c->fork, home));
+    for (cudaStream_t s : c->side) SBDX_CUDA(c, cudaStreamWaitEvent(s, c->fork, 0));
+    return 0;
+  }
+  void on(int k) { c->stream = c->side[k]; }
+  void main() { c->stream = home; }
+  int join() {
+    c->stream = home;
+    for (int k = 0; k < 2; ++k) {
+      SBDX_CUDA(c, cudaEventRecord(c->join[k], c->side[k]));
+      SBDX_CUDA(c, cudaStreamWaitEvent(home, c->join[k], 0));
+    }
+    return 0;
+  }
+};
 
 template <typename T>
 int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
@@ -1995,26 +2229,36 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
   };
   int rc = 0;
   mark(0);
-  {
-    dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((na + 31) / 32));
-    phase_split_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(X, na, nb, c->d_a, c->d_b, xp, xpt, c->xsa, c->xsb);
-    SBDX_LAUNCHED(c);
+  if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, tune.ab_code == 71))) return rc;
+  // the beta singles' Coulomb terms and the diagonal: in the packed alpha-beta
+  // kernel and the combine, or in the same-spin kernels beside an unpacked one
+  const bool packed = tune.ab_code == 71;
+  const V* DtA = Db;
+  const V* DtB = packed ? nullptr : Da;
+  if (packed && !c->profiling) {
+    SideBySide f(c);
+    if ((rc = f.fork())) return rc;
+    f.on(0);
+    rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, valA, DtA, c->db_stride, nullptr, c->d_y);
+    f.on(1);
+    if (!rc) rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, valB, DtB, c->da_stride, nullptr, c->d_yt);
+    f.main();
+    if (!rc) rc = run_ab_packed<T>(c);
+    const int rj = f.join();
+    if (rc || rj) return rc ? rc : rj;
+    return launch_combine<T>(c, X, 0, na, S, true);
   }
   mark(1);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, na, nb, c->xsa, ca, valA, Db, c->db_stride, c->d_hii, c->d_y)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, valA, DtA, c->db_stride, packed ? nullptr : c->d_hii,
+                           c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt, nb, na, c->xsb, cb, valB, Da, c->da_stride, nullptr, c->d_yt)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, valB, DtB, c->da_stride, nullptr, c->d_yt)))
     return rc;
   mark(3);
   if ((rc = run_ab_v6<T>(c, tune.ab_code, xp))) return rc;
   mark(4);
-  {
-    dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((na + 31) / 32));
-    combine_phase_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(c->d_y, c->d_yt, na, nb, c->d_a, c->d_b, S, c->xsa,
-                                                                 c->xsb);
-    SBDX_LAUNCHED(c);
-  }
+  if ((rc = launch_combine<T>(c, X, 0, na, S, packed))) return rc;
   mark(5);
   if (c->profiling) {
     // reported in the phase order alpha same-spin, transpose (here the phase
@@ -2089,7 +2333,7 @@ int run_sigma_v5(Ctx* c, const T* X, T* S) {
 // 1 M (code 34 against 24).
 Tune default_tune(const Ctx* c, bool f64) {
   const size_t D = c->na * c->nb;
-  if (f64) return D >= kBlkMinDets64 ? Tune{32, 71} : Tune{22, 71};
+  if (f64) return D >= kBlkMinDets64 ? Tune{34, 71} : Tune{22, 71};
   return D >= kBlkMinDets32 ? Tune{34, 71} : Tune{24, 71};
 }
 
@@ -2129,17 +2373,18 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
   const Conn& cb = c->conn[1];
   const Conn& rc_items = c->range_conn;
   Conn ra = ca;  // the alpha lists with the range's same-spin work items
-  ra.blk = rc_items.blk;
+  for (int q = 0; q < 2; ++q) ra.blk[q] = rc_items.blk[q];
   ra.same_item = rc_items.same_item;
   ra.n_same_item = rc_items.n_same_item;
   ra.same_split = rc_items.same_split;
+  ra.same_slot = rc_items.same_slot;
+  ra.same_done = rc_items.same_done;
   ra.n_same_split = rc_items.n_same_split;
   ra.n_same_part = rc_items.n_same_part;
   ra.same_ypart = rc_items.same_ypart;
   const V* valA = f64 ? (const V*)ca.val : (const V*)ca.val32;
   const V* valB = f64 ? (const V*)cb.val : (const V*)cb.val32;
   const V* Db = f64 ? (const V*)c->d_Db : (const V*)c->d_Db32;
-  const V* Da = f64 ? (const V*)c->d_Da : (const V*)c->d_Da32;
   T* xp = reinterpret_cast<T*>(c->d_xp);
   T* xpt = reinterpret_cast<T*>(c->d_xt);
   auto mark = [&](int k) {
@@ -2147,28 +2392,19 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
   };
   int rc = 0;
   mark(0);
-  {
-    dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((na + 31) / 32));
-    phase_split_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(X, na, nb, c->d_a, c->d_b, xp, xpt, c->xsa, c->xsb);
-    SBDX_LAUNCHED(c);
-  }
+  if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, true))) return rc;
   mark(1);
   if (nr == 0) return 0;
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, na, nb, c->xsa, ra, valA, Db, c->db_stride, c->d_hii, c->d_y)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ra, valA, Db, c->db_stride, nullptr, c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt + a0, nb, nr, c->xsb, cb, valB, Da + a0, c->da_stride, nullptr,
+  if ((rc = run_same_v6<T>(c, tune.same_code, xpt + a0, nr, c->xsb, cb, valB, (const V*)nullptr, 0, nullptr,
                            c->d_yt + a0)))
     return rc;
   mark(3);
-  if ((rc = run_ab_v7<T>(c, xp, &rc_items))) return rc;
+  if ((rc = run_ab_packed<T>(c, &rc_items))) return rc;
   mark(4);
-  {
-    dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((nr + 31) / 32));
-    combine_phase_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(c->d_y + a0 * c->xsa, c->d_yt + a0, nr, nb,
-                                                                 c->d_a + a0, c->d_b, S, c->xsa, c->xsb);
-    SBDX_LAUNCHED(c);
-  }
+  if ((rc = launch_combine<T>(c, X, a0, nr, S, true))) return rc;
   mark(5);
   if (c->profiling) {  // the phase order of run_sigma_v6
     const int from[kSigmaPhases] = {1, 0, 2, 3, 4};
@@ -2185,26 +2421,37 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
 
 }  // namespace
 
+// The Coulomb tables of the alpha-first sigma (Ctx::d_Db, d_Dr).
 int build_coulomb_tables(Ctx* c) {
-  cudaFree(c->d_Da); cudaFree(c->d_Db); cudaFree(c->d_Da32); cudaFree(c->d_Db32);
-  c->d_Da = c->d_Db = nullptr;
-  c->d_Da32 = c->d_Db32 = nullptr;
-  c->da_stride = pad8(c->na);
   c->db_stride = pad8(c->nb);
-  const size_t na_el = c->npair * c->da_stride, nb_el = c->npair * c->db_stride;
-  SBDX_CUDA(c, cudaMalloc(&c->d_Da, sizeof(double) * na_el));
+  const size_t nb_el = c->npair * c->db_stride;
   SBDX_CUDA(c, cudaMalloc(&c->d_Db, sizeof(double) * nb_el));
-  SBDX_CUDA(c, cudaMalloc(&c->d_Da32, sizeof(float) * na_el));
   SBDX_CUDA(c, cudaMalloc(&c->d_Db32, sizeof(float) * nb_el));
-  SBDX_CUDA(c, cudaMemsetAsync(c->d_Da, 0, sizeof(double) * na_el, c->stream));
+  SBDX_CUDA(c, cudaMalloc(&c->d_Dr, sizeof(double) * c->na * c->vstride));
+  SBDX_CUDA(c, cudaMalloc(&c->d_Dr32, sizeof(float) * c->na * c->vstride32));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Db, 0, sizeof(double) * nb_el, c->stream));
-  SBDX_CUDA(c, cudaMemsetAsync(c->d_Da32, 0, sizeof(float) * na_el, c->stream));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Db32, 0, sizeof(float) * nb_el, c->stream));
-  dim3 ga((unsigned)((c->na + 255) / 256), (unsigned)c->npair);
-  coulomb_table_kernel<<<ga, 256, 0, c->stream>>>(c->d_G, c->L, c->d_a, c->na, c->da_stride, c->d_Da, c->d_Da32);
-  SBDX_LAUNCHED(c);
-  dim3 gb((unsigned)((c->nb + 255) / 256), (unsigned)c->npair);
+  const dim3 gb((unsigned)((c->nb + 255) / 256), (unsigned)c->npair);
   coulomb_table_kernel<<<gb, 256, 0, c->stream>>>(c->d_G, c->L, c->d_b, c->nb, c->db_stride, c->d_Db, c->d_Db32);
+  SBDX_LAUNCHED(c);
+  coulomb_row_sum_kernel<<<(unsigned)c->na, 256, 0, c->stream>>>(c->d_V, c->npair, c->vstride, c->vstride32, c->L, c->d_a,
+                                                                 c->d_Dr, c->d_Dr32);
+  SBDX_LAUNCHED(c);
+  return 0;
+}
+
+int ensure_coulomb_a(Ctx* c) {
+  if (c->d_Da) return 0;
+  c->da_stride = pad8(c->na);
+  const size_t na_el = c->npair * c->da_stride;
+  SBDX_CUDA(c, cudaMalloc(&c->d_Da32, sizeof(float) * na_el));
+  SBDX_CUDA(c, cudaMemsetAsync(c->d_Da32, 0, sizeof(float) * na_el, c->stream));
+  double* Da = nullptr;
+  SBDX_CUDA(c, cudaMalloc(&Da, sizeof(double) * na_el));
+  c->d_Da = Da;
+  SBDX_CUDA(c, cudaMemsetAsync(c->d_Da, 0, sizeof(double) * na_el, c->stream));
+  const dim3 ga((unsigned)((c->na + 255) / 256), (unsigned)c->npair);
+  coulomb_table_kernel<<<ga, 256, 0, c->stream>>>(c->d_G, c->L, c->d_a, c->na, c->da_stride, c->d_Da, c->d_Da32);
   SBDX_LAUNCHED(c);
   return 0;
 }
@@ -2247,8 +2494,18 @@ int ensure_sigma_scratch(Ctx* c) {
     return 0;
   };
   int rc;
-  if ((rc = get(&c->d_xt)) || (rc = get(&c->d_xp)) || (rc = get((void**)&c->d_y)) || (rc = get((void**)&c->d_yt)))
+  if ((rc = get(&c->d_xt)) || (rc = get(&c->d_xp)) || (rc = get((void**)&c->d_y)) || (rc = get((void**)&c->d_yt)) ||
+      (rc = get((void**)&c->d_yab)))
     return rc;
+  if (!c->fork) {
+    for (auto& x : c->side) SBDX_CUDA(c, cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    for (auto& e : c->join) SBDX_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    SBDX_CUDA(c, cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
+  }
+  if (c->ab.xs && !c->d_xk) {
+    SBDX_CUDA(c, cudaMalloc(&c->d_xk, sizeof(double) * c->na * c->ab.xs));
+    SBDX_CUDA(c, cudaMemsetAsync(c->d_xk, 0, sizeof(double) * c->na * c->ab.xs, c->stream));
+  }
   return 0;
 }
 
@@ -2261,7 +2518,7 @@ int autotune(Ctx* c) {
   clear_sigma_graphs(c);
   if (!c->have_conn && (rc = build_connectivity(c))) return rc;
   if (!c->have_hii && (rc = diag_terms(c))) return rc;
-  if ((rc = ensure_sigma_scratch(c))) return rc;
+  if ((rc = ensure_sigma_scratch(c)) || (rc = ensure_sell(c)) || (rc = ensure_coulomb_a(c))) return rc;
   const size_t D = c->na * c->nb;
   void *X = nullptr, *S = nullptr;
   SBDX_CUDA(c, pool_alloc(c, &X, sizeof(double) * D));
@@ -2401,10 +2658,6 @@ int sigma_rows_device(Ctx* c, int precision, const void* X, void* S, size_t a0, 
   const bool f64 = precision == 0;
   Tune t = effective_tune(c, f64);
   if (!is_v6(t)) t = default_tune(c, f64);  // the row range runs the alpha-first kernels
-  if (!ab7_fits(c)) {
-    c->err = "sigma_rows: the packed alpha-beta kernel cannot stage this problem's rows";
-    return SBDX_ERR_ARG;
-  }
   if (!c->have_range || c->range_a0 != a0 || c->range_a1 != a1) {
     if ((rc = build_row_range(c, a0, a1))) return rc;
   }
@@ -2429,6 +2682,7 @@ int sigma_device(Ctx* c, int precision, const void* X, void* S) {
   }
   if (precision == 0 && c->stored.val != nullptr)
     return stored_sigma(c, static_cast<const double*>(X), static_cast<double*>(S));
+  if (effective_tune(c, precision == 0).ab_code != 71 && ((rc = ensure_sell(c)) || (rc = ensure_coulomb_a(c)))) return rc;
   if (c->use_graphs && !c->profiling && c->stream != nullptr) {
     rc = sigma_graph(c, precision, X, S);
     if (rc >= 0) return rc;
@@ -2517,8 +2771,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
   double* dout = static_cast<double*>(c->d_io_out);
   const Tune t = effective_tune(c, true);
   const int K = io_chunk_count(c);
-  const bool pipe = K >= 2 && c->stored.val == nullptr && is_v6(t) && t.ab_code == 71 && ab7_fits(c) &&
-                    !c->profiling;
+  const bool pipe = K >= 2 && c->stored.val == nullptr && is_v6(t) && t.ab_code == 71 && !c->profiling;
   if (!pipe) {  // one copy in, the sigma, one copy out
     SBDX_CUDA(c, cudaMemcpyAsync(din, hC, sizeof(double) * D, cudaMemcpyHostToDevice, c->stream));
     if ((rc = sigma_device(c, SBDX_FP64, din, dout))) return rc;
@@ -2547,38 +2800,31 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
   for (size_t i = 0; i < n; ++i) {  // per arrived chunk: phase split, beta same-spin on its columns
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
     SBDX_CUDA(c, cudaStreamWaitEvent(c->stream, ev[i], 0));
-    const dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((nr + 31) / 32));
-    phase_split_kernel<double><<<grid, dim3(32, 8), 0, c->stream>>>(din + a0 * nb, nr, nb, c->d_a + a0, c->d_b,
-                                                                     xp + a0 * c->xsa, xpt + a0, c->xsa, c->xsb);
-    SBDX_LAUNCHED(c);
-    if ((rc = run_same_v6<double>(c, t.same_code, xpt + a0, nb, nr, c->xsb, cb, cb.val, c->d_Da + a0, c->da_stride,
-                                  nullptr, c->d_yt + a0)))
+    if ((rc = launch_split<double>(c, din, a0, nr, xp, xpt, true))) return rc;
+    if ((rc = run_same_v6<double>(c, t.same_code, xpt + a0, nr, c->xsb, cb, cb.val, (const double*)nullptr, 0, nullptr,
+                                  c->d_yt + a0)))
       return rc;
   }
   // the alpha-beta product of all rows in one launch (its work items keep
-  // the whole grid busy, longest first) into a zeroed Y, then per chunk the
-  // alpha same-spin items of its rows added to Y, and the combine
-  SBDX_CUDA(c, cudaMemsetAsync(c->d_y, 0, sizeof(double) * na * c->xsa, c->stream));
-  if ((rc = run_ab_v7<double>(c, xp))) return rc;
+  // the whole grid busy, longest first), then per chunk the alpha same-spin
+  // items of its rows and the combine
+  if ((rc = run_ab_packed<double>(c))) return rc;
   for (size_t i = 0; i < n; ++i) {
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
     const Conn& it = c->io_items[i];
     Conn ra = ca;
-    ra.blk = it.blk;
+    for (int q = 0; q < 2; ++q) ra.blk[q] = it.blk[q];
     ra.same_item = it.same_item;
     ra.n_same_item = it.n_same_item;
     ra.same_split = it.same_split;
+    ra.same_slot = it.same_slot;
+    ra.same_done = it.same_done;
     ra.n_same_split = it.n_same_split;
     ra.n_same_part = it.n_same_part;
     ra.same_ypart = it.same_ypart;
-    if ((rc = run_same_v6<double>(c, t.same_code, xp, na, nb, c->xsa, ra, ca.val, c->d_Db, c->db_stride, c->d_hii,
-                                  c->d_y, 1)))
+    if ((rc = run_same_v6<double>(c, t.same_code, xp, nb, c->xsa, ra, ca.val, c->d_Db, c->db_stride, nullptr, c->d_y)))
       return rc;
-    const dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((nr + 31) / 32));
-    combine_phase_kernel<double><<<grid, dim3(32, 8), 0, c->stream>>>(c->d_y + a0 * c->xsa, c->d_yt + a0, nr, nb,
-                                                                       c->d_a + a0, c->d_b, dout + a0 * nb, c->xsa,
-                                                                       c->xsb);
-    SBDX_LAUNCHED(c);
+    if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true))) return rc;
     SBDX_CUDA(c, cudaEventRecord(ev[n + i], c->stream));
   }
   for (size_t i = 0; i < n; ++i) {  // each chunk out as soon as it is ready

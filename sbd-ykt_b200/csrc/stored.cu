@@ -184,6 +184,7 @@ void release_stored(Ctx* c) {
 int build_stored(Ctx* c) {
   if (!c->have_conn) { int rc = build_connectivity(c); if (rc) return rc; }
   if (!c->have_hii) { int rc = diag_terms(c); if (rc) return rc; }
+  if (int rc = ensure_coulomb_a(c)) return rc;
   release_stored(c);
   const size_t na = c->na, nb = c->nb, D = na * nb;
   if (D > (size_t)UINT32_MAX) {  // the columns are 32-bit determinant indices

@@ -1,0 +1,59 @@
+"""The sigma's kernels at the edges of their tiles, against the oracle.
+
+The packed alpha-beta kernel (code 71) gives a thread one ket lane of 256,
+512 or 1024 and splits long lists over lanes, groups of alpha singles hold 10
+(FP64) or 20 (FP32), and the blocked same-spin kernels take 8 or 4 bra strings
+and 512 or 1024 columns; one string, odd counts and counts one off those
+sizes go through every remainder. Tolerances: FP64 1e-12 of the largest
+element (sums of some 1e3 terms, each rounded to 1.1e-16); FP32 storage 2e-6
+(vectors and integrals rounded to 6e-8, some 1e3 terms of mixed sign).
+"""
+import numpy as np
+import pytest
+
+import sbdx
+from sbdx import synth
+from oracle import Port
+
+pytestmark = pytest.mark.gpu
+
+# L, alpha and beta electrons, Na, Nb
+SIZES = [
+    (6, 1, 1, 1, 1),        # one determinant, no excitation
+    (8, 2, 3, 1, 9),        # one alpha string
+    (8, 3, 2, 9, 1),        # one beta string
+    (12, 4, 4, 33, 255),
+    (12, 4, 4, 40, 257),
+    (14, 4, 4, 65, 512),
+    (14, 5, 4, 17, 513),
+    (16, 4, 5, 130, 1025),
+    (24, 5, 5, 1025, 31),
+    (58, 7, 7, 90, 640),    # the most integral rows per group that fit beside y
+]
+
+
+@pytest.fixture(scope="module")
+def port():
+    return Port()
+
+
+@pytest.mark.parametrize("codes", [(0, 0), (22, 71), (32, 71), (34, 71)])
+@pytest.mark.parametrize("size", SIZES)
+def test_sigma_matches_oracle_at_tile_edges(size, codes, port):
+    torch = pytest.importorskip("torch")
+    prob = synth.random_problem(*size, seed=sum(size))
+    C = np.random.default_rng(5).standard_normal(prob.D)
+    x32 = torch.from_numpy(C.astype(np.float32)).cuda()
+    s32 = torch.empty_like(x32)
+    with sbdx.Context(0) as ctx:
+        ctx.load(prob)
+        ctx.set_tuning(*codes)
+        S = ctx.sigma(C)
+        again = ctx.sigma(C)
+        ctx.sigma_device(sbdx.SBDX_FP32, x32.data_ptr(), s32.data_ptr())
+        torch.cuda.synchronize()
+    ref = port.sigma(prob, C)
+    top = np.abs(ref).max()
+    assert np.abs(S - ref).max() <= 1e-12 * top
+    assert np.array_equal(S, again)  # one summation order
+    assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top

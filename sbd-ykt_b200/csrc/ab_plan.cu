@@ -9,10 +9,11 @@
 // the singles of all kets into steps:
 //   - a ket with many singles is split over several lanes, lanes are ordered
 //     longest list first and cut into batches of one lane per thread;
-//   - in a step every lane of the batch takes one of its singles (or none),
-//     and no two of them update the same y slot, so no atomics are needed and
-//     every sum has one order; a bra string that a batch reaches in more steps
-//     than it has gets several slots, added in slot order at the end;
+//   - in a step every lane of the batch takes one of its singles (or none);
+//     in a window of kAbWindow steps no two singles update the same y slot, so
+//     the updates need no atomics and one synchronisation per window, and
+//     every sum has one order; a bra string that a batch reaches more often
+//     than it has windows gets several slots, added in slot order at the end;
 //   - a quarter-warp's 128-bit integral gathers take one wavefront per distinct
 //     pair in its most used 16-byte bank slot (pair mod 8), a half-warp's
 //     64-bit y accesses one per lane in its most used bank pair (slot mod 16):
@@ -68,10 +69,14 @@ struct Order {
       rs ^= rs >> 12; rs ^= rs << 25; rs ^= rs >> 27;
       return (uint32_t)(((rs * 0x2545f4914f6cdd1dull) >> 32) * (uint64_t)m >> 32);
     };
+    const int n8 = (n + 15) & ~15;   // row stride: whole half-warps
     std::vector<uint16_t> gp;  // [step][lane] pair, kNone when idle
     std::vector<uint32_t> gy;  // y slot (bit 31: sign)
     std::vector<uint32_t> gb;  // local bra
-    std::vector<uint8_t> vc, yc, used;
+    // singles per bank slot, one byte each: distinct pairs of a quarter-warp's
+    // step by pair mod 8, y slots of a half-warp's step by slot mod 16
+    std::vector<uint64_t> vc, yc;
+    std::vector<uint8_t> used;
     std::vector<uint32_t> len(n), deg;
     std::vector<Single> left = B.list;
     size_t rem = left.size();
@@ -80,35 +85,29 @@ struct Order {
     for (const Single& s : left) ++deg[s.slot0];
     int T = 0;
     auto grow = [&]() {
-      gp.resize((size_t)(T + 1) * n, kNone);
-      gy.resize((size_t)(T + 1) * n, 0);
-      gb.resize((size_t)(T + 1) * n, 0);
-      vc.resize((size_t)(T + 1) * nq * 8, 0);
-      yc.resize((size_t)(T + 1) * nh * 16, 0);
-      used.resize((size_t)(T + 1) * ny, 0);
+      gp.resize((size_t)(T + 1) * n8, kNone);
+      gy.resize((size_t)(T + 1) * n8, 0);
+      gb.resize((size_t)(T + 1) * n8, 0);
+      vc.resize((size_t)(T + 1) * nq, 0);
+      yc.resize((size_t)(T + 1) * nh * 2, 0);
+      used.resize((size_t)(T / kAbWindow + 1) * ny, 0);
     };
+    auto one = [](uint32_t x) { return 1ull << (8 * x); };
+    // whether another lane of lane i's quarter-warp takes the same pair in step m
     auto dup = [&](int m, int i, uint16_t pq) {
-      const int q0 = i & ~7, q1 = std::min(n, q0 + 8);
-      for (int z = q0; z < q1; ++z)
-        if (z != i && gp[(size_t)m * n + z] == pq) return true;
-      return false;
+      const uint16_t* g = &gp[(size_t)m * n8 + (i & ~7)];
+      int c = 0;
+      for (int z = 0; z < 8; ++z) c += g[z] == pq;
+      return c > (g[i & 7] == pq ? 1 : 0);
     };
+    auto ybank = [&](int m, int i, uint32_t y) -> uint64_t& { return yc[((size_t)m * nh + (i >> 4)) * 2 + ((y >> 3) & 1)]; };
     auto put = [&](int m, int i, uint16_t pq, uint32_t y, uint32_t bra) {
-      if (!dup(m, i, pq)) ++vc[((size_t)m * nq + (i >> 3)) * 8 + (pq & 7)];
-      const uint32_t s = y & 0x7fffffffu;
-      ++yc[((size_t)m * nh + (i >> 4)) * 16 + (s & 15)];
-      used[(size_t)m * ny + s] = 1;
-      gp[(size_t)m * n + i] = pq;
-      gy[(size_t)m * n + i] = y;
-      gb[(size_t)m * n + i] = bra;
-    };
-    auto take = [&](int m, int i) {
-      const uint16_t pq = gp[(size_t)m * n + i];
-      const uint32_t s = gy[(size_t)m * n + i] & 0x7fffffffu;
-      gp[(size_t)m * n + i] = kNone;
-      if (!dup(m, i, pq)) --vc[((size_t)m * nq + (i >> 3)) * 8 + (pq & 7)];
-      --yc[((size_t)m * nh + (i >> 4)) * 16 + (s & 15)];
-      used[(size_t)m * ny + s] = 0;
+      if (!dup(m, i, pq)) vc[(size_t)m * nq + (i >> 3)] += one(pq & 7);
+      ybank(m, i, y) += one(y & 7);
+      used[(size_t)(m / kAbWindow) * ny + (y & 0x7fffffffu)] = 1;
+      gp[(size_t)m * n8 + i] = pq;
+      gy[(size_t)m * n8 + i] = y;
+      gb[(size_t)m * n8 + i] = bra;
     };
     // greedy: per step, lanes with the most singles left choose first
     std::vector<int> ord(n), bucket;
@@ -129,20 +128,20 @@ struct Order {
         const int i = ord[j];
         if (len[i] == 0) break;  // the rest are empty too
         Single* l = left.data() + B.beg[i];
-        const uint8_t* cv = &vc[((size_t)m * nq + (i >> 3)) * 8];
-        const uint8_t* cy = &yc[((size_t)m * nh + (i >> 4)) * 16];
+        const uint64_t cv = vc[(size_t)m * nq + (i >> 3)];
+        const uint64_t* cy = &yc[((size_t)m * nh + (i >> 4)) * 2];
         int best = -1;
         uint32_t by = 0;
         float bc = 1e30f;
         for (uint32_t t = 0; t < len[i]; ++t) {
           const int ns = slots_of(l[t].slot0);
           const float pref = 0.02f * (float)deg[l[t].slot0] / (float)ns;  // crowded bra strings early
-          const float cvv = 5.0f * (float)(dup(m, i, l[t].pq) ? 0 : cv[l[t].pq & 7]);
+          const float cvv = 5.0f * (float)(dup(m, i, l[t].pq) ? 0 : (int)((cv >> (8 * (l[t].pq & 7))) & 0xff));
           if (cvv - pref >= bc) continue;
           for (int k = 0; k < ns; ++k) {
             const uint32_t s = slot(l[t].slot0, k);
-            if (used[(size_t)m * ny + s]) continue;
-            const float cost = cvv + 2.0f * (float)cy[s & 15] - pref;
+            if (used[(size_t)(m / kAbWindow) * ny + s]) continue;
+            const float cost = cvv + 2.0f * (float)((cy[(s >> 3) & 1] >> (8 * (s & 7))) & 0xff) - pref;
             if (cost < bc) { bc = cost; best = (int)t; by = s; }
           }
         }
@@ -159,51 +158,73 @@ struct Order {
     B.wsteps.assign(nw, 0);
     for (int m = 0; m < T; ++m)
       for (int i = 0; i < n; ++i)
-        if (gp[(size_t)m * n + i] != kNone) B.wsteps[i >> 5] = (uint32_t)(m + 1);
-    auto cost = [&](int m, int i) {
-      const uint8_t* v = &vc[((size_t)m * nq + (i >> 3)) * 8];
-      const uint8_t* y = &yc[((size_t)m * nh + (i >> 4)) * 16];
-      int a = 1, b = 1;
-      for (int x = 0; x < 8; ++x) a = std::max(a, (int)v[x]);
-      for (int x = 0; x < 16; ++x) b = std::max(b, (int)y[x]);
-      return 5 * a + 2 * b;
+        if (gp[(size_t)m * n8 + i] != kNone) B.wsteps[i >> 5] = (uint32_t)(m + 1);
+    // the largest byte of v (0 and 1 both cost one wavefront)
+    auto most = [](uint64_t v) {
+      int k = 1;
+      while ((v + (uint64_t)(127 - k) * 0x0101010101010101ull) & 0x8080808080808080ull) ++k;
+      return k;
     };
-    const long long moves = (long long)(effort * (double)B.list.size());
+    auto cost = [&](uint64_t v, uint64_t y0, uint64_t y1) { return 5 * most(v) + 2 * std::max(most(y0), most(y1)); };
+    // half-warp by half-warp (their steps stay in cache), kPasses times over
+    constexpr int kPasses = 3;
+    const long long moves = (long long)(effort * (double)B.list.size() / (kPasses * nh)) * kPasses * nh;
     for (long long it = 0; it < moves; ++it) {
-      const int i = (int)rnd((uint32_t)n);
+      const int h0 = 16 * (int)(it / (moves / (kPasses * nh)) % nh);
+      const int i = h0 + (int)rnd((uint32_t)std::min(16, n - h0));
       const uint32_t tw = B.wsteps[i >> 5];
       if (tw < 2) continue;
       const int m1 = (int)rnd(tw), m2 = (int)rnd(tw);
-      const uint16_t pa = gp[(size_t)m1 * n + i], pb = gp[(size_t)m2 * n + i];
-      if (m1 == m2 || (pa == kNone && pb == kNone)) continue;
-      const uint32_t ya = gy[(size_t)m1 * n + i], yb = gy[(size_t)m2 * n + i];
-      const uint32_t ba = gb[(size_t)m1 * n + i], bb = gb[(size_t)m2 * n + i];
-      const int c0 = cost(m1, i) + cost(m2, i);
-      if (pa != kNone) take(m1, i);
-      if (pb != kNone) take(m2, i);
-      auto pick = [&](uint32_t bra, uint32_t y, int m, uint32_t& out) {
+      const size_t p1 = (size_t)m1 * n8 + i, p2 = (size_t)m2 * n8 + i;
+      const uint16_t pa = gp[p1], pb = gp[p2];
+      if (m1 == m2 || pa == pb) continue;
+      const uint32_t ya = gy[p1], yb = gy[p2];
+      uint64_t &v1 = vc[(size_t)m1 * nq + (i >> 3)], &v2 = vc[(size_t)m2 * nq + (i >> 3)];
+      if ((it & 7) != 0 && most(v1) == 1) continue;  // mostly steps with a conflict to resolve
+      uint64_t *y1 = &yc[((size_t)m1 * nh + (i >> 4)) * 2], *y2 = &yc[((size_t)m2 * nh + (i >> 4)) * 2];
+      uint64_t n1 = v1, n2 = v2, a1[2] = {y1[0], y1[1]}, a2[2] = {y2[0], y2[1]};
+      const int w1 = m1 / kAbWindow, w2 = m2 / kAbWindow;
+      // slots in the other window (the two singles vacate theirs)
+      auto pick = [&](uint32_t bra, uint32_t y, int w, uint32_t vacant, bool has, uint32_t& out) {
+        if (w1 == w2) { out = y; return true; }
         const int ns = slots_of(bra), st = ns > 1 ? (int)rnd((uint32_t)ns) : 0;
         for (int k = 0; k < ns; ++k) {
-          const uint32_t s = slot(bra, (st + k) % ns);
-          if (!used[(size_t)m * ny + s]) { out = s | (y & 0x80000000u); return true; }
+          const uint32_t s = slot(bra, ns > 1 ? (st + k) % ns : 0);
+          if (!used[(size_t)w * ny + s] || (has && s == (vacant & 0x7fffffffu))) {
+            out = s | (y & 0x80000000u);
+            return true;
+          }
         }
         return false;
       };
       uint32_t na = 0, nb = 0;
-      bool ok = (pa == kNone || pick(ba, ya, m2, na)) && (pb == kNone || pick(bb, yb, m1, nb));
-      if (ok) {
-        if (pa != kNone) put(m2, i, pa, na, ba);
-        if (pb != kNone) put(m1, i, pb, nb, bb);
-        if (cost(m1, i) + cost(m2, i) > c0) {
-          if (pa != kNone) take(m2, i);
-          if (pb != kNone) take(m1, i);
-          ok = false;
-        }
+      if (pa != kNone && !pick(gb[p1], ya, w2, yb, pb != kNone, na)) continue;
+      if (pb != kNone && !pick(gb[p2], yb, w1, ya, pa != kNone, nb)) continue;
+      if (pa != kNone) {
+        if (!dup(m1, i, pa)) n1 -= one(pa & 7);
+        if (!dup(m2, i, pa)) n2 += one(pa & 7);
+        a1[(ya >> 3) & 1] -= one(ya & 7);
+        a2[(na >> 3) & 1] += one(na & 7);
       }
-      if (!ok) {
-        if (pa != kNone) put(m1, i, pa, ya, ba);
-        if (pb != kNone) put(m2, i, pb, yb, bb);
+      if (pb != kNone) {
+        if (!dup(m2, i, pb)) n2 -= one(pb & 7);
+        if (!dup(m1, i, pb)) n1 += one(pb & 7);
+        a2[(yb >> 3) & 1] -= one(yb & 7);
+        a1[(nb >> 3) & 1] += one(nb & 7);
       }
+      if (cost(n1, a1[0], a1[1]) + cost(n2, a2[0], a2[1]) > cost(v1, y1[0], y1[1]) + cost(v2, y2[0], y2[1])) continue;
+      v1 = n1; v2 = n2;
+      y1[0] = a1[0]; y1[1] = a1[1];
+      y2[0] = a2[0]; y2[1] = a2[1];
+      if (w1 != w2) {
+        if (pa != kNone) used[(size_t)w1 * ny + (ya & 0x7fffffffu)] = 0;
+        if (pb != kNone) used[(size_t)w2 * ny + (yb & 0x7fffffffu)] = 0;
+        if (pa != kNone) used[(size_t)w2 * ny + (na & 0x7fffffffu)] = 1;
+        if (pb != kNone) used[(size_t)w1 * ny + (nb & 0x7fffffffu)] = 1;
+      }
+      gp[p1] = pb; gp[p2] = pa;
+      gy[p1] = nb; gy[p2] = na;
+      std::swap(gb[p1], gb[p2]);
     }
     // records; an idle lane repeats a gather address of its quarter-warp (a broadcast)
     B.steps = T;
@@ -212,13 +233,13 @@ struct Order {
     for (int m = 0; m < T; ++m)
       for (int i = 0; i < nt; ++i) {
         uint32_t r = kAbPad;
-        if (i < n && gp[(size_t)m * n + i] != kNone) {
-          const uint32_t y = gy[(size_t)m * n + i];
-          r = (uint32_t)gp[(size_t)m * n + i] | ((y & 0xffffu) << 12) | (y & 0x80000000u);
+        if (i < n && gp[(size_t)m * n8 + i] != kNone) {
+          const uint32_t y = gy[(size_t)m * n8 + i];
+          r = (uint32_t)gp[(size_t)m * n8 + i] | ((y & 0xffffu) << 12) | (y & 0x80000000u);
         } else {
           const int q0 = i & ~7, q1 = std::min(n, q0 + 8);
           for (int z = q0; z < q1; ++z)
-            if (gp[(size_t)m * n + z] != kNone) { r = kAbPad | gp[(size_t)m * n + z]; break; }
+            if (gp[(size_t)m * n8 + z] != kNone) { r = kAbPad | gp[(size_t)m * n8 + z]; break; }
         }
         B.rec[((size_t)(m >> 2) * nt + i) * 4 + (m & 3)] = r;
       }
@@ -277,7 +298,7 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
     const int nt = small ? (vk.size() <= 256 ? 256 : 512) : (vk.size() <= 512 ? 512 : 1024);
     const size_t nbatch = std::max<size_t>(1, (vk.size() + nt - 1) / nt);
     const double effort =
-        std::min(50.0, (double)alpha_singles * (double)total / 4e8);  // 2.4e10 pairs: 50 moves per record
+        std::min(120.0, (double)alpha_singles * (double)total / 2e8);  // 2.4e10 pairs: 120 moves per record
     struct PanelWork {
       int nmain = 0, nex = 0, ny = 0;
       std::vector<uint32_t> s0, ex_row, ex_off;
@@ -315,8 +336,9 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
         for (const Single& s : B.list) ++deg[s.slot0];
         for (const Single& s : B.list) {
           if (deg[s.slot0] == 0) continue;
-          // strings reached in nearly every step of the batch get more slots
-          const uint32_t x = (uint32_t)((deg[s.slot0] + 0.85 * B.maxlen - 1e-9) / (0.85 * B.maxlen));
+          // strings reached in nearly every window of the batch get more slots
+          const double win = 0.85 * ((B.maxlen + kAbWindow - 1) / kAbWindow);
+          const uint32_t x = (uint32_t)((deg[s.slot0] + win - 1e-9) / win);
           need[s.slot0] = std::max(need[s.slot0], x);
           deg[s.slot0] = 0;
         }

@@ -61,6 +61,7 @@ struct SellPanel {
 // kAbPad: no single. Record m of thread t of batch b sits at
 // rec[4 * (boff[b] + (m / 4) * threads + t) + m % 4].
 constexpr uint32_t kAbPad = 1u << 30;
+constexpr int kAbWindow = 2;  // steps whose updates of y are disjoint (divides 4)
 struct AbPanel {
   uint32_t* rec = nullptr;
   uint64_t* boff = nullptr;     // [nbatch], in blocks of four records
@@ -471,6 +472,8 @@ int build_stored(Ctx* c);
 void release_stored(Ctx* c);
 int stored_sigma(Ctx* c, const double* X, double* S);
 int ensure_sigma_scratch(Ctx* c);
+// phi o W (FP64, na x nb) into d_xp (row stride xsa) and its transpose into d_xt (row stride xsb).
+int phase_vectors(Ctx* c, const double* W);
 void clear_sigma_graphs(Ctx* c);
 int ensure_reduction(Ctx* c, size_t n);
 int autotune(Ctx* c);

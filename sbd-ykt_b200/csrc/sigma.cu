@@ -1768,10 +1768,10 @@ struct AbArgs {
   int* err;
 };
 
-// Step order of the updates of y: one arrival per warp and step on an
-// mbarrier. A warp waits for step s - 1 before it updates y in step s, so the
-// integral gathers of step s run while slower warps finish step s - 1; with a
-// full barrier per step the shared-memory pipe drains at each one. Phases end
+// Order of the updates of y: one arrival per warp and window on an mbarrier. A
+// warp waits for window w - 1 before it updates y in window w, so the integral
+// gathers of window w run while slower warps finish window w - 1; with a full
+// barrier per step the shared-memory pipe drains at each one. Phases end
 // by arrivals of this CTA's own warps alone; the wait is bounded all the same.
 __device__ __forceinline__ void step_init(uint32_t bar, uint32_t warps) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(warps) : "memory");
@@ -1802,40 +1802,68 @@ __device__ __forceinline__ void ab_sweep(const AbArgs<T>& a, const typename RowP
   using RP = RowPack<T>;
   constexpr int VR = RP::kRows, R = NH * VR;
   const int warp = threadIdx.x >> 5;
+  T c[R];
+  auto load_c = [&](int b) {
+    const bool live = a.wsteps[b * (NT / 32) + warp] > 0;
+    const T* xb = a.Xk + (size_t)b * NT + threadIdx.x;
+#pragma unroll
+    for (int r = 0; r < R; ++r) c[r] = (r < nr && live) ? __ldg(xb + (size_t)s_ket[r] * a.xs) : (T)0;
+  };
+  load_c(0);
   for (int b = 0; b < a.nbatch; ++b) {
     const int steps = (int)a.bsteps[b];
     const int wst = (int)a.wsteps[b * (NT / 32) + warp];
-    T c[R];
-    const T* xb = a.Xk + (size_t)b * NT + threadIdx.x;
-#pragma unroll
-    for (int r = 0; r < R; ++r) c[r] = (r < nr && wst > 0) ? __ldg(xb + (size_t)s_ket[r] * a.xs) : (T)0;
     const uint4* rp = a.rec + a.boff[b] + threadIdx.x;
-    uint4 cur = steps > 0 ? __ldg(rp) : make_uint4(kAbPad, kAbPad, kAbPad, kAbPad);
+    uint4 cur = wst > 0 ? __ldg(rp) : make_uint4(kAbPad, kAbPad, kAbPad, kAbPad);
+    bool more = b + 1 < a.nbatch;  // the next batch's ket values are still to be loaded
     for (int m0 = 0; m0 < steps; m0 += 4) {
-      const uint4 nxt = m0 + 4 < wst ? __ldg(rp + (size_t)(m0 / 4 + 1) * NT) : cur;
-      const uint32_t recs[4] = {cur.x, cur.y, cur.z, cur.w};
+      if (m0 < wst) {
+        const uint4 nxt = m0 + 4 < wst ? __ldg(rp + (size_t)(m0 / 4 + 1) * NT) : cur;
+        const uint32_t recs[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (m0 + q >= steps) break;
-        const uint32_t rec = recs[q];
-        const bool live = m0 + q < wst;  // warp-uniform
-        double t[2] = {0.0, 0.0};
-        if (live) {
-          const typename RP::P* v = vs + (rec & 0xfffu);
+        for (int w0 = 0; w0 < 4; w0 += kAbWindow) {
+          if (m0 + w0 >= steps) break;
+          double t[kAbWindow][2];
 #pragma unroll
-          for (int h = 0; h < NH; ++h) RP::dot(v[(size_t)h * a.vstr], c + h * VR, t);
+          for (int q = 0; q < kAbWindow; ++q) {
+            t[q][0] = t[q][1] = 0.0;
+            if (m0 + w0 + q < wst) {  // warp-uniform
+              const typename RP::P* v = vs + (recs[w0 + q] & 0xfffu);
+#pragma unroll
+              for (int h = 0; h < NH; ++h) RP::dot(v[(size_t)h * a.vstr], c + h * VR, t[q]);
+            }
+          }
+          if (more && m0 + w0 + kAbWindow >= wst) {  // this batch's values are used up
+            load_c(b + 1);
+            more = false;
+          }
+          step_wait(bar, ph, a.err);  // the previous window's updates of y are done
+#pragma unroll
+          for (int q = 0; q < kAbWindow; ++q) {
+            const uint32_t rec = recs[w0 + q];
+            if (m0 + w0 + q < wst && !(rec & kAbPad)) {
+              double* yp = y + ((rec >> 12) & 0xffffu);
+              *yp += flip_sign(t[q][0] + t[q][1], rec >> 31);
+            }
+          }
+          __syncwarp();
+          if ((threadIdx.x & 31) == 0) step_arrive(bar);
+          ++ph;
         }
-        step_wait(bar, ph, a.err);  // the previous step's updates of y are done
-        if (live && !(rec & kAbPad)) {
-          double* yp = y + ((rec >> 12) & 0xffffu);
-          *yp += flip_sign(t[0] + t[1], rec >> 31);
+        cur = nxt;
+      } else {
+        if (more) {
+          load_c(b + 1);
+          more = false;
         }
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) step_arrive(bar);
-        ++ph;
+        for (int w0 = 0; w0 < 4 && m0 + w0 < steps; w0 += kAbWindow) {
+          step_wait(bar, ph, a.err);
+          if ((threadIdx.x & 31) == 0) step_arrive(bar);
+          ++ph;
+        }
       }
-      cur = nxt;
     }
+    if (more) load_c(b + 1);  // a batch without steps
   }
 }
 
@@ -1848,8 +1876,8 @@ __device__ __forceinline__ void ab_sweep(const AbArgs<T>& a, const typename RowP
 // y[ib] += s * sum_r s_r (pq_r|rs) C'[ja_r, jb], y in shared memory. The
 // Coulomb terms of the beta singles with the alpha string ride along as one
 // more "single" ja = ia whose integral row is Dr. The
-// schedule (AbPlan) never lets two threads of a step update the same slot, so
-// a barrier per step orders the updates: no atomics, one summation order.
+// schedule (AbPlan) never lets two threads of a window of steps update the same
+// slot, so the updates need no atomics and have one summation order.
 //
 // Bound: the shared-memory pipe. Staging integrals instead of ket rows lets a
 // group hold 10 (FP64) or 20 (FP32) alpha singles instead of the 2 or 4 whose
@@ -1865,7 +1893,7 @@ __global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
   __shared__ uint32_t s_ket[kAbPacks * 4], s_pq[kAbPacks * 4];
   __shared__ __align__(8) uint64_t s_bar;
   const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
-  uint32_t ph = 0;  // steps finished by this warp
+  uint32_t ph = 0;  // windows finished by this warp
   if (threadIdx.x == 0) step_init(bar, NT / 32);
   const uint4 item = a.items[blockIdx.x];
   const size_t ia = item.x;
@@ -2454,6 +2482,10 @@ int ensure_coulomb_a(Ctx* c) {
   coulomb_table_kernel<<<ga, 256, 0, c->stream>>>(c->d_G, c->L, c->d_a, c->na, c->da_stride, c->d_Da, c->d_Da32);
   SBDX_LAUNCHED(c);
   return 0;
+}
+
+int phase_vectors(Ctx* c, const double* W) {
+  return launch_split<double>(c, W, 0, c->na, reinterpret_cast<double*>(c->d_xp), reinterpret_cast<double*>(c->d_xt), false);
 }
 
 int build_g_table(Ctx* c) {

@@ -310,15 +310,16 @@ project_kernel(const TV* __restrict__ V, size_t ldv, int m, XSet<TX> X, int nx, 
   }
 }
 
-// out[k] = sum_b partial[k * nblk + b] (fixed order, deterministic)
-__global__ void finalize_kernel(const double* __restrict__ partial, int nblk, int m, double* __restrict__ out) {
+// out[k] = sum_b partial[k * nblk + b] (fixed order, deterministic), CTA k. One
+// CTA walking all sums took 0.6 us for each (29.4 us for the 48 dots of 24 x
+// 2 vectors; 3 us with a CTA per sum).
+__global__ void finalize_kernel(const double* __restrict__ partial, int nblk, double* __restrict__ out) {
   __shared__ double sh[kRedThreads / 32];
-  for (int k = 0; k < m; ++k) {
-    double v = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += partial[(size_t)k * nblk + b];
-    const double t = block_sum(v, sh);
-    if (threadIdx.x == 0) out[k] = t;
-  }
+  const size_t k = blockIdx.x;
+  double v = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += partial[k * nblk + b];
+  const double t = block_sum(v, sh);
+  if (threadIdx.x == 0) out[k] = t;
 }
 
 // W = u0*W0 + sum_k u[k] C_k ;  R = E0*W - (u0*HW0 + sum_k u[k] HC_k)
@@ -603,7 +604,7 @@ int project(Ctx* c, Work& wk, const TV* V, size_t ldv, int m, const XSet<TX>& X,
     }
   }
   SBDX_LAUNCHED(c);
-  finalize_kernel<<<1, kRedThreads, 0, c->stream>>>(wk.partial, (int)g, m * nx, out);
+  finalize_kernel<<<(unsigned)(m * nx), kRedThreads, 0, c->stream>>>(wk.partial, (int)g, out);
   SBDX_LAUNCHED(c);
   return 0;
 }
@@ -627,7 +628,7 @@ int multidot2(Ctx* c, Work& wk, const TV* V, size_t ldv, int m, const TX* x0, co
 
 // out[k] = sum of the nblk partials of row k (nblk = the producing grid).
 int finalize(Ctx* c, Work& wk, int m, double* out, unsigned nblk = kRedBlocks) {
-  finalize_kernel<<<1, kRedThreads, 0, c->stream>>>(wk.partial, (int)nblk, m, out);
+  finalize_kernel<<<(unsigned)(m), kRedThreads, 0, c->stream>>>(wk.partial, (int)nblk, out);
   SBDX_LAUNCHED(c);
   return 0;
 }
@@ -1729,9 +1730,9 @@ int davidson_block(Ctx* c, const sbdx_davidson_params& p, int k, double* dW, dou
       unsigned ga = kRedBlocks;
       if ((rc = launch_update_anchors<TC>(c, wk, k, W, HW, C, HC, nv, Xd, s + kbTheta, D, Wn, HWn, R, &ga))) return rc;
       // |W'_r|^2 -> kbNW2 + r, |R_r|^2 -> kbNR2 + r
-      finalize_kernel<<<1, kRedThreads, 0, c->stream>>>(wk.partial, (int)ga, k, s + kbNW2);
+      finalize_kernel<<<(unsigned)(k), kRedThreads, 0, c->stream>>>(wk.partial, (int)ga, s + kbNW2);
       SBDX_LAUNCHED(c);
-      finalize_kernel<<<1, kRedThreads, 0, c->stream>>>(wk.partial + (size_t)k * ga, (int)ga, k, s + kbNR2);
+      finalize_kernel<<<(unsigned)(k), kRedThreads, 0, c->stream>>>(wk.partial + (size_t)k * ga, (int)ga, s + kbNR2);
       SBDX_LAUNCHED(c);
       // A holds [W | HW | W' | HW']; the swaps exchange the halves, HW = W + k*D
       std::swap(W, Wn);
@@ -2346,9 +2347,9 @@ int davidson_block_graph(Ctx* c, const sbdx_davidson_params& p, int k, double* d
     SBDX_LAUNCHED(c);
     unsigned ga = kRedBlocks;
     if ((r2 = launch_update_anchors<TC>(c, wk, k, W, HW, C, HC, nv, Xd, s + kbTheta, D, Wn, HWn, R, &ga))) return r2;
-    finalize_kernel<<<1, kRedThreads, 0, c->stream>>>(wk.partial, (int)ga, k, s + kbNW2);
+    finalize_kernel<<<(unsigned)(k), kRedThreads, 0, c->stream>>>(wk.partial, (int)ga, s + kbNW2);
     SBDX_LAUNCHED(c);
-    finalize_kernel<<<1, kRedThreads, 0, c->stream>>>(wk.partial + (size_t)k * ga, (int)ga, k, s + kbNR2);
+    finalize_kernel<<<(unsigned)(k), kRedThreads, 0, c->stream>>>(wk.partial + (size_t)k * ga, (int)ga, s + kbNR2);
     SBDX_LAUNCHED(c);
     post_update_kernel<<<1, 256, 0, c->stream>>>(k, nv, nact, ld, dM, dS, Xd, s + kbTheta, s + kbNW2, s + kbNR2, fs,
                                                  dead, dst);

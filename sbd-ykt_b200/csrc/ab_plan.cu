@@ -248,11 +248,11 @@ struct Order {
 
 }  // namespace
 
-void free_ab_plan(AbPlan& P) {
-  cudaFree(P.vket);
+void free_ab_plan(Ctx* c, AbPlan& P) {
+  dev_free(c, P.vket);
   for (AbPanel& q : P.panels) {
-    cudaFree(q.rec); cudaFree(q.boff); cudaFree(q.bsteps); cudaFree(q.wsteps);
-    cudaFree(q.ex_row); cudaFree(q.ex_off);
+    dev_free(c, q.rec); dev_free(c, q.boff); dev_free(c, q.bsteps); dev_free(c, q.wsteps);
+    dev_free(c, q.ex_row); dev_free(c, q.ex_off);
   }
   P = AbPlan{};
 }
@@ -263,7 +263,7 @@ void free_ab_plan(AbPlan& P) {
 int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::vector<uint64_t>& off,
                   const std::vector<uint64_t>& rec, uint64_t alpha_singles) {
   AbPlan& P = c->ab;
-  free_ab_plan(P);
+  free_ab_plan(c, P);
   uint64_t total = 0;
   for (size_t r = 0; r < n; ++r) total += hs[r];
   P.vstr = (uint32_t)((c->npair + 7) & ~(size_t)7);
@@ -392,7 +392,7 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
     for (size_t i = 0; i < vk.size(); ++i) vket[i] = vk[i].ket;
     auto up = [&](const auto& h, auto** d) -> int {
       using E = typename std::decay<decltype(h[0])>::type;
-      SBDX_CUDA(c, cudaMalloc(d, sizeof(E) * std::max<size_t>(1, h.size())));
+      SBDX_CUDA(c, dev_alloc(c, d, sizeof(E) * std::max<size_t>(1, h.size())));
       if (!h.empty()) SBDX_CUDA(c, cudaMemcpyAsync(*d, h.data(), sizeof(E) * h.size(), cudaMemcpyHostToDevice, c->stream));
       return 0;
     };

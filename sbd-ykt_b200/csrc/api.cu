@@ -42,8 +42,14 @@ cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes) {
 
 void pool_trim(Ctx* c) {
   if (!c->pool || !c->own_pool) return;
-  cudaStreamSynchronize(c->stream);
-  cudaMemPoolTrimTo(c->pool, 0);
+  uint64_t reserved = 0, in_use = 0;
+  if (cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &in_use) != cudaSuccess)
+    reserved = UINT64_MAX, in_use = 0;
+  if (reserved - in_use <= kPoolKeep) return;
+  cudaStreamSynchronize(c->stream);  // the releases queued on the stream
+  cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &in_use);
+  cudaMemPoolTrimTo(c->pool, (size_t)in_use + kPoolKeep);
 }
 
 int check_device_error(Ctx* c) {
@@ -52,7 +58,7 @@ int check_device_error(Ctx* c) {
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
   if (h == 0) return 0;
   SBDX_CUDA(c, cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-  c->err = "device watchdog: a wait timed out in the alpha-beta sigma kernel (code " +
+  c->err = "device watchdog: a wait timed out in a sigma kernel (code " +
            std::to_string(h) + ")";
   return SBDX_ERR_CUDA;
 }
@@ -70,15 +76,15 @@ namespace {
 
 void free_vector_state(Ctx* c) {
   sbdx::clear_sigma_graphs(c);
-  cudaFree(c->d_hii); c->d_hii = nullptr; c->have_hii = false;
-  cudaFree(c->d_xt); c->d_xt = nullptr;
-  cudaFree(c->d_xp); c->d_xp = nullptr;
-  cudaFree(c->d_y); c->d_y = nullptr;
-  cudaFree(c->d_yt); c->d_yt = nullptr;
-  cudaFree(c->d_yab); c->d_yab = nullptr;
-  cudaFree(c->d_io_in); c->d_io_in = nullptr;
-  cudaFree(c->d_io_out); c->d_io_out = nullptr;
-  cudaFree(c->d_wf); c->d_wf = nullptr; c->wf_roots = 0; c->wf_cap = 0;
+  dev_free(c, c->d_hii); c->d_hii = nullptr; c->have_hii = false;
+  dev_free(c, c->d_xt); c->d_xt = nullptr;
+  dev_free(c, c->d_xp); c->d_xp = nullptr;
+  dev_free(c, c->d_y); c->d_y = nullptr;
+  dev_free(c, c->d_yt); c->d_yt = nullptr;
+  dev_free(c, c->d_yab); c->d_yab = nullptr;
+  dev_free(c, c->d_io_in); c->d_io_in = nullptr;
+  dev_free(c, c->d_io_out); c->d_io_out = nullptr;
+  dev_free(c, c->d_wf); c->d_wf = nullptr; c->wf_roots = 0; c->wf_cap = 0;
 }
 
 // Room for k resident result vectors (contents of earlier solves are dropped).
@@ -86,10 +92,10 @@ int ensure_wf(Ctx* c, int k) {
   const size_t D = c->na * c->nb;
   c->wf_roots = 0;
   if (c->wf_cap < k) {
-    cudaFree(c->d_wf);
+    dev_free(c, c->d_wf);
     c->d_wf = nullptr;
     c->wf_cap = 0;
-    cudaError_t e = cudaMalloc(&c->d_wf, sizeof(double) * D * (size_t)k);
+    cudaError_t e = dev_alloc(c, &c->d_wf, sizeof(double) * D * (size_t)k);
     if (e != cudaSuccess) {
       cudaGetLastError();
       c->err = "davidson: no device memory for " + std::to_string(k) + " result vector(s) of " + std::to_string(D) +
@@ -103,8 +109,8 @@ int ensure_wf(Ctx* c, int k) {
 
 int ensure_io(Ctx* c) {
   const size_t D = c->na * c->nb;
-  if (!c->d_io_in) SBDX_CUDA(c, cudaMalloc(&c->d_io_in, sizeof(double) * D));
-  if (!c->d_io_out) SBDX_CUDA(c, cudaMalloc(&c->d_io_out, sizeof(double) * D));
+  if (!c->d_io_in) SBDX_CUDA(c, dev_alloc(c, &c->d_io_in, sizeof(double) * D));
+  if (!c->d_io_out) SBDX_CUDA(c, dev_alloc(c, &c->d_io_out, sizeof(double) * D));
   return 0;
 }
 
@@ -174,9 +180,11 @@ int sbdx_ctx_destroy(sbdx_ctx* ctx) {
   cudaStreamSynchronize(c->stream);
   sbdx::free_connectivity(c);
   sbdx::free_vector_state(c);
-  cudaFree(c->d_h); cudaFree(c->d_eri); cudaFree(c->d_eri32); cudaFree(c->d_G); cudaFree(c->d_G32);
-  cudaFree(c->d_V); cudaFree(c->d_V32); cudaFree(c->d_err);
-  cudaFree(c->d_a); cudaFree(c->d_b); cudaFree(c->d_red);
+  for (void* p : {(void*)c->d_h, (void*)c->d_eri, (void*)c->d_eri32, (void*)c->d_G, (void*)c->d_G32, (void*)c->d_V,
+                  (void*)c->d_V32, (void*)c->d_a, (void*)c->d_b, (void*)c->d_red})
+    sbdx::dev_free(c, p);
+  cudaFree(c->d_err);
+  cudaStreamSynchronize(c->stream);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   for (auto& e : {c->fork, c->join[0], c->join[1]})
@@ -255,9 +263,22 @@ int sbdx_autotune(sbdx_ctx* ctx, int* same_vec, int* ab_rows) {
 int sbdx_set_stream(sbdx_ctx* ctx, void* stream) {
   return sbdx::guarded(ctx, [&](Ctx* c) {
     sbdx::clear_sigma_graphs(c);
+    // buffers used on the old stream are released on the new one, after the old one's work
+    const cudaStream_t next = (cudaStream_t)stream;
+    if (next != c->stream) {
+      cudaEvent_t e = nullptr;
+      const bool ok = cudaSetDevice(c->device) == cudaSuccess &&
+                      cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess &&
+                      cudaEventRecord(e, c->stream) == cudaSuccess && cudaStreamWaitEvent(next, e, 0) == cudaSuccess;
+      if (!ok) {
+        cudaGetLastError();
+        cudaDeviceSynchronize();
+      }
+      if (e) cudaEventDestroy(e);
+    }
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
     c->own_stream = false;
-    c->stream = (cudaStream_t)stream;
+    c->stream = next;
     return SBDX_OK;
   });
 }
@@ -278,7 +299,7 @@ int sbdx_set_integrals(sbdx_ctx* ctx, int norb, double I0, const double* h, cons
       if (!std::isfinite(eri[k])) { c->err = "set_integrals: non-finite two-electron integral"; return SBDX_ERR_NUMERIC; }
     if (cudaSetDevice(c->device) != cudaSuccess) { c->err = "cudaSetDevice failed"; return SBDX_ERR_CUDA; }
     cudaStreamSynchronize(c->stream);
-    cudaFree(c->d_h); cudaFree(c->d_eri); cudaFree(c->d_eri32);
+    sbdx::dev_free(c, c->d_h); sbdx::dev_free(c, c->d_eri); sbdx::dev_free(c, c->d_eri32);
     c->d_h = nullptr; c->d_eri = nullptr; c->d_eri32 = nullptr;
     c->L = norb;
     c->I0 = I0;
@@ -288,19 +309,19 @@ int sbdx_set_integrals(sbdx_ctx* ctx, int norb, double I0, const double* h, cons
     c->h_eri.assign(eri, eri + neri);
     std::vector<float> e32(neri);
     for (size_t k = 0; k < neri; ++k) e32[k] = (float)eri[k];
-    SBDX_CUDA(c, cudaMalloc(&c->d_h, sizeof(double) * norb * norb));
-    SBDX_CUDA(c, cudaMalloc(&c->d_eri, sizeof(double) * neri));
-    SBDX_CUDA(c, cudaMalloc(&c->d_eri32, sizeof(float) * neri));
-    SBDX_CUDA(c, cudaMemcpy(c->d_h, h, sizeof(double) * norb * norb, cudaMemcpyHostToDevice));
-    SBDX_CUDA(c, cudaMemcpy(c->d_eri, eri, sizeof(double) * neri, cudaMemcpyHostToDevice));
-    SBDX_CUDA(c, cudaMemcpy(c->d_eri32, e32.data(), sizeof(float) * neri, cudaMemcpyHostToDevice));
+    SBDX_CUDA(c, sbdx::dev_alloc(c, &c->d_h, sizeof(double) * norb * norb));
+    SBDX_CUDA(c, sbdx::dev_alloc(c, &c->d_eri, sizeof(double) * neri));
+    SBDX_CUDA(c, sbdx::dev_alloc(c, &c->d_eri32, sizeof(float) * neri));
+    SBDX_CUDA(c, cudaMemcpyAsync(c->d_h, h, sizeof(double) * norb * norb, cudaMemcpyHostToDevice, c->stream));
+    SBDX_CUDA(c, cudaMemcpyAsync(c->d_eri, eri, sizeof(double) * neri, cudaMemcpyHostToDevice, c->stream));
+    SBDX_CUDA(c, cudaMemcpyAsync(c->d_eri32, e32.data(), sizeof(float) * neri, cudaMemcpyHostToDevice, c->stream));
     int rc = sbdx::build_g_table(c);
     if (rc) return rc;
     SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
     c->have_integrals = true;
     // matrix elements cached in the connectivity and the diagonal depend on the integrals
     sbdx::free_connectivity(c);
-    cudaFree(c->d_hii); c->d_hii = nullptr; c->have_hii = false;
+    sbdx::dev_free(c, c->d_hii); c->d_hii = nullptr; c->have_hii = false;
     return SBDX_OK;
   });
 }
@@ -321,16 +342,18 @@ int sbdx_set_strings(sbdx_ctx* ctx, const uint64_t* alpha, size_t na, const uint
     cudaStreamSynchronize(c->stream);
     sbdx::free_connectivity(c);
     sbdx::free_vector_state(c);
-    cudaFree(c->d_a); cudaFree(c->d_b);
+    sbdx::dev_free(c, c->d_a); sbdx::dev_free(c, c->d_b);
     c->d_a = nullptr; c->d_b = nullptr;
     c->na = na;
     c->nb = nb;
     c->h_a.assign(alpha, alpha + na);
     c->h_b.assign(beta, beta + nb);
-    SBDX_CUDA(c, cudaMalloc(&c->d_a, sizeof(uint64_t) * na));
-    SBDX_CUDA(c, cudaMalloc(&c->d_b, sizeof(uint64_t) * nb));
-    SBDX_CUDA(c, cudaMemcpy(c->d_a, alpha, sizeof(uint64_t) * na, cudaMemcpyHostToDevice));
-    SBDX_CUDA(c, cudaMemcpy(c->d_b, beta, sizeof(uint64_t) * nb, cudaMemcpyHostToDevice));
+    SBDX_CUDA(c, sbdx::dev_alloc(c, &c->d_a, sizeof(uint64_t) * na));
+    SBDX_CUDA(c, sbdx::dev_alloc(c, &c->d_b, sizeof(uint64_t) * nb));
+    SBDX_CUDA(c, cudaMemcpyAsync(c->d_a, alpha, sizeof(uint64_t) * na, cudaMemcpyHostToDevice, c->stream));
+    SBDX_CUDA(c, cudaMemcpyAsync(c->d_b, beta, sizeof(uint64_t) * nb, cudaMemcpyHostToDevice, c->stream));
+    SBDX_CUDA(c, cudaStreamSynchronize(c->stream));  // the caller's arrays are free to change
+    sbdx::pool_trim(c);
     c->have_strings = true;
     return SBDX_OK;
   });
@@ -383,9 +406,10 @@ int sbdx_get_connectivity(sbdx_ctx* ctx, int spin, uint64_t* slen, uint64_t* dle
     const sbdx::Conn& cn = c->conn[spin];
     std::vector<uint32_t> ns(cn.n), nd(cn.n), ket(cn.total);
     SBDX_CUDA(c, cudaSetDevice(c->device));
-    SBDX_CUDA(c, cudaMemcpy(ns.data(), cn.nsing, sizeof(uint32_t) * cn.n, cudaMemcpyDeviceToHost));
-    SBDX_CUDA(c, cudaMemcpy(nd.data(), cn.ndoub, sizeof(uint32_t) * cn.n, cudaMemcpyDeviceToHost));
-    if (cn.total) SBDX_CUDA(c, cudaMemcpy(ket.data(), cn.ket, sizeof(uint32_t) * cn.total, cudaMemcpyDeviceToHost));
+    SBDX_CUDA(c, cudaMemcpyAsync(ns.data(), cn.nsing, sizeof(uint32_t) * cn.n, cudaMemcpyDeviceToHost, c->stream));
+    SBDX_CUDA(c, cudaMemcpyAsync(nd.data(), cn.ndoub, sizeof(uint32_t) * cn.n, cudaMemcpyDeviceToHost, c->stream));
+    if (cn.total) SBDX_CUDA(c, cudaMemcpyAsync(ket.data(), cn.ket, sizeof(uint32_t) * cn.total, cudaMemcpyDeviceToHost, c->stream));
+    SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
     for (size_t r = 0; r < cn.n; ++r) {
       if (slen) slen[r] = ns[r];
       if (dlen) dlen[r] = nd[r];
@@ -558,10 +582,10 @@ int sbdx_rdm(sbdx_ctx* ctx, const double* W, double* one, double* two) {
     const size_t D = c->na * c->nb, L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
     SBDX_CUDA(c, cudaMemcpyAsync(c->d_io_in, W, sizeof(double) * D, cudaMemcpyHostToDevice, c->stream));
     double *d_one = nullptr, *d_two = nullptr;
-    SBDX_CUDA(c, cudaMalloc(&d_one, sizeof(double) * 2 * L2));
+    SBDX_CUDA(c, sbdx::dev_alloc(c, &d_one, sizeof(double) * 2 * L2));
     if (two) {
-      cudaError_t e = cudaMalloc(&d_two, sizeof(double) * 4 * L4);
-      if (e != cudaSuccess) { cudaFree(d_one); sbdx::set_cuda_err(c, e, "cudaMalloc(2-RDM)"); return SBDX_ERR_NOMEM; }
+      cudaError_t e = sbdx::dev_alloc(c, &d_two, sizeof(double) * 4 * L4);
+      if (e != cudaSuccess) { sbdx::dev_free(c, d_one); sbdx::set_cuda_err(c, e, "allocation of the 2-RDM"); return SBDX_ERR_NOMEM; }
     }
     rc = sbdx::rdm_device(c, (const double*)c->d_io_in, d_one, d_two);
     if (!rc) {
@@ -570,8 +594,8 @@ int sbdx_rdm(sbdx_ctx* ctx, const double* W, double* one, double* two) {
       if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) { sbdx::set_cuda_err(c, e, "rdm copy-out"); rc = SBDX_ERR_CUDA; }
     }
-    cudaFree(d_one);
-    cudaFree(d_two);
+    sbdx::dev_free(c, d_one);
+    sbdx::dev_free(c, d_two);
     return rc;
   });
 }
@@ -654,10 +678,10 @@ int sbdx_rdm_device(sbdx_ctx* ctx, const double* dW, double* one, double* two) {
     if (rc) return rc;
     const size_t L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
     double *d_one = nullptr, *d_two = nullptr;
-    SBDX_CUDA(c, cudaMalloc(&d_one, sizeof(double) * 2 * L2));
+    SBDX_CUDA(c, sbdx::dev_alloc(c, &d_one, sizeof(double) * 2 * L2));
     if (two) {
-      cudaError_t e = cudaMalloc(&d_two, sizeof(double) * 4 * L4);
-      if (e != cudaSuccess) { cudaFree(d_one); sbdx::set_cuda_err(c, e, "cudaMalloc(2-RDM)"); return SBDX_ERR_NOMEM; }
+      cudaError_t e = sbdx::dev_alloc(c, &d_two, sizeof(double) * 4 * L4);
+      if (e != cudaSuccess) { sbdx::dev_free(c, d_one); sbdx::set_cuda_err(c, e, "allocation of the 2-RDM"); return SBDX_ERR_NOMEM; }
     }
     rc = sbdx::rdm_device(c, dW, d_one, d_two);
     if (!rc) {
@@ -666,8 +690,8 @@ int sbdx_rdm_device(sbdx_ctx* ctx, const double* dW, double* one, double* two) {
       if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
       if (e != cudaSuccess) { sbdx::set_cuda_err(c, e, "rdm copy-out"); rc = SBDX_ERR_CUDA; }
     }
-    cudaFree(d_one);
-    cudaFree(d_two);
+    sbdx::dev_free(c, d_one);
+    sbdx::dev_free(c, d_two);
     return rc;
   });
 }

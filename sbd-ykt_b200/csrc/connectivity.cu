@@ -182,18 +182,18 @@ conn_fill_kernel(int spin, const uint64_t* __restrict__ s, size_t n, const uint6
   }
 }
 
-void free_conn(Conn& c) {
-  cudaFree(c.nsing); cudaFree(c.ndoub); cudaFree(c.off); cudaFree(c.ket);
-  cudaFree(c.val); cudaFree(c.val32); cudaFree(c.omask); cudaFree(c.info);
-  cudaFree(c.srec); cudaFree(c.order); cudaFree(c.spos);
-  cudaFree(c.sell); cudaFree(c.soff); cudaFree(c.slen);
-  SellPanel& p = c.bal;
-  cudaFree(p.sell); cudaFree(p.soff); cudaFree(p.slen); cudaFree(p.vrow); cudaFree(p.vslot);
-  cudaFree(p.split_row); cudaFree(p.split_slot);
-  cudaFree(c.ab_item); cudaFree(c.ab_split); cudaFree(c.ab_slot); cudaFree(c.ab_done); cudaFree(c.ypart);
-  cudaFree(c.same_item); cudaFree(c.same_split); cudaFree(c.same_slot); cudaFree(c.same_done); cudaFree(c.same_ypart);
-  for (SameBlocks& b : c.blk) free_blocks(b);
-  c = Conn{};
+void free_conn(Ctx* c, Conn& cn) {
+  dev_free(c, cn.nsing); dev_free(c, cn.ndoub); dev_free(c, cn.off); dev_free(c, cn.ket);
+  dev_free(c, cn.val); dev_free(c, cn.val32); dev_free(c, cn.omask); dev_free(c, cn.info);
+  dev_free(c, cn.srec); dev_free(c, cn.order); dev_free(c, cn.spos);
+  dev_free(c, cn.sell); dev_free(c, cn.soff); dev_free(c, cn.slen);
+  SellPanel& p = cn.bal;
+  dev_free(c, p.sell); dev_free(c, p.soff); dev_free(c, p.slen); dev_free(c, p.vrow); dev_free(c, p.vslot);
+  dev_free(c, p.split_row); dev_free(c, p.split_slot);
+  dev_free(c, cn.ab_item); dev_free(c, cn.ab_split); dev_free(c, cn.ab_slot); dev_free(c, cn.ab_done); dev_free(c, cn.ypart);
+  dev_free(c, cn.same_item); dev_free(c, cn.same_split); dev_free(c, cn.same_slot); dev_free(c, cn.same_done); dev_free(c, cn.same_ypart);
+  for (SameBlocks& b : cn.blk) free_blocks(c, b);
+  cn = Conn{};
 }
 
 // Splits rows of `len` work units longer than cap into items (see
@@ -223,15 +223,15 @@ void split_rows(const std::vector<uint32_t>& len, uint32_t cap, bool keep_empty,
 
 int upload_items(Ctx* c, const std::vector<uint4>& items, const std::vector<uint4>& split, int nslot, size_t ncol,
                  uint4** d_items, uint4** d_split, double** d_part) {
-  SBDX_CUDA(c, cudaMalloc(d_items, sizeof(uint4) * std::max<size_t>(1, items.size())));
-  SBDX_CUDA(c, cudaMalloc(d_split, sizeof(uint4) * std::max<size_t>(1, split.size())));
+  SBDX_CUDA(c, dev_alloc(c, d_items, sizeof(uint4) * std::max<size_t>(1, items.size())));
+  SBDX_CUDA(c, dev_alloc(c, d_split, sizeof(uint4) * std::max<size_t>(1, split.size())));
   if (!items.empty())
     SBDX_CUDA(c, cudaMemcpyAsync(*d_items, items.data(), sizeof(uint4) * items.size(), cudaMemcpyHostToDevice,
                                  c->stream));
   if (!split.empty()) {
     SBDX_CUDA(c, cudaMemcpyAsync(*d_split, split.data(), sizeof(uint4) * split.size(), cudaMemcpyHostToDevice,
                                  c->stream));
-    SBDX_CUDA(c, cudaMalloc(d_part, sizeof(double) * (size_t)nslot * std::max<size_t>(8, pad8(ncol))));
+    SBDX_CUDA(c, dev_alloc(c, d_part, sizeof(double) * (size_t)nslot * std::max<size_t>(8, pad8(ncol))));
   }
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));  // host vectors die at return
   return 0;
@@ -244,8 +244,8 @@ int upload_slots(Ctx* c, const std::vector<uint4>& split, int nslot, size_t stri
   std::vector<uint32_t> of(nslot);
   for (size_t q = 0; q < split.size(); ++q)
     for (uint32_t k = 0; k < split[q].z; ++k) of[split[q].y + k] = (uint32_t)q;
-  SBDX_CUDA(c, cudaMalloc(d_slot, sizeof(uint32_t) * of.size()));
-  SBDX_CUDA(c, cudaMalloc(d_done, sizeof(uint32_t) * split.size() * strips));
+  SBDX_CUDA(c, dev_alloc(c, d_slot, sizeof(uint32_t) * of.size()));
+  SBDX_CUDA(c, dev_alloc(c, d_done, sizeof(uint32_t) * split.size() * strips));
   SBDX_CUDA(c, cudaMemcpyAsync(*d_slot, of.data(), sizeof(uint32_t) * of.size(), cudaMemcpyHostToDevice, c->stream));
   SBDX_CUDA(c, cudaMemsetAsync(*d_done, 0, sizeof(uint32_t) * split.size() * strips, c->stream));
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -383,7 +383,7 @@ union_kernel(const uint32_t* __restrict__ rows, size_t n, const uint64_t* __rest
 // (partial rows have stride pad8(ncol)).
 int build_same_blocks(Ctx* c, const Conn& cn, const std::vector<uint64_t>& strings, size_t row0, size_t n, size_t ncol,
                       int width, SameBlocks& B) {
-  free_blocks(B);
+  free_blocks(c, B);
   if (n == 0) return 0;
   // rows in bit-reversed string order, cut into blocks
   std::vector<std::pair<uint64_t, uint32_t>> rkey(n);
@@ -392,18 +392,18 @@ int build_same_blocks(Ctx* c, const Conn& cn, const std::vector<uint64_t>& strin
   const size_t nblk = (n + width - 1) / width;
   std::vector<uint32_t> rows(nblk * width, kNoRow);
   for (size_t i = 0; i < n; ++i) rows[i] = (uint32_t)(row0 + rkey[i].second);
-  SBDX_CUDA(c, cudaMalloc(&B.rows, sizeof(uint32_t) * rows.size()));
-  SBDX_CUDA(c, cudaMalloc(&B.uoff, sizeof(uint64_t) * (nblk + 1)));
+  SBDX_CUDA(c, dev_alloc(c, &B.rows, sizeof(uint32_t) * rows.size()));
+  SBDX_CUDA(c, dev_alloc(c, &B.uoff, sizeof(uint64_t) * (nblk + 1)));
   SBDX_CUDA(c, cudaMemcpyAsync(B.rows, rows.data(), sizeof(uint32_t) * rows.size(), cudaMemcpyHostToDevice, c->stream));
   uint32_t* d_cnt = nullptr;
-  SBDX_CUDA(c, cudaMalloc(&d_cnt, sizeof(uint32_t) * nblk));
+  SBDX_CUDA(c, dev_alloc(c, &d_cnt, sizeof(uint32_t) * nblk));
   union_kernel<<<(unsigned)nblk, 256, 0, c->stream>>>(B.rows, cn.n, cn.off, cn.ket, cn.val, cn.val32, cn.info, width,
                                                       d_cnt, nullptr, nullptr, nullptr, nullptr);
   ++c->launches;
   std::vector<uint32_t> cnt(nblk);
   cudaError_t e = cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(uint32_t) * nblk, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  cudaFree(d_cnt);
+  dev_free(c, d_cnt);
   SBDX_CUDA(c, e);
   std::vector<uint64_t> uoff(nblk + 1, 0);
   for (size_t b = 0; b < nblk; ++b) uoff[b + 1] = uoff[b] + ((cnt[b] + 7) & ~7u);
@@ -426,10 +426,10 @@ int build_same_blocks(Ctx* c, const Conn& cn, const std::vector<uint64_t>& strin
   B.n_item = items.size();
   B.n_split = (int)split.size();
   B.n_part = nslot;
-  SBDX_CUDA(c, cudaMalloc(&B.uket, sizeof(uint32_t) * nu1));
+  SBDX_CUDA(c, dev_alloc(c, &B.uket, sizeof(uint32_t) * nu1));
   const bool f64 = width == kBlkRows64;
   const size_t vbytes = (f64 ? sizeof(double) : sizeof(float)) * width * nu1;
-  SBDX_CUDA(c, cudaMalloc(f64 ? (void**)&B.uval : (void**)&B.uval32, vbytes));
+  SBDX_CUDA(c, dev_alloc(c, f64 ? (void**)&B.uval : (void**)&B.uval32, vbytes));
   SBDX_CUDA(c, cudaMemsetAsync(f64 ? (void*)B.uval : (void*)B.uval32, 0, vbytes, c->stream));
   SBDX_CUDA(c, cudaMemcpyAsync(B.uoff, uoff.data(), sizeof(uint64_t) * (nblk + 1), cudaMemcpyHostToDevice, c->stream));
   union_kernel<<<(unsigned)nblk, 256, 0, c->stream>>>(B.rows, cn.n, cn.off, cn.ket, cn.val, cn.val32, cn.info, width,
@@ -550,13 +550,13 @@ int build_balanced_sell(Ctx* c, SellPanel& P, size_t n, const std::vector<uint32
   P.cap = (int)cap;
   P.slices_per_warp = ks;
   if (split_row.empty()) split_row.push_back(0);
-  SBDX_CUDA(c, cudaMalloc(&P.sell, sizeof(uint64_t) * sell.size()));
-  SBDX_CUDA(c, cudaMalloc(&P.soff, sizeof(uint64_t) * (ns + 1)));
-  SBDX_CUDA(c, cudaMalloc(&P.slen, sizeof(uint32_t) * slen.size()));
-  SBDX_CUDA(c, cudaMalloc(&P.vrow, sizeof(uint32_t) * vrow.size()));
-  SBDX_CUDA(c, cudaMalloc(&P.vslot, sizeof(uint32_t) * vslot.size()));
-  SBDX_CUDA(c, cudaMalloc(&P.split_row, sizeof(uint32_t) * split_row.size()));
-  SBDX_CUDA(c, cudaMalloc(&P.split_slot, sizeof(uint32_t) * split_slot.size()));
+  SBDX_CUDA(c, dev_alloc(c, &P.sell, sizeof(uint64_t) * sell.size()));
+  SBDX_CUDA(c, dev_alloc(c, &P.soff, sizeof(uint64_t) * (ns + 1)));
+  SBDX_CUDA(c, dev_alloc(c, &P.slen, sizeof(uint32_t) * slen.size()));
+  SBDX_CUDA(c, dev_alloc(c, &P.vrow, sizeof(uint32_t) * vrow.size()));
+  SBDX_CUDA(c, dev_alloc(c, &P.vslot, sizeof(uint32_t) * vslot.size()));
+  SBDX_CUDA(c, dev_alloc(c, &P.split_row, sizeof(uint32_t) * split_row.size()));
+  SBDX_CUDA(c, dev_alloc(c, &P.split_slot, sizeof(uint32_t) * split_slot.size()));
   SBDX_CUDA(c, cudaMemcpyAsync(P.sell, sell.data(), sizeof(uint64_t) * sell.size(), cudaMemcpyHostToDevice, c->stream));
   SBDX_CUDA(c, cudaMemcpyAsync(P.soff, soff.data(), sizeof(uint64_t) * (ns + 1), cudaMemcpyHostToDevice, c->stream));
   SBDX_CUDA(c, cudaMemcpyAsync(P.slen, slen.data(), sizeof(uint32_t) * slen.size(), cudaMemcpyHostToDevice, c->stream));
@@ -584,13 +584,13 @@ int single_records(Ctx* c, const Conn& cn, std::vector<uint64_t>& rec) {
 // without the sigma's work items, SELL layouts, ket positions and blocks.
 int build_one(Ctx* c, int spin, bool full) {
   Conn& cn = c->conn[spin];
-  free_conn(cn);
+  free_conn(c, cn);
   const size_t n = spin == 0 ? c->na : c->nb;
   const uint64_t* s = spin == 0 ? c->d_a : c->d_b;
   cn.n = n;
-  SBDX_CUDA(c, cudaMalloc(&cn.nsing, sizeof(uint32_t) * n));
-  SBDX_CUDA(c, cudaMalloc(&cn.ndoub, sizeof(uint32_t) * n));
-  SBDX_CUDA(c, cudaMalloc(&cn.off, sizeof(uint64_t) * (n + 1)));
+  SBDX_CUDA(c, dev_alloc(c, &cn.nsing, sizeof(uint32_t) * n));
+  SBDX_CUDA(c, dev_alloc(c, &cn.ndoub, sizeof(uint32_t) * n));
+  SBDX_CUDA(c, dev_alloc(c, &cn.off, sizeof(uint64_t) * (n + 1)));
   conn_count_kernel<<<(unsigned)n, kConnThreads, 0, c->stream>>>(s, n, cn.nsing, cn.ndoub);
   SBDX_LAUNCHED(c);
   std::vector<uint32_t> hs(n), hd(n);
@@ -602,14 +602,14 @@ int build_one(Ctx* c, int spin, bool full) {
   cn.total = off[n];
   SBDX_CUDA(c, cudaMemcpyAsync(cn.off, off.data(), sizeof(uint64_t) * (n + 1), cudaMemcpyHostToDevice, c->stream));
   const size_t t = cn.total ? cn.total : 1;
-  SBDX_CUDA(c, cudaMalloc(&cn.ket, sizeof(uint32_t) * t));
-  SBDX_CUDA(c, cudaMalloc(&cn.val, sizeof(double) * t));
-  SBDX_CUDA(c, cudaMalloc(&cn.val32, sizeof(float) * t));
-  SBDX_CUDA(c, cudaMalloc(&cn.omask, sizeof(uint64_t) * t));
-  SBDX_CUDA(c, cudaMalloc(&cn.info, sizeof(uint32_t) * t));
-  SBDX_CUDA(c, cudaMalloc(&cn.srec, sizeof(uint64_t) * t));
-  SBDX_CUDA(c, cudaMalloc(&cn.spos, sizeof(uint32_t) * t));
-  SBDX_CUDA(c, cudaMalloc(&cn.order, sizeof(uint32_t) * n));
+  SBDX_CUDA(c, dev_alloc(c, &cn.ket, sizeof(uint32_t) * t));
+  SBDX_CUDA(c, dev_alloc(c, &cn.val, sizeof(double) * t));
+  SBDX_CUDA(c, dev_alloc(c, &cn.val32, sizeof(float) * t));
+  SBDX_CUDA(c, dev_alloc(c, &cn.omask, sizeof(uint64_t) * t));
+  SBDX_CUDA(c, dev_alloc(c, &cn.info, sizeof(uint32_t) * t));
+  SBDX_CUDA(c, dev_alloc(c, &cn.srec, sizeof(uint64_t) * t));
+  SBDX_CUDA(c, dev_alloc(c, &cn.spos, sizeof(uint32_t) * t));
+  SBDX_CUDA(c, dev_alloc(c, &cn.order, sizeof(uint32_t) * n));
   conn_fill_kernel<<<(unsigned)n, kConnThreads, 0, c->stream>>>(spin, s, n, cn.off, cn.nsing, c->L, c->d_h,
                                                                  c->d_eri, cn.ket, cn.val, cn.val32,
                                                                  cn.omask, cn.info, cn.srec, cn.spos);
@@ -651,9 +651,9 @@ int build_one(Ctx* c, int spin, bool full) {
 
 }  // namespace
 
-void free_blocks(SameBlocks& b) {
-  cudaFree(b.rows); cudaFree(b.uoff); cudaFree(b.uket); cudaFree(b.uval); cudaFree(b.uval32);
-  cudaFree(b.item); cudaFree(b.split); cudaFree(b.slot); cudaFree(b.done); cudaFree(b.ypart);
+void free_blocks(Ctx* c, SameBlocks& b) {
+  dev_free(c, b.rows); dev_free(c, b.uoff); dev_free(c, b.uket); dev_free(c, b.uval); dev_free(c, b.uval32);
+  dev_free(c, b.item); dev_free(c, b.split); dev_free(c, b.slot); dev_free(c, b.done); dev_free(c, b.ypart);
   b = SameBlocks{};
 }
 
@@ -687,12 +687,12 @@ int ensure_sell(Ctx* c) {
         const uint32_t r = order[sl * 32 + l];
         for (uint32_t m = 0; m < hs[r]; ++m) sell[soff[sl] + 32ull * m + l] = rec[off[r] + m];
       }
-    cudaFree(cn.sell); cudaFree(cn.soff); cudaFree(cn.slen);
+    dev_free(c, cn.sell); dev_free(c, cn.soff); dev_free(c, cn.slen);
     cn.sell = nullptr; cn.soff = nullptr; cn.slen = nullptr;
     cn.nslice = ns;
-    SBDX_CUDA(c, cudaMalloc(&cn.sell, sizeof(uint64_t) * sell.size()));
-    SBDX_CUDA(c, cudaMalloc(&cn.soff, sizeof(uint64_t) * (ns + 1)));
-    SBDX_CUDA(c, cudaMalloc(&cn.slen, sizeof(uint32_t) * (ns ? ns : 1)));
+    SBDX_CUDA(c, dev_alloc(c, &cn.sell, sizeof(uint64_t) * sell.size()));
+    SBDX_CUDA(c, dev_alloc(c, &cn.soff, sizeof(uint64_t) * (ns + 1)));
+    SBDX_CUDA(c, dev_alloc(c, &cn.slen, sizeof(uint32_t) * (ns ? ns : 1)));
     SBDX_CUDA(c, cudaMemcpyAsync(cn.sell, sell.data(), sizeof(uint64_t) * sell.size(), cudaMemcpyHostToDevice, c->stream));
     SBDX_CUDA(c, cudaMemcpyAsync(cn.soff, soff.data(), sizeof(uint64_t) * (ns + 1), cudaMemcpyHostToDevice, c->stream));
     if (ns) SBDX_CUDA(c, cudaMemcpyAsync(cn.slen, slen.data(), sizeof(uint32_t) * ns, cudaMemcpyHostToDevice, c->stream));
@@ -703,11 +703,11 @@ int ensure_sell(Ctx* c) {
   return 0;
 }
 
-void free_range_items(Conn& r) {
-  for (SameBlocks& b : r.blk) free_blocks(b);
-  cudaFree(r.same_item); cudaFree(r.same_split); cudaFree(r.same_slot); cudaFree(r.same_done); cudaFree(r.same_ypart);
+void free_range_items(Ctx* c, Conn& r) {
+  for (SameBlocks& b : r.blk) free_blocks(c, b);
+  dev_free(c, r.same_item); dev_free(c, r.same_split); dev_free(c, r.same_slot); dev_free(c, r.same_done); dev_free(c, r.same_ypart);
   r.same_slot = r.same_done = nullptr;
-  cudaFree(r.ab_item); cudaFree(r.ab_split); cudaFree(r.ab_slot); cudaFree(r.ab_done); cudaFree(r.ypart);
+  dev_free(c, r.ab_item); dev_free(c, r.ab_split); dev_free(c, r.ab_slot); dev_free(c, r.ab_done); dev_free(c, r.ypart);
   r.same_item = r.same_split = r.ab_item = r.ab_split = nullptr;
   r.ab_slot = r.ab_done = nullptr;
   r.same_ypart = r.ypart = nullptr;
@@ -716,7 +716,7 @@ void free_range_items(Conn& r) {
 }
 
 void free_row_range(Ctx* c) {
-  free_range_items(c->range_conn);
+  free_range_items(c, c->range_conn);
   c->range_a0 = c->range_a1 = 0;
   c->have_range = false;
 }
@@ -727,7 +727,7 @@ void free_row_range(Ctx* c) {
 // build_ab_items over that range, their caps derived from the range's own
 // work.
 int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r) {
-  free_range_items(r);
+  free_range_items(c, r);
   const Conn& ca = c->conn[0];
   const size_t n = a1 - a0;
   std::vector<uint32_t> hs(n ? n : 1), hd(n ? n : 1);
@@ -760,16 +760,16 @@ void free_connectivity(Ctx* c) {
   release_stored(c);  // its elements come from the connectivity
   free_row_range(c);
   free_io_chunks(c);
-  free_conn(c->conn[0]);
-  free_conn(c->conn[1]);
-  free_ab_plan(c->ab);
-  cudaFree(c->d_xk);  // sized by the schedule
+  free_conn(c, c->conn[0]);
+  free_conn(c, c->conn[1]);
+  free_ab_plan(c, c->ab);
+  dev_free(c, c->d_xk);  // sized by the schedule
   c->d_xk = nullptr;
-  cudaFree(c->d_Dr); cudaFree(c->d_Dr32);
+  dev_free(c, c->d_Dr); dev_free(c, c->d_Dr32);
   c->d_Dr = nullptr;
   c->d_Dr32 = nullptr;
   c->have_sell = false;
-  cudaFree(c->d_Da); cudaFree(c->d_Db); cudaFree(c->d_Da32); cudaFree(c->d_Db32);
+  dev_free(c, c->d_Da); dev_free(c, c->d_Db); dev_free(c, c->d_Da32); dev_free(c, c->d_Db32);
   c->d_Da = c->d_Db = nullptr;
   c->d_Da32 = c->d_Db32 = nullptr;
   c->have_conn = false;
@@ -787,7 +787,10 @@ int build_connectivity(Ctx* c, bool full) {
   rc = build_one(c, 1, full);
   if (rc) return rc;
   c->have_lists = true;
-  if (!full) return 0;
+  if (!full) {
+    pool_trim(c);
+    return 0;
+  }
   rc = build_coulomb_tables(c);
   if (rc) return rc;
   c->have_conn = true;

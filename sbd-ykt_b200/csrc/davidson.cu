@@ -75,7 +75,7 @@ __device__ __forceinline__ void block_sums(const double (&v)[N], int n, double* 
 
 // Four consecutive elements as doubles. The vector kernels below take this
 // path for element quads when D % 4 == 0: every vector of the solvers starts
-// at a cudaMalloc base plus a multiple of D elements, so quads are 16-byte
+// at an allocation's base plus a multiple of D elements, so quads are 16-byte
 // aligned; the remaining elements (or all, when D % 4 != 0) go one by one.
 __device__ __forceinline__ void ld4(const float* p, double (&o)[4]) {
   const float4 v = __ldg(reinterpret_cast<const float4*>(p));
@@ -543,7 +543,24 @@ struct Work {
   double* partial = nullptr;  // reduction partials
   double* scal = nullptr;     // device scalars
   double* u = nullptr;        // Ritz coefficients
-  ~Work() { cudaFree(partial); cudaFree(scal); cudaFree(u); }
+};
+
+// A solve's device buffers, released on its stream; the pool keeps a bounded
+// part of them for the next solve.
+struct SolveBuffers {
+  Ctx* c;
+  std::vector<void*> p;
+  explicit SolveBuffers(Ctx* ctx) : c(ctx) {}
+  ~SolveBuffers() {
+    for (void* q : p) dev_free(c, q);
+    pool_trim(c);
+  }
+  template <typename T>
+  cudaError_t get(T** d, size_t bytes) {
+    const cudaError_t e = dev_alloc(c, d, bytes);
+    if (e == cudaSuccess) p.push_back(*d);
+    return e;
+  }
 };
 
 // Device scalar slots
@@ -675,14 +692,14 @@ int davidson_fp64(Ctx* c, const sbdx_davidson_params& p, double* dW, sbdx_davids
   const size_t D = c->na * c->nb;
   const int nb = p.max_nb;
   Work wk;
-  SBDX_CUDA(c, cudaMalloc(&wk.partial, sizeof(double) * kRedBlocks * (nb + 2)));
-  SBDX_CUDA(c, cudaMalloc(&wk.scal, sizeof(double) * (kDots + 2 * nb + 16)));
-  SBDX_CUDA(c, cudaMalloc(&wk.u, sizeof(double) * (nb + 1)));
+  SolveBuffers g(c);
+  SBDX_CUDA(c, g.get(&wk.partial, sizeof(double) * kRedBlocks * (nb + 2)));
+  SBDX_CUDA(c, g.get(&wk.scal, sizeof(double) * (kDots + 2 * nb + 16)));
+  SBDX_CUDA(c, g.get(&wk.u, sizeof(double) * (nb + 1)));
   double *C = nullptr, *HC = nullptr, *R = nullptr;
-  SBDX_CUDA(c, cudaMalloc(&C, sizeof(double) * D * nb));
-  SBDX_CUDA(c, cudaMalloc(&HC, sizeof(double) * D * nb));
-  SBDX_CUDA(c, cudaMalloc(&R, sizeof(double) * D));
-  struct Guard { double *a, *b, *r; ~Guard() { cudaFree(a); cudaFree(b); cudaFree(r); } } g{C, HC, R};
+  SBDX_CUDA(c, g.get(&C, sizeof(double) * D * nb));
+  SBDX_CUDA(c, g.get(&HC, sizeof(double) * D * nb));
+  SBDX_CUDA(c, g.get(&R, sizeof(double) * D));
   double* s = wk.scal;
   std::vector<double> H((size_t)nb * nb, 0.0), U((size_t)nb * nb), E(nb), hcol(nb + 1);
   const auto t0 = std::chrono::steady_clock::now();
@@ -1056,20 +1073,17 @@ int davidson_mixed(Ctx* c, const sbdx_davidson_params& p, double* dW, sbdx_david
   const int keep = nc >= 3 ? nc / 3 : 0;
   const int period = p.defect_every > 0 ? p.defect_every : 0;
   Work wk;
-  SBDX_CUDA(c, cudaMalloc(&wk.partial, sizeof(double) * kRedBlocks * (2 * nc + 4)));  // multidot2: 2 per vector
-  SBDX_CUDA(c, cudaMalloc(&wk.scal, sizeof(double) * (kDots + 2 * nc + 16)));
-  SBDX_CUDA(c, cudaMalloc(&wk.u, sizeof(double) * (nc + 2)));
+  SolveBuffers g(c);
+  SBDX_CUDA(c, g.get(&wk.partial, sizeof(double) * kRedBlocks * (2 * nc + 4)));  // multidot2: 2 per vector
+  SBDX_CUDA(c, g.get(&wk.scal, sizeof(double) * (kDots + 2 * nc + 16)));
+  SBDX_CUDA(c, g.get(&wk.u, sizeof(double) * (nc + 2)));
   float *C = nullptr, *HC = nullptr;
   double *AW = nullptr, *R = nullptr, *V = nullptr;
-  SBDX_CUDA(c, cudaMalloc(&C, sizeof(float) * D * nc));
-  SBDX_CUDA(c, cudaMalloc(&HC, sizeof(float) * D * nc));
-  SBDX_CUDA(c, cudaMalloc(&AW, sizeof(double) * D * 2));  // [W | HW] anchor pair
-  SBDX_CUDA(c, cudaMalloc(&R, sizeof(double) * D));
-  SBDX_CUDA(c, cudaMalloc(&V, sizeof(double) * D));
-  struct Guard {
-    float *a, *b; double *c, *d, *e;
-    ~Guard() { cudaFree(a); cudaFree(b); cudaFree(c); cudaFree(d); cudaFree(e); }
-  } g{C, HC, AW, R, V};
+  SBDX_CUDA(c, g.get(&C, sizeof(float) * D * nc));
+  SBDX_CUDA(c, g.get(&HC, sizeof(float) * D * nc));
+  SBDX_CUDA(c, g.get(&AW, sizeof(double) * D * 2));  // [W | HW] anchor pair
+  SBDX_CUDA(c, g.get(&R, sizeof(double) * D));
+  SBDX_CUDA(c, g.get(&V, sizeof(double) * D));
   double* W = AW;
   double* HW = AW + D;
   double* s = wk.scal;

@@ -85,7 +85,7 @@ int diag_terms(Ctx* c) {
     return 3;
   }
   const size_t na = c->na, nb = c->nb, D = na * nb;
-  if (!c->d_hii) SBDX_CUDA(c, cudaMalloc(&c->d_hii, sizeof(double) * D));
+  if (!c->d_hii) SBDX_CUDA(c, dev_alloc(c, &c->d_hii, sizeof(double) * D));
   double *Ea = nullptr, *Eb = nullptr, *Jb = nullptr;
   SBDX_CUDA(c, pool_alloc(c, (void**)&Ea, sizeof(double) * na));
   SBDX_CUDA(c, pool_alloc(c, (void**)&Eb, sizeof(double) * nb));

@@ -323,10 +323,11 @@ struct Ctx {
   // CUDA graph per iteration (sbdx_set_graph_steps)
   bool graph_steps = false;
   bool own_stream = false;  // stream created by the library (destroyed with the context)
-  // pool of the solvers' stream-ordered scratch. It keeps its memory between
-  // allocations (no unmap/map of gigabytes per solve, which stalls the other
-  // streams of a batch); a context that owns it trims it after each solve, a
-  // batch shares one pool among its subspaces and trims it after the batch.
+  // pool of the context's device buffers and the solvers' stream-ordered
+  // scratch. It keeps its memory between allocations (no unmap/map of gigabytes
+  // per solve, which stalls the other streams of a batch); a context that owns
+  // it trims it after each solve to kPoolKeep unused bytes, a batch shares one
+  // pool among its subspaces and trims it after the batch.
   cudaMemPool_t pool = nullptr;
   bool own_pool = false;
   std::vector<SigmaGraph> graphs;
@@ -438,7 +439,7 @@ __host__ __device__ __forceinline__ uint64_t other_range(int spin, int x, int y)
 // other alpha-beta kernels (built when a launch code first asks for them).
 int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::vector<uint64_t>& off,
                   const std::vector<uint64_t>& rec, uint64_t alpha_singles);
-void free_ab_plan(AbPlan& P);
+void free_ab_plan(Ctx* c, AbPlan& P);
 int ensure_sell(Ctx* c);
 int ensure_coulomb_a(Ctx* c);
 int build_coulomb_tables(Ctx* c);
@@ -451,8 +452,8 @@ int build_row_range(Ctx* c, size_t a0, size_t a1);
 void free_row_range(Ctx* c);
 // The work items of rows [a0, a1) into r, and their release.
 int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r);
-void free_range_items(Conn& r);
-void free_blocks(SameBlocks& b);
+void free_range_items(Ctx* c, Conn& r);
+void free_blocks(Ctx* c, SameBlocks& b);
 // The host-buffer sigma's chunks (their work items, copy stream, events).
 void free_io_chunks(Ctx* c);
 // S = H C for host buffers (FP64), the copies overlapped with the kernels.
@@ -482,7 +483,22 @@ int autotune(Ctx* c);
 int check_device_error(Ctx* c);
 // Stream-ordered allocation from the context's pool (created on first use).
 cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes);
-// Returns the free memory of an owned pool to the device (syncs the stream).
+// The same for any element type, and its release on the context stream. Every
+// device buffer of a context but the stored Hamiltonian comes from here:
+// cudaMalloc and cudaFree take 0.1 ms each and synchronise the device, which
+// cost a diag call on 400 x 400 strings 17 of 29 ms.
+template <typename T>
+cudaError_t dev_alloc(Ctx* c, T** p, size_t bytes) {
+  return pool_alloc(c, reinterpret_cast<void**>(p), bytes ? bytes : 16);
+}
+inline void dev_free(Ctx* c, void* p) {
+  if (p && cudaFreeAsync(p, c->stream) != cudaSuccess) {  // e.g. a stream its owner has destroyed
+    cudaGetLastError();
+    cudaFree(p);
+  }
+}
+// Returns the unused memory of an owned pool beyond kPoolKeep to the device.
+constexpr size_t kPoolKeep = size_t(1) << 30;
 void pool_trim(Ctx* c);
 // A pool that keeps its memory, on `device`.
 cudaError_t make_pool(int device, cudaMemPool_t* pool);

@@ -2453,10 +2453,10 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
 int build_coulomb_tables(Ctx* c) {
   c->db_stride = pad8(c->nb);
   const size_t nb_el = c->npair * c->db_stride;
-  SBDX_CUDA(c, cudaMalloc(&c->d_Db, sizeof(double) * nb_el));
-  SBDX_CUDA(c, cudaMalloc(&c->d_Db32, sizeof(float) * nb_el));
-  SBDX_CUDA(c, cudaMalloc(&c->d_Dr, sizeof(double) * c->na * c->vstride));
-  SBDX_CUDA(c, cudaMalloc(&c->d_Dr32, sizeof(float) * c->na * c->vstride32));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_Db, sizeof(double) * nb_el));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_Db32, sizeof(float) * nb_el));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_Dr, sizeof(double) * c->na * c->vstride));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_Dr32, sizeof(float) * c->na * c->vstride32));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Db, 0, sizeof(double) * nb_el, c->stream));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Db32, 0, sizeof(float) * nb_el, c->stream));
   const dim3 gb((unsigned)((c->nb + 255) / 256), (unsigned)c->npair);
@@ -2472,10 +2472,10 @@ int ensure_coulomb_a(Ctx* c) {
   if (c->d_Da) return 0;
   c->da_stride = pad8(c->na);
   const size_t na_el = c->npair * c->da_stride;
-  SBDX_CUDA(c, cudaMalloc(&c->d_Da32, sizeof(float) * na_el));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_Da32, sizeof(float) * na_el));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Da32, 0, sizeof(float) * na_el, c->stream));
   double* Da = nullptr;
-  SBDX_CUDA(c, cudaMalloc(&Da, sizeof(double) * na_el));
+  SBDX_CUDA(c, dev_alloc(c, &Da, sizeof(double) * na_el));
   c->d_Da = Da;
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Da, 0, sizeof(double) * na_el, c->stream));
   const dim3 ga((unsigned)((c->na + 255) / 256), (unsigned)c->npair);
@@ -2490,23 +2490,23 @@ int phase_vectors(Ctx* c, const double* W) {
 
 int build_g_table(Ctx* c) {
   const size_t n = c->npair * (size_t)c->L;
-  cudaFree(c->d_G);
-  cudaFree(c->d_G32);
+  dev_free(c, c->d_G);
+  dev_free(c, c->d_G32);
   c->d_G = nullptr;
   c->d_G32 = nullptr;
-  SBDX_CUDA(c, cudaMalloc(&c->d_G, sizeof(double) * n));
-  SBDX_CUDA(c, cudaMalloc(&c->d_G32, sizeof(float) * n));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_G, sizeof(double) * n));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_G32, sizeof(float) * n));
   g_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->d_eri, c->L, c->npair, c->d_G, c->d_G32);
   SBDX_LAUNCHED(c);
   const size_t nv = c->npair * c->npair;
   c->vstride = (c->npair + 1) / 2 * 2;
   c->vstride32 = (c->npair + 3) / 4 * 4;
-  cudaFree(c->d_V);
-  cudaFree(c->d_V32);
+  dev_free(c, c->d_V);
+  dev_free(c, c->d_V32);
   c->d_V = nullptr;
   c->d_V32 = nullptr;
-  SBDX_CUDA(c, cudaMalloc(&c->d_V, sizeof(double) * c->npair * c->vstride));
-  SBDX_CUDA(c, cudaMalloc(&c->d_V32, sizeof(float) * c->npair * c->vstride32));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_V, sizeof(double) * c->npair * c->vstride));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_V32, sizeof(float) * c->npair * c->vstride32));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_V, 0, sizeof(double) * c->npair * c->vstride, c->stream));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_V32, 0, sizeof(float) * c->npair * c->vstride32, c->stream));
   unpack_eri_kernel<<<(unsigned)((nv + 255) / 256), 256, 0, c->stream>>>(c->d_eri, c->npair, c->vstride,
@@ -2521,7 +2521,7 @@ int ensure_sigma_scratch(Ctx* c) {
   const size_t n = std::max(c->na * c->xsa, c->nb * c->xsb);  // >= D
   auto get = [&](void** p) -> int {
     if (*p) return 0;
-    SBDX_CUDA(c, cudaMalloc(p, sizeof(double) * n));
+    SBDX_CUDA(c, dev_alloc(c, p, sizeof(double) * n));
     SBDX_CUDA(c, cudaMemsetAsync(*p, 0, sizeof(double) * n, c->stream));  // padding columns start at zero
     return 0;
   };
@@ -2535,7 +2535,7 @@ int ensure_sigma_scratch(Ctx* c) {
     SBDX_CUDA(c, cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
   }
   if (c->ab.xs && !c->d_xk) {
-    SBDX_CUDA(c, cudaMalloc(&c->d_xk, sizeof(double) * c->na * c->ab.xs));
+    SBDX_CUDA(c, dev_alloc(c, &c->d_xk, sizeof(double) * c->na * c->ab.xs));
     SBDX_CUDA(c, cudaMemsetAsync(c->d_xk, 0, sizeof(double) * c->na * c->ab.xs, c->stream));
   }
   return 0;
@@ -2783,7 +2783,7 @@ int build_io_chunks(Ctx* c, const std::vector<size_t>& bounds) {
 }  // namespace
 
 void free_io_chunks(Ctx* c) {
-  for (auto& r : c->io_items) free_range_items(r);
+  for (auto& r : c->io_items) free_range_items(c, r);
   c->io_items.clear();
   c->io_bounds.clear();
   for (auto e : c->io_events)

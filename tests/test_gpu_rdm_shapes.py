@@ -25,7 +25,7 @@ SIZES = [
     (12, 4, 4, 129, 33),
     (40, 8, 8, 300, 12),      # mixed excitation ranks, lists of very different lengths
     (14, 4, 4, 5, 950),       # six, four, two and one alpha single at a time
-    (16, 4, 4, 5, 2500),
+    (16, 4, 5, 5, 2500),
     (16, 2, 5, 5, 3700),
     (18, 2, 5, 4, 7300),
 ]

@@ -358,7 +358,7 @@ union_kernel(const uint32_t* __restrict__ rows, size_t n, const uint64_t* __rest
           const uint32_t wd = (uint32_t)((x - w0) >> 5), bit = (uint32_t)((x - w0) & 31);
           const uint64_t at = uoff[b] + pre[wd] + __popc(bits[wd] & ((1u << bit) - 1u));
           const bool neg = (info[e] & kInfoNeg) != 0;
-          if (uval != nullptr) uval[at * width + k] = neg ? -val[e] : val[e];
+          if (uval != nullptr) uval[(at >> 2) * (4 * width) + k * 4 + (at & 3)] = neg ? -val[e] : val[e];
           else uval32[at * width + k] = neg ? -val32[e] : val32[e];
         }
       }

@@ -94,7 +94,8 @@ constexpr uint32_t kNoRow = 0xffffffffu;
 // FP64 kernel, four for the FP32 one). Per block the union of its strings' single- and double-excitation kets, ascending, padded
 // to a multiple of 8 entries with zero values, with one signed same-spin value
 // per string of the block (zero where that string does not connect).
-// Values: [entry][string].
+// Values: FP64 in groups of four entries, [group][string][entry], the A
+// operands of m8n8k4 in lane order; FP32 [entry][string].
 // Work items {block, first union entry, one past the last, 1 + partial slot
 // or 0}, longest first; a block with more union entries than the cap is
 // split, and the last of its CTAs to finish sums the parts' partial rows
@@ -509,5 +510,6 @@ int lowest_diagonal(Ctx* c, int k, std::vector<size_t>& idx);
 
 // Device error codes written to Ctx::d_err.
 constexpr int kErrWatchdogAb = 1;  // alpha-beta kernels: a wait (TMA completion, step order) timed out
+constexpr int kErrWatchdogSame = 2;  // blocked same-spin kernel: a wait for its copies timed out
 
 }  // namespace sbdx

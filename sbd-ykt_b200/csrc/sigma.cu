@@ -36,6 +36,15 @@ namespace {
 
 constexpr int kSameThreads = 256;
 
+// D += A B on the FP64 tensor pipe: A 8 x 4 (lane: row lane >> 2, k lane & 3),
+// B 4 x 8 (k lane & 3, column lane >> 2), D row lane >> 2, columns 2 (lane & 3)
+// + {0, 1}.
+__device__ __forceinline__ void dmma_m8n8k4(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
 template <typename T> struct Prec;
 template <> struct Prec<double> { using V = double; };
 template <> struct Prec<float> { using V = float; };
@@ -1012,6 +1021,7 @@ int run_ab(Ctx* c, const T* X) {
 //   1. alpha same-spin on Xp -> Y                     (sigma_same_*_kernel)
 //   2. beta same-spin on Xpt -> Yt                    (sigma_same_*_kernel)
 //   3. alpha x beta on Xk -> Yab                      (sigma_ab_kernel)
+//   (steps 1 to 3 side by side where the context's streams allow it)
 //   4. S = phi o (Y + Yab + Yt^T) + hii o X           (combine_phase_kernel)
 // Step 1 includes the Coulomb terms of the alpha singles with the beta string,
 // step 3 those of the beta singles with the alpha string (one more integral
@@ -1363,12 +1373,19 @@ sigma_same_v6f_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, cons
   if (item.w) same_split_sum<VEC>(split, slot_split, done, item.w - 1, 1, ypart, ldx, c0, active, Y, r);
 }
 
+// VEC consecutive elements in the storage type.
+template <typename T, int VEC> struct LoadT;
+template <int VEC> struct LoadT<double, VEC> {
+  static __device__ __forceinline__ void load(const double* p, double* o) { VecIO<double, VEC>::load(p, o); }
+};
+template <int VEC> struct LoadT<float, VEC> {
+  static __device__ __forceinline__ void load(const float* p, float* o) { VecF<VEC>::load(p, o); }
+};
+
 // Blocked same-spin products: CTA = (work item of SameBlocks, strip of
 // columns). Every ket row strip of the block's union is loaded once and
 // applied to all bra strings of the block with their signed values (zero
-// where a string does not connect). With Dt, a block's first item adds the
-// Coulomb terms of its strings' singles (the constant part of a single is in
-// the union).
+// where a string does not connect).
 
 // Stages up to kSameThreads union entries (kets and values).
 template <int ROWS, typename V>
@@ -1383,124 +1400,215 @@ __device__ __forceinline__ void stage_union(uint32_t* s_ket, V* s_val, const uin
   __syncthreads();
 }
 
-// FP64, eight strings per block. A thread owns P pairs of columns, pair p at
-// 64 p + 2 (lane) of its warp's 64 P columns, so every 16-byte load of a warp
-// covers 512 contiguous bytes (a quarter-warp that reads several lines pays a
-// wavefront for each). Loads run kAhead entries ahead of the products.
-template <int P>
+// Y[r, c] += sum over the singles e of string r of s_e Dt[pq_e, c] X[ket_e, c]: the
+// Coulomb terms that the blocked kernels leave out (the constant part of a
+// single is in their unions). CTA = (string row0 + blockIdx.x, strip), 16 bytes of
+// consecutive columns per thread, the loads of kAhead singles before their
+// products. FP32: sums over kRun singles in FP32, then FP64. Reads two strips
+// per single from L2 (19.7 GB at 8000 x 8000 strings, FP64). Inside the matrix
+// kernel the same loads wait for the row with the most singles of eight, and
+// their registers spill (8000 x 8000, FP64: 7.3 ms for both, 5.1 + 1.3 ms apart).
+template <typename T>
+__global__ void __launch_bounds__(kSameThreads, 4)
+sigma_coulomb_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, size_t row0, const uint64_t* __restrict__ off,
+                     const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
+                     const uint32_t* __restrict__ info, const T* __restrict__ Dt, size_t dstride,
+                     double* __restrict__ Y) {
+  constexpr int PW = 16 / sizeof(T), kAhead = 4;
+  __shared__ uint32_t s_ket[kSameThreads], s_pq[kSameThreads];
+  const size_t r = row0 + blockIdx.x;
+  const size_t c0 = ((size_t)blockIdx.y * kSameThreads + threadIdx.x) * PW;
+  const uint64_t e0 = off[r];
+  const int ns = (int)nsing[r];
+  if (ns == 0) return;
+  const bool active = c0 < ncol;
+  double acc[PW];
+#pragma unroll
+  for (int v = 0; v < PW; ++v) acc[v] = 0.0;
+  for (int base = 0; base < ns; base += kSameThreads) {
+    const int cnt = min(kSameThreads, ns - base);
+    __syncthreads();
+    if ((int)threadIdx.x < cnt) {
+      const uint32_t inf = info[e0 + base + threadIdx.x];
+      s_ket[threadIdx.x] = ket[e0 + base + threadIdx.x];
+      s_pq[threadIdx.x] = ((inf >> 12) & 0xfffu) | (inf & kInfoNeg);
+    }
+    __syncthreads();
+    if (!active) continue;
+    T pf[PW];
+    for (int b0 = 0; b0 < cnt; b0 += kAhead) {
+      T x[kAhead][PW], d[kAhead][PW];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        const int b = min(b0 + u, cnt - 1);
+        LoadT<T, PW>::load(X + (size_t)s_ket[b] * ldx + c0, x[u]);
+        LoadT<T, PW>::load(Dt + (size_t)(s_pq[b] & 0xfffu) * dstride + c0, d[u]);
+      }
+      if (b0 % kRun == 0)
+#pragma unroll
+        for (int v = 0; v < PW; ++v) pf[v] = (T)0;
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (b0 + u < cnt) {
+          const bool neg = (s_pq[b0 + u] >> 31) != 0;
+#pragma unroll
+          for (int v = 0; v < PW; ++v) pf[v] = fma(neg ? -d[u][v] : d[u][v], x[u][v], pf[v]);
+        }
+      if (b0 % kRun + kAhead == kRun || b0 + kAhead >= cnt)
+#pragma unroll
+        for (int v = 0; v < PW; ++v) acc[v] += (double)pf[v];
+    }
+  }
+  if (!active) return;
+#pragma unroll
+  for (int v = 0; v < PW; v += 2) {
+    double2* y = reinterpret_cast<double2*>(Y + r * ldx + c0 + v);
+    double2 t = *y;
+    t.x += acc[v];
+    t.y += acc[v + 1];
+    *y = t;
+  }
+}
+
+// FP64, eight strings per block: the strings times four union entries are the A
+// operand of m8n8k4, four ket rows times eight columns its B operand, so the
+// product is a dense (8 x entries)(entries x columns) sum on the FP64 tensor
+// pipe. TMA bulk copies bring the strips of kMmaG entries and their values to
+// shared memory, a ring of kMmaStages stages that the warps refill in turn. A
+// warp owns 128 columns: lane l reads ket l & 3's columns 16 i + 2 (l >> 2) + {0,
+// 1} in one 16-byte load per i, the operands of an even and an odd tile; it ends
+// with string l >> 2, columns 16 i + 4 (l & 3) .. + 3. Rows in shared memory are
+// 32 bytes longer than the strip, so the four kets that a quarter-warp reads
+// lie in different banks. Bound: the FP64 tensor pipe (67% busy at 4800 x 4800);
+// padding of the unions counts as work there. 8000 x 8000: 5.1 ms for the beta
+// side, where CUDA-core products of four strings per block took 7.5 ms and of
+// eight 6.0 ms (issue slots, 60% of the FP64 pipe); with the B operands loaded
+// straight from global memory, a wavefront per ket and quarter-warp, 8.0 ms;
+// with two stages 6.8 ms; with kMmaI = 4 (shorter strips, the A operands read
+// twice as often) 5.5 ms.
+constexpr int kMmaI = 8;  // loads, of two 8-column tiles each, per lane and four entries
+constexpr int kMmaCols = 16 * kMmaI * (kSameThreads / 32), kMmaG = 32 / kMmaI, kMmaPitch = kMmaCols + 4;
+constexpr size_t kMmaStageBytes = sizeof(double) * kMmaG * (kMmaPitch + kBlkRows64);
+constexpr int kMmaStages = 3;
+
+// Bounded wait by polls (each suspends the thread for a while in hardware).
+__device__ __forceinline__ bool mbar_wait_polls(uint64_t* bar, uint32_t parity) {
+  for (int it = 0; it < (1 << 20); ++it)
+    if (mbar_try_wait(bar, parity)) return true;
+  return false;
+}
+
 __global__ void __launch_bounds__(kSameThreads, 2)
-sigma_same_blk_kernel(const double* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
-                      const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
-                      const uint32_t* __restrict__ info, const double* __restrict__ Dt, size_t dstride,
+sigma_same_mma_kernel(const double* __restrict__ X, size_t ncol, size_t ldx,
                       const uint32_t* __restrict__ brows, const uint64_t* __restrict__ uoff,
                       const uint32_t* __restrict__ uket, const double* __restrict__ uval,
                       const uint4* __restrict__ items, const uint4* __restrict__ split,
                       const uint32_t* __restrict__ slot_split, uint32_t* __restrict__ done,
-                      double* __restrict__ ypart, double* __restrict__ Y) {
-  constexpr int ROWS = kBlkRows64, kAhead = 8 / P;
-  __shared__ uint32_t s_ket[kSameThreads + 8];
-  __shared__ __align__(16) double s_val[kSameThreads * ROWS];
+                      double* __restrict__ ypart, double* __restrict__ Y, int* __restrict__ err) {
+  constexpr int ROWS = kBlkRows64, G = kMmaG, NS = kMmaStages, kWarps = kSameThreads / 32;
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[NS], empty[NS];
   const uint4 item = items[blockIdx.x];  // block, union range, partial slot
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t c0 = ((size_t)blockIdx.y * (kSameThreads / 32) + warp) * (64 * P) + 2 * lane;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   // columns up to ncol rounded up to 8: the rows' padding, never another range's columns
-  const size_t lim = (ncol + 7) & ~(size_t)7;
-  const bool active = c0 - 2 * lane < ncol;  // warp-uniform
-  bool in[P];
-#pragma unroll
-  for (int p = 0; p < P; ++p) in[p] = c0 + 64 * p < lim;
-  const double* xc = X + c0;
-  double acc[ROWS][P][2];
-#pragma unroll
-  for (int k = 0; k < ROWS; ++k)
-#pragma unroll
-    for (int p = 0; p < P; ++p) acc[k][p][0] = acc[k][p][1] = 0.0;
-  auto load = [&](uint32_t kt, double2 (&o)[P]) {
-    const double* x = xc + (size_t)kt * ldx;
-#pragma unroll
-    for (int p = 0; p < P; ++p)
-      o[p] = in[p] ? __ldg(reinterpret_cast<const double2*>(x + 64 * p)) : make_double2(0.0, 0.0);
+  const size_t lim = (ncol + 7) & ~(size_t)7, s0 = (size_t)blockIdx.y * kMmaCols, cw = s0 + 16 * kMmaI * warp;
+  const bool active = cw < ncol;  // warp-uniform
+  const int n_stage = (int)((item.z - item.y) / G);  // the unions are padded to 8 entries
+  const uint64_t beg = uoff[item.x] + item.y;
+  const uint32_t r = brows[item.x * ROWS + g];
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < NS; ++k) {
+      mbar_init(&full[k], 1);
+      mbar_init(&empty[k], kWarps);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  // stage k's copies (G strips and their values) by one warp; kt: the lane's ket
+  const uint32_t bytes = (uint32_t)(min((size_t)kMmaCols, lim - s0) * sizeof(double));
+  constexpr uint32_t vbytes = G * ROWS * sizeof(double);
+  auto tile = [&](int b) { return reinterpret_cast<double*>(smem + b * kMmaStageBytes); };
+  auto fill_ket = [&](int k) { return lane < G ? __ldg(uket + beg + (uint64_t)k * G + lane) : 0u; };
+  auto fill = [&](int k, int b, uint32_t kt) {
+    if (lane == 0) mbar_arrive_expect_tx(&full[b], G * bytes + vbytes);
+    __syncwarp();
+    if (lane < G) tma_load_1d(tile(b) + (size_t)lane * kMmaPitch, X + (size_t)kt * ldx + s0, bytes, &full[b]);
+    else if (lane == G) tma_load_1d(tile(b) + (size_t)G * kMmaPitch, uval + (beg + (uint64_t)k * G) * ROWS, vbytes, &full[b]);
   };
-  const uint64_t ub = uoff[item.x];
-  const uint64_t beg = ub + item.y, end = ub + item.z;
-  for (uint64_t base = beg; base < end; base += kSameThreads) {
-    const int cnt = (int)min((uint64_t)kSameThreads, end - base);  // a multiple of 8
-    stage_union<ROWS>(s_ket, s_val, uket, uval, base, cnt);
-    if (!active) continue;
-    double2 x[kAhead][P];
+  if (warp == 0)
+    for (int k = 0; k < min(NS, n_stage); ++k) fill(k, k, fill_ket(k));
+  double acc[kMmaI][2][2];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) load(s_ket[u], x[u]);
-#pragma unroll 1
-    for (int e0 = 0; e0 < cnt; e0 += 8) {
+  for (int i = 0; i < kMmaI; ++i) acc[i][0][0] = acc[i][0][1] = acc[i][1][0] = acc[i][1][1] = 0.0;
+  int b = 0, last = NS - 1;  // buffers of stages k and k - 1
+  uint32_t ph = 0, lph = 1;  // parities of their phases
+  for (int k = 0; k < n_stage; ++k) {
+    // warp k mod 8 refills the buffer of stage k - 1, which the others have
+    // finished or are about to
+    const bool mine = k > 0 && k - 1 + NS < n_stage && warp == (k & (kWarps - 1));
+    const uint32_t kt = mine ? fill_ket(k - 1 + NS) : 0u;
+    bool ok = mbar_wait_polls(&full[b], ph);
+    if (ok) {
+      if (active) {
+        const double* x = tile(b) + (size_t)q * kMmaPitch + 16 * kMmaI * warp + 2 * g;
+        const double* w = tile(b) + (size_t)G * kMmaPitch + lane;
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int e = e0 + u;
-        const double* w = s_val + e * ROWS;
+        for (int u = 0; u < G / 4; ++u) {
+          const double a = w[4 * ROWS * u];
+          double2 xv[kMmaI];
 #pragma unroll
-        for (int k = 0; k < ROWS; k += 2) {
-          const double2 wk = *reinterpret_cast<const double2*>(w + k);
+          for (int i = 0; i < kMmaI; ++i) xv[i] = *reinterpret_cast<const double2*>(x + (size_t)4 * u * kMmaPitch + 16 * i);
 #pragma unroll
-          for (int p = 0; p < P; ++p) {
-            acc[k][p][0] = fma(wk.x, x[u % kAhead][p].x, acc[k][p][0]);
-            acc[k][p][1] = fma(wk.x, x[u % kAhead][p].y, acc[k][p][1]);
-            acc[k + 1][p][0] = fma(wk.y, x[u % kAhead][p].x, acc[k + 1][p][0]);
-            acc[k + 1][p][1] = fma(wk.y, x[u % kAhead][p].y, acc[k + 1][p][1]);
+          for (int i = 0; i < kMmaI; ++i) {
+            dmma_m8n8k4(acc[i][0], a, xv[i].x);
+            dmma_m8n8k4(acc[i][1], a, xv[i].y);
           }
         }
-        load(s_ket[min(e + kAhead, cnt - 1)], x[u % kAhead]);
       }
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&empty[b])) : "memory");
+      if (mine) ok = mbar_wait_polls(&empty[last], lph);
     }
+    if (!__all_sync(0xffffffffu, ok)) {  // flag it; the copies in flight land before shared memory is given up
+      if (lane == 0) atomicExch(err, kErrWatchdogSame);
+      for (int j = k; j < min(k + NS, n_stage); ++j) mbar_wait_polls(&full[j % NS], (uint32_t)((j / NS) & 1));
+      break;
+    }
+    if (mine) fill(k - 1 + NS, last, kt);
+    last = b;
+    lph = ph;
+    if (++b == NS) { b = 0; ph ^= 1; }
   }
-  if (Dt != nullptr && item.y == 0 && active) {
+  bool on[kMmaI];
 #pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-      const uint32_t r = brows[item.x * ROWS + k];
-      if (r == kNoRow) continue;
-      const uint64_t e0 = off[r];
-      const int ns = (int)nsing[r];
-#pragma unroll 4
-      for (int s = 0; s < ns; ++s) {
-        const uint32_t inf = __ldg(info + e0 + s);
-        const double* d = Dt + (size_t)((inf >> 12) & 0xfffu) * dstride + c0;
-        double2 x[P];
-        load(__ldg(ket + e0 + s), x);
+  for (int i = 0; i < kMmaI; ++i) on[i] = active && cw + 16 * i + 4 * q < lim;
+  // columns 4 q .. 4 q + 3 of each i: {even tile, odd tile} x {0, 1}
+  double* y = (item.w ? ypart + ((size_t)(item.w - 1) * ROWS + g) * ldx : Y + (size_t)r * ldx) + cw;
+  if (item.w || r != kNoRow) {
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-          const double2 dv = in[p] ? __ldg(reinterpret_cast<const double2*>(d + 64 * p)) : make_double2(0.0, 0.0);
-          acc[k][p][0] = fma(flip_sign(dv.x, inf >> 31), x[p].x, acc[k][p][0]);
-          acc[k][p][1] = fma(flip_sign(dv.y, inf >> 31), x[p].y, acc[k][p][1]);
-        }
+    for (int i = 0; i < kMmaI; ++i)
+      if (on[i]) {
+        double2* o = reinterpret_cast<double2*>(y + 16 * i + 4 * q);
+        o[0] = make_double2(acc[i][0][0], acc[i][1][0]);
+        o[1] = make_double2(acc[i][0][1], acc[i][1][1]);
       }
-    }
-  }
-  if (active) {
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-      const uint32_t r = brows[item.x * ROWS + k];
-      if (item.w == 0 && r == kNoRow) continue;
-      double* y = (item.w ? ypart + ((size_t)(item.w - 1) * ROWS + k) * ldx : Y + (size_t)r * ldx) + c0;
-#pragma unroll
-      for (int p = 0; p < P; ++p)
-        if (in[p]) *reinterpret_cast<double2*>(y + 64 * p) = make_double2(acc[k][p][0], acc[k][p][1]);
-    }
   }
   if (item.w == 0) return;
   const uint32_t sq = slot_split[item.w - 1];
   const uint4 sp = split[sq];
-  if (!last_part(done, (size_t)sq * gridDim.y + blockIdx.y, sp.z) || !active) return;
-  for (int k = 0; k < ROWS; ++k) {
-    const uint32_t r = brows[item.x * ROWS + k];
-    if (r == kNoRow) continue;
-    for (int p = 0; p < P; ++p) {
-      if (c0 + 64 * p >= lim) continue;
-      double2 t = make_double2(0.0, 0.0);
-      for (uint32_t z = 0; z < sp.z; ++z) {
-        const double2 u = __ldcg(reinterpret_cast<const double2*>(ypart + ((size_t)(sp.y + z) * ROWS + k) * ldx + c0 + 64 * p));
-        t.x += u.x;
-        t.y += u.y;
-      }
-      *reinterpret_cast<double2*>(Y + (size_t)r * ldx + c0 + 64 * p) = t;
+  if (!last_part(done, (size_t)sq * gridDim.y + blockIdx.y, sp.z) || r == kNoRow) return;
+  for (int i = 0; i < kMmaI; ++i) {
+    const size_t c = cw + 16 * i + 4 * q;
+    if (!on[i]) continue;
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    for (uint32_t p = 0; p < sp.z; ++p) {
+      const double2* o = reinterpret_cast<const double2*>(ypart + ((size_t)(sp.y + p) * ROWS + g) * ldx + c);
+      const double2 u = __ldcg(o), v = __ldcg(o + 1);
+      t[0] += u.x; t[1] += u.y; t[2] += v.x; t[3] += v.y;
     }
+    double2* o = reinterpret_cast<double2*>(Y + (size_t)r * ldx + c);
+    o[0] = make_double2(t[0], t[1]);
+    o[1] = make_double2(t[2], t[3]);
   }
 }
 
@@ -1508,13 +1616,14 @@ sigma_same_blk_kernel(const double* __restrict__ X, size_t ncol, size_t ldx, con
 // kRun union entries (or of kRun singles), each run's sum added to the FP64
 // row accumulator. The unions are padded to whole runs, so the run's ket
 // strips are all loaded before the first product and no product is guarded.
+// Four strings: a ket value is converted once for four products, which the FP32
+// pipe then bounds; the tensor pipe has no FP32 type without a loss of bits.
+// 8000 x 8000: 3.3 ms for the beta side (4.4 ms with the singles in lists of
+// their own and with guarded products; 4.3 ms with the strips brought by TMA).
 template <int VEC>
 __global__ void __launch_bounds__(kSameThreads, 3)
-sigma_same_blkf_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
-                       const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
-                       const uint32_t* __restrict__ info, const float* __restrict__ Dt, size_t dstride,
-                       const uint32_t* __restrict__ brows,
-                       const uint64_t* __restrict__ uoff, const uint32_t* __restrict__ uket,
+sigma_same_blkf_kernel(const float* __restrict__ X, size_t ncol, size_t ldx,
+                       const uint32_t* __restrict__ brows, const uint64_t* __restrict__ uoff, const uint32_t* __restrict__ uket,
                        const float* __restrict__ uval, const uint4* __restrict__ items,
                        const uint4* __restrict__ split, const uint32_t* __restrict__ slot_split,
                        uint32_t* __restrict__ done, double* __restrict__ ypart, double* __restrict__ Y) {
@@ -1557,32 +1666,6 @@ sigma_same_blkf_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, con
       for (int k = 0; k < ROWS; ++k)
 #pragma unroll
         for (int v = 0; v < VEC; ++v) acc[k][v] += (double)pf[k][v];
-    }
-  }
-  if (Dt != nullptr && item.y == 0 && active) {
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k) {
-      const uint32_t r = brows[item.x * ROWS + k];
-      if (r == kNoRow) continue;
-      const uint64_t e0 = off[r];
-      const int ns = (int)nsing[r];
-      for (int s0 = 0; s0 < ns; s0 += kRun) {
-        const int s1 = min(s0 + kRun, ns);
-        float pf[VEC];
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) pf[v] = 0.f;
-#pragma unroll 4
-        for (int s = s0; s < s1; ++s) {
-          const uint32_t inf = __ldg(info + e0 + s);
-          float x[VEC], d[VEC];
-          VecF<VEC>::load(xc + (size_t)__ldg(ket + e0 + s) * ldx, x);
-          VecF<VEC>::load(Dt + (size_t)((inf >> 12) & 0xfffu) * dstride + c0, d);
-#pragma unroll
-          for (int v = 0; v < VEC; ++v) pf[v] = fmaf((inf >> 31) ? -d[v] : d[v], x[v], pf[v]);
-        }
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) acc[k][v] += (double)pf[v];
-      }
     }
   }
   if (active) {
@@ -1883,7 +1966,13 @@ __device__ __forceinline__ void ab_sweep(const AbArgs<T>& a, const typename RowP
 // group hold 10 (FP64) or 20 (FP32) alpha singles instead of the 2 or 4 whose
 // ket rows of 8000 strings fit, and replaces the ket gather of every pair by
 // registers: per record of a group one 16-byte gather per pack and one
-// read-add-write of y, against two 16-byte gathers per pack.
+// read-add-write of y, against two 16-byte gathers per pack. The pipe is 78% busy
+// at 8000 x 8000 (62% at 613 x 1187). 8000 x 8000: 17.4 -> 13.6 ms FP64, 9.6 ->
+// 8.4 ms FP32. Measured and not taken: a barrier per step instead of the
+// mbarrier (13.8 against 12.9 ms at the time), ket strings sorted by string or
+// pair indices spread over the banks by the schedule (no change), the Coulomb
+// terms of the alpha singles here (5.5 ms more), the first ket values loaded
+// before the integrals are staged (no change FP64, 0.2 ms more FP32).
 template <typename T, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
   using RP = RowPack<T>;
@@ -2063,59 +2152,55 @@ int launch_same_v6(Ctx* c, const T* X, size_t ncol, size_t ldx, const Conn& cn, 
   return 0;
 }
 
-template <int P>
-int launch_same_blkd(Ctx* c, const double* X, size_t ncol, size_t ldx, const Conn& cn, const double* Dt, size_t dstride,
-                     double* Y) {
-  const SameBlocks& B = cn.blk[0];
-  constexpr size_t cols = (size_t)kSameThreads * 2 * P;
-  const dim3 grid((unsigned)B.n_item, (unsigned)((ncol + cols - 1) / cols));
-  sigma_same_blk_kernel<P><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, cn.off, cn.nsing, cn.ket, cn.info, Dt,
-                                                                 dstride, B.rows, B.uoff, B.uket, B.uval, B.item, B.split,
-                                                                 B.slot, B.done, B.ypart, Y);
+int launch_same_blk(Ctx* c, int, const double* X, size_t ncol, size_t ldx, const SameBlocks& B, double* Y) {
+  constexpr size_t smem = kMmaStageBytes * kMmaStages;
+  SBDX_CUDA(c, cudaFuncSetAttribute(sigma_same_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const dim3 grid((unsigned)B.n_item, (unsigned)((ncol + kMmaCols - 1) / kMmaCols));
+  sigma_same_mma_kernel<<<grid, kSameThreads, smem, c->stream>>>(X, ncol, ldx, B.rows, B.uoff, B.uket, B.uval, B.item,
+                                                                 B.split, B.slot, B.done, B.ypart, Y, c->d_err);
   SBDX_LAUNCHED(c);
   return 0;
 }
 
-int launch_same_blk(Ctx* c, int vec, const double* X, size_t ncol, size_t ldx, const Conn& cn, const double* Dt,
-                    size_t dstride, double* Y) {
-  if (vec >= 4) return launch_same_blkd<2>(c, X, ncol, ldx, cn, Dt, dstride, Y);
-  return launch_same_blkd<1>(c, X, ncol, ldx, cn, Dt, dstride, Y);
-}
-
 template <int VEC>
-int launch_same_blkf(Ctx* c, const float* X, size_t ncol, size_t ldx, const Conn& cn, const float* Dt, size_t dstride,
-                     double* Y) {
-  const SameBlocks& B = cn.blk[1];
+int launch_same_blkf(Ctx* c, const float* X, size_t ncol, size_t ldx, const SameBlocks& B, double* Y) {
   const dim3 grid((unsigned)B.n_item, (unsigned)((ncol + (size_t)kSameThreads * VEC - 1) / ((size_t)kSameThreads * VEC)));
-  sigma_same_blkf_kernel<VEC><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, cn.off, cn.nsing, cn.ket, cn.info, Dt,
-                                                                    dstride, B.rows, B.uoff, B.uket, B.uval32, B.item,
+  sigma_same_blkf_kernel<VEC><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, B.rows, B.uoff, B.uket, B.uval32, B.item,
                                                                     B.split, B.slot, B.done, B.ypart, Y);
   SBDX_LAUNCHED(c);
   return 0;
 }
 
-int launch_same_blk(Ctx* c, int vec, const float* X, size_t ncol, size_t ldx, const Conn& cn, const float* Dt,
-                    size_t dstride, double* Y) {
-  if (vec >= 4) return launch_same_blkf<4>(c, X, ncol, ldx, cn, Dt, dstride, Y);
-  if (vec == 2) return launch_same_blkf<2>(c, X, ncol, ldx, cn, Dt, dstride, Y);
-  return launch_same_blkf<1>(c, X, ncol, ldx, cn, Dt, dstride, Y);
+int launch_same_blk(Ctx* c, int vec, const float* X, size_t ncol, size_t ldx, const SameBlocks& B, double* Y) {
+  if (vec >= 4) return launch_same_blkf<4>(c, X, ncol, ldx, B, Y);
+  if (vec == 2) return launch_same_blkf<2>(c, X, ncol, ldx, B, Y);
+  return launch_same_blkf<1>(c, X, ncol, ldx, B, Y);
 }
 
 // Same-spin codes: 21, 22, 24, 28 = 1, 2, 4, 8 columns per thread of the
 // one-string kernels, narrowed to the widest vector that divides the row
 // stride and keeps 16-byte alignment (the internal vectors have strides
 // padded to 8 elements, so only a misaligned base narrows). 31, 32, 34, 38:
-// the blocked kernels with 2 or 4 (FP64), 1, 2 or 4 (FP32) columns per thread;
-// they leave the diagonal out, so with hii (an unpacked alpha-beta code) the one-string kernels run.
+// the blocked kernels, whose FP64 form has one shape (128 columns per warp) and
+// whose FP32 form takes up to 4 columns per thread; they leave the diagonal out, so with hii (an unpacked alpha-beta code) the one-string kernels run.
 template <typename T>
-int run_same_v6(Ctx* c, int code, const T* X, size_t ncol, size_t ldx, const Conn& cn,
+int run_same_v6(Ctx* c, int code, const T* X, size_t ncol, size_t ldx, const Conn& cn, size_t row0, size_t nrow,
                 const typename Prec<T>::V* val, const typename Prec<T>::V* Dt, size_t dstride, const double* hii,
                 double* Y) {
   int vec = code % 10;
   const bool aligned = (reinterpret_cast<uintptr_t>(X) % 16) == 0;
   while (vec > 1 && (!aligned || ldx % vec != 0 || (Dt != nullptr && dstride % vec != 0))) vec >>= 1;
-  if (code / 10 == 3 && cn.blk[0].nblk > 0 && hii == nullptr && aligned)
-    return launch_same_blk(c, vec, X, ncol, ldx, cn, Dt, dstride, Y);
+  if (code / 10 == 3 && cn.blk[0].nblk > 0 && hii == nullptr && aligned) {
+    const int rc = launch_same_blk(c, vec, X, ncol, ldx, cn.blk[std::is_same<T, double>::value ? 0 : 1], Y);
+    if (rc || Dt == nullptr || nrow == 0) return rc;
+    // the singles' Coulomb terms
+    constexpr size_t cols = (size_t)kSameThreads * 16 / sizeof(T);
+    const dim3 grid((unsigned)nrow, (unsigned)((ncol + cols - 1) / cols));
+    sigma_coulomb_kernel<T><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, row0, cn.off, cn.nsing, cn.ket, cn.info,
+                                                                  Dt, dstride, Y);
+    SBDX_LAUNCHED(c);
+    return 0;
+  }
   if (vec >= 8) return launch_same_v6<T, 8>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
   if (vec >= 4) return launch_same_v6<T, 4>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
   if (vec == 2) return launch_same_v6<T, 2>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
@@ -2267,9 +2352,9 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
     SideBySide f(c);
     if ((rc = f.fork())) return rc;
     f.on(0);
-    rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, valA, DtA, c->db_stride, nullptr, c->d_y);
+    rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, nullptr, c->d_y);
     f.on(1);
-    if (!rc) rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, valB, DtB, c->da_stride, nullptr, c->d_yt);
+    if (!rc) rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, nullptr, c->d_yt);
     f.main();
     if (!rc) rc = run_ab_packed<T>(c);
     const int rj = f.join();
@@ -2277,11 +2362,11 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
     return launch_combine<T>(c, X, 0, na, S, true);
   }
   mark(1);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, valA, DtA, c->db_stride, packed ? nullptr : c->d_hii,
+  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, packed ? nullptr : c->d_hii,
                            c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, valB, DtB, c->da_stride, nullptr, c->d_yt)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, nullptr, c->d_yt)))
     return rc;
   mark(3);
   if ((rc = run_ab_v6<T>(c, tune.ab_code, xp))) return rc;
@@ -2353,12 +2438,12 @@ int run_sigma_v5(Ctx* c, const T* X, T* S) {
   return 0;
 }
 
-// Default launch codes: the alpha-first kernels; the blocked same-spin kernel
-// above a size where its four-strings-per-CTA grid still fills the GPU, the
-// one-string-per-CTA kernel below it. Crossovers measured on B200 over the
-// 64 subspaces of the batched workload and the 400x400 to 8000x8000
-// workloads: FP64 about 2 M determinants (code 32 against 22), FP32 about
-// 1 M (code 34 against 24).
+// Default launch codes: the alpha-first kernels; the blocked same-spin kernels
+// above a size where the grid of their blocks still fills the GPU and the
+// strings of a block share excitations, the one-string-per-CTA kernel below it.
+// Measured on both sides of the lines (alpha and beta same-spin, us): FP64,
+// 2000 x 2000: 278 and 205 blocked, 385 and 351 by strings; FP32, 613 x 1187:
+// 97 and 44 blocked, 58 and 47 by strings.
 Tune default_tune(const Ctx* c, bool f64) {
   const size_t D = c->na * c->nb;
   if (f64) return D >= kBlkMinDets64 ? Tune{34, 71} : Tune{22, 71};
@@ -2423,10 +2508,10 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
   if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, true))) return rc;
   mark(1);
   if (nr == 0) return 0;
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ra, valA, Db, c->db_stride, nullptr, c->d_y)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ra, a0, nr, valA, Db, c->db_stride, nullptr, c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt + a0, nr, c->xsb, cb, valB, (const V*)nullptr, 0, nullptr,
+  if ((rc = run_same_v6<T>(c, tune.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, valB, (const V*)nullptr, 0, nullptr,
                            c->d_yt + a0)))
     return rc;
   mark(3);
@@ -2833,7 +2918,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
     SBDX_CUDA(c, cudaStreamWaitEvent(c->stream, ev[i], 0));
     if ((rc = launch_split<double>(c, din, a0, nr, xp, xpt, true))) return rc;
-    if ((rc = run_same_v6<double>(c, t.same_code, xpt + a0, nr, c->xsb, cb, cb.val, (const double*)nullptr, 0, nullptr,
+    if ((rc = run_same_v6<double>(c, t.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, cb.val, (const double*)nullptr, 0, nullptr,
                                   c->d_yt + a0)))
       return rc;
   }
@@ -2854,7 +2939,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     ra.n_same_split = it.n_same_split;
     ra.n_same_part = it.n_same_part;
     ra.same_ypart = it.same_ypart;
-    if ((rc = run_same_v6<double>(c, t.same_code, xp, nb, c->xsa, ra, ca.val, c->d_Db, c->db_stride, nullptr, c->d_y)))
+    if ((rc = run_same_v6<double>(c, t.same_code, xp, nb, c->xsa, ra, a0, nr, ca.val, c->d_Db, c->db_stride, nullptr, c->d_y)))
       return rc;
     if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true))) return rc;
     SBDX_CUDA(c, cudaEventRecord(ev[n + i], c->stream));

@@ -335,6 +335,31 @@ __global__ void finalize_kernel(const double* __restrict__ partial, int nblk, do
   if (threadIdx.x == 0) out[k] = t;
 }
 
+// The end of a reduction kernel with at most a few sums: the last CTA to arrive
+// adds the CTA partials of every row in the order of finalize_kernel (one
+// launch less per sum: a step of a small solve is bound by its launches; a
+// full solve at 400 x 400: 9.9 -> 9.4 ms, five roots: 30.5 -> 28.5 ms). ctr
+// is zero between launches; with out null the partials are left as they are.
+__device__ __forceinline__ void finish_sums(const double* partial, int rows, double* out, uint32_t* ctr, double* sh) {
+  if (out == nullptr) return;
+  __shared__ int s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(ctr, 1u) + 1 == gridDim.x;
+    if (s_last) *ctr = 0;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int k = 0; k < rows; ++k) {
+    double v = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) v += __ldcg(partial + (size_t)k * gridDim.x + b);
+    const double t = block_sum(v, sh);
+    if (threadIdx.x == 0) out[k] = t;
+  }
+}
+
 // W = u0*W0 + sum_k u[k] C_k ;  R = E0*W - (u0*HW0 + sum_k u[k] HC_k)
 // (W0/HW0 optional FP64 anchor). partial norms of W (slot 0) and R (slot 1).
 template <typename TV>
@@ -342,7 +367,7 @@ __global__ void __launch_bounds__(kRedThreads)
 combine_kernel(const TV* __restrict__ C, const TV* __restrict__ HC, size_t ldv, int m,
                const double* __restrict__ u, const double* __restrict__ W0, const double* __restrict__ HW0,
                double u0, const double* __restrict__ E0p, size_t D, double* __restrict__ W,
-               double* __restrict__ R, double* __restrict__ partial) {
+               double* __restrict__ R, double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   __shared__ double su[64];
   for (int k = threadIdx.x; k < m; k += blockDim.x) su[k] = u[k];
@@ -397,6 +422,7 @@ combine_kernel(const TV* __restrict__ C, const TV* __restrict__ HC, size_t ldv, 
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
   t = block_sum(nr, sh);
   if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = t;
+  finish_sums(partial, 2, out, ctr, sh);
 }
 
 // v = (R / |R|) / (E0 - d) with the reference guard (davidson.h:855-862);
@@ -405,7 +431,7 @@ template <typename TV>
 __global__ void __launch_bounds__(kRedThreads)
 precond_kernel(const double* R, const double* __restrict__ dii, const double* __restrict__ E0p,
                const double* __restrict__ nrm2, size_t D, double* v, const TV* __restrict__ V0,
-               const double* __restrict__ V0d, double* __restrict__ partial) {
+               const double* __restrict__ V0d, double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   const double E0 = *E0p;
   const double inv = 1.0 / sqrt(*nrm2);
@@ -436,13 +462,15 @@ precond_kernel(const double* R, const double* __restrict__ dii, const double* __
   }
   const double t = block_sum(acc, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  finish_sums(partial, 1, out, ctr, sh);
 }
 
 // v -= olap * Vk ; partial <Vn, v> (Vn = next basis vector) or <v, v> if Vn null.
 template <typename TV>
 __global__ void __launch_bounds__(kRedThreads)
 axpy_dot_kernel(double* __restrict__ v, const TV* __restrict__ Vk, const double* __restrict__ Vkd,
-                const double* __restrict__ olap_p, const TV* __restrict__ Vn, size_t D, double* __restrict__ partial) {
+                const double* __restrict__ olap_p, const TV* __restrict__ Vn, size_t D, double* __restrict__ partial,
+                double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   const double olap = -(*olap_p);
   double acc = 0.0;
@@ -473,6 +501,7 @@ axpy_dot_kernel(double* __restrict__ v, const TV* __restrict__ Vk, const double*
   }
   const double t = block_sum(acc, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  finish_sums(partial, 1, out, ctr, sh);
 }
 
 // out = (TV)(v / sqrt(nrm2))
@@ -486,7 +515,7 @@ __global__ void scale_store_kernel(const TI* v, const double* __restrict__ nrm2,
 // r = HW - E W (FP64), partial |r|^2
 __global__ void __launch_bounds__(kRedThreads)
 residual_kernel(const double* __restrict__ W, const double* __restrict__ HW, const double* __restrict__ Ep,
-                size_t D, double* __restrict__ r, double* __restrict__ partial) {
+                size_t D, double* __restrict__ r, double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   const double E = *Ep;
   double acc = 0.0;
@@ -497,6 +526,7 @@ residual_kernel(const double* __restrict__ W, const double* __restrict__ HW, con
   }
   const double t = block_sum(acc, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  finish_sums(partial, 1, out, ctr, sh);
 }
 
 // ---- host symmetric eigensolver (stand-in for LAPACK dsyev 'V','U') ---------
@@ -556,6 +586,7 @@ struct Work {
   double* partial = nullptr;  // reduction partials
   double* scal = nullptr;     // device scalars
   double* u = nullptr;        // Ritz coefficients
+  uint32_t* ctr = nullptr;    // arrivals of finish_sums
 };
 
 // A solve's device buffers, released on its stream; the pool keeps a bounded
@@ -675,10 +706,8 @@ int expand(Ctx* c, Work& wk, const double* R, const double* Wd, const TV* V, int
   double* s = wk.scal;
   // the first basis vector is the FP64 anchor when Wd != null
   precond_kernel<TV><<<kRedBlocks, kRedThreads, 0, c->stream>>>(R, c->d_hii, s + kE0, s + kNR, D, v,
-                                                                Wd ? nullptr : V, Wd, wk.partial);
+                                                                Wd ? nullptr : V, Wd, wk.partial, s + kOlap, wk.ctr);
   SBDX_LAUNCHED(c);
-  int rc = finalize(c, wk, 1, s + kOlap);
-  if (rc) return rc;
   const int nbasis = nv + (Wd ? 1 : 0);
   for (int k = 0; k < nbasis; ++k) {
     const bool anchor = Wd && k == 0;
@@ -686,10 +715,8 @@ int expand(Ctx* c, Work& wk, const double* R, const double* Wd, const TV* V, int
     const TV* vk = anchor ? nullptr : V + (size_t)vi * D;
     const TV* vn = (k + 1 < nbasis) ? V + (size_t)(Wd ? k : k + 1) * D : nullptr;
     axpy_dot_kernel<TV><<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, vk, anchor ? Wd : nullptr, s + kOlap, vn, D,
-                                                                   wk.partial);
+                                                                   wk.partial, vn ? s + kOlap : s + kNV, wk.ctr);
     SBDX_LAUNCHED(c);
-    rc = finalize(c, wk, 1, vn ? s + kOlap : s + kNV);
-    if (rc) return rc;
   }
   scale_store_kernel<TV, double><<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, s + kNV, D, dst);
   SBDX_LAUNCHED(c);
@@ -710,6 +737,8 @@ int davidson_fp64(Ctx* c, const sbdx_davidson_params& p, double* dW, sbdx_davids
   SBDX_CUDA(c, g.get(&wk.partial, sizeof(double) * kRedBlocks * (nb + 2)));
   SBDX_CUDA(c, g.get(&wk.scal, sizeof(double) * (kDots + 2 * nb + 16)));
   SBDX_CUDA(c, g.get(&wk.u, sizeof(double) * (nb + 1)));
+  SBDX_CUDA(c, g.get(&wk.ctr, sizeof(uint32_t)));
+  SBDX_CUDA(c, cudaMemsetAsync(wk.ctr, 0, sizeof(uint32_t), c->stream));
   double *C = nullptr, *HC = nullptr, *R = nullptr;
   SBDX_CUDA(c, g.get(&C, sizeof(double) * D * nb));
   SBDX_CUDA(c, g.get(&HC, sizeof(double) * D * nb));
@@ -741,9 +770,8 @@ int davidson_fp64(Ctx* c, const sbdx_davidson_params& p, double* dW, sbdx_davids
       SBDX_CUDA(c, cudaMemcpyAsync(wk.u, up.data(), sizeof(double) * (ib + 1), cudaMemcpyHostToDevice, c->stream));
       SBDX_CUDA(c, cudaMemcpyAsync(s + kE0, &E[0], sizeof(double), cudaMemcpyHostToDevice, c->stream));
       combine_kernel<double><<<kRedBlocks, kRedThreads, 0, c->stream>>>(C, HC, D, ib + 1, wk.u, nullptr, nullptr,
-                                                                        0.0, s + kE0, D, dW, R, wk.partial);
+                                                                        0.0, s + kE0, D, dW, R, wk.partial, s + kNW, wk.ctr);
       SBDX_LAUNCHED(c);
-      if ((rc = finalize(c, wk, 2, s + kNW))) return rc;
       double nrm[2];
       SBDX_CUDA(c, cudaMemcpyAsync(nrm, s + kNW, sizeof(double) * 2, cudaMemcpyDeviceToHost, c->stream));
       SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -854,7 +882,7 @@ __device__ __forceinline__ double precond_inv(double E0, double d) {
 __global__ void __launch_bounds__(kRedThreads)
 olsen_precond_kernel(const double* __restrict__ R, const double* __restrict__ W, const double* __restrict__ dii,
                      const double* __restrict__ E0p, const double* __restrict__ nr2, size_t D, double* __restrict__ v,
-                     double* __restrict__ partial) {
+                     double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   const double E0 = *E0p;
   const double inv = 1.0 / sqrt(*nr2);
@@ -887,6 +915,7 @@ olsen_precond_kernel(const double* __restrict__ R, const double* __restrict__ W,
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
   t = block_sum(b, sh);
   if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = t;
+  finish_sums(partial, 2, out, ctr, sh);
 }
 
 // Pass 2: v -= (a/b) P W, so that v is orthogonal to W; partial <W, v> (about
@@ -894,7 +923,7 @@ olsen_precond_kernel(const double* __restrict__ R, const double* __restrict__ W,
 __global__ void __launch_bounds__(kRedThreads)
 olsen_apply_kernel(double* __restrict__ v, const double* __restrict__ W, const double* __restrict__ dii,
                    const double* __restrict__ E0p, const double* __restrict__ ab, size_t D,
-                   double* __restrict__ partial) {
+                   double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   const double E0 = *E0p;
   const double eps = ab[1] != 0.0 ? ab[0] / ab[1] : 0.0;
@@ -925,13 +954,14 @@ olsen_apply_kernel(double* __restrict__ v, const double* __restrict__ W, const d
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
   t = block_sum(nn, sh);
   if (threadIdx.x == 0) partial[gridDim.x + blockIdx.x] = t;
+  finish_sums(partial, 2, out, ctr, sh);
 }
 
 // Classical Gram-Schmidt update: v -= o[0] W + sum_k o[k+1] V_k; partial |v|^2.
 template <typename TV>
 __global__ void __launch_bounds__(kRedThreads)
 gs_subtract_kernel(double* __restrict__ v, const double* __restrict__ W, const TV* __restrict__ V, size_t ldv, int m,
-                   const double* __restrict__ o, size_t D, double* __restrict__ partial) {
+                   const double* __restrict__ o, size_t D, double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   __shared__ double so[65];
   for (int k = threadIdx.x; k <= m; k += blockDim.x) so[k] = o[k];
@@ -963,6 +993,7 @@ gs_subtract_kernel(double* __restrict__ v, const double* __restrict__ W, const T
   }
   const double t = block_sum(nn, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  finish_sums(partial, 1, out, ctr, sh);
 }
 
 // Expansion vector of the mixed solver: Olsen-corrected preconditioned
@@ -976,21 +1007,18 @@ int expand_olsen(Ctx* c, Work& wk, const double* R, const double* W, const float
                  double* o, float* dst) {
   double* s = wk.scal;
   olsen_precond_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(R, W, c->d_hii, s + kE0, s + kNR, D, v,
-                                                                  wk.partial);
+                                                                  wk.partial, s + kAB, wk.ctr);
   SBDX_LAUNCHED(c);
-  int rc = finalize(c, wk, 2, s + kAB);
-  if (rc) return rc;
-  olsen_apply_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, W, c->d_hii, s + kE0, s + kAB, D, wk.partial);
+  int rc = 0;
+  olsen_apply_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, W, c->d_hii, s + kE0, s + kAB, D, wk.partial, s + kOlap, wk.ctr);  // kOlap = <W, v>, kNV = |v|^2
   SBDX_LAUNCHED(c);
-  if ((rc = finalize(c, wk, 2, s + kOlap))) return rc;  // kOlap = <W, v>, kNV = |v|^2
   double before = 0.0;
   SBDX_CUDA(c, cudaMemcpyAsync(&before, s + kNV, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   for (int pass = 0; pass < 2; ++pass) {
     if ((rc = multidot<double, double>(c, wk, W, D, 1, v, D, o))) return rc;
     if (nv > 0 && (rc = multidot<float, double>(c, wk, V, D, nv, v, D, o + 1))) return rc;
-    gs_subtract_kernel<float><<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, W, V, D, nv, o, D, wk.partial);
+    gs_subtract_kernel<float><<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, W, V, D, nv, o, D, wk.partial, s + kNV, wk.ctr);
     SBDX_LAUNCHED(c);
-    if ((rc = finalize(c, wk, 1, s + kNV))) return rc;
     double after = 0.0;
     SBDX_CUDA(c, cudaMemcpyAsync(&after, s + kNV, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1091,6 +1119,8 @@ int davidson_mixed(Ctx* c, const sbdx_davidson_params& p, double* dW, sbdx_david
   SBDX_CUDA(c, g.get(&wk.partial, sizeof(double) * kRedBlocks * (2 * nc + 4)));  // multidot2: 2 per vector
   SBDX_CUDA(c, g.get(&wk.scal, sizeof(double) * (kDots + 2 * nc + 16)));
   SBDX_CUDA(c, g.get(&wk.u, sizeof(double) * (nc + 2)));
+  SBDX_CUDA(c, g.get(&wk.ctr, sizeof(uint32_t)));
+  SBDX_CUDA(c, cudaMemsetAsync(wk.ctr, 0, sizeof(uint32_t), c->stream));
   float *C = nullptr, *HC = nullptr;
   double *AW = nullptr, *R = nullptr, *V = nullptr;
   SBDX_CUDA(c, g.get(&C, sizeof(float) * D * nc));
@@ -1118,9 +1148,8 @@ int davidson_mixed(Ctx* c, const sbdx_davidson_params& p, double* dW, sbdx_david
     if (r2) return r2;
     info.n_sigma64++;
     if ((r2 = multidot<double, double>(c, wk, W, D, 1, HW, D, s + kE))) return r2;
-    residual_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(W, HW, s + kE, D, R, wk.partial);
+    residual_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(W, HW, s + kE, D, R, wk.partial, s + kNR, wk.ctr);
     SBDX_LAUNCHED(c);
-    if ((r2 = finalize(c, wk, 1, s + kNR))) return r2;
     SBDX_CUDA(c, cudaMemcpyAsync(s + kE0, s + kE, sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     double h2[2];
     SBDX_CUDA(c, cudaMemcpyAsync(&h2[0], s + kE, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1292,7 +1321,7 @@ constexpr int kMaxRoots = 4;
 template <typename TV>
 __global__ void __launch_bounds__(kRedThreads)
 gs_subtract_block_kernel(double* __restrict__ v, const double* __restrict__ A, int na, const TV* __restrict__ V,
-                         int m, const double* __restrict__ o, size_t D, double* __restrict__ partial) {
+                         int m, const double* __restrict__ o, size_t D, double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   __shared__ double so[72];
   for (int k = threadIdx.x; k < na + m; k += blockDim.x) so[k] = o[k];
@@ -1328,6 +1357,7 @@ gs_subtract_block_kernel(double* __restrict__ v, const double* __restrict__ A, i
   }
   const double t = block_sum(nn, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = t;
+  finish_sums(partial, 1, out, ctr, sh);
 }
 
 // For each root r < K: W'_r = sum_a X[a][r] W_a + sum_j X[K+j][r] C_j, the same
@@ -1445,7 +1475,7 @@ update_anchors_kernel(const double* __restrict__ W, const double* __restrict__ H
 // R_r = E_r W_r - HW_r for r < k (E in device memory), partial |R_r|^2.
 __global__ void __launch_bounds__(kRedThreads)
 residual_block_kernel(const double* __restrict__ W, const double* __restrict__ HW, const double* __restrict__ E,
-                      int k, size_t D, double* __restrict__ R, double* __restrict__ partial) {
+                      int k, size_t D, double* __restrict__ R, double* __restrict__ partial, double* out, uint32_t* ctr) {
   __shared__ double sh[kRedThreads / 32];
   for (int r = 0; r < k; ++r) {
     const double e = E[r];
@@ -1458,6 +1488,7 @@ residual_block_kernel(const double* __restrict__ W, const double* __restrict__ H
     const double t = block_sum(acc, sh);
     if (threadIdx.x == 0) partial[(size_t)r * gridDim.x + blockIdx.x] = t;
   }
+  finish_sums(partial, k, out, ctr, sh);
 }
 
 // Lowest k eigenpairs of M x = theta S x (n x n, upper triangles of the ld-
@@ -1513,21 +1544,18 @@ template <typename TC>
 int expand_block(Ctx* c, Work& wk, const double* Rr, const double* Wr, const double* A, int k, const TC* V, int nv,
                  size_t D, double* v, double* o, const double* thetap, const double* nr2p, TC* dst) {
   double* s = wk.scal;
-  olsen_precond_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(Rr, Wr, c->d_hii, thetap, nr2p, D, v, wk.partial);
+  olsen_precond_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(Rr, Wr, c->d_hii, thetap, nr2p, D, v, wk.partial, s + kbAB, wk.ctr);
   SBDX_LAUNCHED(c);
-  int rc = finalize(c, wk, 2, s + kbAB);
-  if (rc) return rc;
-  olsen_apply_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, Wr, c->d_hii, thetap, s + kbAB, D, wk.partial);
+  int rc = 0;
+  olsen_apply_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, Wr, c->d_hii, thetap, s + kbAB, D, wk.partial, s + kbOlap, wk.ctr);  // kbOlap, kbNV
   SBDX_LAUNCHED(c);
-  if ((rc = finalize(c, wk, 2, s + kbOlap))) return rc;  // kbOlap, kbNV
   double before = 0.0;
   SBDX_CUDA(c, cudaMemcpyAsync(&before, s + kbNV, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   for (int pass = 0; pass < 2; ++pass) {
     if ((rc = multidot<double, double>(c, wk, A, D, k, v, D, o))) return rc;
     if (nv > 0 && (rc = multidot<TC, double>(c, wk, V, D, nv, v, D, o + k))) return rc;
-    gs_subtract_block_kernel<TC><<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, A, k, V, nv, o, D, wk.partial);
+    gs_subtract_block_kernel<TC><<<kRedBlocks, kRedThreads, 0, c->stream>>>(v, A, k, V, nv, o, D, wk.partial, s + kbNV, wk.ctr);
     SBDX_LAUNCHED(c);
-    if ((rc = finalize(c, wk, 1, s + kbNV))) return rc;
     double after = 0.0;
     SBDX_CUDA(c, cudaMemcpyAsync(&after, s + kbNV, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1594,6 +1622,8 @@ int davidson_block(Ctx* c, const sbdx_davidson_params& p, int k, double* dW, dou
   SBDX_CUDA(c, alloc((void**)&wpartial, sizeof(double) * kRedBlocks * (2 * nc + 2 * kMaxRoots + 4)));
   SBDX_CUDA(c, alloc((void**)&wscal, sizeof(double) * (kbDots + (size_t)(k + 2) * nc + 64)));
   SBDX_CUDA(c, alloc((void**)&wu, sizeof(double) * ((size_t)(k + nc) * k + k + nc + 8)));
+  SBDX_CUDA(c, alloc((void**)&wk.ctr, sizeof(uint32_t)));
+  SBDX_CUDA(c, cudaMemsetAsync(wk.ctr, 0, sizeof(uint32_t), c->stream));
   TC *C = nullptr, *HC = nullptr;
   double *A = nullptr, *R = nullptr, *V = nullptr;
   SBDX_CUDA(c, alloc((void**)&C, sizeof(TC) * D * nc));
@@ -1624,7 +1654,7 @@ int davidson_block(Ctx* c, const sbdx_davidson_params& p, int k, double* dW, dou
     for (int pass = 0; pass < 2 && r > 0; ++pass) {
       if ((rc = multidot<double, double>(c, wk, W, D, r, wr, D, gso))) return rc;
       gs_subtract_block_kernel<double><<<kRedBlocks, kRedThreads, 0, c->stream>>>(wr, W, r, (const double*)nullptr, 0,
-                                                                                gso, D, wk.partial);
+                                                                                gso, D, wk.partial, nullptr, nullptr);
       SBDX_LAUNCHED(c);
     }
     if ((rc = multidot<double, double>(c, wk, wr, D, 1, wr, D, s + kbNV))) return rc;
@@ -1661,9 +1691,8 @@ int davidson_block(Ctx* c, const sbdx_davidson_params& p, int k, double* dW, dou
       }
     for (int r = 0; r < k; ++r) h[r] = M[r + (size_t)ld * r] / S[r + (size_t)ld * r];
     SBDX_CUDA(c, cudaMemcpyAsync(s + kbTheta, h.data(), sizeof(double) * k, cudaMemcpyHostToDevice, c->stream));
-    residual_block_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(W, HW, s + kbTheta, k, D, R, wk.partial);
+    residual_block_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(W, HW, s + kbTheta, k, D, R, wk.partial, s + kbNR2, wk.ctr);
     SBDX_LAUNCHED(c);
-    if ((r2 = finalize(c, wk, k, s + kbNR2))) return r2;
     SBDX_CUDA(c, cudaMemcpyAsync(h.data() + kMaxRoots, s + kbNR2, sizeof(double) * k, cudaMemcpyDeviceToHost, c->stream));
     SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
     for (int r = 0; r < k; ++r) {
@@ -2237,6 +2266,8 @@ int davidson_block_graph(Ctx* c, const sbdx_davidson_params& p, int k, double* d
   SBDX_CUDA(c, alloc((void**)&wpartial, sizeof(double) * kRedBlocks * (2 * nc + 2 * kMaxRoots + 4)));
   SBDX_CUDA(c, alloc((void**)&wscal, sizeof(double) * (kbDots + 2 * (size_t)k * (nc + 2 * k) + 64)));
   SBDX_CUDA(c, alloc((void**)&wu, sizeof(double) * ((size_t)(k + nc) * k + k + nc + 8)));
+  SBDX_CUDA(c, alloc((void**)&wk.ctr, sizeof(uint32_t)));
+  SBDX_CUDA(c, cudaMemsetAsync(wk.ctr, 0, sizeof(uint32_t), c->stream));
   TC *C = nullptr, *HC = nullptr;
   double *A = nullptr, *R = nullptr, *V = nullptr, *dM = nullptr, *dS = nullptr, *misc = nullptr;
   int* dead = nullptr;
@@ -2281,7 +2312,7 @@ int davidson_block_graph(Ctx* c, const sbdx_davidson_params& p, int k, double* d
     for (int pass = 0; pass < 2 && r > 0; ++pass) {
       if ((rc = multidot<double, double>(c, wk, W0, D, r, wr, D, gso))) return rc;
       gs_subtract_block_kernel<double><<<kRedBlocks, kRedThreads, 0, c->stream>>>(wr, W0, r, (const double*)nullptr, 0,
-                                                                                gso, D, wk.partial);
+                                                                                gso, D, wk.partial, nullptr, nullptr);
       SBDX_LAUNCHED(c);
     }
     if ((rc = multidot<double, double>(c, wk, wr, D, 1, wr, D, s + kbNV))) return rc;
@@ -2304,9 +2335,8 @@ int davidson_block_graph(Ctx* c, const sbdx_davidson_params& p, int k, double* d
     }
     refresh_block_kernel<<<1, 64, 0, c->stream>>>(k, ld, s + kbDots, dM, dS, s + kbTheta, dst);
     SBDX_LAUNCHED(c);
-    residual_block_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(W, HW, s + kbTheta, k, D, R, wk.partial);
+    residual_block_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(W, HW, s + kbTheta, k, D, R, wk.partial, s + kbNR2, wk.ctr);
     SBDX_LAUNCHED(c);
-    if ((r2 = finalize(c, wk, k, s + kbNR2))) return r2;
     for (int r = 0; r < k && nv > 0; ++r) {
       if ((r2 = multidot<TC, double>(c, wk, C, D, nv, HW + (size_t)r * D, D, s + kbDots + (size_t)r * nv))) return r2;
       if ((r2 = multidot<TC, double>(c, wk, C, D, nv, W + (size_t)r * D, D, s + kbDots + (size_t)(k + r) * nv)))
@@ -2344,20 +2374,17 @@ int davidson_block_graph(Ctx* c, const sbdx_davidson_params& p, int k, double* d
       const double* Rr = R + (size_t)r * D;
       const double* Wr = W + (size_t)r * D;
       olsen_precond_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(Rr, Wr, c->d_hii, s + kbTheta + r,
-                                                                      s + kbNR2 + r, D, V, wk.partial);
+                                                                      s + kbNR2 + r, D, V, wk.partial, s + kbAB, wk.ctr);
       SBDX_LAUNCHED(c);
-      if ((r2 = finalize(c, wk, 2, s + kbAB))) return r2;
       olsen_apply_kernel<<<kRedBlocks, kRedThreads, 0, c->stream>>>(V, Wr, c->d_hii, s + kbTheta + r, s + kbAB, D,
-                                                                    wk.partial);
+                                                                    wk.partial, s + kbOlap, wk.ctr);  // kbOlap, kbNV
       SBDX_LAUNCHED(c);
-      if ((r2 = finalize(c, wk, 2, s + kbOlap))) return r2;  // kbOlap, kbNV
       SBDX_CUDA(c, cudaMemcpyAsync(before, s + kbNV, sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
       for (int pass = 0; pass < 2; ++pass) {
         if ((r2 = multidot<double, double>(c, wk, W, D, k, V, D, gso))) return r2;
         if (nv > 0 && (r2 = multidot<TC, double>(c, wk, C, D, nv, V, D, gso + k))) return r2;
-        gs_subtract_block_kernel<TC><<<kRedBlocks, kRedThreads, 0, c->stream>>>(V, W, k, C, nv, gso, D, wk.partial);
+        gs_subtract_block_kernel<TC><<<kRedBlocks, kRedThreads, 0, c->stream>>>(V, W, k, C, nv, gso, D, wk.partial, s + kbNV, wk.ctr);
         SBDX_LAUNCHED(c);
-        if ((r2 = finalize(c, wk, 1, s + kbNV))) return r2;
       }
       const int j = nv;
       TC* Cb = C + (size_t)j * D;

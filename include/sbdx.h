@@ -116,8 +116,9 @@ int sbdx_get_connectivity(sbdx_ctx* ctx, int spin, uint64_t* slen, uint64_t* dle
 /* Stored Hamiltonian, the reference's method 1 (chemistry/tpb/sbdiag.h:275-330:
  * makeQCham, chemistry/tpb/qcham.h:10-312, then the stored-element mult,
  * chemistry/tpb/mult.h:13-123). Builds every off-diagonal H_IJ on the device
- * (CSR over determinant rows, FP64 values with the determinant phases, 32-bit
- * columns: 12 bytes per element) after the connectivity and the diagonal;
+ * (FP64 values with the determinant phases, 8 bytes per element, in blocks of one
+ * alpha string and up to 32 beta strings that share their column lists; lists shorter
+ * than the block's longest are padded) after the connectivity and the diagonal;
  * from then on every FP64 sigma of this context (sbdx_sigma, sbdx_sigma_device
  * with SBDX_FP64, the Davidson solvers' FP64 products) is its sparse product,
  * and FP32 sigmas stay on the fly. *nnz (may be NULL) receives the number of

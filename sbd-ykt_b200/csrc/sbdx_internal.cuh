@@ -194,13 +194,20 @@ constexpr size_t pad8(size_t n) { return (n + 7) / 8 * 8; }
 constexpr int kAbPacks = 5;
 constexpr size_t kAbStaticSmem = 512;
 
-// Stored Hamiltonian (the reference's method 1): off-diagonal elements in CSR
-// over determinant rows, basis phases folded into the values (stored.cu).
+// Stored Hamiltonian (the reference's method 1): off-diagonal elements with the
+// basis phases folded in, in blocks of G determinants (ia; a slice of G beta
+// strings in the order `perm`, most single excitations first). Per block,
+// G values (one per string of the slice) for every alpha same-spin entry of
+// ia, then for every beta single and double of the slice's longest lists, then
+// for every alpha single of ia x every beta single of the slice (stored.cu).
 struct StoredH {
-  uint64_t* rowptr = nullptr;  // [D + 1]
-  uint32_t* col = nullptr;     // [nnz] determinant index ja*nb + jb
-  double* val = nullptr;       // [nnz] H_IJ
-  uint64_t nnz = 0;
+  double* val = nullptr;
+  uint64_t* rowbase = nullptr;  // [na] first value of the blocks of ia
+  uint32_t* perm = nullptr;     // [nb + 32] beta string of each position (kNoRow beyond nb)
+  uint32_t* idx = nullptr;      // [G * psd[nslice]] position of each lane's m-th excited string
+  uint32_t *psd = nullptr, *ps = nullptr;  // [nslice + 1] prefix sums of singles + doubles, of singles, per slice
+  int width = 32, nslice = 0;   // G, slices
+  uint64_t nnz = 0;             // off-diagonal elements, padding not counted
 };
 
 // Launch shape of the sigma kernels. Codes (also the C-ABI encoding):

@@ -2,44 +2,46 @@
 // The reference builds every non-zero H_IJ of its bra block as (ih, jh, hij)
 // triplets per task and thread (makeQCham, chemistry/tpb/qcham.h:10-312) and
 // multiplies with them (mult, chemistry/tpb/mult.h:13-123): Wb[ih] += hij *
-// T[jh] after Wb += hii * T. Here the matrix lives on the device in CSR form:
-//   - row I = ia*nb + ib holds, in this order, the alpha same-spin entries of
-//     ia (columns ja*nb + ib), the beta same-spin entries of ib (columns
-//     ia*nb + jb) and the alpha single x beta single pairs (columns
-//     ja*nb + jb), the same elements the on-the-fly sigma evaluates;
+// T[jh] after Wb += hii * T. Here the elements lie in blocks that share their
+// column lists:
+//   - a block is one alpha string ia and a slice of G = 32 beta strings ib, the
+//     strings with the most single excitations first so that the lists of a
+//     slice have like lengths; lane l of a warp owns row (ia, ib_l). Where the
+//     padding would be more than a quarter of the elements (few beta strings,
+//     lists of very different lengths) G is the largest power of two below that,
+//     and a warp takes 32 / G entries of the block at a time (at G = 1 nothing is
+//     padded);
+//   - its values, G per entry and one per row: the alpha same-spin entries of
+//     ia (columns (ja, ib_l): consecutive in the permuted vector), the beta
+//     singles and doubles of the slice (columns (ia, jb)), and the pairs of an
+//     alpha single of ia and a beta single (columns (ja, jb)), the same elements
+//     the on-the-fly sigma evaluates; shorter lists are padded with zeros;
+//   - the column lists are per slice (jb) and per alpha string (ja), so an
+//     element costs its 8 bytes;
 //   - the values carry the determinant phases, H_IJ = phi_I phi_J H'_IJ with
-//     H' the alpha-first-basis matrix of the sigma kernels, so the product
-//     acts on vectors in determinant order with no phase pass;
-//   - the diagonal stays in the context's hii vector;
-//   - column indices are 32-bit (at most 2^32 - 1 determinants), values
-//     FP64: 12 bytes per stored element.
-// Building it costs one count kernel, a device prefix sum and one fill kernel
-// (a warp per row, coalesced writes). The product is one warp per row, lanes
-// over the row's elements, a fixed-order shuffle sum (deterministic): HBM
-// bound on the 12 bytes per element; the vector gathers hit L2 for the
-// problem sizes a stored matrix fits.
+//     H' the alpha-first-basis matrix of the sigma kernels; the diagonal stays
+//     in the context's hii vector.
+// The product permutes the vector's columns, then a CTA per alpha string and
+// group of slices streams the values, with the vector row that the current
+// entries gather from in shared memory. Deterministic (a lane sums its row in
+// one order). Bound: HBM, 8 bytes per element, and the latency of a warp's
+// stream. 1000 x 1000 strings, 575 M elements: 1.12 ms (4.1 TB/s); as CSR, 12 bytes
+// per element, a warp per row and 32 gather wavefronts per 32 elements, 1.62 ms.
+// Tighter register bounds spill (1.7 to 2.8 ms at 4 values in flight), 16 values
+// in flight took 1.24 ms, several slices per warp 2.0 ms: the warp with the
+// longest lists holds up the others at every staged row.
 #include "sbdx.h"
 #include "sbdx_internal.cuh"
 
-#include <cub/device/device_scan.cuh>
-
+#include <algorithm>
 #include <string>
+#include <vector>
 
 namespace sbdx {
 namespace {
 
-constexpr int kStoredThreads = 256;  // 8 rows (warps) per CTA
-
-__global__ void stored_count_kernel(const uint64_t* __restrict__ a_off, const uint32_t* __restrict__ a_ns,
-                                    const uint64_t* __restrict__ b_off, const uint32_t* __restrict__ b_ns, size_t na,
-                                    size_t nb, uint64_t* __restrict__ cnt) {
-  const size_t D = na * nb;
-  for (size_t I = (size_t)blockIdx.x * blockDim.x + threadIdx.x; I <= D; I += (size_t)gridDim.x * blockDim.x) {
-    if (I == D) { cnt[D] = 0; continue; }
-    const size_t ia = I / nb, ib = I - ia * nb;
-    cnt[I] = (a_off[ia + 1] - a_off[ia]) + (b_off[ib + 1] - b_off[ib]) + (uint64_t)a_ns[ia] * b_ns[ib];
-  }
-}
+constexpr int kStoredThreads = 256;  // 8 warps
+constexpr int kStoredBatch = 8;      // values a lane has in flight
 
 // Same-spin element of entry e (first `ns` entries of the row are singles):
 // sign * (value + opposite-spin Coulomb term of a single, table row pq).
@@ -49,136 +51,181 @@ __device__ __forceinline__ double same_element(uint32_t inf, double v, bool sing
   return (inf >> 31) ? -v : v;
 }
 
+// First value of block (ia, s), in entries of G values from rowbase: the blocks
+// of ia follow each other, the entries of ia (ne of them, nas singles) per slice
+// plus the slices' own lists.
+__device__ __forceinline__ uint64_t block_entry(uint64_t ne, uint64_t nas, int s, const uint32_t* __restrict__ psd,
+                                                const uint32_t* __restrict__ ps) {
+  return ne * s + psd[s] + nas * ps[s];
+}
+
+// A warp per block.
 __global__ void __launch_bounds__(kStoredThreads)
-stored_fill_kernel(size_t na, size_t nb, const uint64_t* __restrict__ astr, const uint64_t* __restrict__ bstr,
+stored_fill_kernel(const uint64_t* __restrict__ astr, const uint64_t* __restrict__ bstr,
                    const uint64_t* __restrict__ a_off, const uint32_t* __restrict__ a_ns,
                    const uint32_t* __restrict__ a_ket, const double* __restrict__ a_val,
                    const uint32_t* __restrict__ a_info, const uint64_t* __restrict__ b_off,
                    const uint32_t* __restrict__ b_ns, const uint32_t* __restrict__ b_ket,
                    const double* __restrict__ b_val, const uint32_t* __restrict__ b_info,
                    const double* __restrict__ Da, size_t da_stride, const double* __restrict__ Db, size_t db_stride,
-                   const double* __restrict__ V, size_t vstride, const uint64_t* __restrict__ rowptr,
-                   uint32_t* __restrict__ col, double* __restrict__ val) {
-  const size_t D = na * nb;
-  const int lane = threadIdx.x & 31;
-  const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
-  for (size_t I = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); I < D; I += warps) {
-    const size_t ia = I / nb, ib = I - ia * nb;
-    const uint64_t ppa = prefix_parity(astr[ia]);
-    const uint64_t bI = bstr[ib];
+                   const double* __restrict__ V, size_t vstride, const uint64_t* __restrict__ rowbase,
+                   const uint32_t* __restrict__ perm, const uint32_t* __restrict__ psd,
+                   const uint32_t* __restrict__ ps, int nslice, int G, double* __restrict__ val) {
+  const uint32_t lane = threadIdx.x & 31, col = lane & (G - 1), sub = lane / G, step = 32 / G;
+  const size_t ia = blockIdx.x;
+  const uint64_t a0 = a_off[ia], ne = a_off[ia + 1] - a0, nas = a_ns[ia];
+  const uint64_t ppa = prefix_parity(astr[ia]);
+  for (int s = blockIdx.y * (kStoredThreads / 32) + (threadIdx.x >> 5); s < nslice;
+       s += gridDim.y * (kStoredThreads / 32)) {
+    double* out = val + rowbase[ia] + G * block_entry(ne, nas, s, psd, ps) + col;
+    const uint32_t ib = perm[G * s + col];
+    const bool in = ib != kNoRow;
+    const uint64_t bI = in ? bstr[ib] : 0ull;
     const uint32_t phI = basis_phase(ppa, bI);
-    uint64_t out = rowptr[I];
     // alpha same-spin: (ja, ib)
-    const uint64_t a0 = a_off[ia], na_e = a_off[ia + 1] - a0, nas = a_ns[ia];
-    for (uint64_t k = lane; k < na_e; k += 32) {
+    for (uint64_t k = sub; k < ne; k += step) {
       const uint64_t e = a0 + k;
-      const uint32_t ja = a_ket[e];
-      double v = same_element(a_info[e], a_val[e], k < nas, Db, db_stride, ib);
-      if (phI ^ basis_phase(prefix_parity(astr[ja]), bI)) v = -v;
-      col[out + k] = (uint32_t)(ja * nb + ib);
-      val[out + k] = v;
+      double v = in ? same_element(a_info[e], a_val[e], k < nas, Db, db_stride, ib) : 0.0;
+      if (phI ^ basis_phase(prefix_parity(astr[a_ket[e]]), bI)) v = -v;
+      out[G * k] = v;
     }
-    out += na_e;
-    // beta same-spin: (ia, jb)
-    const uint64_t b0 = b_off[ib], nb_e = b_off[ib + 1] - b0, nbs = b_ns[ib];
-    for (uint64_t k = lane; k < nb_e; k += 32) {
-      const uint64_t e = b0 + k;
-      const uint32_t jb = b_ket[e];
-      double v = same_element(b_info[e], b_val[e], k < nbs, Da, da_stride, ia);
-      if (phI ^ basis_phase(ppa, bstr[jb])) v = -v;
-      col[out + k] = (uint32_t)(ia * nb + jb);
-      val[out + k] = v;
+    out += G * ne;
+    // beta same-spin: (ia, jb), singles then doubles, each padded to the slice's longest list
+    const uint64_t b0 = in ? b_off[ib] : 0, nbs = in ? b_ns[ib] : 0, nbd = in ? b_off[ib + 1] - b0 - nbs : 0;
+    const uint32_t ls = ps[s + 1] - ps[s], ld = psd[s + 1] - psd[s] - ls;
+    for (uint32_t m = sub; m < ls + ld; m += step) {
+      const bool single = m < ls, has = single ? m < nbs : m - ls < nbd;
+      double v = 0.0;
+      if (has) {
+        const uint64_t e = b0 + (single ? m : nbs + m - ls);
+        v = same_element(b_info[e], b_val[e], single, Da, da_stride, ia);
+        if (phI ^ basis_phase(ppa, bstr[b_ket[e]])) v = -v;
+      }
+      out[G * (size_t)m] = v;
     }
-    out += nb_e;
+    out += G * (size_t)(ls + ld);
     // alpha single x beta single: (ja, jb), s_a s_b (a i|b j)
-    const uint64_t npairs = nas * nbs;
-    for (uint64_t p = lane; p < npairs; p += 32) {
-      const uint64_t ka = p / nbs, kb = p - ka * nbs;
-      const uint32_t ia_inf = a_info[a0 + ka], ib_inf = b_info[b0 + kb];
-      const uint32_t ja = a_ket[a0 + ka], jb = b_ket[b0 + kb];
-      double v = V[(size_t)((ia_inf >> 12) & 0xfffu) * vstride + ((ib_inf >> 12) & 0xfffu)];
-      const uint32_t flip = (ia_inf >> 31) ^ (ib_inf >> 31) ^ phI ^ basis_phase(prefix_parity(astr[ja]), bstr[jb]);
-      col[out + p] = (uint32_t)(ja * nb + jb);
-      val[out + p] = flip ? -v : v;
+    for (uint64_t ka = 0; ka < nas; ++ka, out += G * (size_t)ls) {
+      const uint32_t inf = a_info[a0 + ka];
+      const double* row = V + (size_t)((inf >> 12) & 0xfffu) * vstride;
+      const uint64_t ppj = prefix_parity(astr[a_ket[a0 + ka]]);
+      for (uint32_t m = sub; m < ls; m += step) {
+        double v = 0.0;
+        if (m < nbs) {
+          const uint32_t ib_inf = b_info[b0 + m];
+          v = row[(ib_inf >> 12) & 0xfffu];
+          if ((inf >> 31) ^ (ib_inf >> 31) ^ phI ^ basis_phase(ppj, bstr[b_ket[b0 + m]])) v = -v;
+        }
+        out[G * (size_t)m] = v;
+      }
     }
   }
 }
 
-// S = hii o X + H_offdiag X, a warp per row. The matrix streams through in
-// chunks of 128 elements (four per lane); the columns and values of the next
-// chunk, or of the next row's first chunk, are loaded while the vector
-// gathers of the current one are in flight, so the stream always has a chunk
-// in flight. Partial sums in fixed lane and chunk order, then a fixed
-// shuffle tree (deterministic).
-__global__ void __launch_bounds__(kStoredThreads)
-stored_spmv_kernel(size_t D, const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col,
-                   const double* __restrict__ val, const double* __restrict__ hii, const double* __restrict__ X,
-                   double* __restrict__ S) {
-  const int lane = threadIdx.x & 31;
-  const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
-  size_t I = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (I >= D) return;
-  uint64_t k0 = rowptr[I], k1 = rowptr[I + 1];
-  // the chunk in hand: columns and values of elements k0 + lane + 32 u
-  uint32_t c[4];
-  double v[4];
-  auto fetch = [&](uint64_t base, uint64_t end, uint32_t* cc, double* vv) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const uint64_t k = base + lane + 32 * u;
-      const bool in = k < end;
-      cc[u] = in ? __ldg(col + k) : 0u;
-      vv[u] = in ? __ldg(val + k) : 0.0;
+// Xq[ia, t] = X[ia, perm[t]], rows of stride xs (zero beyond nb).
+__global__ void permute_columns_kernel(const double* __restrict__ X, size_t nb, const uint32_t* __restrict__ perm,
+                                       size_t xs, double* __restrict__ Xq) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= xs) return;
+  Xq[blockIdx.y * xs + t] = t < nb ? X[blockIdx.y * nb + perm[t]] : 0.0;
+}
+
+// S = hii o X + H_offdiag X: CTA = (alpha string, 8 slices, one per warp). Xq: X
+// with permuted columns. A block's values are one stream that the warp reads in
+// batches, the next batch (of the next section too) loaded before the current
+// one is used. The vector row that the entries gather from is staged with
+// cp.async while the row before it is in use (kStaged), two buffers of xs
+// doubles; without room it is read from global memory.
+template <bool kStaged, int G>
+__global__ void __launch_bounds__(kStoredThreads, 3)
+stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, const uint32_t* __restrict__ a_ns,
+                      const uint32_t* __restrict__ a_ket, const uint64_t* __restrict__ rowbase,
+                      const uint32_t* __restrict__ perm, const uint32_t* __restrict__ idx,
+                      const uint32_t* __restrict__ psd, const uint32_t* __restrict__ ps, int nslice,
+                      const double* __restrict__ val, const double* __restrict__ hii, const double* __restrict__ X,
+                      const double* __restrict__ Xq, double* __restrict__ S) {
+  extern __shared__ __align__(16) double rows[];  // [2][xs] when staged
+  constexpr int kB = kStoredBatch, P = 32 / G;  // P entries per warp and load
+  const int lane = threadIdx.x & 31, col = lane & (G - 1), sub = lane / G;
+  const size_t ia = blockIdx.x;
+  const uint64_t a0 = a_off[ia];
+  const int ne = (int)(a_off[ia + 1] - a0), nas = (int)a_ns[ia];
+  auto stage = [&](int buf, size_t row) {
+    if constexpr (kStaged) {
+      for (size_t t = 2 * threadIdx.x; t < xs; t += 2 * kStoredThreads) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(rows + buf * xs + t);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(Xq + row * xs + t) : "memory");
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
   };
-  fetch(k0, k1, c, v);
-  uint64_t k = k0;
-  double a[4] = {0.0, 0.0, 0.0, 0.0};
-  for (;;) {
-    // the gathers of the chunk in hand first (they need only its columns)
-    double x[4];
+  stage(0, ia);
+  const int s = (int)blockIdx.y * (kStoredThreads / 32) + (threadIdx.x >> 5);
+  const bool active = s < nslice;
+  const int lb = active ? (int)(psd[s + 1] - psd[s]) : 0, ls = active ? (int)(ps[s + 1] - ps[s]) : 0;
+  const int na_e = active ? ne : 0;
+  // sections: -2 alpha same-spin entries, -1 beta same-spin, j >= 0 alpha single j with the beta singles
+  auto size = [&](int j) { return j == -2 ? na_e : j == -1 ? lb : j < nas ? ls : 0; };
+  const double* p = active ? val + rowbase[ia] + G * block_entry((uint64_t)ne, (uint64_t)nas, s, psd, ps) + lane : val;
+  const uint32_t* ix = idx + (active ? (uint64_t)G * psd[s] : 0ull) + lane;
+  const double* xcol = Xq + min((size_t)G * (active ? s : 0) + col, xs - 1);  // values beyond nb are zero
+  double cur[kB], acc = 0.0;
+  auto load = [&](double (&o)[kB], int n) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) x[u] = k + lane + 32 * u < k1 ? __ldg(X + c[u]) : 0.0;
-    // the next chunk: the rest of this row, or the next row of this warp
-    uint64_t kn = k + 128, e = k1;
-    size_t In = I;
-    if (kn >= k1) {
-      In = I + warps;
-      kn = In < D ? rowptr[In] : 0;
-      e = In < D ? rowptr[In + 1] : 0;
+    for (int u = 0; u < kB; ++u) o[u] = P * u + sub < n ? __ldcs(p + 32 * u) : 0.0;
+    p += G * (int64_t)n;
+  };
+  load(cur, min(kB * P, na_e > 0 ? na_e : lb));  // without beta entries there are no pairs either
+  for (int j = -2; j < nas; ++j) {
+    const double* r = nullptr;
+    if (j >= -1) {
+      const int buf = (j + 1) & 1;
+      if constexpr (kStaged) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();  // the row is in, and the other buffer's row is no longer read
+        if (j + 1 < nas) stage(buf ^ 1, a_ket[a0 + j + 1]);
+        r = rows + buf * xs;
+      } else {
+        r = Xq + (j < 0 ? ia : (size_t)a_ket[a0 + j]) * xs;
+      }
     }
-    uint32_t cn[4];
-    double vn[4];
-    fetch(kn, e, cn, vn);
+    const int n = size(j);
+    for (int m = 0; m < n; m += kB * P) {
+      const int cnt = n - m - sub;  // entries of the lane's from here: those of P * u < cnt
+      double nxt[kB];
+      load(nxt, min(kB * P, m + kB * P < n ? n - m - kB * P : size(j + 1)));
+      if (j == -2) {
+        double x[kB];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) a[u] = fma(v[u], x[u], a[u]);  // out-of-range lanes add 0 * 0
-    if (In != I) {  // row I complete
-      double acc = (a[0] + a[1]) + (a[2] + a[3]);
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-      if (lane == 0) S[I] = fma(hii[I], X[I], acc);
-      if (In >= D) return;
-      I = In;
-      k1 = e;
-      a[0] = a[1] = a[2] = a[3] = 0.0;
+        for (int u = 0; u < kB; ++u) x[u] = P * u < cnt ? __ldg(xcol + (size_t)__ldg(a_ket + a0 + m + sub + P * u) * xs) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kB; ++u) acc = fma(cur[u], x[u], acc);
+      } else {
+        uint32_t t[kB];
+#pragma unroll
+        for (int u = 0; u < kB; ++u) t[u] = P * u < cnt ? __ldg(ix + G * m + 32 * u) : 0u;
+#pragma unroll
+        for (int u = 0; u < kB; ++u)
+          if (P * u < cnt) acc = fma(cur[u], r[t[u]], acc);
+      }
+#pragma unroll
+      for (int u = 0; u < kB; ++u) cur[u] = nxt[u];
     }
-    k = kn;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) { c[u] = cn[u]; v[u] = vn[u]; }
   }
-}
-
-unsigned grid_for(size_t warps_needed) {
-  const size_t ctas = (warps_needed + (kStoredThreads / 32) - 1) / (kStoredThreads / 32);
-  return (unsigned)std::min<size_t>(std::max<size_t>(ctas, 1), 148ull * 64);
+#pragma unroll
+  for (int o = 16; o >= G; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  const uint32_t ib = active && sub == 0 ? perm[G * s + col] : kNoRow;
+  if (ib == kNoRow) return;
+  const size_t I = ia * nb + ib;
+  S[I] = fma(hii[I], X[I], acc);
 }
 
 }  // namespace
 
 void release_stored(Ctx* c) {
-  cudaFree(c->stored.rowptr);
-  cudaFree(c->stored.col);
-  cudaFree(c->stored.val);
-  c->stored = StoredH{};
+  StoredH& H = c->stored;
+  for (void* p : {(void*)H.val, (void*)H.rowbase, (void*)H.perm, (void*)H.idx, (void*)H.psd, (void*)H.ps}) cudaFree(p);
+  H = StoredH{};
 }
 
 int build_stored(Ctx* c) {
@@ -187,57 +234,133 @@ int build_stored(Ctx* c) {
   if (int rc = ensure_coulomb_a(c)) return rc;
   release_stored(c);
   const size_t na = c->na, nb = c->nb, D = na * nb;
-  if (D > (size_t)UINT32_MAX) {  // the columns are 32-bit determinant indices
+  if (D > (size_t)UINT32_MAX) {  // a limit that callers can rely on, whatever the layout
     c->err = "build_hamiltonian: " + std::to_string(D) +
-             " determinants exceed the 32-bit column indices of the stored matrix (at most 4294967295)";
+             " determinants exceed the stored matrix's 4294967295";
     return SBDX_ERR_ARG;
   }
   const Conn& ca = c->conn[0];
   const Conn& cb = c->conn[1];
-  StoredH& H = c->stored;
-  SBDX_CUDA(c, cudaMalloc(&H.rowptr, sizeof(uint64_t) * (D + 1)));
-  {
-    uint64_t* cnt = nullptr;  // row lengths, then their exclusive prefix sum into rowptr
-    SBDX_CUDA(c, pool_alloc(c, (void**)&cnt, sizeof(uint64_t) * (D + 1)));
-    const unsigned g = (unsigned)std::min<size_t>((D + 256) / 256, 148ull * 32);
-    stored_count_kernel<<<g, 256, 0, c->stream>>>(ca.off, ca.nsing, cb.off, cb.nsing, na, nb, cnt);
-    SBDX_LAUNCHED(c);
-    size_t tmp = 0;
-    cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, tmp, cnt, H.rowptr, D + 1, c->stream);
-    void* dtmp = nullptr;
-    if (e == cudaSuccess) e = pool_alloc(c, &dtmp, tmp);
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(dtmp, tmp, cnt, H.rowptr, D + 1, c->stream);
-    if (dtmp) cudaFreeAsync(dtmp, c->stream);
-    cudaFreeAsync(cnt, c->stream);
-    SBDX_CUDA(c, e);
-  }
-  uint64_t nnz = 0;
-  SBDX_CUDA(c, cudaMemcpyAsync(&nnz, H.rowptr + D, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream));
+  std::vector<uint32_t> as(na), bs(nb), bd(nb), bket(std::max<size_t>(1, cb.total));
+  std::vector<uint64_t> aoff(na + 1), boff(nb + 1);
+  auto down = [&](void* h, const void* d, size_t bytes) {
+    return cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->stream);
+  };
+  SBDX_CUDA(c, down(as.data(), ca.nsing, sizeof(uint32_t) * na));
+  SBDX_CUDA(c, down(bs.data(), cb.nsing, sizeof(uint32_t) * nb));
+  SBDX_CUDA(c, down(bd.data(), cb.ndoub, sizeof(uint32_t) * nb));
+  SBDX_CUDA(c, down(aoff.data(), ca.off, sizeof(uint64_t) * (na + 1)));
+  SBDX_CUDA(c, down(boff.data(), cb.off, sizeof(uint64_t) * (nb + 1)));
+  if (cb.total) SBDX_CUDA(c, down(bket.data(), cb.ket, sizeof(uint32_t) * cb.total));
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
-  const size_t n = nnz ? nnz : 1;
-  if (cudaMalloc(&H.col, sizeof(uint32_t) * n) != cudaSuccess || cudaMalloc(&H.val, sizeof(double) * n) != cudaSuccess) {
+  // beta strings with the most singles, then doubles, first
+  uint64_t sa = 0, sb = 0;
+  for (uint32_t x : as) sa += x;
+  for (uint32_t x : bs) sb += x;
+  const uint64_t nnz = ca.total * nb + na * (uint64_t)cb.total + sa * sb;
+  std::vector<uint32_t> perm(nb + 32, kNoRow), pos(nb), psd, ps;
+  for (size_t t = 0; t < nb; ++t) perm[t] = (uint32_t)t;
+  std::sort(perm.begin(), perm.begin() + nb, [&](uint32_t x, uint32_t y) {
+    return bs[x] != bs[y] ? bs[x] > bs[y] : bd[x] != bd[y] ? bd[x] > bd[y] : x < y;
+  });
+  for (size_t t = 0; t < nb; ++t) pos[perm[t]] = (uint32_t)t;
+  size_t G = 32, ns = 0;
+  uint64_t total = 0;
+  for (;; G /= 2) {
+    ns = (nb + G - 1) / G;
+    ps.assign(ns + 1, 0);
+    psd.assign(ns + 1, 0);
+    for (size_t s = 0; s < ns; ++s) {
+      uint32_t ls = 0, ld = 0;
+      for (size_t t = G * s; t < std::min(nb, G * s + G); ++t) {
+        ls = std::max(ls, bs[perm[t]]);
+        ld = std::max(ld, bd[perm[t]]);
+      }
+      ps[s + 1] = ps[s] + ls;
+      psd[s + 1] = psd[s] + ls + ld;
+    }
+    total = G * (ca.total * ns + na * (uint64_t)psd[ns] + sa * ps[ns]);
+    if (G == 1 || total <= nnz + nnz / 4) break;
+  }
+  std::vector<uint32_t> idx(std::max<size_t>(1, G * psd[ns]), 0);
+  for (size_t t = 0; t < nb; ++t) {
+    const size_t s = t / G, ls = ps[s + 1] - ps[s];
+    const uint32_t b = perm[t];
+    uint32_t* o = idx.data() + G * psd[s] + t % G;
+    // padding reads the row's own column, which its elements touch anyway, so an
+    // infinity elsewhere stays where the matrix puts it
+    for (uint32_t m = 0; m < psd[s + 1] - psd[s]; ++m) o[G * m] = (uint32_t)t;
+    for (uint32_t m = 0; m < bs[b] + bd[b]; ++m)
+      o[G * (m < bs[b] ? (size_t)m : ls + m - bs[b])] = pos[bket[boff[b] + m]];
+  }
+  std::vector<uint64_t> rowbase(na);
+  uint64_t base = 0;
+  for (size_t a = 0; a < na; ++a) {
+    rowbase[a] = base;
+    base += G * ((aoff[a + 1] - aoff[a]) * ns + psd[ns] + (uint64_t)as[a] * ps[ns]);
+  }
+  StoredH& H = c->stored;
+  auto up = [&](auto** d, const auto& h) -> cudaError_t {
+    const size_t bytes = sizeof(h[0]) * h.size();
+    const cudaError_t e = cudaMalloc(d, bytes);
+    return e != cudaSuccess ? e : cudaMemcpyAsync(*d, h.data(), bytes, cudaMemcpyHostToDevice, c->stream);
+  };
+  H.nslice = (int)ns;
+  H.width = (int)G;
+  if (cudaMalloc(&H.val, sizeof(double) * std::max<uint64_t>(1, total)) != cudaSuccess ||
+      up(&H.rowbase, rowbase) != cudaSuccess || up(&H.perm, perm) != cudaSuccess || up(&H.idx, idx) != cudaSuccess ||
+      up(&H.psd, psd) != cudaSuccess || up(&H.ps, ps) != cudaSuccess) {
     cudaGetLastError();
+    cudaStreamSynchronize(c->stream);
     release_stored(c);
     c->err = "build_hamiltonian: the stored matrix (" + std::to_string(nnz) + " elements, " +
-             std::to_string((12.0 * (double)nnz + 8.0 * (double)D) / 1e9) + " GB) does not fit in device memory";
+             std::to_string(8.0 * (double)total / 1e9) + " GB) does not fit in device memory";
     return SBDX_ERR_NOMEM;
   }
-  stored_fill_kernel<<<grid_for(D), kStoredThreads, 0, c->stream>>>(
-      na, nb, c->d_a, c->d_b, ca.off, ca.nsing, ca.ket, ca.val, ca.info, cb.off, cb.nsing, cb.ket, cb.val, cb.info,
-      c->d_Da, c->da_stride, c->d_Db, c->db_stride, c->d_V, c->vstride, H.rowptr, H.col, H.val);
+  const dim3 grid((unsigned)na, (unsigned)std::min<size_t>((ns + 7) / 8, 65535));
+  stored_fill_kernel<<<grid, kStoredThreads, 0, c->stream>>>(
+      c->d_a, c->d_b, ca.off, ca.nsing, ca.ket, ca.val, ca.info, cb.off, cb.nsing, cb.ket, cb.val, cb.info, c->d_Da,
+      c->da_stride, c->d_Db, c->db_stride, c->d_V, c->vstride, H.rowbase, H.perm, H.psd, H.ps, (int)ns, (int)G, H.val);
   SBDX_LAUNCHED(c);
-  SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
+  SBDX_CUDA(c, cudaStreamSynchronize(c->stream));  // host vectors die at return
   H.nnz = nnz;
   clear_sigma_graphs(c);
   return 0;
 }
 
+// The permuted vector lies in the sigma's scratch (d_xp, row stride xsa).
 int stored_sigma(Ctx* c, const double* X, double* S) {
-  const size_t D = c->na * c->nb;
-  stored_spmv_kernel<<<grid_for(D), kStoredThreads, 0, c->stream>>>(D, c->stored.rowptr, c->stored.col,
-                                                                    c->stored.val, c->d_hii, X, S);
-  SBDX_LAUNCHED(c);
-  return 0;
+  const StoredH& H = c->stored;
+  const size_t xs = c->xsa, smem = 2 * sizeof(double) * xs;
+  double* Xq = reinterpret_cast<double*>(c->d_xp);
+  // alpha rows in launches of at most 65535 (the y extent of a grid)
+  for (size_t a = 0; a < c->na; a += 65535) {
+    const dim3 grid((unsigned)((xs + 255) / 256), (unsigned)std::min<size_t>(65535, c->na - a));
+    permute_columns_kernel<<<grid, 256, 0, c->stream>>>(X + a * c->nb, c->nb, H.perm, xs, Xq + a * xs);
+    SBDX_LAUNCHED(c);
+  }
+  constexpr int per = kStoredThreads / 32;
+  const dim3 grid((unsigned)c->na, (unsigned)((H.nslice + per - 1) / per));
+  const Conn& ca = c->conn[0];
+  auto launch = [&](auto kernel, size_t bytes) -> int {
+    SBDX_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAbSmemBudget));
+    kernel<<<grid, kStoredThreads, bytes, c->stream>>>(c->nb, xs, ca.off, ca.nsing, ca.ket, H.rowbase, H.perm, H.idx,
+                                                       H.psd, H.ps, H.nslice, H.val, c->d_hii, X, Xq, S);
+    SBDX_LAUNCHED(c);
+    return 0;
+  };
+  // a CTA's rows gather from the staged one about as many elements as it has,
+  // or more; narrow slices of many strings use too little of it
+  const bool staged = smem <= kAbSmemBudget && (H.width == 32 || c->nb <= 64 * (size_t)H.width);
+  auto pick = [&](auto st, auto unst) -> int { return staged ? launch(st, smem) : launch(unst, 0); };
+  switch (H.width) {
+    case 32: return pick(stored_product_kernel<true, 32>, stored_product_kernel<false, 32>);
+    case 16: return pick(stored_product_kernel<true, 16>, stored_product_kernel<false, 16>);
+    case 8: return pick(stored_product_kernel<true, 8>, stored_product_kernel<false, 8>);
+    case 4: return pick(stored_product_kernel<true, 4>, stored_product_kernel<false, 4>);
+    case 2: return pick(stored_product_kernel<true, 2>, stored_product_kernel<false, 2>);
+    default: return pick(stored_product_kernel<true, 1>, stored_product_kernel<false, 1>);
+  }
 }
 
 }  // namespace sbdx

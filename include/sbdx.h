@@ -171,8 +171,9 @@ int sbdx_diag_terms_noalloc(int norb, double I0, const double* d_h, const double
  * overlapped with the product's kernels (page-locked host buffers let them
  * overlap; pageable ones give the same result, serialised). */
 int sbdx_sigma(sbdx_ctx* ctx, const double* C, double* S);
-/* Chunks of that pipeline: 0 = automatic (about 8 M determinants per chunk,
- * at most 8; none below about 12.6 M determinants), 1 = no pipeline (one copy in, the
+/* Chunks of that pipeline: 0 = automatic (page-locked buffers, from about 2 M
+ * determinants: three, one more for every 4 M; pageable ones: about 8 M
+ * determinants per chunk, none below about 12.6 M; at most 8), 1 = no pipeline (one copy in, the
  * product, one copy out), K >= 2 = K chunks of equal alpha-row counts. The
  * pipeline runs with the default alpha-first launch codes and no stored
  * Hamiltonian; otherwise sbdx_sigma copies around one whole product. */

@@ -2824,16 +2824,35 @@ int sigma_device(Ctx* c, int precision, const void* X, void* S) {
 
 namespace {
 
-constexpr size_t kIoChunkDets = size_t(8) << 20;  // determinants per chunk in automatic mode
-constexpr int kIoMaxChunks = 8;
+// Automatic chunk count: three from kIoMinDets determinants, one more for each
+// kIoChunkDets, kIoMaxChunks at most. More chunks expose less of the copies but
+// cost launches and the tails of the chunked kernels. Page-locked buffers, us
+// with 1, 3, 4, 6 and 8 chunks: 2.25 M determinants 1317, 1245, 1267, 1408,
+// 1613; 6.25 M 3430, 3107, 3078, 3044, 3274; 16 M 9598, 8658, 8451, 8382, 8631;
+// 64 M (4, 6, 8, 12) 41.4, 40.7, 40.6 and 43 ms.
+constexpr size_t kIoMinDets = size_t(2) << 20, kIoChunkDets = size_t(4) << 20;
+// Pageable copies block the host, so more chunks only cost there (2.25 M: 2461
+// against 2545, 11.6 M: 28.8 against 29.8 ms): one for each 8 M.
+constexpr int kIoMinChunks = 3, kIoMaxChunks = 8;
 
-int io_chunk_count(const Ctx* c) {
+bool page_locked(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost;
+}
+
+int io_chunk_count(const Ctx* c, bool locked) {
   if (c->io_chunks_req == 1) return 1;
   const size_t D = c->na * c->nb;
-  // automatic: the nearest whole number of kIoChunkDets chunks (64 M
-  // determinants: 8 chunks, 40.6 ms end to end against 41.4 ms with 7)
-  int k = c->io_chunks_req >= 2 ? c->io_chunks_req
-                                : (int)std::min<size_t>(kIoMaxChunks, (D + kIoChunkDets / 2) / kIoChunkDets);
+  int k = c->io_chunks_req;
+  if (k < 2) {
+    const size_t n = locked ? (D < kIoMinDets ? 1 : kIoMinChunks + D / kIoChunkDets)
+                            : (D + kIoChunkDets) / (2 * kIoChunkDets);
+    k = (int)std::min<size_t>(kIoMaxChunks, n);
+  }
   k = std::min<int>(k, (int)(c->na / 8));  // at least 8 rows per chunk
   return std::max(k, 1);
 }
@@ -2887,7 +2906,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
   double* din = static_cast<double*>(c->d_io_in);
   double* dout = static_cast<double*>(c->d_io_out);
   const Tune t = effective_tune(c, true);
-  const int K = io_chunk_count(c);
+  const int K = io_chunk_count(c, page_locked(hC) && page_locked(hS));
   const bool pipe = K >= 2 && c->stored.val == nullptr && is_v6(t) && t.ab_code == 71 && !c->profiling;
   if (!pipe) {  // one copy in, the sigma, one copy out
     SBDX_CUDA(c, cudaMemcpyAsync(din, hC, sizeof(double) * D, cudaMemcpyHostToDevice, c->stream));

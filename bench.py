@@ -15,9 +15,10 @@ host buffers, the host->device copy of C and the device->host copy of S inside
 every step. `roofline` describes the dominant kernel of the sigma (the
 alpha-beta kernel), which gathers from rows staged in shared memory and is
 bound by the shared-memory pipe: its conflict-free shared bytes per launch
-(one ket and one integral element per alpha-single x beta-single det-pair,
-2*s_c*P_ab) over its CUDA-event time, against 128 bytes per clock per SM at
-the sampled SM clock. `roofline.hbm` keeps the SpMV byte model (one vector
+(one integral element per alpha-single x beta-single det-pair and one 16-byte
+update of the bra row per group of R = 80/s_c alpha singles,
+(s_c + 16/R)*P_ab) over its CUDA-event time, against 128 bytes per clock per SM
+at the sampled SM clock. `roofline.hbm` keeps the SpMV byte model (one vector
 gather per pair plus the partial-sigma read-modify-write, P_ab*s_c + 16*D)
 against the measured HBM copy bandwidth, and the DRAM bytes ncu measured;
 `roofline.sigma` gives the model for the whole sigma,
@@ -221,15 +222,16 @@ def roofline_bytes(prob, dp, s_c: int, s_h: int = 8) -> float:
 
 # CUDA kernel of each sigma phase (alpha-first path) and its ncu summary file
 PHASE_KERNELS = {"alpha_same_spin": "sigma_same_v6", "transpose": "phase_split", "beta_same_spin": "sigma_same_v6",
-                 "alpha_beta": "sigma_ab_v7", "combine": "combine_phase"}
+                 "alpha_beta": "sigma_ab", "combine": "combine_phase"}
 
 
 def ab_smem_bytes(dp, s_c: int) -> float:
-    """Shared-memory bytes the alpha-beta kernel must load: per alpha-single x
-    beta-single det-pair one element of the staged ket row and one of the
-    staged integral row (2 * s_c), at one 128-byte wavefront per 8 lanes of a
-    16-byte load, i.e. without bank conflicts."""
-    return 2.0 * s_c * dp["alpha_beta"]
+    """Shared-memory bytes the alpha-beta kernel must move without bank
+    conflicts: per alpha-single x beta-single det-pair one element of the staged
+    integral row (s_c), and per beta single and group of 80 / s_c alpha singles,
+    whose ket values are in registers, one read and one write of the bra row in
+    FP64."""
+    return (s_c + 16.0 * s_c / 80) * dp["alpha_beta"]
 
 
 def phase_bytes(prob, dp, s_c: int) -> dict:
@@ -417,8 +419,8 @@ def run_stored(args, hbm: float) -> dict:
     whose matrix fits in HBM: build time, element count, the FP64 product
     against the on-the-fly sigma of the same context (CUDA events, 10
     products after 3 warm-up ones; the matrix is far larger than L2). Bytes
-    of a product: 12 per stored element (column + value) plus the row
-    pointers and three D-vectors (input, diagonal, output)."""
+    of a product: 8 per stored element plus three D-vectors (input, diagonal,
+    output)."""
     import torch
 
     import sbdx
@@ -455,10 +457,10 @@ def run_stored(args, hbm: float) -> dict:
         ms_st = time_sigma()
         rel = float((S - S_fly).abs().max() / S_fly.abs().max())
         ctx.release_hamiltonian()
-    nbytes = 12 * nnz + 8 * (prob.D + 1) + 24 * prob.D
+    nbytes = 8 * nnz + 24 * prob.D
     gbs = nbytes / (ms_st * 1e-3) / 1e9
     return {"workload": args.stored, "desc": workload_desc(args.stored), "dets": int(prob.D), "elements": nnz,
-            "matrix_gb": (12 * nnz + 8 * (prob.D + 1)) / 1e9, "build_seconds": build_s,
+            "matrix_gb": 8 * nnz / 1e9, "build_seconds": build_s,
             "ms_stored_product": ms_st, "ms_on_the_fly_sigma": ms_fly, "gbs": gbs, "frac_of_hbm": gbs / hbm,
             "max_rel_diff_vs_on_the_fly": rel}
 
@@ -692,11 +694,12 @@ def run_sharded(args, rank, world, local):
     B = roofline_bytes(prob, dp, 8)
     gbs = B / world / (ms * 1e-3) / 1e9
     # the alpha-beta kernel of this rank's shard against the shared-memory
-    # pipe, as at N = 1: 16 conflict-free bytes per alpha-beta det-pair
+    # pipe, as at N = 1 (ab_smem_bytes)
     ab_pairs = float(sa[a0:a1].sum()) * float(sb.sum())
     ab_ms = phases.get("alpha_beta", 0.0)
     smem_peak = smem_peak_gbs((clocks or {}).get("sm_mhz") or 1965.0)
-    ab_gbs = 16.0 * ab_pairs / (ab_ms * 1e-3) / 1e9 if ab_ms > 0 else None
+    ab_bytes = ab_smem_bytes({"alpha_beta": ab_pairs}, 8)
+    ab_gbs = ab_bytes / (ab_ms * 1e-3) / 1e9 if ab_ms > 0 else None
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms, "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "f64",
@@ -708,8 +711,8 @@ def run_sharded(args, rank, world, local):
                    "l2": f"inputs larger than L2 (C = {8 * prob.D / 1e6:.0f} MB > 126 MB), no flush"},
         "roofline": {"bound": "smem", "achieved": ab_gbs, "peak": smem_peak, "unit": "GB/s",
                      "frac": ab_gbs / smem_peak if ab_gbs else None, "traffic": None,
-                     "kernel": "sigma_ab_v7", "phase": "alpha_beta", "shard": [a0, a1],
-                     "ms_per_launch": ab_ms, "smem_bytes_per_launch": 16.0 * ab_pairs,
+                     "kernel": "sigma_ab", "phase": "alpha_beta", "shard": [a0, a1],
+                     "ms_per_launch": ab_ms, "smem_bytes_per_launch": ab_bytes,
                      "peak_kind": "128 B/clk/SM x SMs x sampled SM clock (rank 0's shard)",
                      "phases": phases,
                      "hbm": {"model": "whole sigma of a row shard (SpMV byte model / N per GPU)", "gbs": gbs,
@@ -909,11 +912,11 @@ def run_ours(args, rank, world, local):
     if dominant == "alpha_beta" and tune[1] // 10 != 7:
         kern = "sigma_ab_v6"  # codes 61-64: unpacked staged rows
     if dominant in ("alpha_same_spin", "beta_same_spin") and tune[0] // 10 == 3:
-        kern = "sigma_same_blk"  # codes 31-38: blocks of 4 bra strings
+        kern = "sigma_same_mma"  # codes 31-38: blocks of 8 bra strings on the FP64 tensor pipe
     # The alpha-beta kernel gathers from rows staged in shared memory; DRAM
-    # moves a few percent of the SpMV byte model (profiles/sigma_ab_v7_cfg2.md),
+    # moves a few percent of the SpMV byte model (profiles/sigma_ab_cfg2.md),
     # so its bound is the shared-memory pipe: frac = conflict-free shared bytes
-    # (two 8-byte elements per det-pair) / time / (128 B per clock per SM).
+    # (ab_smem_bytes) / time / (128 B per clock per SM).
     sm_mhz = (clocks or {}).get("sm_mhz") or 1965.0
     smem_peak = smem_peak_gbs(sm_mhz)
     traffic = traffic_per_launch(kern, args.workload)

@@ -206,7 +206,12 @@ struct StoredH {
   uint32_t* perm = nullptr;     // [nb + 32] beta string of each position (kNoRow beyond nb)
   uint32_t* idx = nullptr;      // [G * psd[nslice]] position of each lane's m-th excited string
   uint32_t *psd = nullptr, *ps = nullptr;  // [nslice + 1] prefix sums of singles + doubles, of singles, per slice
-  int width = 32, nslice = 0;   // G, slices
+  uint4* item = nullptr;        // [nitem] {ia, group of slices, alpha singles first | end << 16, 1 + slot or 0}
+  uint2* split = nullptr;       // per split item {first slot, slots}
+  uint32_t *slot_split = nullptr, *done = nullptr;
+  double* part = nullptr;       // partial rows, 256 per slot
+  uint32_t nitem = 0;
+  int width = 32, nslice = 0, warps = 8;  // G, slices, slices per CTA
   uint64_t nnz = 0;             // off-diagonal elements, padding not counted
 };
 

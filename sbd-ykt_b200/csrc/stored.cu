@@ -130,7 +130,9 @@ __global__ void permute_columns_kernel(const double* __restrict__ X, size_t nb, 
   Xq[blockIdx.y * xs + t] = t < nb ? X[blockIdx.y * nb + perm[t]] : 0.0;
 }
 
-// S = hii o X + H_offdiag X: CTA = (alpha string, 8 slices, one per warp). Xq: X
+// S = hii o X + H_offdiag X: CTA = work item (alpha string, up to 8 slices, one per
+// warp; or a range of the alpha singles of that, the partial rows added in item
+// order by the last of them to finish), longest first. Xq: X
 // with permuted columns. A block's values are one stream that the warp reads in
 // batches, the next batch (of the next section too) loaded before the current
 // one is used. The vector row that the entries gather from is staged with
@@ -143,47 +145,54 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
                       const uint32_t* __restrict__ perm, const uint32_t* __restrict__ idx,
                       const uint32_t* __restrict__ psd, const uint32_t* __restrict__ ps, int nslice,
                       const double* __restrict__ val, const double* __restrict__ hii, const double* __restrict__ X,
-                      const double* __restrict__ Xq, double* __restrict__ S) {
+                      const double* __restrict__ Xq, double* __restrict__ S, const uint4* __restrict__ items,
+                      const uint2* __restrict__ split, const uint32_t* __restrict__ slot_split,
+                      uint32_t* __restrict__ done, double* __restrict__ part) {
   extern __shared__ __align__(16) double rows[];  // [2][xs] when staged
   constexpr int kB = kStoredBatch, P = 32 / G;  // P entries per warp and load
   const int lane = threadIdx.x & 31, col = lane & (G - 1), sub = lane / G;
-  const size_t ia = blockIdx.x;
+  const uint4 item = items[blockIdx.x];  // ia, slice group, alpha singles [z & 0xffff, z >> 16), slot
+  const size_t ia = item.x;
+  const int j0 = (int)(item.z & 0xffffu), j1 = (int)(item.z >> 16);
+  const bool first = j0 == 0;  // the item with the same-spin entries
   const uint64_t a0 = a_off[ia];
   const int ne = (int)(a_off[ia + 1] - a0), nas = (int)a_ns[ia];
   auto stage = [&](int buf, size_t row) {
     if constexpr (kStaged) {
-      for (size_t t = 2 * threadIdx.x; t < xs; t += 2 * kStoredThreads) {
+      for (size_t t = 2 * threadIdx.x; t < xs; t += 2 * blockDim.x) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(rows + buf * xs + t);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(Xq + row * xs + t) : "memory");
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
   };
-  stage(0, ia);
-  const int s = (int)blockIdx.y * (kStoredThreads / 32) + (threadIdx.x >> 5);
+  if (first) stage(0, ia);
+  else stage((j0 + 1) & 1, a_ket[a0 + j0]);
+  const int s = (int)item.y * (int)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const bool active = s < nslice;
   const int lb = active ? (int)(psd[s + 1] - psd[s]) : 0, ls = active ? (int)(ps[s + 1] - ps[s]) : 0;
   const int na_e = active ? ne : 0;
   // sections: -2 alpha same-spin entries, -1 beta same-spin, j >= 0 alpha single j with the beta singles
-  auto size = [&](int j) { return j == -2 ? na_e : j == -1 ? lb : j < nas ? ls : 0; };
+  auto size = [&](int j) { return j == -2 ? na_e : j == -1 ? lb : j < j1 ? ls : 0; };
   const double* p = active ? val + rowbase[ia] + G * block_entry((uint64_t)ne, (uint64_t)nas, s, psd, ps) + lane : val;
   const uint32_t* ix = idx + (active ? (uint64_t)G * psd[s] : 0ull) + lane;
   const double* xcol = Xq + min((size_t)G * (active ? s : 0) + col, xs - 1);  // values beyond nb are zero
+  if (!first) p += G * ((int64_t)ne + lb + (int64_t)j0 * ls);
   double cur[kB], acc = 0.0;
   auto load = [&](double (&o)[kB], int n) {
 #pragma unroll
     for (int u = 0; u < kB; ++u) o[u] = P * u + sub < n ? __ldcs(p + 32 * u) : 0.0;
     p += G * (int64_t)n;
   };
-  load(cur, min(kB * P, na_e > 0 ? na_e : lb));  // without beta entries there are no pairs either
-  for (int j = -2; j < nas; ++j) {
+  load(cur, min(kB * P, !first ? ls : na_e > 0 ? na_e : lb));  // without beta entries there are no pairs either
+  for (int j = first ? -2 : j0; j < j1; ++j) {
     const double* r = nullptr;
     if (j >= -1) {
       const int buf = (j + 1) & 1;
       if constexpr (kStaged) {
         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();  // the row is in, and the other buffer's row is no longer read
-        if (j + 1 < nas) stage(buf ^ 1, a_ket[a0 + j + 1]);
+        if (j + 1 < j1) stage(buf ^ 1, a_ket[a0 + j + 1]);
         r = rows + buf * xs;
       } else {
         r = Xq + (j < 0 ? ia : (size_t)a_ket[a0 + j]) * xs;
@@ -215,6 +224,23 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
 #pragma unroll
   for (int o = 16; o >= G; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   const uint32_t ib = active && sub == 0 ? perm[G * s + col] : kNoRow;
+  if (item.w != 0) {
+    __shared__ bool s_last;
+    const uint32_t slot = item.w - 1, id = slot_split[slot];
+    const uint2 sp = split[id];  // first slot, number of slots
+    part[(size_t)slot * kStoredThreads + threadIdx.x] = acc;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_last = atomicAdd(done + id, 1u) + 1 == sp.y;
+      if (s_last) done[id] = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    acc = 0.0;
+    for (uint32_t k = 0; k < sp.y; ++k) acc += __ldcg(part + (size_t)(sp.x + k) * kStoredThreads + threadIdx.x);
+  }
   if (ib == kNoRow) return;
   const size_t I = ia * nb + ib;
   S[I] = fma(hii[I], X[I], acc);
@@ -224,7 +250,9 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
 
 void release_stored(Ctx* c) {
   StoredH& H = c->stored;
-  for (void* p : {(void*)H.val, (void*)H.rowbase, (void*)H.perm, (void*)H.idx, (void*)H.psd, (void*)H.ps}) cudaFree(p);
+  for (void* p : {(void*)H.val, (void*)H.rowbase, (void*)H.perm, (void*)H.idx, (void*)H.psd, (void*)H.ps,
+                  (void*)H.item, (void*)H.split, (void*)H.slot_split, (void*)H.done, (void*)H.part})
+    cudaFree(p);
   H = StoredH{};
 }
 
@@ -299,6 +327,57 @@ int build_stored(Ctx* c) {
     rowbase[a] = base;
     base += G * ((aoff[a + 1] - aoff[a]) * ns + psd[ns] + (uint64_t)as[a] * ps[ns]);
   }
+  // work items: a CTA walks its entries batch by batch, so the strings with the
+  // most excitations would be a serial chain much longer than the rest (1000 x 150
+  // strings, L = 24: 417 us without the split, 204 with it); items above a quarter of an SM slot's share are
+  // split over their alpha singles
+  constexpr size_t kMinCap = 48, kMaxWarps = kStoredThreads / 32;  // cap in batches
+  const size_t ng = (ns + kMaxWarps - 1) / kMaxWarps, warps = (ns + ng - 1) / ng;  // few idle warps
+  const auto batches = [&](uint64_t n) { return (n * G + 32 * kStoredBatch - 1) / (32 * kStoredBatch); };
+  std::vector<uint64_t> mls(ng, 0), mlb(ng, 0);
+  for (size_t s = 0; s < ns; ++s) {
+    mls[s / warps] = std::max<uint64_t>(mls[s / warps], ps[s + 1] - ps[s]);
+    mlb[s / warps] = std::max<uint64_t>(mlb[s / warps], psd[s + 1] - psd[s]);
+  }
+  auto fixed = [&](size_t a, size_t g) { return batches(aoff[a + 1] - aoff[a]) + batches(mlb[g]) + 1; };
+  auto per = [&](size_t g) { return batches(mls[g]) + 1; };
+  uint64_t cost = 0;
+  for (size_t a = 0; a < na; ++a)
+    for (size_t g = 0; g < ng; ++g) cost += fixed(a, g) + as[a] * per(g);
+  int nsm = 0;
+  SBDX_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+  const uint64_t cap = std::max<uint64_t>(kMinCap, cost / (4 * 3 * (uint64_t)nsm));
+  struct Item { uint64_t cost; uint4 v; };
+  std::vector<Item> list;
+  std::vector<uint2> split;
+  std::vector<uint32_t> slot_split;
+  for (size_t a = 0; a < na; ++a)
+    for (size_t g = 0; g < ng; ++g) {
+      const uint64_t f = fixed(a, g), q = per(g), t = f + as[a] * q;
+      const uint32_t n = as[a];
+      const uint32_t parts = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((t + cap - 1) / cap, n));
+      if (parts == 1) {
+        list.push_back({t, make_uint4((uint32_t)a, (uint32_t)g, n << 16, 0)});
+        continue;
+      }
+      split.push_back(make_uint2((uint32_t)slot_split.size(), parts));
+      // the first part holds the same-spin entries and fewer singles (one at least)
+      const uint64_t share = t / parts;
+      uint32_t j = (uint32_t)std::min<uint64_t>(n - (parts - 1), std::max<uint64_t>(1, share > f ? (share - f) / q : 1));
+      for (uint32_t k = 0, lo = 0; k < parts; ++k) {
+        list.push_back({(k == 0 ? f : 0) + (j - lo) * q,
+                        make_uint4((uint32_t)a, (uint32_t)g, lo | (j << 16), 1 + (uint32_t)slot_split.size())});
+        slot_split.push_back((uint32_t)split.size() - 1);
+        lo = j;
+        if (k + 1 < parts) j = lo + (n - lo) / (parts - 1 - k);
+      }
+    }
+  std::stable_sort(list.begin(), list.end(), [](const Item& x, const Item& y) { return x.cost > y.cost; });
+  std::vector<uint4> item(list.size());
+  for (size_t k = 0; k < list.size(); ++k) item[k] = list[k].v;
+  const size_t nslot = slot_split.size();
+  if (split.empty()) { split.resize(1); slot_split.resize(1); }
+  std::vector<uint32_t> done(split.size(), 0);
   StoredH& H = c->stored;
   auto up = [&](auto** d, const auto& h) -> cudaError_t {
     const size_t bytes = sizeof(h[0]) * h.size();
@@ -307,9 +386,14 @@ int build_stored(Ctx* c) {
   };
   H.nslice = (int)ns;
   H.width = (int)G;
+  H.warps = (int)warps;
+  H.nitem = (uint32_t)item.size();
   if (cudaMalloc(&H.val, sizeof(double) * std::max<uint64_t>(1, total)) != cudaSuccess ||
       up(&H.rowbase, rowbase) != cudaSuccess || up(&H.perm, perm) != cudaSuccess || up(&H.idx, idx) != cudaSuccess ||
-      up(&H.psd, psd) != cudaSuccess || up(&H.ps, ps) != cudaSuccess) {
+      up(&H.psd, psd) != cudaSuccess || up(&H.ps, ps) != cudaSuccess || up(&H.item, item) != cudaSuccess ||
+      up(&H.split, split) != cudaSuccess || up(&H.slot_split, slot_split) != cudaSuccess ||
+      up(&H.done, done) != cudaSuccess ||
+      cudaMalloc(&H.part, sizeof(double) * kStoredThreads * std::max<size_t>(1, nslot)) != cudaSuccess) {
     cudaGetLastError();
     cudaStreamSynchronize(c->stream);
     release_stored(c);
@@ -339,13 +423,12 @@ int stored_sigma(Ctx* c, const double* X, double* S) {
     permute_columns_kernel<<<grid, 256, 0, c->stream>>>(X + a * c->nb, c->nb, H.perm, xs, Xq + a * xs);
     SBDX_LAUNCHED(c);
   }
-  constexpr int per = kStoredThreads / 32;
-  const dim3 grid((unsigned)c->na, (unsigned)((H.nslice + per - 1) / per));
   const Conn& ca = c->conn[0];
   auto launch = [&](auto kernel, size_t bytes) -> int {
     SBDX_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAbSmemBudget));
-    kernel<<<grid, kStoredThreads, bytes, c->stream>>>(c->nb, xs, ca.off, ca.nsing, ca.ket, H.rowbase, H.perm, H.idx,
-                                                       H.psd, H.ps, H.nslice, H.val, c->d_hii, X, Xq, S);
+    kernel<<<H.nitem, 32 * H.warps, bytes, c->stream>>>(c->nb, xs, ca.off, ca.nsing, ca.ket, H.rowbase, H.perm, H.idx,
+                                                       H.psd, H.ps, H.nslice, H.val, c->d_hii, X, Xq, S, H.item,
+                                                       H.split, H.slot_split, H.done, H.part);
     SBDX_LAUNCHED(c);
     return 0;
   };

@@ -28,6 +28,7 @@ SIZES = [
     (14, 4, 4, 20, 255),
     (14, 4, 4, 20, 257),
     (40, 8, 8, 40, 300),     # lists of very different lengths
+    (24, 5, 5, 30, 700),     # long lists split over their alpha singles
     (20, 2, 5, 3, 14600),    # a row that does not fit twice
 ]
 

@@ -42,7 +42,7 @@ def build_lib(force: bool = False) -> str:
     links libsbdx.so; sources whose object is newer than them and than the
     shared headers are not recompiled."""
     srcs = sorted(glob.glob(os.path.join(HERE, "csrc", "*.cu")))
-    hdrs = sorted(glob.glob(os.path.join(HERE, "csrc", "*.cuh"))) + [os.path.join(ROOT, "include", "sbdx.h")]
+    hdrs = sorted(glob.glob(os.path.join(HERE, "csrc", "*.cuh")) + glob.glob(os.path.join(HERE, "csrc", "*.h"))) + [os.path.join(ROOT, "include", "sbdx.h")]
     if not force and not _stale(LIB, srcs + hdrs):
         return LIB
     objdir = os.path.join(HERE, "_build")

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "sbdx.h"
+#include "ab_order.h"
 #include <cstdint>
 #include <cstddef>
 #include <string>
@@ -56,12 +57,9 @@ struct SellPanel {
   int slices_per_warp = 8;         // 8, 12 or 16: virtual rows per CTA = 1024 * this
 };
 
-// Schedule of the packed alpha-beta kernel (built by ab_plan.cu). A record is
-// one beta single: bits 0-11 pair index, 12-27 y slot, 31 same-spin sign,
-// kAbPad: no single. Record m of thread t of batch b sits at
+// Schedule of the packed alpha-beta kernel (built by ab_plan.cu; a record:
+// ab_order.h). Record m of thread t of batch b sits at
 // rec[4 * (boff[b] + (m / 4) * threads + t) + m % 4].
-constexpr uint32_t kAbPad = 1u << 30;
-constexpr int kAbWindow = 2;  // steps whose updates of y are disjoint (divides 4)
 struct AbPanel {
   uint32_t* rec = nullptr;
   uint64_t* boff = nullptr;     // [nbatch], in blocks of four records

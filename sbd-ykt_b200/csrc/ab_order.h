@@ -83,6 +83,12 @@ struct AbOrder {
   uint32_t slot(uint32_t i, int k) const { return k == 0 ? i : (uint32_t)nmain + s0[i] + (uint32_t)(k - 1); }
 
   void run(AbBatch& B, uint64_t seed) const {
+    if (B.list.empty()) {  // no lane, or none with a single: no step
+      B.steps = 0;
+      B.wsteps.assign((nt + 31) / 32, 0);
+      B.rec.clear();
+      return;
+    }
     const int n = B.n, nq = (n + 7) / 8, nh = (n + 15) / 16;
     uint64_t rs = seed * 0x9e3779b97f4a7c15ull + 0x1234567ull;
     auto rnd = [&](uint32_t m) -> uint32_t {  // xorshift64*

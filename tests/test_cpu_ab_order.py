@@ -16,7 +16,7 @@ def program(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("what", ["jobs"])
+@pytest.mark.parametrize("what", ["jobs", "order"])
 def test_schedule(program, what):
     """jobs: an exception on a worker thread reaches the caller, with every
     thread joined (a host allocation that fails must not end the program).

@@ -1182,6 +1182,7 @@ __device__ __forceinline__ void same_split_sum(const uint4* split, const uint32_
   double t[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) t[v] = 0.0;
+#pragma unroll 4
   for (uint32_t p = 0; p < sp.z; ++p)
 #pragma unroll
     for (int v = 0; v < VEC; ++v) t[v] += __ldcg(ypart + (size_t)(sp.y + p) * k_rows * ldx + c0 + v);
@@ -1197,6 +1198,11 @@ __device__ __forceinline__ void same_split_sum(const uint4* split, const uint32_
 // Coulomb table element of its column) and one FMA. X and Y rows have stride ldx, a multiple
 // of VEC (padding columns up to ldx are computed and never read); hii has
 // stride ncol.
+// Bound by the latency of the ket loads from L2: four entries' loads are
+// issued before their products (written as one loop of single entries the
+// compiler keeps two in flight: 8000 x 150 strings, 7 electrons in 58
+// orbitals, FP64 alpha side 370 -> 296 us; 150 x 4000, 5 in 24, beta side 160
+// -> 131 us; eight at a time 333 and 147 us).
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kSameThreads)
 sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
@@ -1208,6 +1214,7 @@ sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uin
                      double* __restrict__ Y) {
   __shared__ uint32_t s_ket[kSameThreads], s_pq[kSameThreads];
   __shared__ double s_val[kSameThreads];
+  constexpr int kAhead = 4;
   const uint4 item = items[blockIdx.x];  // bra string, entry range, output row
   const size_t r = item.x;
   double* __restrict__ Yrow = item.w ? ypart + (size_t)(item.w - 1) * ldx : Y + r * ldx;
@@ -1238,7 +1245,7 @@ sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uin
     }
     __syncthreads();
     if (!active) continue;
-    for (int e = 0; e < nsb; ++e) {
+    auto single = [&](int e) {
       const uint32_t pqs = s_pq[e];
       const double hv = s_val[e];
       double x[VEC], d[VEC];
@@ -1246,14 +1253,24 @@ sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uin
       VecIO<T, VEC>::load(Dt + (size_t)(pqs & 0xfffu) * dstride + c0, d);
 #pragma unroll
       for (int v = 0; v < VEC; ++v) acc[v] = fma(hv + flip_sign(d[v], pqs >> 31), x[v], acc[v]);
+    };
+#pragma unroll 2
+    for (int e = 0; e < nsb; ++e) single(e);
+    int e = nsb;
+    for (; e + kAhead <= cnt; e += kAhead) {  // the ket values of a run in flight together
+      double x[kAhead][VEC];
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) VecIO<T, VEC>::load(X + (size_t)s_ket[e + u] * ldx + c0, x[u]);
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) acc[v] = fma(s_val[e + u], x[u][v], acc[v]);
     }
-#pragma unroll 4
-    for (int e = nsb; e < cnt; ++e) {
-      const double hv = s_val[e];
+    for (; e < cnt; ++e) {
       double x[VEC];
       VecIO<T, VEC>::load(X + (size_t)s_ket[e] * ldx + c0, x);
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) acc[v] = fma(hv, x[v], acc[v]);
+      for (int v = 0; v < VEC; ++v) acc[v] = fma(s_val[e], x[v], acc[v]);
     }
   }
   if (active) {

@@ -69,8 +69,7 @@ long long sbdx_phase_times(sbdx_ctx* ctx, double* ms, int n);
  * determinant ordering, conjugated by the +-1 basis phase):
  *   same_code: 21/22/24/28 = 1/2/4/8 columns per thread, one bra string per
  *              CTA; 31/32/34/38 = blocks of 8 (FP64) or 4 (FP32) bra strings
- *              that walk the union of their excitation lists once (beside
- *              ab_code 61-64 they run the one-string kernel of that width);
+ *              that walk the union of their excitation lists once;
  *   ab_code:   61-64 = 1-4 staged ket rows of the balanced alpha-beta kernel,
  *              71 = a ket string per thread, its values for up to 10 (FP64) or
  *              20 (FP32) alpha singles in registers, integrals in shared memory.

@@ -1027,8 +1027,7 @@ int run_ab(Ctx* c, const T* X) {
 // step 3 those of the beta singles with the alpha string (one more integral
 // row per alpha string), so step 2 is a product with a constant sparse matrix.
 // The unpacked alpha-beta kernels (codes 61-64) evaluate the pairs only, add
-// them to Y, and leave both Coulomb terms and the diagonal to the same-spin
-// kernels (Dt, hii).
+// them to Y, and leave both Coulomb terms to the same-spin kernels (Dt).
 
 // Blocks ibx < ntx split one 32 x 32 tile; the further ones write 256 columns
 // of 32 rows of Xk, phi o X with its columns in the lane order of the packed
@@ -1082,8 +1081,8 @@ __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb
 }
 
 // S[ia, ib] = phi(ia, ib) (Y[ia, ib] + Yab[ia, ib] + Yt[ib, ia]) + hii[ia, ib]
-// X[ia, ib], stored in T; Y, Yab and Yt have row strides xsa, xsa and xsb.
-// With Yab null: S = phi o (Y + Yt^T).
+// X[ia, ib], stored in T; Y, Yab and Yt have row strides xsa, xsa and xsb. Yab
+// is null where the alpha-beta kernel has added its part to Y.
 template <typename T>
 __global__ void combine_phase_kernel(const double* __restrict__ Y, const double* __restrict__ Yab,
                                      const double* __restrict__ Yt, const double* __restrict__ hii,
@@ -1107,11 +1106,9 @@ __global__ void combine_phase_kernel(const double* __restrict__ Y, const double*
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const size_t ia = ia0 + k, ib = ib0 + tx;
     if (ia < na && ib < nb) {
-      double y = Y[ia * xsa + ib] + tile[k][tx], d = 0.0;
-      if (Yab != nullptr) {
-        y += Yab[ia * xsa + ib];
-        d = hii[ia * nb + ib] * (double)X[ia * nb + ib];
-      }
+      double y = Y[ia * xsa + ib] + tile[k][tx];
+      if (Yab != nullptr) y += Yab[ia * xsa + ib];
+      const double d = hii[ia * nb + ib] * (double)X[ia * nb + ib];
       S[ia * nb + ib] = (T)(basis_phase(s_pa[k], s_b[tx]) ? d - y : d + y);
     }
   }
@@ -1196,8 +1193,7 @@ __device__ __forceinline__ void same_split_sum(const uint4* split, const uint32_
 // entries of its row (ket, signed value, signed pair index) in shared memory;
 // per pair a double costs one FMA and a single, when Dt is given, one add (the
 // Coulomb table element of its column) and one FMA. X and Y rows have stride ldx, a multiple
-// of VEC (padding columns up to ldx are computed and never read); hii has
-// stride ncol.
+// of VEC (padding columns up to ldx are computed and never read).
 // Bound by the latency of the ket loads from L2: four entries' loads are
 // issued before their products (written as one loop of single entries the
 // compiler keeps two in flight: 8000 x 150 strings, 7 electrons in 58
@@ -1208,7 +1204,7 @@ __global__ void __launch_bounds__(kSameThreads)
 sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
                      const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
                      const typename Prec<T>::V* __restrict__ val, const uint32_t* __restrict__ info,
-                     const typename Prec<T>::V* __restrict__ Dt, size_t dstride, const double* __restrict__ hii,
+                     const typename Prec<T>::V* __restrict__ Dt, size_t dstride,
                      const uint4* __restrict__ items, const uint4* __restrict__ split,
                      const uint32_t* __restrict__ slot_split, uint32_t* __restrict__ done, double* __restrict__ ypart,
                      double* __restrict__ Y) {
@@ -1223,12 +1219,6 @@ sigma_same_v6_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, const uin
   double acc[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) acc[v] = 0.0;
-  if (hii != nullptr && item.y == 0 && active) {
-    double x[VEC];
-    VecIO<T, VEC>::load(X + r * ldx + c0, x);
-#pragma unroll
-    for (int v = 0; v < VEC; ++v) acc[v] = c0 + v < ncol ? hii[r * ncol + c0 + v] * x[v] : 0.0;
-  }
   const uint64_t beg = off[r] + item.y, end = off[r] + item.z, send = off[r] + nsing[r];
   const unsigned t = threadIdx.x;
   for (uint64_t base = beg; base < end; base += kSameThreads) {
@@ -1314,7 +1304,7 @@ __global__ void __launch_bounds__(kSameThreads)
 sigma_same_v6f_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, const uint64_t* __restrict__ off,
                       const uint32_t* __restrict__ nsing, const uint32_t* __restrict__ ket,
                       const float* __restrict__ val, const uint32_t* __restrict__ info, const float* __restrict__ Dt,
-                      size_t dstride, const double* __restrict__ hii, const uint4* __restrict__ items,
+                      size_t dstride, const uint4* __restrict__ items,
                       const uint4* __restrict__ split, const uint32_t* __restrict__ slot_split,
                       uint32_t* __restrict__ done, double* __restrict__ ypart, double* __restrict__ Y) {
   __shared__ uint32_t s_ket[kSameThreads], s_pq[kSameThreads];
@@ -1327,12 +1317,6 @@ sigma_same_v6f_kernel(const float* __restrict__ X, size_t ncol, size_t ldx, cons
   double acc[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) acc[v] = 0.0;
-  if (hii != nullptr && item.y == 0 && active) {
-    float x[VEC];
-    VecF<VEC>::load(X + r * ldx + c0, x);
-#pragma unroll
-    for (int v = 0; v < VEC; ++v) acc[v] = c0 + v < ncol ? hii[r * ncol + c0 + v] * (double)x[v] : 0.0;
-  }
   const uint64_t beg = off[r] + item.y, end = off[r] + item.z, send = off[r] + nsing[r];
   const unsigned t = threadIdx.x;
   for (uint64_t base = beg; base < end; base += kSameThreads) {
@@ -2152,17 +2136,17 @@ int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
 
 template <typename T, int VEC>
 int launch_same_v6(Ctx* c, const T* X, size_t ncol, size_t ldx, const Conn& cn, const typename Prec<T>::V* val,
-                   const typename Prec<T>::V* Dt, size_t dstride, const double* hii, double* Y) {
+                   const typename Prec<T>::V* Dt, size_t dstride, double* Y) {
   if (cn.n_same_item == 0) return 0;
   dim3 grid((unsigned)cn.n_same_item,
             (unsigned)((ncol + (size_t)kSameThreads * VEC - 1) / ((size_t)kSameThreads * VEC)));
   if constexpr (std::is_same<T, float>::value) {
     sigma_same_v6f_kernel<VEC><<<grid, kSameThreads, 0, c->stream>>>(
-        X, ncol, ldx, cn.off, cn.nsing, cn.ket, val, cn.info, Dt, dstride, hii, cn.same_item, cn.same_split,
+        X, ncol, ldx, cn.off, cn.nsing, cn.ket, val, cn.info, Dt, dstride, cn.same_item, cn.same_split,
         cn.same_slot, cn.same_done, cn.same_ypart, Y);
   } else {
     sigma_same_v6_kernel<T, VEC><<<grid, kSameThreads, 0, c->stream>>>(
-        X, ncol, ldx, cn.off, cn.nsing, cn.ket, val, cn.info, Dt, dstride, hii, cn.same_item, cn.same_split,
+        X, ncol, ldx, cn.off, cn.nsing, cn.ket, val, cn.info, Dt, dstride, cn.same_item, cn.same_split,
         cn.same_slot, cn.same_done, cn.same_ypart, Y);
   }
   SBDX_LAUNCHED(c);
@@ -2199,15 +2183,14 @@ int launch_same_blk(Ctx* c, int vec, const float* X, size_t ncol, size_t ldx, co
 // stride and keeps 16-byte alignment (the internal vectors have strides
 // padded to 8 elements, so only a misaligned base narrows). 31, 32, 34, 38:
 // the blocked kernels, whose FP64 form has one shape (128 columns per warp) and
-// whose FP32 form takes up to 4 columns per thread; they leave the diagonal out, so with hii (an unpacked alpha-beta code) the one-string kernels run.
+// whose FP32 form takes up to 4 columns per thread.
 template <typename T>
 int run_same_v6(Ctx* c, int code, const T* X, size_t ncol, size_t ldx, const Conn& cn, size_t row0, size_t nrow,
-                const typename Prec<T>::V* val, const typename Prec<T>::V* Dt, size_t dstride, const double* hii,
-                double* Y) {
+                const typename Prec<T>::V* val, const typename Prec<T>::V* Dt, size_t dstride, double* Y) {
   int vec = code % 10;
   const bool aligned = (reinterpret_cast<uintptr_t>(X) % 16) == 0;
   while (vec > 1 && (!aligned || ldx % vec != 0 || (Dt != nullptr && dstride % vec != 0))) vec >>= 1;
-  if (code / 10 == 3 && cn.blk[0].nblk > 0 && hii == nullptr && aligned) {
+  if (code / 10 == 3 && cn.blk[0].nblk > 0 && aligned) {
     const int rc = launch_same_blk(c, vec, X, ncol, ldx, cn.blk[std::is_same<T, double>::value ? 0 : 1], Y);
     if (rc || Dt == nullptr || nrow == 0) return rc;
     // the singles' Coulomb terms
@@ -2218,10 +2201,10 @@ int run_same_v6(Ctx* c, int code, const T* X, size_t ncol, size_t ldx, const Con
     SBDX_LAUNCHED(c);
     return 0;
   }
-  if (vec >= 8) return launch_same_v6<T, 8>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
-  if (vec >= 4) return launch_same_v6<T, 4>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
-  if (vec == 2) return launch_same_v6<T, 2>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
-  return launch_same_v6<T, 1>(c, X, ncol, ldx, cn, val, Dt, dstride, hii, Y);
+  if (vec >= 8) return launch_same_v6<T, 8>(c, X, ncol, ldx, cn, val, Dt, dstride, Y);
+  if (vec >= 4) return launch_same_v6<T, 4>(c, X, ncol, ldx, cn, val, Dt, dstride, Y);
+  if (vec == 2) return launch_same_v6<T, 2>(c, X, ncol, ldx, cn, val, Dt, dstride, Y);
+  return launch_same_v6<T, 1>(c, X, ncol, ldx, cn, val, Dt, dstride, Y);
 }
 
 template <typename T, int R, int KS>
@@ -2360,8 +2343,8 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
   int rc = 0;
   mark(0);
   if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, tune.ab_code == 71))) return rc;
-  // the beta singles' Coulomb terms and the diagonal: in the packed alpha-beta
-  // kernel and the combine, or in the same-spin kernels beside an unpacked one
+  // the beta singles' Coulomb terms: in the packed alpha-beta kernel, or in the
+  // same-spin kernels beside an unpacked one
   const bool packed = tune.ab_code == 71;
   const V* DtA = Db;
   const V* DtB = packed ? nullptr : Da;
@@ -2369,9 +2352,9 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
     SideBySide f(c);
     if ((rc = f.fork())) return rc;
     f.on(0);
-    rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, nullptr, c->d_y);
+    rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, c->d_y);
     f.on(1);
-    if (!rc) rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, nullptr, c->d_yt);
+    if (!rc) rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt);
     f.main();
     if (!rc) rc = run_ab_packed<T>(c);
     const int rj = f.join();
@@ -2379,11 +2362,10 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
     return launch_combine<T>(c, X, 0, na, S, true);
   }
   mark(1);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, packed ? nullptr : c->d_hii,
-                           c->d_y)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, nullptr, c->d_yt)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt)))
     return rc;
   mark(3);
   if ((rc = run_ab_v6<T>(c, tune.ab_code, xp))) return rc;
@@ -2525,11 +2507,10 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
   if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, true))) return rc;
   mark(1);
   if (nr == 0) return 0;
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ra, a0, nr, valA, Db, c->db_stride, nullptr, c->d_y)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ra, a0, nr, valA, Db, c->db_stride, c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, valB, (const V*)nullptr, 0, nullptr,
-                           c->d_yt + a0)))
+  if ((rc = run_same_v6<T>(c, tune.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, valB, (const V*)nullptr, 0, c->d_yt + a0)))
     return rc;
   mark(3);
   if ((rc = run_ab_packed<T>(c, &rc_items))) return rc;
@@ -2954,7 +2935,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
     SBDX_CUDA(c, cudaStreamWaitEvent(c->stream, ev[i], 0));
     if ((rc = launch_split<double>(c, din, a0, nr, xp, xpt, true))) return rc;
-    if ((rc = run_same_v6<double>(c, t.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, cb.val, (const double*)nullptr, 0, nullptr,
+    if ((rc = run_same_v6<double>(c, t.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, cb.val, (const double*)nullptr, 0,
                                   c->d_yt + a0)))
       return rc;
   }
@@ -2975,7 +2956,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     ra.n_same_split = it.n_same_split;
     ra.n_same_part = it.n_same_part;
     ra.same_ypart = it.same_ypart;
-    if ((rc = run_same_v6<double>(c, t.same_code, xp, nb, c->xsa, ra, a0, nr, ca.val, c->d_Db, c->db_stride, nullptr, c->d_y)))
+    if ((rc = run_same_v6<double>(c, t.same_code, xp, nb, c->xsa, ra, a0, nr, ca.val, c->d_Db, c->db_stride, c->d_y)))
       return rc;
     if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true))) return rc;
     SBDX_CUDA(c, cudaEventRecord(ev[n + i], c->stream));

@@ -57,3 +57,29 @@ def test_sigma_matches_oracle_at_tile_edges(size, codes, port):
     assert np.abs(S - ref).max() <= 1e-12 * top
     assert np.array_equal(S, again)  # one summation order
     assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top
+
+
+@pytest.mark.parametrize("same", [22, 32, 34])
+@pytest.mark.parametrize("size", [(12, 4, 4, 40, 257), (14, 5, 4, 17, 513), (24, 5, 5, 150, 31), (8, 3, 2, 9, 1)])
+def test_sigma_beside_unpacked_alpha_beta_kernels(size, same, port):
+    """Both same-spin families beside the unpacked alpha-beta kernels (codes
+    61-64): the oracle's values, and the blocked kernels really run there (they
+    leave the singles' Coulomb terms to one more kernel per spin)."""
+    torch = pytest.importorskip("torch")
+    prob = synth.random_problem(*size, seed=sum(size))
+    C = np.random.default_rng(6).standard_normal(prob.D)
+    x32 = torch.from_numpy(C.astype(np.float32)).cuda()
+    s32 = torch.empty_like(x32)
+    ref = port.sigma(prob, C)
+    top = np.abs(ref).max()
+    with sbdx.Context(0) as ctx:
+        ctx.load(prob)
+        for ab in (61, 62, 64):
+            ctx.set_tuning(same, ab)
+            S = ctx.sigma(C)
+            before = ctx.launches
+            ctx.sigma_device(sbdx.SBDX_FP32, x32.data_ptr(), s32.data_ptr())
+            torch.cuda.synchronize()
+            assert ctx.launches - before == (7 if same > 30 else 5)
+            assert np.abs(S - ref).max() <= 1e-12 * top
+            assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top

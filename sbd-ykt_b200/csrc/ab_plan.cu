@@ -31,7 +31,7 @@
 namespace sbdx {
 
 void free_ab_plan(Ctx* c, AbPlan& P) {
-  dev_free(c, P.vket);
+  dev_free(c, P.vket); dev_free(c, P.pairs); dev_free(c, P.V); dev_free(c, P.V32);
   for (AbPanel& q : P.panels) {
     dev_free(c, q.rec); dev_free(c, q.boff); dev_free(c, q.bsteps); dev_free(c, q.wsteps);
     dev_free(c, q.ex_row); dev_free(c, q.ex_off);
@@ -48,7 +48,23 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
   free_ab_plan(c, P);
   uint64_t total = 0;
   for (size_t r = 0; r < n; ++r) total += hs[r];
-  P.vstr = (uint32_t)((c->npair + 7) & ~(size_t)7);
+  // The pairs in use. A sample of 150 strings has singles for a few of the 1711
+  // pairs of 58 orbitals, and staging the integrals of all of them took longer
+  // than using them: alpha-beta time of 8000 x 150 strings (7 electrons) 1549 us
+  // FP64 and 1073 us FP32 with all pairs, 406 and 291 us with these; 5000 x 200
+  // 991 and 677, 516 and 345 us; 8000 x 8000, where nearly all are used, the same.
+  std::vector<uint32_t> pairs, pair_at(c->npair, 0);
+  for (size_t r = 0; r < n; ++r)
+    for (uint32_t e = 0; e < hs[r]; ++e) pair_at[(rec[off[r] + e] >> 16) & 0xfffu] = 1;
+  for (size_t t = 0; t < c->npair; ++t)
+    if (pair_at[t]) {
+      pair_at[t] = (uint32_t)pairs.size();
+      pairs.push_back((uint32_t)t);
+    }
+  P.npu = (int)pairs.size();
+  P.vstride = (pairs.size() + 1) / 2 * 2;
+  P.vstride32 = (pairs.size() + 3) / 4 * 4;
+  P.vstr = (uint32_t)((pairs.size() + 7) & ~(size_t)7);
   // lanes: (ket, part of its list); lists above 1.5 times the mean are split
   struct VKet { uint32_t ket, part, parts, len; };
   const uint32_t cap = std::max<uint32_t>(16, (uint32_t)((3 * total + 2 * n - 1) / (2 * std::max<size_t>(n, 1))));
@@ -108,7 +124,7 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
             // this part's share of the panel's sub-list
             if ((uint64_t)m * vk[i].parts / in == vk[i].part) {
               const uint32_t loc = (uint32_t)(ib / (4 * np) * 4 + ib % 4);
-              B.list.push_back({loc, (uint16_t)((r[e] >> 16) & 0xfffu), (uint8_t)((r[e] >> 40) & 1u)});
+              B.list.push_back({loc, (uint16_t)pair_at[(r[e] >> 16) & 0xfffu], (uint8_t)((r[e] >> 40) & 1u)});
             }
             ++m;
           }
@@ -169,7 +185,7 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
       return 0;
     };
     int rc = up(vket, &P.vket);
-    if (rc) return rc;
+    if (rc || (rc = up(pairs, &P.pairs))) return rc;
     P.panels.resize(np);
     for (size_t q = 0; q < np; ++q) {
       PanelWork& w = W[q];

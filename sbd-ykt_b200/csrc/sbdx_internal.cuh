@@ -73,7 +73,14 @@ struct AbPlan {
   uint32_t* vket = nullptr;  // [xs] ket string of each lane
   size_t xs = 0;             // nbatch * threads: row stride of Ctx::d_xk
   int threads = 0, nbatch = 0, np = 0;
-  uint32_t vstr = 0;         // packs per staged integral row (pairs padded to 8)
+  // the pairs that a beta single has, ascending: the records' pair index counts
+  // them, and the integrals (all rows, V[pq * vstride + t]) keep these columns only
+  uint32_t* pairs = nullptr;  // [npu]
+  int npu = 0;
+  uint32_t vstr = 0;          // packs per staged integral row (npu padded to 8)
+  double* V = nullptr;        // [npair x vstride]
+  float* V32 = nullptr;       // [npair x vstride32]
+  size_t vstride = 0, vstride32 = 0;
   std::vector<AbPanel> panels;
 };
 
@@ -275,8 +282,8 @@ struct Ctx {
   double *d_Da = nullptr, *d_Db = nullptr;
   float *d_Da32 = nullptr, *d_Db32 = nullptr;
   size_t da_stride = 0, db_stride = 0;
-  // the beta singles' term in the packed alpha-beta kernel: Da by string,
-  // [na x vstride] (FP32: [na x vstride32])
+  // the beta singles' term in the packed alpha-beta kernel: Da by string, over
+  // the plan's pairs, [na x ab.vstride] (FP32: [na x ab.vstride32])
   double* d_Dr = nullptr;
   float* d_Dr32 = nullptr;
   // sigma scratch (sized for D): transposed input, FP64 partial outputs

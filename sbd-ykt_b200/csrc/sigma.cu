@@ -1132,8 +1132,19 @@ __global__ void coulomb_table_kernel(const double* __restrict__ G, int L, const 
   D32[pq * stride + k] = (float)v;
 }
 
+// The integrals over the pairs in use: row pq = (pq|pairs[t]), t < n.
+__global__ void gather_pairs_kernel(const double* __restrict__ V, size_t vstride, const uint32_t* __restrict__ pairs,
+                                    int n, size_t vs, size_t vs32, double* __restrict__ out, float* __restrict__ out32) {
+  const size_t pq = blockIdx.x;
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    const double v = V[pq * vstride + pairs[t]];
+    out[pq * vs + t] = v;
+    out32[pq * vs32 + t] = (float)v;
+  }
+}
+
 // The table by string: row k = sum over the orbitals p of string k of the
-// integral row (pp|..).
+// integral row (pp|..) over npair pairs.
 __global__ void coulomb_row_sum_kernel(const double* __restrict__ V, size_t npair, size_t vs, size_t vs32, int L,
                                        const uint64_t* __restrict__ s, double* __restrict__ D,
                                        float* __restrict__ D32) {
@@ -1804,7 +1815,7 @@ sigma_ab_v6_kernel(const T* __restrict__ Xp, size_t nb, size_t ldx, const uint64
 }
 
 // 16-byte packs of the packed alpha-beta kernel: element e of pack h of pair
-// index pq is the signed integral s_alpha(ja) (a i|pq) of alpha single
+// index pq (of the pairs in use) is the signed integral s_alpha(ja) (a i|pq) of alpha single
 // h * kRows + e of the group.
 template <typename T> struct RowPack;
 template <> struct RowPack<double> {
@@ -1836,7 +1847,7 @@ struct AbArgs {
   size_t xs, ldx;    // ldx: row stride of Y and the partial rows
   const uint64_t* a_off;
   const uint32_t *a_ns, *a_ket, *a_info;
-  const T* Vt;       // unpacked integrals, row stride vstride
+  const T* Vt;       // integrals over the pairs in use, row stride vstride
   const T* Dr;       // [na] rows of the integral row of the alpha string itself, row stride vstride
   size_t vstride;
   int npair;
@@ -2100,9 +2111,9 @@ int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
     a.a_ket = ca.ket;
     a.a_info = ca.info;
     a.Dr = f64 ? (const T*)c->d_Dr : (const T*)c->d_Dr32;
-    a.Vt = f64 ? (const T*)c->d_V : (const T*)c->d_V32;
-    a.vstride = f64 ? c->vstride : c->vstride32;
-    a.npair = (int)c->npair;
+    a.Vt = f64 ? (const T*)P.V : (const T*)P.V32;
+    a.vstride = f64 ? P.vstride : P.vstride32;
+    a.npair = P.npu;
     a.vstr = P.vstr;
     a.max_packs = ab_packs(c, p);
     a.nbatch = P.nbatch;
@@ -2538,14 +2549,20 @@ int build_coulomb_tables(Ctx* c) {
   const size_t nb_el = c->npair * c->db_stride;
   SBDX_CUDA(c, dev_alloc(c, &c->d_Db, sizeof(double) * nb_el));
   SBDX_CUDA(c, dev_alloc(c, &c->d_Db32, sizeof(float) * nb_el));
-  SBDX_CUDA(c, dev_alloc(c, &c->d_Dr, sizeof(double) * c->na * c->vstride));
-  SBDX_CUDA(c, dev_alloc(c, &c->d_Dr32, sizeof(float) * c->na * c->vstride32));
+  AbPlan& P = c->ab;
+  SBDX_CUDA(c, dev_alloc(c, &P.V, sizeof(double) * c->npair * P.vstride));
+  SBDX_CUDA(c, dev_alloc(c, &P.V32, sizeof(float) * c->npair * P.vstride32));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_Dr, sizeof(double) * c->na * P.vstride));
+  SBDX_CUDA(c, dev_alloc(c, &c->d_Dr32, sizeof(float) * c->na * P.vstride32));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Db, 0, sizeof(double) * nb_el, c->stream));
   SBDX_CUDA(c, cudaMemsetAsync(c->d_Db32, 0, sizeof(float) * nb_el, c->stream));
   const dim3 gb((unsigned)((c->nb + 255) / 256), (unsigned)c->npair);
   coulomb_table_kernel<<<gb, 256, 0, c->stream>>>(c->d_G, c->L, c->d_b, c->nb, c->db_stride, c->d_Db, c->d_Db32);
   SBDX_LAUNCHED(c);
-  coulomb_row_sum_kernel<<<(unsigned)c->na, 256, 0, c->stream>>>(c->d_V, c->npair, c->vstride, c->vstride32, c->L, c->d_a,
+  gather_pairs_kernel<<<(unsigned)c->npair, 256, 0, c->stream>>>(c->d_V, c->vstride, P.pairs, P.npu, P.vstride,
+                                                                  P.vstride32, P.V, P.V32);
+  SBDX_LAUNCHED(c);
+  coulomb_row_sum_kernel<<<(unsigned)c->na, 256, 0, c->stream>>>(P.V, (size_t)P.npu, P.vstride, P.vstride32, c->L, c->d_a,
                                                                  c->d_Dr, c->d_Dr32);
   SBDX_LAUNCHED(c);
   return 0;

@@ -83,3 +83,24 @@ def test_sigma_beside_unpacked_alpha_beta_kernels(size, same, port):
             assert ctx.launches - before == (7 if same > 30 else 5)
             assert np.abs(S - ref).max() <= 1e-12 * top
             assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top
+
+
+@pytest.mark.parametrize("size", [(58, 7, 7, 600, 40), (64, 3, 2, 90, 8), (64, 5, 5, 33, 300), (30, 4, 1, 50, 30)])
+def test_sigma_with_few_pairs_in_use(size, port):
+    """The alpha-beta kernel keeps the integrals of the pairs that a beta single
+    has: few of many orbitals' pairs, counts off the pack sizes, one electron
+    (every beta pair of strings connected)."""
+    torch = pytest.importorskip("torch")
+    prob = synth.random_problem(*size, seed=sum(size))
+    C = np.random.default_rng(7).standard_normal(prob.D)
+    x32 = torch.from_numpy(C.astype(np.float32)).cuda()
+    s32 = torch.empty_like(x32)
+    with sbdx.Context(0) as ctx:
+        ctx.load(prob)
+        S = ctx.sigma(C)
+        ctx.sigma_device(sbdx.SBDX_FP32, x32.data_ptr(), s32.data_ptr())
+        torch.cuda.synchronize()
+    ref = port.sigma(prob, C)
+    top = np.abs(ref).max()
+    assert np.abs(S - ref).max() <= 1e-12 * top
+    assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top

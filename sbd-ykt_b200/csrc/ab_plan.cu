@@ -187,6 +187,7 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
     int rc = up(vket, &P.vket);
     if (rc || (rc = up(pairs, &P.pairs))) return rc;
     P.panels.resize(np);
+    P.steps.assign(nbatch, 0);
     for (size_t q = 0; q < np; ++q) {
       PanelWork& w = W[q];
       AbPanel& A = P.panels[q];
@@ -198,6 +199,7 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
       for (AbBatch& B : w.b) {
         boff.push_back(all.size() / 4);
         bsteps.push_back((uint32_t)B.steps);
+        P.steps[bsteps.size() - 1] += (uint64_t)B.steps;
         B.wsteps.resize(nt / 32, 0);
         wsteps.insert(wsteps.end(), B.wsteps.begin(), B.wsteps.end());
         all.insert(all.end(), B.rec.begin(), B.rec.end());

@@ -182,6 +182,11 @@ conn_fill_kernel(int spin, const uint64_t* __restrict__ s, size_t n, const uint6
   }
 }
 
+void free_ab_items(Ctx* c, AbItems& a) {
+  dev_free(c, a.item); dev_free(c, a.split); dev_free(c, a.slot); dev_free(c, a.done); dev_free(c, a.ypart);
+  a = AbItems{};
+}
+
 void free_conn(Ctx* c, Conn& cn) {
   dev_free(c, cn.nsing); dev_free(c, cn.ndoub); dev_free(c, cn.off); dev_free(c, cn.ket);
   dev_free(c, cn.val); dev_free(c, cn.val32); dev_free(c, cn.omask); dev_free(c, cn.info);
@@ -190,14 +195,14 @@ void free_conn(Ctx* c, Conn& cn) {
   SellPanel& p = cn.bal;
   dev_free(c, p.sell); dev_free(c, p.soff); dev_free(c, p.slen); dev_free(c, p.vrow); dev_free(c, p.vslot);
   dev_free(c, p.split_row); dev_free(c, p.split_slot);
-  dev_free(c, cn.ab_item); dev_free(c, cn.ab_split); dev_free(c, cn.ab_slot); dev_free(c, cn.ab_done); dev_free(c, cn.ypart);
+  for (AbItems& a : cn.ab) free_ab_items(c, a);
   dev_free(c, cn.same_item); dev_free(c, cn.same_split); dev_free(c, cn.same_slot); dev_free(c, cn.same_done); dev_free(c, cn.same_ypart);
   for (SameBlocks& b : cn.blk) free_blocks(c, b);
   cn = Conn{};
 }
 
-// Splits rows of `len` work units longer than cap into items (see
-// Conn::ab_item): {row, first unit, one past the last, 1 + slot or 0},
+// Splits rows of `len` work units longer than cap into items: {row, first
+// unit, one past the last, 1 + slot or 0},
 // longest first; split rows as {row, first slot, parts, 0}. Empty rows get an
 // item only with keep_empty (a kernel that assigns its output row).
 // Rows are numbered from row0 (len[i] belongs to row row0 + i).
@@ -441,31 +446,72 @@ int build_same_blocks(Ctx* c, const Conn& cn, const std::vector<uint64_t>& strin
   return upload_items(c, items, split, nslot * width, ncol, &B.item, &B.split, &B.ypart);
 }
 
-// Work items of the packed alpha-beta kernel (see Conn::ab_item; partial rows
-// have the padded stride pad8(nb) of the sigma's alpha-major vectors). A CTA
+// Work items of the packed alpha-beta kernel (see AbItems; partial rows have
+// the padded stride pad8(nb) of the sigma's alpha-major vectors). A CTA
 // handles one item and the kernel lasts about as long as the busiest SM, so
 // a few strings with many singles (near-Aufbau strings of a small sample
 // connect to ten times the mean) would set its duration: strings are split
 // into items of at most cap singles, cap = a quarter of the mean work per SM
-// rounded up to a multiple of 20 (one full group of the FP32 kernel, two of
-// the FP64 one), and items run longest first. Large samples have many strings
-// per SM and split nothing.
-int build_ab_items(Ctx* c, Conn& cn, std::vector<uint32_t> hs, size_t nb, size_t row0 = 0) {
+// rounded up to whole groups of the kernel (10 singles in FP64, 20 with FP32
+// storage), and items run longest first. Large samples have many strings per
+// SM and split nothing. Where the items are fewer than the CTAs that the GPU
+// holds, they are split over the schedule's batches too, into ranges of like
+// numbers of steps, from four batches on (below, the partial rows cost what the
+// split saves: 400 x 400 strings, two batches, 39 -> 45 us). Alpha-beta time
+// with groups of 20 and whole batches / with both (us, FP64): 100 x 20000
+// strings (7 electrons in 58 orbitals) 1265 / 553; 3 x 9000 (5 in 24) 204 / 58;
+// 150 x 4000 240 / 158; 200 x 5000 (8 in 40) 189 / 153; two and four items per
+// resident CTA 165 and 182.
+int build_ab_items(Ctx* c, AbItems (&out)[2], std::vector<uint32_t> hs, size_t nb, size_t row0 = 0) {
+  const AbPlan& P = c->ab;
   const uint64_t nsm = (uint64_t)sm_count(c);
+  const uint64_t resident = nsm * (P.threads == 256 ? 4 : P.threads == 512 ? 2 : 1);
   uint64_t total = 0;
   for (uint32_t& h : hs) total += ++h;  // the string itself counts as one more
   const uint64_t quarter = (total + 4 * nsm - 1) / (4 * nsm);
-  const uint32_t cap = (uint32_t)std::max<uint64_t>(20, (quarter + 19) / 20 * 20);
-  std::vector<uint4> items, split;
-  int slot = 0;
-  split_rows(hs, cap, true, items, split, slot, row0);  // every row's output is assigned
-  cn.item_cap = (int)cap;
-  cn.n_item = items.size();
-  cn.n_split = (int)split.size();
-  cn.n_part = slot;
-  const int rc = upload_slots(c, split, slot, 1, &cn.ab_slot, &cn.ab_done);
-  if (rc) return rc;
-  return upload_items(c, items, split, slot, nb, &cn.ab_item, &cn.ab_split, &cn.ypart);
+  for (int q = 0; q < 2; ++q) {
+    const uint64_t group = kAbPacks * (q == 0 ? 2 : 4);
+    const uint32_t cap = (uint32_t)std::max<uint64_t>(group, (quarter + group - 1) / group * group);
+    uint64_t whole = 0;
+    for (uint32_t h : hs) whole += (h + cap - 1) / cap;
+    const uint64_t want = whole && P.nbatch >= 4 ? (resident + whole - 1) / whole : 1;
+    const int ways = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)P.nbatch));
+    // batch ranges of like numbers of steps
+    std::vector<uint32_t> cut(1, 0);
+    std::vector<uint64_t> sum(P.steps.size() + 1, 0);
+    for (size_t b = 0; b < P.steps.size(); ++b) sum[b + 1] = sum[b] + P.steps[b];
+    for (int w = 1; w < ways; ++w) {
+      uint32_t b = cut.back() + 1;
+      while (b + (uint32_t)(ways - w) < (uint32_t)P.nbatch && sum[b] * ways < sum.back() * w) ++b;
+      cut.push_back(b);
+    }
+    cut.push_back((uint32_t)P.nbatch);
+    struct Item { uint64_t cost; uint4 v; };
+    std::vector<Item> list;
+    std::vector<uint4> split;
+    int slot = 0;
+    for (size_t i = 0; i < hs.size(); ++i) {
+      const uint32_t r = (uint32_t)(row0 + i), parts = (hs[i] + cap - 1) / cap;
+      const bool many = parts * (uint32_t)ways > 1;
+      if (many) split.push_back(make_uint4(r, (uint32_t)slot, parts * (uint32_t)ways, 0u));
+      for (uint32_t k = 0; k < parts; ++k)
+        for (int w = 0; w < ways; ++w) {
+          const uint32_t s0 = k * cap, s1 = std::min(hs[i], s0 + cap);
+          list.push_back({(s1 - s0) * (sum[cut[w + 1]] - sum[cut[w]] + 1),
+                          make_uint4(r, s0 | (s1 << 16), cut[w] | (cut[w + 1] << 16), many ? (uint32_t)++slot : 0u)});
+        }
+    }
+    std::stable_sort(list.begin(), list.end(), [](const Item& x, const Item& y) { return x.cost > y.cost; });
+    std::vector<uint4> items(list.size());
+    for (size_t k = 0; k < list.size(); ++k) items[k] = list[k].v;
+    AbItems& A = out[q];
+    A.n = items.size();
+    A.n_split = (int)split.size();
+    A.n_part = slot;
+    int rc = upload_slots(c, split, slot, 1, &A.slot, &A.done);
+    if (rc || (rc = upload_items(c, items, split, slot, nb, &A.item, &A.split, &A.ypart))) return rc;
+  }
+  return 0;
 }
 
 // Balanced SELL-32 of the single records (see SellPanel). The cap starts at
@@ -631,7 +677,6 @@ int build_one(Ctx* c, int spin, bool full) {
       if ((rc = build_same_blocks(c, cn, spin == 0 ? c->h_a : c->h_b, 0, n, spin == 0 ? c->nb : c->na,
                                   q == 0 ? kBlkRows64 : kBlkRows32, cn.blk[q])))
         return rc;
-    if (spin == 0 && (rc = build_ab_items(c, cn, hs, c->nb))) return rc;
   }
   if (spin == 1) {
     std::vector<uint64_t> rec;
@@ -642,7 +687,8 @@ int build_one(Ctx* c, int spin, bool full) {
     SBDX_CUDA(c, cudaMemcpyAsync(ha.data(), c->conn[0].nsing, sizeof(uint32_t) * c->na, cudaMemcpyDeviceToHost, c->stream));
     SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
     for (uint32_t h : ha) alpha_singles += h;
-    if ((rc = build_ab_plan(c, n, hs, off, rec, alpha_singles))) return rc;
+    if ((rc = build_ab_plan(c, n, hs, off, rec, alpha_singles)) || (rc = build_ab_items(c, c->conn[0].ab, ha, c->nb)))
+      return rc;
   }
   // the host copy of `off` must stay alive until the async copy ran
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -707,12 +753,11 @@ void free_range_items(Ctx* c, Conn& r) {
   for (SameBlocks& b : r.blk) free_blocks(c, b);
   dev_free(c, r.same_item); dev_free(c, r.same_split); dev_free(c, r.same_slot); dev_free(c, r.same_done); dev_free(c, r.same_ypart);
   r.same_slot = r.same_done = nullptr;
-  dev_free(c, r.ab_item); dev_free(c, r.ab_split); dev_free(c, r.ab_slot); dev_free(c, r.ab_done); dev_free(c, r.ypart);
-  r.same_item = r.same_split = r.ab_item = r.ab_split = nullptr;
-  r.ab_slot = r.ab_done = nullptr;
-  r.same_ypart = r.ypart = nullptr;
-  r.n_same_item = r.n_item = 0;
-  r.n_same_split = r.n_same_part = r.n_split = r.n_part = 0;
+  for (AbItems& a : r.ab) free_ab_items(c, a);
+  r.same_item = r.same_split = nullptr;
+  r.same_ypart = nullptr;
+  r.n_same_item = 0;
+  r.n_same_split = r.n_same_part = 0;
 }
 
 void free_row_range(Ctx* c) {
@@ -742,7 +787,7 @@ int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r) {
   if (rc) return rc;
   for (int q = 0; q < 2; ++q)
     if ((rc = build_same_blocks(c, ca, c->h_a, a0, n, c->nb, q == 0 ? kBlkRows64 : kBlkRows32, r.blk[q]))) return rc;
-  return build_ab_items(c, r, hs, c->nb, a0);
+  return build_ab_items(c, r.ab, hs, c->nb, a0);
 }
 
 int build_row_range(Ctx* c, size_t a0, size_t a1) {

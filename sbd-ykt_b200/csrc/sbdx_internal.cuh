@@ -82,6 +82,7 @@ struct AbPlan {
   float* V32 = nullptr;       // [npair x vstride32]
   size_t vstride = 0, vstride32 = 0;
   std::vector<AbPanel> panels;
+  std::vector<uint64_t> steps;  // [nbatch] over all panels
 };
 
 // Bra strings per block of the blocked same-spin kernels, and the determinant
@@ -122,6 +123,24 @@ struct SameBlocks {
   double* ypart = nullptr;   // [n_part * width * pad8(ncol)]
 };
 
+// Work items of the packed alpha-beta kernel for one precision, one CTA each,
+// longest first: {bra alpha string, first single | one past the last << 16,
+// first batch | one past the last << 16, 1 + partial-row slot or 0}, where the
+// index after a string's last single stands for the string itself (see
+// sigma_ab_kernel), so every string has an item. A string of several items has
+// a partial row for each (ypart[slot * pad8(nb) ..], FP64), which the last of
+// its CTAs to finish adds up into the output in slot order; the others write
+// the output directly.
+struct AbItems {
+  uint4* item = nullptr;     // [n]
+  size_t n = 0;
+  uint4* split = nullptr;    // [n_split]: {string, first slot, parts, 0}
+  uint32_t* slot = nullptr;  // [n_part]: entry of split
+  uint32_t* done = nullptr;  // [n_split]: items finished (zero between launches)
+  int n_split = 0, n_part = 0;
+  double* ypart = nullptr;   // [n_part * pad8(nb)]
+};
+
 struct Conn {
   size_t n = 0;          // number of bra strings
   size_t total = 0;      // number of entries
@@ -154,21 +173,7 @@ struct Conn {
   // balanced SELL-32 of the single-excitation records (beta spin only), read
   // by the alpha-first kernel with unpacked rows
   SellPanel bal;
-  // work items of the packed alpha-beta kernel (alpha spin only), one CTA
-  // each, longest first: {bra alpha string, first single, one past the last
-  // single, 1 + partial-row slot or 0}, where the index after a string's last
-  // single stands for the string itself (see sigma_ab_kernel), so every
-  // string has an item. A string with more singles than the
-  // cap is split into items of at most `item_cap` singles whose partial rows
-  // (ypart[slot * pad8(nb) ..], FP64) the last of its CTAs to finish adds to
-  // up into the output in slot order; the others write the output directly.
-  uint4* ab_item = nullptr;    // [n_item]
-  size_t n_item = 0;
-  uint4* ab_split = nullptr;   // [n_split]: {string, first slot, parts, 0}
-  uint32_t* ab_slot = nullptr; // [n_part]: entry of ab_split
-  uint32_t* ab_done = nullptr; // [n_split]: items finished (zero between launches)
-  int n_split = 0, n_part = 0, item_cap = 0;
-  double* ypart = nullptr;     // [n_part * pad8(nb)]
+  AbItems ab[2];  // (alpha spin only) FP64, FP32
   // work items of the alpha-first same-spin kernel (either spin), the same
   // scheme over the row's entries (singles then doubles): {bra string, first
   // entry, one past the last entry, 1 + partial-row slot or 0}. Partial rows

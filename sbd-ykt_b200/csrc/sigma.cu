@@ -1852,7 +1852,7 @@ struct AbArgs {
   size_t vstride;
   int npair;
   uint32_t vstr;     // packs per staged integral row
-  int max_packs, nbatch, np, panel, nmain, nex, ny;
+  int max_packs, np, panel, nmain, nex, ny;
   const uint4* rec;
   const uint64_t* boff;
   const uint32_t *bsteps, *wsteps, *ex_row, *ex_off;
@@ -1889,11 +1889,11 @@ __device__ __forceinline__ void step_wait(uint32_t bar, uint32_t ph, int* err) {
   atomicExch(err, kErrWatchdogAb);  // gives up: the result is flagged, nothing waits for it
 }
 
-// All batches of one group of nr alpha singles held in NH packs.
+// Batches b0 .. b1 - 1 of one group of nr alpha singles held in NH packs.
 template <typename T, int NT, int NH>
 __device__ __forceinline__ void ab_sweep(const AbArgs<T>& a, const typename RowPack<T>::P* __restrict__ vs,
-                                         double* __restrict__ y, const uint32_t* s_ket, int nr, uint32_t bar,
-                                         uint32_t& ph) {
+                                         double* __restrict__ y, const uint32_t* s_ket, int nr, int b0, int b1,
+                                         uint32_t bar, uint32_t& ph) {
   using RP = RowPack<T>;
   constexpr int VR = RP::kRows, R = NH * VR;
   const int warp = threadIdx.x >> 5;
@@ -1904,13 +1904,13 @@ __device__ __forceinline__ void ab_sweep(const AbArgs<T>& a, const typename RowP
 #pragma unroll
     for (int r = 0; r < R; ++r) c[r] = (r < nr && live) ? __ldg(xb + (size_t)s_ket[r] * a.xs) : (T)0;
   };
-  load_c(0);
-  for (int b = 0; b < a.nbatch; ++b) {
+  load_c(b0);
+  for (int b = b0; b < b1; ++b) {
     const int steps = (int)a.bsteps[b];
     const int wst = (int)a.wsteps[b * (NT / 32) + warp];
     const uint4* rp = a.rec + a.boff[b] + threadIdx.x;
     uint4 cur = wst > 0 ? __ldg(rp) : make_uint4(kAbPad, kAbPad, kAbPad, kAbPad);
-    bool more = b + 1 < a.nbatch;  // the next batch's ket values are still to be loaded
+    bool more = b + 1 < b1;  // the next batch's ket values are still to be loaded
     for (int m0 = 0; m0 < steps; m0 += 4) {
       if (m0 < wst) {
         const uint4 nxt = m0 + 4 < wst ? __ldg(rp + (size_t)(m0 / 4 + 1) * NT) : cur;
@@ -1963,7 +1963,8 @@ __device__ __forceinline__ void ab_sweep(const AbArgs<T>& a, const typename RowP
 }
 
 // Alpha single x beta single in the alpha-first basis. One CTA per work item:
-// a bra alpha string, or a range of the singles of a long one (Conn::ab_item).
+// a bra alpha string, or a range of its singles and of the schedule's batches
+// (AbItems).
 // Per group of up to kAbPacks * kRows alpha singles (ja_r, pq_r, s_r) of the
 // item, the signed integral rows s_r (pq_r|..) are staged in shared memory as
 // 16-byte packs; a thread owns one ket string jb at a time, with C'[ja_r, jb]
@@ -2002,18 +2003,19 @@ __global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
   P* vs = reinterpret_cast<P*>(smem + (((size_t)a.ny * 8 + 15) & ~(size_t)15));  // [packs][vstr]
   for (int i = threadIdx.x; i < a.ny; i += NT) y[i] = 0.0;
   const uint64_t e0 = a.a_off[ia];
-  const int n = (int)(item.z - item.y), ns = (int)a.a_ns[ia];
+  const int first = (int)(item.y & 0xffffu), n = (int)(item.y >> 16) - first, ns = (int)a.a_ns[ia];
+  const int b0 = (int)(item.z & 0xffffu), b1 = (int)(item.z >> 16);
   const int rmax = a.max_packs * VR;
   const int ng = (n + rmax - 1) / rmax;
   const int per = ng > 0 ? ((n + ng - 1) / ng + VR - 1) / VR * VR : VR;  // balanced groups of whole packs
   for (int k0 = 0; k0 < n; k0 += per) {
     const int nr = min(per, n - k0), nh = (nr + VR - 1) / VR;
-    const int nd = min(nr, ns - (int)item.y - k0);  // the rest (at most one) is the string itself
+    const int nd = min(nr, ns - first - k0);  // the rest (at most one) is the string itself
     __syncthreads();  // the integrals of the group before are no longer read
     if ((int)threadIdx.x < nh * VR) {
       uint32_t ket = (uint32_t)ia, pqs = 0;
       if ((int)threadIdx.x < nd) {
-        const uint64_t ent = e0 + item.y + k0 + threadIdx.x;
+        const uint64_t ent = e0 + first + k0 + threadIdx.x;
         const uint32_t inf = a.a_info[ent];
         ket = a.a_ket[ent];
         pqs = ((inf >> 12) & 0xfffu) | (inf & kInfoNeg);
@@ -2040,11 +2042,11 @@ __global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
     }
     __syncthreads();
     switch (nh) {
-      case 1: ab_sweep<T, NT, 1>(a, vs, y, s_ket, nr, bar, ph); break;
-      case 2: ab_sweep<T, NT, 2>(a, vs, y, s_ket, nr, bar, ph); break;
-      case 3: ab_sweep<T, NT, 3>(a, vs, y, s_ket, nr, bar, ph); break;
-      case 4: ab_sweep<T, NT, 4>(a, vs, y, s_ket, nr, bar, ph); break;
-      default: ab_sweep<T, NT, 5>(a, vs, y, s_ket, nr, bar, ph); break;
+      case 1: ab_sweep<T, NT, 1>(a, vs, y, s_ket, nr, b0, b1, bar, ph); break;
+      case 2: ab_sweep<T, NT, 2>(a, vs, y, s_ket, nr, b0, b1, bar, ph); break;
+      case 3: ab_sweep<T, NT, 3>(a, vs, y, s_ket, nr, b0, b1, bar, ph); break;
+      case 4: ab_sweep<T, NT, 4>(a, vs, y, s_ket, nr, b0, b1, bar, ph); break;
+      default: ab_sweep<T, NT, 5>(a, vs, y, s_ket, nr, b0, b1, bar, ph); break;
     }
   }
   __syncthreads();
@@ -2096,9 +2098,9 @@ int launch_ab(Ctx* c, const AbArgs<T>& args, size_t n_item, size_t smem) {
 template <typename T>
 int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
   const Conn& ca = c->conn[0];
-  const Conn& it = items ? *items : ca;
-  if (it.n_item == 0) return 0;
   const bool f64 = std::is_same<T, double>::value;
+  const AbItems& it = (items ? *items : ca).ab[f64 ? 0 : 1];
+  if (it.n == 0) return 0;
   const AbPlan& P = c->ab;
   for (size_t q = 0; q < P.panels.size(); ++q) {
     const AbPanel& p = P.panels[q];
@@ -2116,7 +2118,6 @@ int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
     a.npair = P.npu;
     a.vstr = P.vstr;
     a.max_packs = ab_packs(c, p);
-    a.nbatch = P.nbatch;
     a.np = P.np;
     a.panel = (int)q;
     a.nmain = p.nmain;
@@ -2128,18 +2129,18 @@ int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
     a.wsteps = p.wsteps;
     a.ex_row = p.ex_row;
     a.ex_off = p.ex_off;
-    a.items = it.ab_item;
-    a.split = it.ab_split;
-    a.slot_split = it.ab_slot;
-    a.done = it.ab_done;
+    a.items = it.item;
+    a.split = it.split;
+    a.slot_split = it.slot;
+    a.done = it.done;
     a.ypart = it.ypart;
     a.Y = c->d_yab;
     a.err = c->d_err;
     const size_t smem = (((size_t)p.ny * 8 + 15) & ~(size_t)15) + 16 * (size_t)a.max_packs * P.vstr;
     int rc;
-    if (P.threads == 256) rc = launch_ab<T, 256, 4>(c, a, it.n_item, smem);
-    else if (P.threads == 512) rc = launch_ab<T, 512, 2>(c, a, it.n_item, smem);
-    else rc = launch_ab<T, 1024, 1>(c, a, it.n_item, smem);
+    if (P.threads == 256) rc = launch_ab<T, 256, 4>(c, a, it.n, smem);
+    else if (P.threads == 512) rc = launch_ab<T, 512, 2>(c, a, it.n, smem);
+    else rc = launch_ab<T, 1024, 1>(c, a, it.n, smem);
     if (rc) return rc;
   }
   return 0;

@@ -104,3 +104,32 @@ def test_sigma_with_few_pairs_in_use(size, port):
     top = np.abs(ref).max()
     assert np.abs(S - ref).max() <= 1e-12 * top
     assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top
+
+
+@pytest.mark.parametrize("size", [(24, 5, 5, 1, 2100), (24, 5, 5, 3, 5001), (24, 5, 5, 20, 2600), (24, 5, 5, 90, 4100),
+                                  (20, 4, 4, 40, 2049), (30, 5, 5, 9, 1100)])
+def test_sigma_with_few_alpha_strings(size, port):
+    """Few alpha strings against many beta strings: the alpha-beta items are
+    split over the schedule's batches (from four batches on) and their partial
+    rows added in order, in whole and row-range products."""
+    torch = pytest.importorskip("torch")
+    prob = synth.random_problem(*size, seed=sum(size))
+    C = np.random.default_rng(8).standard_normal(prob.D)
+    x = torch.from_numpy(C).cuda()
+    x32 = x.float()
+    s32 = torch.empty_like(x32)
+    ref = port.sigma(prob, C)
+    top = np.abs(ref).max()
+    with sbdx.Context(0) as ctx:
+        ctx.load(prob)
+        S = ctx.sigma(C)
+        again = ctx.sigma(C)
+        ctx.sigma_device(sbdx.SBDX_FP32, x32.data_ptr(), s32.data_ptr())
+        a0 = prob.na // 2 // 8 * 8
+        rows = torch.empty((prob.na - a0, prob.nb), dtype=torch.float64, device="cuda")
+        ctx.sigma_rows_device(sbdx.SBDX_FP64, x.data_ptr(), rows.data_ptr(), a0, prob.na)
+        torch.cuda.synchronize()
+    assert np.abs(S - ref).max() <= 1e-12 * top
+    assert np.array_equal(S, again)
+    assert np.abs(rows.cpu().numpy() - ref.reshape(prob.na, prob.nb)[a0:]).max() <= 1e-12 * top
+    assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top

@@ -453,8 +453,9 @@ int build_same_blocks(Ctx* c, const Conn& cn, const std::vector<uint64_t>& strin
 // connect to ten times the mean) would set its duration: strings are split
 // into items of at most cap singles, cap = a quarter of the mean work per SM
 // rounded up to whole groups of the kernel (10 singles in FP64, 20 with FP32
-// storage), and items run longest first. Large samples have many strings per
-// SM and split nothing. Where the items are fewer than the CTAs that the GPU
+// storage; two groups in FP64 where single ones are short and more than the CTAs
+// that the GPU holds: 400 x 400 strings, 45 against 39 us), and items run longest
+// first. Large samples have many strings per SM and split nothing. Where the items are fewer than the CTAs that the GPU
 // holds, they are split over the schedule's batches too, into ranges of like
 // numbers of steps, from four batches on (below, the partial rows cost what the
 // split saves: 400 x 400 strings, two batches, 39 -> 45 us). Alpha-beta time
@@ -471,9 +472,15 @@ int build_ab_items(Ctx* c, AbItems (&out)[2], std::vector<uint32_t> hs, size_t n
   const uint64_t quarter = (total + 4 * nsm - 1) / (4 * nsm);
   for (int q = 0; q < 2; ++q) {
     const uint64_t group = kAbPacks * (q == 0 ? 2 : 4);
-    const uint32_t cap = (uint32_t)std::max<uint64_t>(group, (quarter + group - 1) / group * group);
+    uint32_t cap = 0;
     uint64_t whole = 0;
-    for (uint32_t h : hs) whole += (h + cap - 1) / cap;
+    auto set_cap = [&](uint64_t unit) {
+      cap = (uint32_t)std::max<uint64_t>(unit, (quarter + unit - 1) / unit * unit);
+      whole = 0;
+      for (uint32_t h : hs) whole += (h + cap - 1) / cap;
+    };
+    set_cap(group);
+    if (q == 0 && P.nbatch < 4 && whole > resident) set_cap(2 * group);
     const uint64_t want = whole && P.nbatch >= 4 ? (resident + whole - 1) / whole : 1;
     const int ways = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)P.nbatch));
     // batch ranges of like numbers of steps

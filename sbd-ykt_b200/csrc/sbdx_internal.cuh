@@ -85,10 +85,12 @@ struct AbPlan {
   std::vector<uint64_t> steps;  // [nbatch] over all panels
 };
 
-// Bra strings per block of the blocked same-spin kernels, and the determinant
-// counts from which the default launch codes use them (FP64, FP32 storage).
+// Bra strings per block of the blocked same-spin kernels, the determinant
+// counts from which the default launch codes use them (FP64, FP32 storage), and
+// the columns of a product that they need for that (FP64).
 constexpr int kBlkRows64 = 8, kBlkRows32 = 4;
 constexpr size_t kBlkMinDets64 = 2000000, kBlkMinDets32 = 1000000;
+constexpr size_t kBlkMinCols64 = 448;
 constexpr uint32_t kNoRow = 0xffffffffu;
 
 // Blocks of the blocked same-spin kernels over the bra strings [row0, row1)
@@ -225,15 +227,11 @@ struct StoredH {
   uint64_t nnz = 0;             // off-diagonal elements, padding not counted
 };
 
-// Launch shape of the sigma kernels. Codes (also the C-ABI encoding):
-//   same-spin: 1/2/4/8 = columns per thread of the prefix-parity-table kernel,
-//              11/12/14 = 1/2/4 columns of the popcount kernel
-//   alpha-beta: 10*variant + staged rows; variant 1 = shared-memory staging,
-//              2 = double-buffered TMA staging, 3 = staging with 512-thread CTAs,
-//              4 = staging with SELL-32 records, 0 = L1 gathers (rows 1-4)
+// Launch shape of the sigma kernels (the codes of sbdx_set_tuning).
 struct Tune {
   int same_code = 0;  // 0 = built-in default for the precision
   int ab_code = 0;
+  bool by_size = false;  // same_code is the default: a product with few columns takes its own
 };
 
 struct Ctx {

@@ -2190,6 +2190,8 @@ int launch_same_blk(Ctx* c, int vec, const float* X, size_t ncol, size_t ldx, co
   return launch_same_blkf<1>(c, X, ncol, ldx, B, Y);
 }
 
+constexpr int kStrings64 = 22;  // the one-string kernel that serves FP64 best
+
 // Same-spin codes: 21, 22, 24, 28 = 1, 2, 4, 8 columns per thread of the
 // one-string kernels, narrowed to the widest vector that divides the row
 // stride and keeps 16-byte alignment (the internal vectors have strides
@@ -2197,8 +2199,10 @@ int launch_same_blk(Ctx* c, int vec, const float* X, size_t ncol, size_t ldx, co
 // the blocked kernels, whose FP64 form has one shape (128 columns per warp) and
 // whose FP32 form takes up to 4 columns per thread.
 template <typename T>
-int run_same_v6(Ctx* c, int code, const T* X, size_t ncol, size_t ldx, const Conn& cn, size_t row0, size_t nrow,
+int run_same_v6(Ctx* c, const Tune& tune, const T* X, size_t ncol, size_t ldx, const Conn& cn, size_t row0, size_t nrow,
                 const typename Prec<T>::V* val, const typename Prec<T>::V* Dt, size_t dstride, double* Y) {
+  int code = tune.same_code;
+  if (tune.by_size && std::is_same<T, double>::value && ncol < kBlkMinCols64) code = kStrings64;
   int vec = code % 10;
   const bool aligned = (reinterpret_cast<uintptr_t>(X) % 16) == 0;
   while (vec > 1 && (!aligned || ldx % vec != 0 || (Dt != nullptr && dstride % vec != 0))) vec >>= 1;
@@ -2364,9 +2368,9 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
     SideBySide f(c);
     if ((rc = f.fork())) return rc;
     f.on(0);
-    rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, c->d_y);
+    rc = run_same_v6<T>(c, tune, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, c->d_y);
     f.on(1);
-    if (!rc) rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt);
+    if (!rc) rc = run_same_v6<T>(c, tune, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt);
     f.main();
     if (!rc) rc = run_ab_packed<T>(c);
     const int rj = f.join();
@@ -2374,10 +2378,10 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
     return launch_combine<T>(c, X, 0, na, S, true);
   }
   mark(1);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, c->d_y)))
+  if ((rc = run_same_v6<T>(c, tune, xp, nb, c->xsa, ca, 0, na, valA, DtA, c->db_stride, c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt)))
+  if ((rc = run_same_v6<T>(c, tune, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt)))
     return rc;
   mark(3);
   if ((rc = run_ab_v6<T>(c, tune.ab_code, xp))) return rc;
@@ -2453,12 +2457,16 @@ int run_sigma_v5(Ctx* c, const T* X, T* S) {
 // above a size where the grid of their blocks still fills the GPU and the
 // strings of a block share excitations, the one-string-per-CTA kernel below it.
 // Measured on both sides of the lines (alpha and beta same-spin, us): FP64,
-// 2000 x 2000: 278 and 205 blocked, 385 and 351 by strings; FP32, 613 x 1187:
-// 97 and 44 blocked, 58 and 47 by strings.
+// 2000 x 2000: 278 and 205 blocked, 368 and 370 by strings; FP32, 613 x 1187:
+// 97 and 44 blocked, 58 and 47 by strings. In FP64 the blocked kernel gives a
+// warp 128 columns of a strip of 1024, so a product with few columns (the other
+// spin's strings, or the rows of a range) leaves most warps idle: 7 electrons
+// in 58 orbitals, us, blocked / by strings: 100 columns of 20000 strings 2345 /
+// 1097, 250 of 8000 560 / 374, 400 of 8000 615 / 574, 500 of 5000 314 / 350.
 Tune default_tune(const Ctx* c, bool f64) {
   const size_t D = c->na * c->nb;
-  if (f64) return D >= kBlkMinDets64 ? Tune{34, 71} : Tune{22, 71};
-  return D >= kBlkMinDets32 ? Tune{34, 71} : Tune{24, 71};
+  if (f64) return D >= kBlkMinDets64 ? Tune{34, 71, true} : Tune{kStrings64, 71, true};
+  return D >= kBlkMinDets32 ? Tune{34, 71, true} : Tune{24, 71, true};
 }
 
 Tune effective_tune(const Ctx* c, bool f64) {
@@ -2467,7 +2475,7 @@ Tune effective_tune(const Ctx* c, bool f64) {
   const bool v6 = same_alpha_first(t.same_code) || (t.ab_code > 60 && t.ab_code < 70) ||
                   t.ab_code == 71 || (t.same_code == 0 && t.ab_code == 0);
   if (v6) {
-    if (t.same_code == 0) t.same_code = d.same_code;
+    if (t.same_code == 0) t.same_code = d.same_code, t.by_size = true;
     if (t.ab_code == 0) t.ab_code = d.ab_code;
   }
   return t;
@@ -2519,10 +2527,10 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
   if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, true))) return rc;
   mark(1);
   if (nr == 0) return 0;
-  if ((rc = run_same_v6<T>(c, tune.same_code, xp, nb, c->xsa, ra, a0, nr, valA, Db, c->db_stride, c->d_y)))
+  if ((rc = run_same_v6<T>(c, tune, xp, nb, c->xsa, ra, a0, nr, valA, Db, c->db_stride, c->d_y)))
     return rc;
   mark(2);
-  if ((rc = run_same_v6<T>(c, tune.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, valB, (const V*)nullptr, 0, c->d_yt + a0)))
+  if ((rc = run_same_v6<T>(c, tune, xpt + a0, nr, c->xsb, cb, 0, nb, valB, (const V*)nullptr, 0, c->d_yt + a0)))
     return rc;
   mark(3);
   if ((rc = run_ab_packed<T>(c, &rc_items))) return rc;
@@ -2953,7 +2961,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
     SBDX_CUDA(c, cudaStreamWaitEvent(c->stream, ev[i], 0));
     if ((rc = launch_split<double>(c, din, a0, nr, xp, xpt, true))) return rc;
-    if ((rc = run_same_v6<double>(c, t.same_code, xpt + a0, nr, c->xsb, cb, 0, nb, cb.val, (const double*)nullptr, 0,
+    if ((rc = run_same_v6<double>(c, t, xpt + a0, nr, c->xsb, cb, 0, nb, cb.val, (const double*)nullptr, 0,
                                   c->d_yt + a0)))
       return rc;
   }
@@ -2974,7 +2982,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     ra.n_same_split = it.n_same_split;
     ra.n_same_part = it.n_same_part;
     ra.same_ypart = it.same_ypart;
-    if ((rc = run_same_v6<double>(c, t.same_code, xp, nb, c->xsa, ra, a0, nr, ca.val, c->d_Db, c->db_stride, c->d_y)))
+    if ((rc = run_same_v6<double>(c, t, xp, nb, c->xsa, ra, a0, nr, ca.val, c->d_Db, c->db_stride, c->d_y)))
       return rc;
     if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true))) return rc;
     SBDX_CUDA(c, cudaEventRecord(ev[n + i], c->stream));

@@ -80,20 +80,29 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
   // of 4 consecutive columns go to the panels in turn, so that every panel
   // gets its share of each list. Slots: the panel's strings plus extras; their
   // room is estimated and checked below.
-  auto fits = [&](int packs, size_t slots) {
-    return 16 * (size_t)packs * P.vstr + sizeof(double) * slots + kAbStaticSmem <= kAbSmemBudget;
+  auto fits = [&](int packs, size_t slots, size_t budget = kAbSmemBudget) {
+    return 16 * (size_t)packs * P.vstr + sizeof(double) * slots + kAbStaticSmem <= budget;
   };
+  // Two CTAs of 512 threads share an SM where three packs fit in half of it: one
+  // stages integrals while the other one uses its own. Alpha-beta time with one
+  // CTA and five packs / two CTAs and three or four, 7 electrons in 58 orbitals,
+  // us: 8000 x 440 strings FP64 2499 / 1863, FP32 1709 / 1215; 3000 x 500 879 /
+  // 743 and 593 / 479; 2000 x 2000 980 / 952 and 648 / 583; with a single pack,
+  // 300 x 8000, 514 / 967.
+  constexpr int kHalfPacks = 3;
+  bool halves = true;
   size_t np = 1;
   for (;; ++np) {
     const size_t per = (n + np - 1) / np + 4, est = per + per / 8 + 512;
     if (fits(kAbPacks, est) || (fits(kAbPacks - 1, est) && kAbPacks > 1)) break;
     if (per <= 8) break;
   }
-  for (;; ++np) {
+  for (;;) {
     const size_t per = (n + np - 1) / np + 4;
-    const bool small = 16 * (size_t)kAbPacks * P.vstr + sizeof(double) * (per + per / 8 + 512) + kAbStaticSmem <=
-                       kAbSmemBudget / 2;
-    const int nt = small ? (vk.size() <= 256 ? 256 : 512) : (vk.size() <= 512 ? 512 : 1024);
+    halves = halves && fits(kHalfPacks, per + per / 8 + 512, kAbSmemBudget / 2);
+    const bool quarters = vk.size() <= 256 && fits(kAbPacks, per + per / 8 + 512, kAbSmemBudget / 2);
+    P.smem = halves ? kAbSmemBudget / 2 : kAbSmemBudget;
+    const int nt = quarters ? 256 : halves || vk.size() <= 512 ? 512 : 1024;
     const size_t nbatch = std::max<size_t>(1, (vk.size() + nt - 1) / nt);
     const double effort =
         std::min(120.0, (double)alpha_singles * (double)total / 2e8);  // 2.4e10 pairs: 120 moves per record
@@ -152,12 +161,16 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
       }
       w.nex = (int)w.ex_row.size();
       w.ny = w.nmain + (int)w.s0[w.nmain];
-      int packs = 0;
-      for (int k = 1; k <= kAbPacks; ++k)
-        if (fits(k, w.ny)) packs = k;
-      if (w.ny > 0xffff || packs < std::min(kAbPacks, 4)) { ok = false; break; }
+      if (w.ny > 0xffff || !fits(halves ? kHalfPacks : kAbPacks - 1, w.ny, P.smem)) { ok = false; break; }
     }
-    if (!ok && np < n / 4 + 1) continue;
+    if (!ok && halves) {  // the extra slots need more room than half an SM
+      halves = false;
+      continue;
+    }
+    if (!ok && np < n / 4 + 1) {
+      ++np;
+      continue;
+    }
     if (!ok) {
       c->err = "build_connectivity: the alpha-beta schedule does not fit in shared memory";
       return SBDX_ERR_ARG;
@@ -188,6 +201,9 @@ int build_ab_plan(Ctx* c, size_t n, const std::vector<uint32_t>& hs, const std::
     if (rc || (rc = up(pairs, &P.pairs))) return rc;
     P.panels.resize(np);
     P.steps.assign(nbatch, 0);
+    P.packs = kAbPacks;
+    for (const PanelWork& w : W)
+      while (P.packs > 1 && !fits(P.packs, w.ny, P.smem)) --P.packs;
     for (size_t q = 0; q < np; ++q) {
       PanelWork& w = W[q];
       AbPanel& A = P.panels[q];

@@ -452,8 +452,8 @@ int build_same_blocks(Ctx* c, const Conn& cn, const std::vector<uint64_t>& strin
 // a few strings with many singles (near-Aufbau strings of a small sample
 // connect to ten times the mean) would set its duration: strings are split
 // into items of at most cap singles, cap = a quarter of the mean work per SM
-// rounded up to whole groups of the kernel (10 singles in FP64, 20 with FP32
-// storage; two groups in FP64 where single ones are short and more than the CTAs
+// rounded up to whole groups of the kernel (up to 10 singles in FP64, 20 with
+// FP32 storage; two groups in FP64 where single ones are short and more than the CTAs
 // that the GPU holds: 400 x 400 strings, 45 against 39 us), and items run longest
 // first. Large samples have many strings per SM and split nothing. Where the items are fewer than the CTAs that the GPU
 // holds, they are split over the schedule's batches too, into ranges of like
@@ -466,12 +466,12 @@ int build_same_blocks(Ctx* c, const Conn& cn, const std::vector<uint64_t>& strin
 int build_ab_items(Ctx* c, AbItems (&out)[2], std::vector<uint32_t> hs, size_t nb, size_t row0 = 0) {
   const AbPlan& P = c->ab;
   const uint64_t nsm = (uint64_t)sm_count(c);
-  const uint64_t resident = nsm * (P.threads == 256 ? 4 : P.threads == 512 ? 2 : 1);
+  const uint64_t resident = nsm * (P.threads == 256 ? 4 : P.smem < kAbSmemBudget ? 2 : 1);
   uint64_t total = 0;
   for (uint32_t& h : hs) total += ++h;  // the string itself counts as one more
   const uint64_t quarter = (total + 4 * nsm - 1) / (4 * nsm);
   for (int q = 0; q < 2; ++q) {
-    const uint64_t group = kAbPacks * (q == 0 ? 2 : 4);
+    const uint64_t group = (uint64_t)P.packs * (q == 0 ? 2 : 4);
     uint32_t cap = 0;
     uint64_t whole = 0;
     auto set_cap = [&](uint64_t unit) {

@@ -73,6 +73,8 @@ struct AbPlan {
   uint32_t* vket = nullptr;  // [xs] ket string of each lane
   size_t xs = 0;             // nbatch * threads: row stride of Ctx::d_xk
   int threads = 0, nbatch = 0, np = 0;
+  size_t smem = 0;           // shared memory that a CTA may take
+  int packs = 0;             // packs per group that fit (kAbPacks at most)
   // the pairs that a beta single has, ascending: the records' pair index counts
   // them, and the integrals (all rows, V[pq * vstride + t]) keep these columns only
   uint32_t* pairs = nullptr;  // [npu]

@@ -2077,13 +2077,6 @@ __global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
   }
 }
 
-// Packs of a group that fit beside a panel's y slots.
-int ab_packs(const Ctx* c, const AbPanel& p) {
-  int k = kAbPacks;
-  while (k > 1 && 16 * (size_t)k * c->ab.vstr + sizeof(double) * (size_t)p.ny + kAbStaticSmem > kAbSmemBudget) --k;
-  return k;
-}
-
 template <typename T, int NT, int MINB>
 int launch_ab(Ctx* c, const AbArgs<T>& args, size_t n_item, size_t smem) {
   SBDX_CUDA(c, cudaFuncSetAttribute(sigma_ab_kernel<T, NT, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2117,7 +2110,7 @@ int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
     a.vstride = f64 ? P.vstride : P.vstride32;
     a.npair = P.npu;
     a.vstr = P.vstr;
-    a.max_packs = ab_packs(c, p);
+    a.max_packs = P.packs;
     a.np = P.np;
     a.panel = (int)q;
     a.nmain = p.nmain;

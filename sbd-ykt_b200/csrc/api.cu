@@ -40,6 +40,33 @@ cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes) {
   return cudaMallocFromPoolAsync(p, bytes, c->pool, c->stream);
 }
 
+cudaError_t direct_alloc(Ctx* c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && c->pool && c->own_pool) {
+    cudaGetLastError();
+    cudaStreamSynchronize(c->stream);  // the releases queued on the stream
+    cudaMemPoolTrimTo(c->pool, 0);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e == cudaSuccess) c->direct.push_back(*p);
+  return e;
+}
+
+void dev_free(Ctx* c, void* p) {
+  if (!p) return;
+  for (size_t k = 0; k < c->direct.size(); ++k)
+    if (c->direct[k] == p) {
+      c->direct[k] = c->direct.back();
+      c->direct.pop_back();
+      cudaFree(p);
+      return;
+    }
+  if (cudaFreeAsync(p, c->stream) != cudaSuccess) {  // e.g. a stream its owner has destroyed
+    cudaGetLastError();
+    cudaFree(p);
+  }
+}
+
 void pool_trim(Ctx* c) {
   if (!c->pool || !c->own_pool) return;
   uint64_t reserved = 0, in_use = 0;
@@ -77,11 +104,7 @@ namespace {
 void free_vector_state(Ctx* c) {
   sbdx::clear_sigma_graphs(c);
   dev_free(c, c->d_hii); c->d_hii = nullptr; c->have_hii = false;
-  dev_free(c, c->d_xt); c->d_xt = nullptr;
-  dev_free(c, c->d_xp); c->d_xp = nullptr;
-  dev_free(c, c->d_y); c->d_y = nullptr;
-  dev_free(c, c->d_yt); c->d_yt = nullptr;
-  dev_free(c, c->d_yab); c->d_yab = nullptr;
+  sbdx::free_sigma_scratch(c);
   dev_free(c, c->d_io_in); c->d_io_in = nullptr;
   dev_free(c, c->d_io_out); c->d_io_out = nullptr;
   dev_free(c, c->d_wf); c->d_wf = nullptr; c->wf_roots = 0; c->wf_cap = 0;

@@ -815,8 +815,6 @@ void free_connectivity(Ctx* c) {
   free_conn(c, c->conn[0]);
   free_conn(c, c->conn[1]);
   free_ab_plan(c, c->ab);
-  dev_free(c, c->d_xk);  // sized by the schedule
-  c->d_xk = nullptr;
   dev_free(c, c->d_Dr); dev_free(c, c->d_Dr32);
   c->d_Dr = nullptr;
   c->d_Dr32 = nullptr;

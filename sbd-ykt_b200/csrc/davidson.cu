@@ -589,11 +589,12 @@ struct Work {
   uint32_t* ctr = nullptr;    // arrivals of finish_sums
 };
 
-// A solve's device buffers, released on its stream; the pool keeps a bounded
-// part of them for the next solve.
+// A solve's device buffers, released on its stream. What the pool keeps for
+// the next solve comes from it, the rest from cudaMalloc (see dev_alloc).
 struct SolveBuffers {
   Ctx* c;
   std::vector<void*> p;
+  size_t pooled = 0;
   explicit SolveBuffers(Ctx* ctx) : c(ctx) {}
   ~SolveBuffers() {
     for (void* q : p) dev_free(c, q);
@@ -601,8 +602,12 @@ struct SolveBuffers {
   }
   template <typename T>
   cudaError_t get(T** d, size_t bytes) {
-    const cudaError_t e = dev_alloc(c, d, bytes);
-    if (e == cudaSuccess) p.push_back(*d);
+    const bool pool = pooled + bytes <= kPoolKeep || (c->pool && !c->own_pool);
+    const cudaError_t e = pool ? pool_alloc(c, reinterpret_cast<void**>(d), bytes)
+                               : direct_alloc(c, reinterpret_cast<void**>(d), bytes);
+    if (e != cudaSuccess) return e;
+    if (pool) pooled += bytes;
+    p.push_back(*d);
     return e;
   }
 };
@@ -1602,42 +1607,20 @@ int davidson_block(Ctx* c, const sbdx_davidson_params& p, int k, double* dW, dou
   const int nc = std::max(std::min(kMixed ? 2 * p.max_nb : p.max_nb, 64 - k), 2 * k);
   const int keep = std::max(k, nc / 3);
   const int period = p.defect_every > 0 ? p.defect_every : 0;
-  // stream-ordered allocations: several solves can run concurrently on their
-  // own streams without a device-wide synchronisation at allocation or release
-  struct AsyncGuard {
-    Ctx* c;
-    std::vector<void*> p;
-    ~AsyncGuard() {
-      for (void* q : p) cudaFreeAsync(q, c->stream);
-      pool_trim(c);
-    }
-  } g{c, {}};
-  auto alloc = [&](void** ptr, size_t bytes) -> cudaError_t {
-    const cudaError_t e = pool_alloc(c, ptr, bytes);
-    if (e == cudaSuccess) g.p.push_back(*ptr);
-    return e;
-  };
-  Work wk;  // its pointers stay owned by g (Work's destructor frees null pointers)
-  double *wpartial = nullptr, *wscal = nullptr, *wu = nullptr;
-  SBDX_CUDA(c, alloc((void**)&wpartial, sizeof(double) * kRedBlocks * (2 * nc + 2 * kMaxRoots + 4)));
-  SBDX_CUDA(c, alloc((void**)&wscal, sizeof(double) * (kbDots + (size_t)(k + 2) * nc + 64)));
-  SBDX_CUDA(c, alloc((void**)&wu, sizeof(double) * ((size_t)(k + nc) * k + k + nc + 8)));
-  SBDX_CUDA(c, alloc((void**)&wk.ctr, sizeof(uint32_t)));
+  SolveBuffers g(c);  // in a batch all from its pool: no device-wide synchronisation at allocation or release
+  Work wk;
+  SBDX_CUDA(c, g.get(&wk.partial, sizeof(double) * kRedBlocks * (2 * nc + 2 * kMaxRoots + 4)));
+  SBDX_CUDA(c, g.get(&wk.scal, sizeof(double) * (kbDots + (size_t)(k + 2) * nc + 64)));
+  SBDX_CUDA(c, g.get(&wk.u, sizeof(double) * ((size_t)(k + nc) * k + k + nc + 8)));
+  SBDX_CUDA(c, g.get(&wk.ctr, sizeof(uint32_t)));
   SBDX_CUDA(c, cudaMemsetAsync(wk.ctr, 0, sizeof(uint32_t), c->stream));
   TC *C = nullptr, *HC = nullptr;
   double *A = nullptr, *R = nullptr, *V = nullptr;
-  SBDX_CUDA(c, alloc((void**)&C, sizeof(TC) * D * nc));
-  SBDX_CUDA(c, alloc((void**)&HC, sizeof(TC) * D * nc));
-  SBDX_CUDA(c, alloc((void**)&A, sizeof(double) * D * 4 * k));  // W | HW | W' | HW'
-  SBDX_CUDA(c, alloc((void**)&R, sizeof(double) * D * k));
-  SBDX_CUDA(c, alloc((void**)&V, sizeof(double) * D));
-  struct Borrow {
-    Work& w;
-    ~Borrow() { w.partial = w.scal = w.u = nullptr; }
-  } borrow{wk};
-  wk.partial = wpartial;
-  wk.scal = wscal;
-  wk.u = wu;
+  SBDX_CUDA(c, g.get(&C, sizeof(TC) * D * nc));
+  SBDX_CUDA(c, g.get(&HC, sizeof(TC) * D * nc));
+  SBDX_CUDA(c, g.get(&A, sizeof(double) * D * 4 * k));  // W | HW | W' | HW'
+  SBDX_CUDA(c, g.get(&R, sizeof(double) * D * k));
+  SBDX_CUDA(c, g.get(&V, sizeof(double) * D));
   double* W = A;
   double* HW = A + D * k;
   double* Wn = A + 2 * D * k;
@@ -2243,55 +2226,40 @@ int davidson_block_graph(Ctx* c, const sbdx_davidson_params& p, int k, double* d
   const int keep = std::max(k, nc / 3);
   const int period = p.defect_every > 0 ? p.defect_every : 0;
   const int ld = k + nc;
-  struct AsyncGuard {
+  SolveBuffers buf(c);
+  struct Guard {
     Ctx* c;
-    std::vector<void*> p;
     void* host = nullptr;
     std::vector<cudaGraphExec_t> execs;
-    ~AsyncGuard() {
+    ~Guard() {
       cudaStreamSynchronize(c->stream);
       for (cudaGraphExec_t e : execs) cudaGraphExecDestroy(e);
-      for (void* q : p) cudaFreeAsync(q, c->stream);
       if (host) cudaFreeHost(host);
-      pool_trim(c);
     }
-  } g{c, {}};
-  auto alloc = [&](void** ptr, size_t bytes) -> cudaError_t {
-    const cudaError_t e = pool_alloc(c, ptr, bytes);
-    if (e == cudaSuccess) g.p.push_back(*ptr);
-    return e;
-  };
+  } g{c};
   Work wk;
-  double *wpartial = nullptr, *wscal = nullptr, *wu = nullptr;
-  SBDX_CUDA(c, alloc((void**)&wpartial, sizeof(double) * kRedBlocks * (2 * nc + 2 * kMaxRoots + 4)));
-  SBDX_CUDA(c, alloc((void**)&wscal, sizeof(double) * (kbDots + 2 * (size_t)k * (nc + 2 * k) + 64)));
-  SBDX_CUDA(c, alloc((void**)&wu, sizeof(double) * ((size_t)(k + nc) * k + k + nc + 8)));
-  SBDX_CUDA(c, alloc((void**)&wk.ctr, sizeof(uint32_t)));
+  SBDX_CUDA(c, buf.get(&wk.partial, sizeof(double) * kRedBlocks * (2 * nc + 2 * kMaxRoots + 4)));
+  SBDX_CUDA(c, buf.get(&wk.scal, sizeof(double) * (kbDots + 2 * (size_t)k * (nc + 2 * k) + 64)));
+  SBDX_CUDA(c, buf.get(&wk.u, sizeof(double) * ((size_t)(k + nc) * k + k + nc + 8)));
+  SBDX_CUDA(c, buf.get(&wk.ctr, sizeof(uint32_t)));
   SBDX_CUDA(c, cudaMemsetAsync(wk.ctr, 0, sizeof(uint32_t), c->stream));
   TC *C = nullptr, *HC = nullptr;
   double *A = nullptr, *R = nullptr, *V = nullptr, *dM = nullptr, *dS = nullptr, *misc = nullptr;
   int* dead = nullptr;
   GStatus* dst = nullptr;
-  SBDX_CUDA(c, alloc((void**)&C, sizeof(TC) * D * nc));
-  SBDX_CUDA(c, alloc((void**)&HC, sizeof(TC) * D * nc));
-  SBDX_CUDA(c, alloc((void**)&A, sizeof(double) * D * 4 * k));  // anchors: [W | HW] twice, the current by parity
-  SBDX_CUDA(c, alloc((void**)&R, sizeof(double) * D * k));
-  SBDX_CUDA(c, alloc((void**)&V, sizeof(double) * D));
-  SBDX_CUDA(c, alloc((void**)&dM, sizeof(double) * ld * ld));
-  SBDX_CUDA(c, alloc((void**)&dS, sizeof(double) * ld * ld));
-  SBDX_CUDA(c, alloc((void**)&misc, sizeof(double) * 16));  // fs[4], before
-  SBDX_CUDA(c, alloc((void**)&dead, sizeof(int) * nc));
-  SBDX_CUDA(c, alloc((void**)&dst, sizeof(GStatus)));
+  SBDX_CUDA(c, buf.get(&C, sizeof(TC) * D * nc));
+  SBDX_CUDA(c, buf.get(&HC, sizeof(TC) * D * nc));
+  SBDX_CUDA(c, buf.get(&A, sizeof(double) * D * 4 * k));  // anchors: [W | HW] twice, the current by parity
+  SBDX_CUDA(c, buf.get(&R, sizeof(double) * D * k));
+  SBDX_CUDA(c, buf.get(&V, sizeof(double) * D));
+  SBDX_CUDA(c, buf.get(&dM, sizeof(double) * ld * ld));
+  SBDX_CUDA(c, buf.get(&dS, sizeof(double) * ld * ld));
+  SBDX_CUDA(c, buf.get(&misc, sizeof(double) * 16));  // fs[4], before
+  SBDX_CUDA(c, buf.get(&dead, sizeof(int) * nc));
+  SBDX_CUDA(c, buf.get(&dst, sizeof(GStatus)));
   GStatus* hst = nullptr;
   SBDX_CUDA(c, cudaMallocHost((void**)&hst, sizeof(GStatus) * kStatusSlots));
   g.host = hst;
-  struct Borrow {
-    Work& w;
-    ~Borrow() { w.partial = w.scal = w.u = nullptr; }
-  } borrow{wk};
-  wk.partial = wpartial;
-  wk.scal = wscal;
-  wk.u = wu;
   double* s = wk.scal;
   double* gso = wk.u;
   double* Xd = wk.u + k + nc + 8;

@@ -93,6 +93,12 @@ struct AbPlan {
 constexpr int kBlkRows64 = 8, kBlkRows32 = 4;
 constexpr size_t kBlkMinDets64 = 2000000, kBlkMinDets32 = 1000000;
 constexpr size_t kBlkMinCols64 = 448;
+// Determinants from which the sigma keeps four vectors of scratch instead of
+// more than six (see Ctx::lean): 1 GB each. The products are then not side by
+// side and the lanes take a pass of their own, which costs 4% at 3000 x 3000
+// strings, 2.7% at 5600 x 5600 and 1.2% at 8000 x 8000 (FP64; FP32 4.5%, 4.5% and
+// 0.5%).
+constexpr size_t kLeanDets = size_t(1) << 27;
 constexpr uint32_t kNoRow = 0xffffffffu;
 
 // Blocks of the blocked same-spin kernels over the bra strings [row0, row1)
@@ -298,10 +304,17 @@ struct Ctx {
   // kernels load whole vectors of columns whatever na and nb are.
   void* d_xt = nullptr;     // nb x xsb elements of the widest type used (8 B)
   void* d_xp = nullptr;     // na x xsa elements (8 B): phi o C, the input in the alpha-first basis
-  void* d_xk = nullptr;     // na x ab.xs elements (8 B): phi o C with its columns in the lane order of `ab`
   double* d_y = nullptr;    // na x xsa FP64: alpha same-spin part of sigma
-  double* d_yab = nullptr;  // na x xsa FP64: opposite-spin part (packed alpha-beta kernel)
   double* d_yt = nullptr;   // nb x xsb FP64: beta same-spin part, beta-major
+  void* d_xk = nullptr;     // na x ab.xs elements (8 B): phi o C with its columns in the lane order of `ab`
+  double* d_yab = nullptr;  // na x xsa FP64: opposite-spin part (packed alpha-beta kernel)
+  // All of them lie in one allocation. Problems of kLeanDets determinants or more
+  // have no d_yab and d_xk: their products run one after another, and the lanes
+  // take the room of two neighbouring vectors that are not in use by then
+  // (run_ab_71, sigma_host).
+  double* d_scratch = nullptr;
+  size_t scratch_size = 0;  // elements
+  bool lean = false;
   size_t xsa = 0, xsb = 0;
   // the three independent products of one sigma run side by side: the packed
   // alpha-beta one on the context stream, the same-spin ones on these
@@ -353,6 +366,7 @@ struct Ctx {
   // pool among its subspaces and trims it after the batch.
   cudaMemPool_t pool = nullptr;
   bool own_pool = false;
+  std::vector<void*> direct;  // large buffers that come from cudaMalloc (dev_alloc)
   std::vector<SigmaGraph> graphs;
   // optional per-phase timing of the sigma (CUDA events on the context stream)
   bool profiling = false;
@@ -496,6 +510,7 @@ int build_stored(Ctx* c);
 void release_stored(Ctx* c);
 int stored_sigma(Ctx* c, const double* X, double* S);
 int ensure_sigma_scratch(Ctx* c);
+void free_sigma_scratch(Ctx* c);
 // phi o W (FP64, na x nb) into d_xp (row stride xsa) and its transpose into d_xt (row stride xsb).
 int phase_vectors(Ctx* c, const double* W);
 void clear_sigma_graphs(Ctx* c);
@@ -506,20 +521,25 @@ int autotune(Ctx* c);
 int check_device_error(Ctx* c);
 // Stream-ordered allocation from the context's pool (created on first use).
 cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes);
-// The same for any element type, and its release on the context stream. Every
-// device buffer of a context but the stored Hamiltonian comes from here:
-// cudaMalloc and cudaFree take 0.1 ms each and synchronise the device, which
-// cost a diag call on 400 x 400 strings 17 of 29 ms.
+// A buffer of its own, outside the pool; on failure the pool's unused memory is
+// given back first and the request repeated.
+cudaError_t direct_alloc(Ctx* c, void** p, size_t bytes);
+// Any buffer of a context but the stored Hamiltonian: small ones from the pool
+// (cudaMalloc and cudaFree take 0.35 and 0.45 ms and synchronise the device,
+// which cost a diag call on 400 x 400 strings 17 of 29 ms), large ones by
+// themselves (a growing pool maps 1 GB in 5 to 6 ms, cudaMalloc in under 1 ms, and
+// both cost the same near 64 MB; the first product on 8000 x 8000 strings took
+// 46 ms with its vectors in the pool and takes 29). The contexts of a
+// batch share a pool, so that no solve synchronises the others, and take all
+// from it.
+constexpr size_t kDirectBytes = size_t(64) << 20;
 template <typename T>
 cudaError_t dev_alloc(Ctx* c, T** p, size_t bytes) {
+  if (bytes >= kDirectBytes && (c->own_pool || !c->pool)) return direct_alloc(c, reinterpret_cast<void**>(p), bytes);
   return pool_alloc(c, reinterpret_cast<void**>(p), bytes ? bytes : 16);
 }
-inline void dev_free(Ctx* c, void* p) {
-  if (p && cudaFreeAsync(p, c->stream) != cudaSuccess) {  // e.g. a stream its owner has destroyed
-    cudaGetLastError();
-    cudaFree(p);
-  }
-}
+// Releases it on the context stream.
+void dev_free(Ctx* c, void* p);
 // Returns the unused memory of an owned pool beyond kPoolKeep to the device.
 constexpr size_t kPoolKeep = size_t(1) << 30;
 void pool_trim(Ctx* c);

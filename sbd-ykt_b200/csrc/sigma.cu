@@ -1029,11 +1029,40 @@ int run_ab(Ctx* c, const T* X) {
 // The unpacked alpha-beta kernels (codes 61-64) evaluate the pairs only, add
 // them to Y, and leave both Coulomb terms to the same-spin kernels (Dt).
 
-// Blocks ibx < ntx split one 32 x 32 tile; the further ones write 256 columns
-// of 32 rows of Xk, phi o X with its columns in the lane order of the packed
-// alpha-beta kernel (vket: the ket string of each lane), so that kernel's
-// loads are coalesced: one gather per element here instead of one per alpha
-// single there.
+// 256 lanes of up to 32 rows of Xk, phi o X with its columns in the lane order
+// of the packed alpha-beta kernel (vket: the ket string of each lane), so that
+// kernel's loads are coalesced: one gather per element here instead of one per
+// alpha single there. v: the thread's lane; x, o: the rows; s_pa: their strings'
+// prefix parities.
+template <typename T>
+__device__ __forceinline__ void lane_rows(const T* __restrict__ x, size_t nb, int rows, size_t v, const uint64_t* s_pa,
+                                          const uint64_t* __restrict__ bstr, const uint32_t* __restrict__ vket,
+                                          T* __restrict__ o, size_t xs) {
+  if (v >= xs) return;
+  const size_t ib = vket[v];
+  const uint64_t beta = bstr[ib];
+#pragma unroll 8
+  for (int k = 0; k < rows; ++k) {
+    const T w = x[(size_t)k * nb + ib];
+    o[(size_t)k * xs + v] = basis_phase(s_pa[k], beta) ? -w : w;
+  }
+}
+
+// The lanes of all rows by themselves (the split kernel's, where Xk takes the
+// room of vectors that are read in between).
+template <typename T>
+__global__ void __launch_bounds__(256)
+lane_order_kernel(const T* __restrict__ X, size_t na, size_t nb, const uint64_t* __restrict__ astr,
+                  const uint64_t* __restrict__ bstr, const uint32_t* __restrict__ vket, T* __restrict__ Xk, size_t xs) {
+  __shared__ uint64_t s_pa[32];
+  const size_t ia0 = (size_t)blockIdx.y * 32;
+  if (threadIdx.x < 32) s_pa[threadIdx.x] = ia0 + threadIdx.x < na ? prefix_parity(astr[ia0 + threadIdx.x]) : 0ull;
+  __syncthreads();
+  lane_rows(X + ia0 * nb, nb, (int)min((size_t)32, na - ia0), (size_t)blockIdx.x * 256 + threadIdx.x, s_pa, bstr, vket,
+            Xk + ia0 * xs, xs);
+}
+
+// Blocks ibx < ntx split one 32 x 32 tile; the further ones write lane_rows.
 template <typename T>
 __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb, const uint64_t* __restrict__ astr,
                                    const uint64_t* __restrict__ bstr, T* __restrict__ Xp, T* __restrict__ Xpt,
@@ -1050,18 +1079,8 @@ __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb
   }
   __syncthreads();
   if (blockIdx.x >= ntx) {
-    const size_t v = (blockIdx.x - ntx) * 256 + threadIdx.y * 32 + tx;
-    if (v >= xs) return;
-    const size_t ib = vket[v];
-    const uint64_t beta = bstr[ib];
-    const int rows = (int)min((size_t)32, na - ia0);
-    const T* x = X + ia0 * nb + ib;
-    T* o = Xk + ia0 * xs + v;
-#pragma unroll 8
-    for (int k = 0; k < rows; ++k) {
-      const T w = x[(size_t)k * nb];
-      o[(size_t)k * xs] = basis_phase(s_pa[k], beta) ? -w : w;
-    }
+    lane_rows(X + ia0 * nb, nb, (int)min((size_t)32, na - ia0), (blockIdx.x - ntx) * 256 + threadIdx.y * 32 + tx, s_pa, bstr,
+              vket, Xk + ia0 * xs, xs);
     return;
   }
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
@@ -1082,12 +1101,13 @@ __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb
 
 // S[ia, ib] = phi(ia, ib) (Y[ia, ib] + Yab[ia, ib] + Yt[ib, ia]) + hii[ia, ib]
 // X[ia, ib], stored in T; Y, Yab and Yt have row strides xsa, xsa and xsb. Yab
-// is null where the alpha-beta kernel has added its part to Y.
-template <typename T>
+// is null where the alpha-beta kernel has added its part to Y; with kInPlace S
+// itself holds it.
+template <typename T, bool kInPlace>
 __global__ void combine_phase_kernel(const double* __restrict__ Y, const double* __restrict__ Yab,
                                      const double* __restrict__ Yt, const double* __restrict__ hii,
                                      const T* __restrict__ X, size_t na, size_t nb, const uint64_t* __restrict__ astr,
-                                     const uint64_t* __restrict__ bstr, T* __restrict__ S, size_t xsa, size_t xsb) {
+                                     const uint64_t* __restrict__ bstr, T* S, size_t xsa, size_t xsb) {
   __shared__ double tile[32][33];
   __shared__ uint64_t s_pa[32], s_b[32];
   const size_t ib0 = (size_t)blockIdx.x * 32, ia0 = (size_t)blockIdx.y * 32;
@@ -1107,7 +1127,8 @@ __global__ void combine_phase_kernel(const double* __restrict__ Y, const double*
     const size_t ia = ia0 + k, ib = ib0 + tx;
     if (ia < na && ib < nb) {
       double y = Y[ia * xsa + ib] + tile[k][tx];
-      if (Yab != nullptr) y += Yab[ia * xsa + ib];
+      if constexpr (kInPlace) y += (double)S[ia * nb + ib];
+      else if (Yab != nullptr) y += Yab[ia * xsa + ib];
       const double d = hii[ia * nb + ib] * (double)X[ia * nb + ib];
       S[ia * nb + ib] = (T)(basis_phase(s_pa[k], s_b[tx]) ? d - y : d + y);
     }
@@ -1844,7 +1865,9 @@ template <> struct RowPack<float> {
 template <typename T>
 struct AbArgs {
   const T* Xk;       // na x xs: phi o C, columns in lane order
-  size_t xs, ldx;    // ldx: row stride of Y and the partial rows
+  size_t xs, ldx;    // ldx: row stride of the partial rows
+  size_t ldy;        // row stride of Y
+  bool add;          // Y += instead of Y =
   const uint64_t* a_off;
   const uint32_t *a_ns, *a_ket, *a_info;
   const T* Vt;       // integrals over the pairs in use, row stride vstride
@@ -2057,9 +2080,12 @@ __global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
   }
   if (a.nex > 0) __syncthreads();
   auto col = [&](int i) -> size_t { return a.np == 1 ? (size_t)i : (size_t)(i / 4) * 4 * a.np + 4 * a.panel + i % 4; };
-  double* __restrict__ Yrow = a.Y + ia * a.ldx;
+  double* __restrict__ Yrow = a.Y + ia * a.ldy;
   if (item.w == 0) {
-    for (int i = threadIdx.x; i < a.nmain; i += NT) Yrow[col(i)] = y[i];
+    for (int i = threadIdx.x; i < a.nmain; i += NT) {
+      const size_t k = col(i);
+      Yrow[k] = a.add ? Yrow[k] + y[i] : y[i];
+    }
     return;
   }
   // a part of a split string: its partial row; the last part to finish adds all in slot order
@@ -2073,7 +2099,7 @@ __global__ void __launch_bounds__(NT, MINB) sigma_ab_kernel(const AbArgs<T> a) {
     const size_t k = col(i);
     double t = 0.0;
     for (uint32_t q = 0; q < s.z; ++q) t += __ldcg(part + (size_t)q * a.ldx + k);
-    Yrow[k] = t;
+    Yrow[k] = a.add ? Yrow[k] + t : t;
   }
 }
 
@@ -2086,10 +2112,11 @@ int launch_ab(Ctx* c, const AbArgs<T>& args, size_t n_item, size_t smem) {
   return 0;
 }
 
-// Yab = the alpha-beta product on Xk (Ctx::d_xk) over the rows of the work
-// items: the alpha connectivity's, or those of a row range (Ctx::range_conn).
+// The alpha-beta product of Xk over the rows of the work items (the alpha
+// connectivity's, or those of a row range, Ctx::range_conn) into Y, row stride
+// ldy, or added to it.
 template <typename T>
-int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
+int run_ab_packed(Ctx* c, const Conn* items, const T* Xk, double* Y, size_t ldy, bool add) {
   const Conn& ca = c->conn[0];
   const bool f64 = std::is_same<T, double>::value;
   const AbItems& it = (items ? *items : ca).ab[f64 ? 0 : 1];
@@ -2098,9 +2125,11 @@ int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
   for (size_t q = 0; q < P.panels.size(); ++q) {
     const AbPanel& p = P.panels[q];
     AbArgs<T> a{};
-    a.Xk = reinterpret_cast<const T*>(c->d_xk);
+    a.Xk = Xk;
     a.xs = P.xs;
     a.ldx = c->xsa;
+    a.ldy = ldy;
+    a.add = add;
     a.a_off = ca.off;
     a.a_ns = ca.nsing;
     a.a_ket = ca.ket;
@@ -2127,7 +2156,7 @@ int run_ab_packed(Ctx* c, const Conn* items = nullptr) {
     a.slot_split = it.slot;
     a.done = it.done;
     a.ypart = it.ypart;
-    a.Y = c->d_yab;
+    a.Y = Y;
     a.err = c->d_err;
     const size_t smem = (((size_t)p.ny * 8 + 15) & ~(size_t)15) + 16 * (size_t)a.max_packs * P.vstr;
     int rc;
@@ -2251,7 +2280,6 @@ int launch_ab_v6_ks(Ctx* c, const T* Xp, size_t smem, size_t xstride) {
 template <typename T>
 int run_ab_v6(Ctx* c, int code, const T* Xp) {
   using V = typename Prec<T>::V;
-  if (code / 10 == 7) return run_ab_packed<T>(c);  // 71
   const bool f64 = std::is_same<T, double>::value;
   const size_t vs = f64 ? c->vstride : c->vstride32;
   const size_t per = 16 / sizeof(T);
@@ -2274,11 +2302,32 @@ int run_ab_v6(Ctx* c, int code, const T* Xp) {
   return launch_ab_v6_ks<T, 1>(c, Xp, smem, xstride);
 }
 
+// Xk of all rows.
+template <typename T>
+int launch_lanes(Ctx* c, const T* X, T* Xk) {
+  const size_t xs = c->ab.xs;
+  const dim3 grid((unsigned)((xs + 255) / 256), (unsigned)((c->na + 31) / 32));
+  lane_order_kernel<T><<<grid, 256, 0, c->stream>>>(X, c->na, c->nb, c->d_a, c->d_b, c->ab.vket, Xk, xs);
+  SBDX_LAUNCHED(c);
+  return 0;
+}
+
+// The alpha-beta product of the items' rows (code 71): into d_yab from the
+// lanes that the split wrote, or, lean, added to d_y from lanes in the room of
+// d_xp and d_xt, once the same-spin products have read those.
+template <typename T>
+int run_ab_71(Ctx* c, const T* X, const Conn* items = nullptr) {
+  if (!c->lean) return run_ab_packed<T>(c, items, reinterpret_cast<const T*>(c->d_xk), c->d_yab, c->xsa, false);
+  T* xk = reinterpret_cast<T*>(c->d_xp);
+  const int rc = launch_lanes<T>(c, X, xk);
+  return rc ? rc : run_ab_packed<T>(c, items, xk, c->d_y, c->xsa, true);
+}
+
 // Phase split of the rows [a0, a0 + nr) (X: the whole input), with their
-// lane-order copy when the packed alpha-beta kernel follows.
+// lane-order copy when the packed alpha-beta kernel reads it beside the others.
 template <typename T>
 int launch_split(Ctx* c, const T* X, size_t a0, size_t nr, T* xp, T* xpt, bool lanes) {
-  const size_t nb = c->nb, xs = lanes ? c->ab.xs : 0;
+  const size_t nb = c->nb, xs = lanes && !c->lean ? c->ab.xs : 0;
   const dim3 grid((unsigned)((nb + 31) / 32 + (xs + 255) / 256), (unsigned)((nr + 31) / 32));
   phase_split_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(
       X + a0 * nb, nr, nb, c->d_a + a0, c->d_b, xp + a0 * c->xsa, xpt + a0, c->xsa, c->xsb, c->ab.vket,
@@ -2288,13 +2337,19 @@ int launch_split(Ctx* c, const T* X, size_t a0, size_t nr, T* xp, T* xpt, bool l
 }
 
 // S (row 0 = alpha string a0) of the rows [a0, a0 + nr); X: the whole input.
+// in_place: S holds the alpha-beta part; otherwise d_yab does after code 71,
+// or d_y.
 template <typename T>
-int launch_combine(Ctx* c, const T* X, size_t a0, size_t nr, T* S, bool packed) {
+int launch_combine(Ctx* c, const T* X, size_t a0, size_t nr, T* S, bool packed, bool in_place = false) {
   const size_t nb = c->nb;
   const dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((nr + 31) / 32));
-  combine_phase_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(
-      c->d_y + a0 * c->xsa, packed ? c->d_yab + a0 * c->xsa : nullptr, c->d_yt + a0, c->d_hii + a0 * nb, X + a0 * nb, nr,
-      nb, c->d_a + a0, c->d_b, S, c->xsa, c->xsb);
+  auto go = [&](auto kernel) {
+    kernel<<<grid, dim3(32, 8), 0, c->stream>>>(c->d_y + a0 * c->xsa, packed && !c->lean ? c->d_yab + a0 * c->xsa : nullptr,
+                                                c->d_yt + a0, c->d_hii + a0 * nb, X + a0 * nb, nr, nb, c->d_a + a0, c->d_b,
+                                                S, c->xsa, c->xsb);
+  };
+  if (in_place) go(combine_phase_kernel<T, true>);
+  else go(combine_phase_kernel<T, false>);
   SBDX_LAUNCHED(c);
   return 0;
 }
@@ -2357,7 +2412,7 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
   const bool packed = tune.ab_code == 71;
   const V* DtA = Db;
   const V* DtB = packed ? nullptr : Da;
-  if (packed && !c->profiling) {
+  if (packed && !c->lean && !c->profiling) {
     SideBySide f(c);
     if ((rc = f.fork())) return rc;
     f.on(0);
@@ -2365,7 +2420,7 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
     f.on(1);
     if (!rc) rc = run_same_v6<T>(c, tune, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt);
     f.main();
-    if (!rc) rc = run_ab_packed<T>(c);
+    if (!rc) rc = run_ab_71<T>(c, X);
     const int rj = f.join();
     if (rc || rj) return rc ? rc : rj;
     return launch_combine<T>(c, X, 0, na, S, true);
@@ -2377,7 +2432,7 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
   if ((rc = run_same_v6<T>(c, tune, xpt, na, c->xsb, cb, 0, nb, valB, DtB, c->da_stride, c->d_yt)))
     return rc;
   mark(3);
-  if ((rc = run_ab_v6<T>(c, tune.ab_code, xp))) return rc;
+  if ((rc = packed ? run_ab_71<T>(c, X) : run_ab_v6<T>(c, tune.ab_code, xp))) return rc;
   mark(4);
   if ((rc = launch_combine<T>(c, X, 0, na, S, packed))) return rc;
   mark(5);
@@ -2526,7 +2581,7 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
   if ((rc = run_same_v6<T>(c, tune, xpt + a0, nr, c->xsb, cb, 0, nb, valB, (const V*)nullptr, 0, c->d_yt + a0)))
     return rc;
   mark(3);
-  if ((rc = run_ab_packed<T>(c, &rc_items))) return rc;
+  if ((rc = run_ab_71<T>(c, X, &rc_items))) return rc;
   mark(4);
   if ((rc = launch_combine<T>(c, X, a0, nr, S, true))) return rc;
   mark(5);
@@ -2620,27 +2675,39 @@ int build_g_table(Ctx* c) {
 int ensure_sigma_scratch(Ctx* c) {
   c->xsa = pad8(c->nb);
   c->xsb = pad8(c->na);
-  const size_t n = std::max(c->na * c->xsa, c->nb * c->xsb);  // >= D
-  auto get = [&](void** p) -> int {
-    if (*p) return 0;
-    SBDX_CUDA(c, dev_alloc(c, p, sizeof(double) * n));
-    SBDX_CUDA(c, cudaMemsetAsync(*p, 0, sizeof(double) * n, c->stream));  // padding columns start at zero
-    return 0;
-  };
-  int rc;
-  if ((rc = get(&c->d_xt)) || (rc = get(&c->d_xp)) || (rc = get((void**)&c->d_y)) || (rc = get((void**)&c->d_yt)) ||
-      (rc = get((void**)&c->d_yab)))
-    return rc;
+  size_t n = std::max(c->na * c->xsa, c->nb * c->xsb);  // >= D
   if (!c->fork) {
     for (auto& x : c->side) SBDX_CUDA(c, cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
     for (auto& e : c->join) SBDX_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     SBDX_CUDA(c, cudaEventCreateWithFlags(&c->fork, cudaEventDisableTiming));
   }
-  if (c->ab.xs && !c->d_xk) {
-    SBDX_CUDA(c, dev_alloc(c, &c->d_xk, sizeof(double) * c->na * c->ab.xs));
-    SBDX_CUDA(c, cudaMemsetAsync(c->d_xk, 0, sizeof(double) * c->na * c->ab.xs, c->stream));
+  // One request (6 vectors of 72 MB by themselves take 2 ms to allocate), and
+  // nothing is cleared: a padding column enters only the products' padding
+  // columns, which nobody reads.
+  c->lean = c->na * c->nb >= kLeanDets;
+  if (c->lean) n = std::max(n, (c->na * c->ab.xs + 1) / 2);  // two vectors hold the lanes
+  n = (n + 15) / 16 * 16;
+  const size_t want = c->lean ? 4 * n : 5 * n + c->na * c->ab.xs;
+  if (!c->d_scratch || c->scratch_size < want) {
+    free_sigma_scratch(c);
+    SBDX_CUDA(c, dev_alloc(c, &c->d_scratch, sizeof(double) * want));
+    c->scratch_size = want;
   }
+  c->d_xp = c->d_scratch;
+  c->d_xt = c->d_scratch + n;
+  c->d_y = c->d_scratch + 2 * n;
+  c->d_yt = c->d_scratch + 3 * n;
+  c->d_yab = c->lean ? nullptr : c->d_scratch + 4 * n;
+  c->d_xk = c->lean ? nullptr : c->d_scratch + 5 * n;
   return 0;
+}
+
+void free_sigma_scratch(Ctx* c) {
+  clear_sigma_graphs(c);
+  dev_free(c, c->d_scratch);
+  c->d_scratch = c->d_y = c->d_yt = c->d_yab = nullptr;
+  c->d_xt = c->d_xp = c->d_xk = nullptr;
+  c->scratch_size = 0;
 }
 
 // Autotuner: for each precision, time the candidate kernel variants and launch
@@ -2833,8 +2900,8 @@ int sigma_device(Ctx* c, int precision, const void* X, void* S) {
 // split of its rows and the beta same-spin product on its columns of the
 // transpose (which read that chunk only). Once every chunk is in, the context
 // stream runs the alpha-beta product of all rows (it reads any ket row), then
-// per chunk the alpha same-spin work items of its rows, added to the
-// alpha-beta result, and the combine of its rows; the copy stream takes each
+// per chunk the alpha same-spin work items of its rows and the combine of its
+// rows; the copy stream takes each
 // finished chunk out while the next one computes. Exposed: the first chunk's
 // copy in, the last chunk's beta same-spin product and the last chunk's copy
 // out.
@@ -2961,7 +3028,13 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
   // the alpha-beta product of all rows in one launch (its work items keep
   // the whole grid busy, longest first), then per chunk the alpha same-spin
   // items of its rows and the combine
-  if ((rc = run_ab_packed<double>(c))) return rc;
+  if (!c->lean) {
+    rc = run_ab_71<double>(c, din);
+  } else {  // the lanes take the room of d_xt and d_y, and the result that of the output
+    if ((rc = launch_lanes<double>(c, din, xpt))) return rc;
+    rc = run_ab_packed<double>(c, nullptr, xpt, dout, nb, false);
+  }
+  if (rc) return rc;
   for (size_t i = 0; i < n; ++i) {
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
     const Conn& it = c->io_items[i];
@@ -2977,7 +3050,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     ra.same_ypart = it.same_ypart;
     if ((rc = run_same_v6<double>(c, t, xp, nb, c->xsa, ra, a0, nr, ca.val, c->d_Db, c->db_stride, c->d_y)))
       return rc;
-    if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true))) return rc;
+    if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true, c->lean))) return rc;
     SBDX_CUDA(c, cudaEventRecord(ev[n + i], c->stream));
   }
   for (size_t i = 0; i < n; ++i) {  // each chunk out as soon as it is ready

@@ -605,9 +605,9 @@ int sbdx_rdm(sbdx_ctx* ctx, const double* W, double* one, double* two) {
     const size_t D = c->na * c->nb, L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
     SBDX_CUDA(c, cudaMemcpyAsync(c->d_io_in, W, sizeof(double) * D, cudaMemcpyHostToDevice, c->stream));
     double *d_one = nullptr, *d_two = nullptr;
-    SBDX_CUDA(c, sbdx::dev_alloc(c, &d_one, sizeof(double) * 2 * L2));
+    SBDX_CUDA(c, sbdx::temp_alloc(c, &d_one, sizeof(double) * 2 * L2));
     if (two) {
-      cudaError_t e = sbdx::dev_alloc(c, &d_two, sizeof(double) * 4 * L4);
+      cudaError_t e = sbdx::temp_alloc(c, &d_two, sizeof(double) * 4 * L4);
       if (e != cudaSuccess) { sbdx::dev_free(c, d_one); sbdx::set_cuda_err(c, e, "allocation of the 2-RDM"); return SBDX_ERR_NOMEM; }
     }
     rc = sbdx::rdm_device(c, (const double*)c->d_io_in, d_one, d_two);
@@ -701,9 +701,9 @@ int sbdx_rdm_device(sbdx_ctx* ctx, const double* dW, double* one, double* two) {
     if (rc) return rc;
     const size_t L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
     double *d_one = nullptr, *d_two = nullptr;
-    SBDX_CUDA(c, sbdx::dev_alloc(c, &d_one, sizeof(double) * 2 * L2));
+    SBDX_CUDA(c, sbdx::temp_alloc(c, &d_one, sizeof(double) * 2 * L2));
     if (two) {
-      cudaError_t e = sbdx::dev_alloc(c, &d_two, sizeof(double) * 4 * L4);
+      cudaError_t e = sbdx::temp_alloc(c, &d_two, sizeof(double) * 4 * L4);
       if (e != cudaSuccess) { sbdx::dev_free(c, d_one); sbdx::set_cuda_err(c, e, "allocation of the 2-RDM"); return SBDX_ERR_NOMEM; }
     }
     rc = sbdx::rdm_device(c, dW, d_one, d_two);

@@ -147,8 +147,9 @@ __global__ void diag_finalize_kernel(int L, const double* __restrict__ Pa, const
   two[1 * L4 + (size_t)q + L * p + L2 * q + L3 * p] += v;
 }
 
-// G = A A^T of the n rows of A (K columns, row stride lda), lower tiles only:
-// CTA = one 64 x 64 tile (bi >= bj), four warps of 32 x 32, m8n8k4 on the FP64
+// G = A A^T of the n rows of A (K columns, row stride lda), lower tiles only,
+// from tile row bi0 on (G's first row is row 64 bi0): CTA = one 64 x 64 tile,
+// four warps of 32 x 32, m8n8k4 on the FP64
 // tensor pipe. The operands pass through shared memory in two stages of 16
 // columns (cp.async, zero beyond n and K); a lane reads two consecutive
 // columns per 16-byte load and uses them as the k-slots of two steps, the same
@@ -161,10 +162,10 @@ __device__ __forceinline__ void dmma_m8n8k4(double (&d)[2], double a, double b) 
       : "d"(a), "d"(b));
 }
 __global__ void __launch_bounds__(128)
-gram_kernel(const double* __restrict__ A, size_t n, size_t K, size_t lda, double* __restrict__ G) {
+gram_kernel(const double* __restrict__ A, size_t n, size_t K, size_t lda, double* __restrict__ G, size_t bi0) {
   __shared__ __align__(16) double sm[2][2][kGramTile][kGramPad];  // [stage][operand]
   // tile t -> (bi, bj), bj <= bi
-  const size_t t = blockIdx.x;
+  const size_t t = blockIdx.x + bi0 * (bi0 + 1) / 2;
   size_t bi = (size_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
   while (bi * (bi + 1) / 2 > t) --bi;
   while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
@@ -224,8 +225,9 @@ gram_kernel(const double* __restrict__ A, size_t n, size_t K, size_t lda, double
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const size_t c = bj * kGramTile + wc + 8 * j + 2 * q;
-      if (c < n) G[r * n + c] = acc[i][j][0];
-      if (c + 1 < n) G[r * n + c + 1] = acc[i][j][1];
+      double* o = G + (r - kGramTile * bi0) * n + c;
+      if (c < n) o[0] = acc[i][j][0];
+      if (c + 1 < n) o[1] = acc[i][j][1];
     }
   }
 }
@@ -239,11 +241,14 @@ __host__ __device__ __forceinline__ uint32_t ps_pat(uint64_t r) { return (uint32
 // Values of one spin's same-spin entries, CTA = bra row: singles packed to
 // srec[soff[r] + k] with value sval, doubles (when dkey is given) to position
 // off[r] - soff[r] + k with pattern key dkey (info bits 0-23) and value dval.
-// value = sign * sum_c W'[r,c] W'[k,c], from the Gram matrix G (lower
-// triangle) or, without it, by a warp per entry. Signs as in OneDiffCorrelation
+// value = sign * sum_c W'[r,c] W'[k,c], from rows [r0, r1) of the Gram
+// matrix's lower triangle (kDense: the entries whose larger string lies there)
+// or by a warp per entry. Signs as in OneDiffCorrelation
 // and TwoDiffCorrelation (correlation.h:49-130).
+template <bool kDense>
 __global__ void __launch_bounds__(128)
-rdm_entries_kernel(const double* __restrict__ W, size_t cols, size_t ldw, const double* __restrict__ G, size_t n,
+rdm_entries_kernel(const double* __restrict__ W, size_t cols, size_t ldw, const double* __restrict__ G, size_t n, size_t r0,
+                   size_t r1,
                    const uint64_t* __restrict__ s_row, const uint64_t* __restrict__ off,
                    const uint64_t* __restrict__ soff, const uint32_t* __restrict__ ket,
                    const uint32_t* __restrict__ info, uint64_t* __restrict__ srec, double* __restrict__ sval,
@@ -254,16 +259,25 @@ rdm_entries_kernel(const double* __restrict__ W, size_t cols, size_t ldw, const 
   const uint32_t todo = dkey != nullptr ? ne : ns;
   const uint64_t sr = s_row[r];
   const int lane = threadIdx.x & 31;
-  const uint32_t first = G != nullptr ? threadIdx.x : threadIdx.x >> 5, step = G != nullptr ? blockDim.x : blockDim.x >> 5;
+  const uint32_t first = kDense ? threadIdx.x : threadIdx.x >> 5, step = kDense ? blockDim.x : blockDim.x >> 5;
   for (uint32_t k = first; k < todo; k += step) {
     const uint32_t kt = ket[e0 + k], inf = info[e0 + k];
     double v = 0.0;
-    if (G != nullptr) {
-      v = r >= kt ? G[r * n + kt] : G[(size_t)kt * n + r];
+    if constexpr (kDense) {
+      const size_t hi = max(r, (size_t)kt), lo = min(r, (size_t)kt);
+      if (hi < r0 || hi >= r1) continue;
+      v = G[(hi - r0) * n + lo];
     } else {
       const double* wr = W + r * ldw;
       const double* wk = W + (size_t)kt * ldw;
-      for (size_t c = lane; c < cols; c += 32) v = fma(wr[c], wk[c], v);
+      double p[4] = {0.0, 0.0, 0.0, 0.0};  // eight loads in flight
+      size_t c = lane;
+      for (; c + 96 < cols; c += 128) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) p[u] = fma(__ldg(wr + c + 32 * u), __ldg(wk + c + 32 * u), p[u]);
+      }
+      for (; c < cols; c += 32) p[0] = fma(__ldg(wr + c), __ldg(wk + c), p[0]);
+      v = (p[0] + p[1]) + (p[2] + p[3]);
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       if (lane != 0) continue;
     }
@@ -561,8 +575,9 @@ rdm_occ_chunk_kernel(const double* __restrict__ W, size_t cols, size_t ldw, cons
 
 // Per row pattern, the sums over its chunks (in chunk order) of every column's
 // parts [vfirst[p], vfirst[p + 1]) (part p itself when vfirst is null):
-// G[row pattern][column], ncol columns from partial rows of nvp parts.
-__global__ void rdm_chunk_sum_kernel(const uint2* __restrict__ apat, int npa, int ncol,
+// G[row pattern][column], ncol columns from partial rows of nvp parts, the
+// first of them that of chunk `chunk0`.
+__global__ void rdm_chunk_sum_kernel(const uint2* __restrict__ apat, int npa, uint32_t chunk0, int ncol,
                                      const uint32_t* __restrict__ vfirst, int nvp, const double* __restrict__ partial,
                                      double* __restrict__ G) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -572,7 +587,7 @@ __global__ void rdm_chunk_sum_kernel(const uint2* __restrict__ apat, int npa, in
   const int v0 = vfirst ? (int)vfirst[p] : p, v1 = vfirst ? (int)vfirst[p + 1] : p + 1;
   double v = 0.0;
   for (uint32_t q = 0; q < ap.y; ++q)
-    for (int x = v0; x < v1; ++x) v += partial[(size_t)(ap.x + q) * nvp + x];
+    for (int x = v0; x < v1; ++x) v += partial[(size_t)(ap.x - chunk0 + q) * nvp + x];
   G[t] = v;
 }
 
@@ -700,17 +715,17 @@ __global__ void backward_eri_kernel(int L, const double* __restrict__ two, doubl
   g[t] = sum;
 }
 
-// Device scratch of one call, from the context's pool, released on its stream.
+// Device scratch of one call, released on the context's stream.
 struct Scratch {
   Ctx* c;
   std::vector<void*> p;
   explicit Scratch(Ctx* ctx) : c(ctx) {}
   ~Scratch() {
-    for (void* q : p) cudaFreeAsync(q, c->stream);
+    for (void* q : p) dev_free(c, q);
   }
   template <typename T>
   cudaError_t get(T** d, size_t n) {
-    const cudaError_t e = pool_alloc(c, reinterpret_cast<void**>(d), sizeof(T) * std::max<size_t>(1, n));
+    const cudaError_t e = temp_alloc(c, d, sizeof(T) * std::max<size_t>(1, n));
     if (e == cudaSuccess) p.push_back(*d);
     return e;
   }
@@ -722,6 +737,14 @@ struct Scratch {
     return cudaMemcpyAsync(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, c->stream);
   }
 };
+
+// At the end of a call, after its scratch: the pool keeps kPoolKeep bytes.
+struct Trim {
+  Ctx* c;
+  ~Trim() { pool_trim(c); }
+};
+
+constexpr size_t kMaxPartials = size_t(256) << 20;  // bytes of chunk partials at a time
 
 }  // namespace
 
@@ -784,35 +807,50 @@ static int rdm_same(Ctx* c, Scratch& sc, int spin, const double* Wm, size_t ldw,
   SBDX_CUDA(c, sc.put(&d_soff, keep));
   SBDX_CUDA(c, sc.get(&S.d_srec, nsing));
   SBDX_CUDA(c, sc.get(&S.d_sval, nsing));
+  Scratch own(c);  // of this spin only
   uint32_t *d_key = nullptr, *d_key2 = nullptr, *d_idx = nullptr, *d_idx2 = nullptr;
   double* d_dval = nullptr;
   if (two && nd) {
-    SBDX_CUDA(c, sc.get(&d_key, nd));
-    SBDX_CUDA(c, sc.get(&d_key2, nd));
-    SBDX_CUDA(c, sc.get(&d_idx, nd));
-    SBDX_CUDA(c, sc.get(&d_idx2, nd));
-    SBDX_CUDA(c, sc.get(&d_dval, nd));
+    SBDX_CUDA(c, own.get(&d_key, nd));
+    SBDX_CUDA(c, own.get(&d_key2, nd));
+    SBDX_CUDA(c, own.get(&d_idx, nd));
+    SBDX_CUDA(c, own.get(&d_idx2, nd));
+    SBDX_CUDA(c, own.get(&d_dval, nd));
   }
   // The Gram matrix costs n^2 cols flops at about 25 TFLOP/s, a dot per entry
   // reads 16 cols bytes at about 10 TB/s: dense from 1 entry in 40 pairs (the
-  // sampled sets hold 4 to 15%), while n^2 doubles stay below 4 GB.
+  // sampled sets hold 4 to 15%), while there is room. Above kGramElems elements
+  // it comes in panels of rows (20000 x 200 strings, 3.2 GB of it: 24 ms a call; in
+  // one piece and given back each time 57 ms).
+  constexpr size_t kGramElems = size_t(1) << 26;
   double* G = nullptr;
-  if (two && (double)cn.total * 40.0 >= (double)n * (double)n && n * n <= (size_t)1 << 29) {
-    SBDX_CUDA(c, sc.get(&G, n * n));
-    const size_t nt = (n + kGramTile - 1) / kGramTile;
-    gram_kernel<<<(unsigned)(nt * (nt + 1) / 2), 128, 0, c->stream>>>(Wm, n, cols, ldw, G);
+  const size_t prow = n * n > kGramElems ? std::max<size_t>(kGramTile, kGramElems / n / kGramTile * kGramTile) : n;
+  if (two && (double)cn.total * 40.0 >= (double)n * (double)n && own.get(&G, prow * n) != cudaSuccess) {
+    cudaGetLastError();
+    G = nullptr;
+  }
+  for (size_t r0 = 0; r0 < n; r0 += G ? prow : n) {
+    const size_t r1 = G ? std::min(n, r0 + prow) : n;
+    if (G) {
+      const size_t b0 = r0 / kGramTile, b1 = (r1 + kGramTile - 1) / kGramTile;
+      gram_kernel<<<(unsigned)((b1 * (b1 + 1) - b0 * (b0 + 1)) / 2), 128, 0, c->stream>>>(Wm, n, cols, ldw, G, b0);
+      SBDX_LAUNCHED(c);
+    }
+    auto entries = [&](auto kernel) {
+      kernel<<<(unsigned)n, 128, 0, c->stream>>>(Wm, cols, ldw, G, n, r0, r1, s_row, cn.off, d_soff, cn.ket, cn.info, S.d_srec,
+                                                 S.d_sval, d_key, d_dval);
+    };
+    if (G) entries(rdm_entries_kernel<true>);
+    else entries(rdm_entries_kernel<false>);
     SBDX_LAUNCHED(c);
   }
-  rdm_entries_kernel<<<(unsigned)n, 128, 0, c->stream>>>(Wm, cols, ldw, G, n, s_row, cn.off, d_soff, cn.ket, cn.info,
-                                                         S.d_srec, S.d_sval, d_key, d_dval);
-  SBDX_LAUNCHED(c);
   if (d_key) {
     iota_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, c->stream>>>(d_idx, nd);
     SBDX_LAUNCHED(c);
     size_t tmp = 0;
     SBDX_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, tmp, d_key, d_key2, d_idx, d_idx2, nd, 0, 24, c->stream));
     unsigned char* d_tmp = nullptr;
-    SBDX_CUDA(c, sc.get(&d_tmp, tmp));
+    SBDX_CUDA(c, own.get(&d_tmp, tmp));
     SBDX_CUDA(c, cub::DeviceRadixSort::SortPairs(d_tmp, tmp, d_key, d_key2, d_idx, d_idx2, nd, 0, 24, c->stream));
     rdm_doubles_finalize_kernel<<<(unsigned)((nd + 255) / 256), 256, 0, c->stream>>>(spin, c->L, d_key2, d_idx2, nd,
                                                                                      d_dval, two);
@@ -872,7 +910,7 @@ static int rdm_singles(Ctx* c, Scratch& sc, int spin, const double* Wm, size_t l
     rdm_occ_chunk_kernel<<<(unsigned)S.chunks.size(), 256, 0, c->stream>>>(Wm, cols, ldw, s_col, L, S.d_chunks, S.d_rec,
                                                                           part);
     SBDX_LAUNCHED(c);
-    rdm_chunk_sum_kernel<<<(unsigned)((ng * L + 255) / 256), 256, 0, c->stream>>>(S.d_cpat, (int)ng, L, nullptr, L, part,
+    rdm_chunk_sum_kernel<<<(unsigned)((ng * L + 255) / 256), 256, 0, c->stream>>>(S.d_cpat, (int)ng, 0u, L, nullptr, L, part,
                                                                                   prof);
     SBDX_LAUNCHED(c);
   }
@@ -884,11 +922,11 @@ static int rdm_singles(Ctx* c, Scratch& sc, int spin, const double* Wm, size_t l
 }
 
 template <int R>
-static int launch_ab_chunks(Ctx* c, const double* W, const SingleGroups& A, const uint32_t* vlen, const uint64_t* voff,
-                            const uint64_t* brec, int nvp, double* part) {
+static int launch_ab_chunks(Ctx* c, const double* W, const SingleGroups& A, uint32_t chunk0, uint32_t chunks,
+                            const uint32_t* vlen, const uint64_t* voff, const uint64_t* brec, int nvp, double* part) {
   SBDX_CUDA(c, cudaFuncSetAttribute(rdm_ab_chunk_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAbSmemBudget));
-  rdm_ab_chunk_kernel<R><<<(unsigned)A.chunks.size(), kAbDetThreads, 2 * sizeof(double) * R * c->nb, c->stream>>>(
-      W, c->nb, c->xsa, A.d_chunks, A.d_rec, vlen, voff, brec, nvp, part);
+  rdm_ab_chunk_kernel<R><<<chunks, kAbDetThreads, 2 * sizeof(double) * R * c->nb, c->stream>>>(
+      W, c->nb, c->xsa, A.d_chunks + chunk0, A.d_rec, vlen, voff, brec, nvp, part);
   SBDX_LAUNCHED(c);
   return 0;
 }
@@ -956,20 +994,37 @@ static int rdm_ab_chunks(Ctx* c, Scratch& sc, const SingleGroups& A, const Singl
   SBDX_CUDA(c, sc.put(&d_bkey, bkey));
   SBDX_CUDA(c, sc.put(&d_amap, amap));
   SBDX_CUDA(c, sc.put(&d_bmap, bmap));
-  SBDX_CUDA(c, sc.get(&part, A.chunks.size() * (size_t)nvp));
+  // ranges of alpha patterns whose chunk partials fit in kMaxPartials (one
+  // pattern at least)
+  std::vector<int> range(1, 0);
+  size_t most = 0;
+  for (int q = 0; q < npa;) {
+    size_t n = A.cpat[q].y;
+    int e = q + 1;
+    while (e < npa && (n + A.cpat[e].y) * nvp * sizeof(double) <= kMaxPartials) n += A.cpat[e++].y;
+    most = std::max(most, n);
+    range.push_back(q = e);
+  }
+  SBDX_CUDA(c, sc.get(&part, most * (size_t)nvp));
   SBDX_CUDA(c, sc.get(&G, (size_t)npa * npb));
   const double* W = reinterpret_cast<const double*>(c->d_xp);
   const size_t row = 2 * sizeof(double) * nb;
-  int rc;
-  if (8 * row <= kAbSmemBudget / 2) rc = launch_ab_chunks<8>(c, W, A, d_vlen, d_voff, d_brec, nvp, part);
-  else if (6 * row <= kAbSmemBudget) rc = launch_ab_chunks<6>(c, W, A, d_vlen, d_voff, d_brec, nvp, part);
-  else if (4 * row <= kAbSmemBudget) rc = launch_ab_chunks<4>(c, W, A, d_vlen, d_voff, d_brec, nvp, part);
-  else if (2 * row <= kAbSmemBudget) rc = launch_ab_chunks<2>(c, W, A, d_vlen, d_voff, d_brec, nvp, part);
-  else rc = launch_ab_chunks<1>(c, W, A, d_vlen, d_voff, d_brec, nvp, part);
-  if (rc) return rc;
+  for (size_t k = 0; k + 1 < range.size(); ++k) {
+    const int q0 = range[k], q1 = range[k + 1];
+    const uint32_t c0 = A.cpat[q0].x, nc = A.cpat[q1 - 1].x + A.cpat[q1 - 1].y - c0;
+    int rc;
+    if (8 * row <= kAbSmemBudget / 2) rc = launch_ab_chunks<8>(c, W, A, c0, nc, d_vlen, d_voff, d_brec, nvp, part);
+    else if (6 * row <= kAbSmemBudget) rc = launch_ab_chunks<6>(c, W, A, c0, nc, d_vlen, d_voff, d_brec, nvp, part);
+    else if (4 * row <= kAbSmemBudget) rc = launch_ab_chunks<4>(c, W, A, c0, nc, d_vlen, d_voff, d_brec, nvp, part);
+    else if (2 * row <= kAbSmemBudget) rc = launch_ab_chunks<2>(c, W, A, c0, nc, d_vlen, d_voff, d_brec, nvp, part);
+    else rc = launch_ab_chunks<1>(c, W, A, c0, nc, d_vlen, d_voff, d_brec, nvp, part);
+    if (rc) return rc;
+    const size_t sums = (size_t)(q1 - q0) * npb;
+    rdm_chunk_sum_kernel<<<(unsigned)((sums + 255) / 256), 256, 0, c->stream>>>(A.d_cpat + q0, q1 - q0, c0, npb, d_vfirst,
+                                                                               nvp, part, G + (size_t)q0 * npb);
+    SBDX_LAUNCHED(c);
+  }
   const size_t npairs = (size_t)npa * npb;
-  rdm_chunk_sum_kernel<<<(unsigned)((npairs + 255) / 256), 256, 0, c->stream>>>(A.d_cpat, npa, npb, d_vfirst, nvp, part, G);
-  SBDX_LAUNCHED(c);
   rdm_ab_write_kernel<<<(unsigned)((npairs + 255) / 256), 256, 0, c->stream>>>(d_akey, npa, d_bkey, npb, d_amap, d_bmap,
                                                                                G, c->L, two);
   SBDX_LAUNCHED(c);
@@ -984,6 +1039,7 @@ int rdm_device(Ctx* c, const double* dW, double* d_one, double* d_two) {
   const size_t na = c->na, nb = c->nb, L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
   SingleGroups S[2];
   std::vector<uint64_t> keep[2];  // host sources of copies, alive until the last synchronisation
+  const Trim trim{c};
   Scratch sc(c);
   double* wa = nullptr;
   SBDX_CUDA(c, sc.get(&wa, na + nb + 3 * L2));
@@ -1025,6 +1081,7 @@ int occupation_device(Ctx* c, const double* dW, double* d_density) {
   int rc = ensure_sigma_scratch(c);
   if (rc) return rc;
   const size_t na = c->na, nb = c->nb, L = (size_t)c->L, L2 = L * L;
+  const Trim trim{c};
   Scratch sc(c);
   double* wa = nullptr;
   SBDX_CUDA(c, sc.get(&wa, na + nb + 2 * L2));
@@ -1045,6 +1102,7 @@ int occupation_device(Ctx* c, const double* dW, double* d_density) {
 }
 
 int alpha_weights_device(Ctx* c, const double* dW, double* d_w) {
+  const Trim trim{c};
   const int rc = weights(c, dW, c->nb, d_w, nullptr, nullptr, nullptr, nullptr, nullptr, 0);
   if (rc) return rc;
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1058,6 +1116,7 @@ int backward_device(Ctx* c, const double* dW, double* dE_dh, double* dE_deri) {
   int rc = build_connectivity(c, false);
   if (rc) return rc;
   const size_t L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
+  const Trim trim{c};
   Scratch sc(c);
   double* one = nullptr;
   SBDX_CUDA(c, sc.get(&one, 2 * L2 + 4 * L4 + c->neri));

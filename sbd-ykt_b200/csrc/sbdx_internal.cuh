@@ -524,7 +524,7 @@ cudaError_t pool_alloc(Ctx* c, void** p, size_t bytes);
 // A buffer of its own, outside the pool; on failure the pool's unused memory is
 // given back first and the request repeated.
 cudaError_t direct_alloc(Ctx* c, void** p, size_t bytes);
-// Any buffer of a context but the stored Hamiltonian: small ones from the pool
+// Any buffer of a context: small ones from the pool
 // (cudaMalloc and cudaFree take 0.35 and 0.45 ms and synchronise the device,
 // which cost a diag call on 400 x 400 strings 17 of 29 ms), large ones by
 // themselves (a growing pool maps 1 GB in 5 to 6 ms, cudaMalloc in under 1 ms, and
@@ -540,6 +540,14 @@ cudaError_t dev_alloc(Ctx* c, T** p, size_t bytes) {
 }
 // Releases it on the context stream.
 void dev_free(Ctx* c, void* p);
+// A buffer that the call which asked for it releases: from the pool, which
+// keeps it for the next call, up to kTempPooled bytes.
+constexpr size_t kTempPooled = size_t(512) << 20;
+template <typename T>
+cudaError_t temp_alloc(Ctx* c, T** p, size_t bytes) {
+  if (bytes > kTempPooled && (c->own_pool || !c->pool)) return direct_alloc(c, reinterpret_cast<void**>(p), bytes);
+  return pool_alloc(c, reinterpret_cast<void**>(p), bytes ? bytes : 16);
+}
 // Returns the unused memory of an owned pool beyond kPoolKeep to the device.
 constexpr size_t kPoolKeep = size_t(1) << 30;
 void pool_trim(Ctx* c);

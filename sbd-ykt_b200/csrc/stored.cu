@@ -252,7 +252,7 @@ void release_stored(Ctx* c) {
   StoredH& H = c->stored;
   for (void* p : {(void*)H.val, (void*)H.rowbase, (void*)H.perm, (void*)H.idx, (void*)H.psd, (void*)H.ps,
                   (void*)H.item, (void*)H.split, (void*)H.slot_split, (void*)H.done, (void*)H.part})
-    cudaFree(p);
+    dev_free(c, p);
   H = StoredH{};
 }
 
@@ -381,19 +381,19 @@ int build_stored(Ctx* c) {
   StoredH& H = c->stored;
   auto up = [&](auto** d, const auto& h) -> cudaError_t {
     const size_t bytes = sizeof(h[0]) * h.size();
-    const cudaError_t e = cudaMalloc(d, bytes);
+    const cudaError_t e = dev_alloc(c, d, bytes);
     return e != cudaSuccess ? e : cudaMemcpyAsync(*d, h.data(), bytes, cudaMemcpyHostToDevice, c->stream);
   };
   H.nslice = (int)ns;
   H.width = (int)G;
   H.warps = (int)warps;
   H.nitem = (uint32_t)item.size();
-  if (cudaMalloc(&H.val, sizeof(double) * std::max<uint64_t>(1, total)) != cudaSuccess ||
+  if (direct_alloc(c, reinterpret_cast<void**>(&H.val), sizeof(double) * std::max<uint64_t>(1, total)) != cudaSuccess ||
       up(&H.rowbase, rowbase) != cudaSuccess || up(&H.perm, perm) != cudaSuccess || up(&H.idx, idx) != cudaSuccess ||
       up(&H.psd, psd) != cudaSuccess || up(&H.ps, ps) != cudaSuccess || up(&H.item, item) != cudaSuccess ||
       up(&H.split, split) != cudaSuccess || up(&H.slot_split, slot_split) != cudaSuccess ||
       up(&H.done, done) != cudaSuccess ||
-      cudaMalloc(&H.part, sizeof(double) * kStoredThreads * std::max<size_t>(1, nslot)) != cudaSuccess) {
+      dev_alloc(c, &H.part, sizeof(double) * kStoredThreads * std::max<size_t>(1, nslot)) != cudaSuccess) {
     cudaGetLastError();
     cudaStreamSynchronize(c->stream);
     release_stored(c);

@@ -179,7 +179,9 @@ int sbdx_sigma(sbdx_ctx* ctx, const double* C, double* S);
 int sbdx_set_io_chunks(sbdx_ctx* ctx, int chunks);
 /* Same on device buffers of na*nb elements of the given precision
  * (SBDX_FP64: double; SBDX_FP32: float storage with FP64 row accumulation),
- * on the context stream. */
+ * on the context stream. An infinity or NaN in C makes those elements of S
+ * non-finite that H connects it with (an infinity may come out as NaN), and no
+ * others. */
 int sbdx_sigma_device(sbdx_ctx* ctx, int precision, const void* dC, void* dS);
 
 /* One shard of the product for a distributed solve: output rows [a0, a1) of

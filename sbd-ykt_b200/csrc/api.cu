@@ -188,10 +188,12 @@ int sbdx_ctx_create(sbdx_ctx** out, int device) {
   sbdx_ctx* ctx = new (std::nothrow) sbdx_ctx();
   if (!ctx) return SBDX_ERR_NOMEM;
   ctx->c.device = device;
-  if (cudaMalloc(&ctx->c.d_err, sizeof(int)) != cudaSuccess || cudaMemset(ctx->c.d_err, 0, sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&ctx->c.d_err, 2 * sizeof(int)) != cudaSuccess ||
+      cudaMemset(ctx->c.d_err, 0, 2 * sizeof(int)) != cudaSuccess) {
     delete ctx;
     return SBDX_ERR_CUDA;
   }
+  ctx->c.d_nonfinite = ctx->c.d_err + 1;
   *out = ctx;
   return SBDX_OK;
 }

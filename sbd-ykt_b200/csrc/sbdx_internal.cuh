@@ -315,6 +315,7 @@ struct Ctx {
   double* d_scratch = nullptr;
   size_t scratch_size = 0;  // elements
   bool lean = false;
+  int* d_nonfinite = nullptr;  // set from the phase split to the combine of an input with an infinity or NaN
   size_t xsa = 0, xsb = 0;
   // the three independent products of one sigma run side by side: the packed
   // alpha-beta one on the context stream, the same-spin ones on these

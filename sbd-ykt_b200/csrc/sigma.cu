@@ -1063,11 +1063,12 @@ lane_order_kernel(const T* __restrict__ X, size_t na, size_t nb, const uint64_t*
 }
 
 // Blocks ibx < ntx split one 32 x 32 tile; the further ones write lane_rows.
+// *nonfinite (unless null) is set where X holds an infinity or NaN.
 template <typename T>
 __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb, const uint64_t* __restrict__ astr,
                                    const uint64_t* __restrict__ bstr, T* __restrict__ Xp, T* __restrict__ Xpt,
                                    size_t xsa, size_t xsb, const uint32_t* __restrict__ vket, T* __restrict__ Xk,
-                                   size_t xs) {
+                                   size_t xs, int* nonfinite) {
   __shared__ T tile[32][33];
   __shared__ uint64_t s_pa[32], s_b[32];
   const size_t ntx = (nb + 31) / 32;
@@ -1083,15 +1084,18 @@ __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb
               vket, Xk + ia0 * xs, xs);
     return;
   }
+  bool odd = false;
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const size_t ia = ia0 + k, ib = ib0 + tx;
     if (ia < na && ib < nb) {
       T v = X[ia * nb + ib];
+      odd |= !isfinite(v);
       if (basis_phase(s_pa[k], s_b[tx])) v = -v;
       Xp[ia * xsa + ib] = v;
       tile[k][tx] = v;
     }
   }
+  if (odd && nonfinite != nullptr) *nonfinite = 1;
   __syncthreads();
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
     const size_t ib = ib0 + k, ia = ia0 + tx;
@@ -1102,12 +1106,13 @@ __global__ void phase_split_kernel(const T* __restrict__ X, size_t na, size_t nb
 // S[ia, ib] = phi(ia, ib) (Y[ia, ib] + Yab[ia, ib] + Yt[ib, ia]) + hii[ia, ib]
 // X[ia, ib], stored in T; Y, Yab and Yt have row strides xsa, xsa and xsb. Yab
 // is null where the alpha-beta kernel has added its part to Y; with kInPlace S
-// itself holds it.
+// itself holds it. *nonfinite (unless null) is cleared.
 template <typename T, bool kInPlace>
 __global__ void combine_phase_kernel(const double* __restrict__ Y, const double* __restrict__ Yab,
                                      const double* __restrict__ Yt, const double* __restrict__ hii,
                                      const T* __restrict__ X, size_t na, size_t nb, const uint64_t* __restrict__ astr,
-                                     const uint64_t* __restrict__ bstr, T* S, size_t xsa, size_t xsb) {
+                                     const uint64_t* __restrict__ bstr, T* S, size_t xsa, size_t xsb,
+                                     int* nonfinite) {
   __shared__ double tile[32][33];
   __shared__ uint64_t s_pa[32], s_b[32];
   const size_t ib0 = (size_t)blockIdx.x * 32, ia0 = (size_t)blockIdx.y * 32;
@@ -1121,6 +1126,7 @@ __global__ void combine_phase_kernel(const double* __restrict__ Y, const double*
     const size_t ib = ib0 + k, ia = ia0 + tx;
     if (ib < nb && ia < na) tile[tx][k] = Yt[ib * xsb + ia];
   }
+  if (nonfinite != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tx == 0 && threadIdx.y == 0) *nonfinite = 0;
   __syncthreads();
 #pragma unroll 4
   for (int k = threadIdx.y; k < 32; k += blockDim.y) {
@@ -1500,6 +1506,36 @@ sigma_coulomb_kernel(const T* __restrict__ X, size_t ncol, size_t ldx, size_t ro
     t.x += acc[v];
     t.y += acc[v + 1];
     *y = t;
+  }
+}
+
+// The blocked kernels multiply the zeros of a block's union too, and zero times
+// an infinity is NaN: where the input holds one (*nonfinite), this kernel
+// evaluates their rows again, string by string, so that it reaches the
+// elements that the matrix connects it with and no others. Otherwise its CTAs end at once
+// (2 us on a side stream beside products of 0.9 ms and more).
+template <typename T>
+__global__ void __launch_bounds__(kSameThreads)
+sigma_same_nonfinite_kernel(const int* __restrict__ nonfinite, const T* __restrict__ X, size_t ncol, size_t ldx, size_t row0,
+                            size_t nrow, const uint64_t* __restrict__ off, const uint32_t* __restrict__ nsing,
+                            const uint32_t* __restrict__ ket, const typename Prec<T>::V* __restrict__ val,
+                            const uint32_t* __restrict__ info, const typename Prec<T>::V* __restrict__ Dt, size_t dstride,
+                            double* __restrict__ Y) {
+  if (*nonfinite == 0) return;
+  const size_t strips = (ncol + kSameThreads - 1) / kSameThreads;
+  for (size_t w = blockIdx.x; w < nrow * strips; w += gridDim.x) {
+    const size_t r = row0 + w / strips, c = w % strips * kSameThreads + threadIdx.x;
+    if (c >= ncol) continue;
+    double acc = 0.0;
+    const uint64_t e0 = off[r], e1 = off[r + 1], send = Dt != nullptr ? e0 + nsing[r] : e0;
+    for (uint64_t e = e0; e < e1; ++e) {
+      const uint32_t inf = info[e];
+      double v = (double)val[e];
+      if (inf >> 31) v = -v;
+      if (e < send) v += flip_sign((double)Dt[(size_t)((inf >> 12) & 0xfffu) * dstride + c], inf >> 31);
+      acc = fma(v, (double)X[(size_t)ket[e] * ldx + c], acc);
+    }
+    Y[r * ldx + c] = acc;
   }
 }
 
@@ -2228,14 +2264,18 @@ int run_same_v6(Ctx* c, const Tune& tune, const T* X, size_t ncol, size_t ldx, c
   int vec = code % 10;
   const bool aligned = (reinterpret_cast<uintptr_t>(X) % 16) == 0;
   while (vec > 1 && (!aligned || ldx % vec != 0 || (Dt != nullptr && dstride % vec != 0))) vec >>= 1;
-  if (code / 10 == 3 && cn.blk[0].nblk > 0 && aligned) {
+  if (code / 10 == 3 && cn.blk[0].nblk > 0 && aligned && nrow > 0) {
     const int rc = launch_same_blk(c, vec, X, ncol, ldx, cn.blk[std::is_same<T, double>::value ? 0 : 1], Y);
-    if (rc || Dt == nullptr || nrow == 0) return rc;
-    // the singles' Coulomb terms
-    constexpr size_t cols = (size_t)kSameThreads * 16 / sizeof(T);
-    const dim3 grid((unsigned)nrow, (unsigned)((ncol + cols - 1) / cols));
-    sigma_coulomb_kernel<T><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, row0, cn.off, cn.nsing, cn.ket, cn.info,
-                                                                  Dt, dstride, Y);
+    if (rc) return rc;
+    if (Dt != nullptr) {  // the singles' Coulomb terms
+      constexpr size_t cols = (size_t)kSameThreads * 16 / sizeof(T);
+      const dim3 grid((unsigned)nrow, (unsigned)((ncol + cols - 1) / cols));
+      sigma_coulomb_kernel<T><<<grid, kSameThreads, 0, c->stream>>>(X, ncol, ldx, row0, cn.off, cn.nsing, cn.ket, cn.info,
+                                                                    Dt, dstride, Y);
+      SBDX_LAUNCHED(c);
+    }
+    sigma_same_nonfinite_kernel<T><<<148, kSameThreads, 0, c->stream>>>(c->d_nonfinite, X, ncol, ldx, row0, nrow, cn.off,
+                                                                        cn.nsing, cn.ket, val, cn.info, Dt, dstride, Y);
     SBDX_LAUNCHED(c);
     return 0;
   }
@@ -2326,27 +2366,27 @@ int run_ab_71(Ctx* c, const T* X, const Conn* items = nullptr) {
 // Phase split of the rows [a0, a0 + nr) (X: the whole input), with their
 // lane-order copy when the packed alpha-beta kernel reads it beside the others.
 template <typename T>
-int launch_split(Ctx* c, const T* X, size_t a0, size_t nr, T* xp, T* xpt, bool lanes) {
+int launch_split(Ctx* c, const T* X, size_t a0, size_t nr, T* xp, T* xpt, bool lanes, int* nonfinite) {
   const size_t nb = c->nb, xs = lanes && !c->lean ? c->ab.xs : 0;
   const dim3 grid((unsigned)((nb + 31) / 32 + (xs + 255) / 256), (unsigned)((nr + 31) / 32));
   phase_split_kernel<T><<<grid, dim3(32, 8), 0, c->stream>>>(
       X + a0 * nb, nr, nb, c->d_a + a0, c->d_b, xp + a0 * c->xsa, xpt + a0, c->xsa, c->xsb, c->ab.vket,
-      reinterpret_cast<T*>(c->d_xk) + a0 * xs, xs);
+      reinterpret_cast<T*>(c->d_xk) + a0 * xs, xs, nonfinite);
   SBDX_LAUNCHED(c);
   return 0;
 }
 
 // S (row 0 = alpha string a0) of the rows [a0, a0 + nr); X: the whole input.
 // in_place: S holds the alpha-beta part; otherwise d_yab does after code 71,
-// or d_y.
+// or d_y. last: nothing reads the input's flag after this.
 template <typename T>
-int launch_combine(Ctx* c, const T* X, size_t a0, size_t nr, T* S, bool packed, bool in_place = false) {
+int launch_combine(Ctx* c, const T* X, size_t a0, size_t nr, T* S, bool packed, bool in_place = false, bool last = true) {
   const size_t nb = c->nb;
   const dim3 grid((unsigned)((nb + 31) / 32), (unsigned)((nr + 31) / 32));
   auto go = [&](auto kernel) {
     kernel<<<grid, dim3(32, 8), 0, c->stream>>>(c->d_y + a0 * c->xsa, packed && !c->lean ? c->d_yab + a0 * c->xsa : nullptr,
                                                 c->d_yt + a0, c->d_hii + a0 * nb, X + a0 * nb, nr, nb, c->d_a + a0, c->d_b,
-                                                S, c->xsa, c->xsb);
+                                                S, c->xsa, c->xsb, last ? c->d_nonfinite : nullptr);
   };
   if (in_place) go(combine_phase_kernel<T, true>);
   else go(combine_phase_kernel<T, false>);
@@ -2406,7 +2446,7 @@ int run_sigma_v6(Ctx* c, const Tune& tune, const T* X, T* S) {
   };
   int rc = 0;
   mark(0);
-  if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, tune.ab_code == 71))) return rc;
+  if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, tune.ab_code == 71, c->d_nonfinite))) return rc;
   // the beta singles' Coulomb terms: in the packed alpha-beta kernel, or in the
   // same-spin kernels beside an unpacked one
   const bool packed = tune.ab_code == 71;
@@ -2572,7 +2612,7 @@ int run_sigma_rows(Ctx* c, const Tune& tune, const T* X, T* S, size_t a0, size_t
   };
   int rc = 0;
   mark(0);
-  if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, true))) return rc;
+  if ((rc = launch_split<T>(c, X, 0, na, xp, xpt, true, c->d_nonfinite))) return rc;
   mark(1);
   if (nr == 0) return 0;
   if ((rc = run_same_v6<T>(c, tune, xp, nb, c->xsa, ra, a0, nr, valA, Db, c->db_stride, c->d_y)))
@@ -2642,7 +2682,7 @@ int ensure_coulomb_a(Ctx* c) {
 }
 
 int phase_vectors(Ctx* c, const double* W) {
-  return launch_split<double>(c, W, 0, c->na, reinterpret_cast<double*>(c->d_xp), reinterpret_cast<double*>(c->d_xt), false);
+  return launch_split<double>(c, W, 0, c->na, reinterpret_cast<double*>(c->d_xp), reinterpret_cast<double*>(c->d_xt), false, nullptr);
 }
 
 int build_g_table(Ctx* c) {
@@ -3020,7 +3060,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
   for (size_t i = 0; i < n; ++i) {  // per arrived chunk: phase split, beta same-spin on its columns
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
     SBDX_CUDA(c, cudaStreamWaitEvent(c->stream, ev[i], 0));
-    if ((rc = launch_split<double>(c, din, a0, nr, xp, xpt, true))) return rc;
+    if ((rc = launch_split<double>(c, din, a0, nr, xp, xpt, true, c->d_nonfinite))) return rc;
     if ((rc = run_same_v6<double>(c, t, xpt + a0, nr, c->xsb, cb, 0, nb, cb.val, (const double*)nullptr, 0,
                                   c->d_yt + a0)))
       return rc;
@@ -3050,7 +3090,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     ra.same_ypart = it.same_ypart;
     if ((rc = run_same_v6<double>(c, t, xp, nb, c->xsa, ra, a0, nr, ca.val, c->d_Db, c->db_stride, c->d_y)))
       return rc;
-    if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true, c->lean))) return rc;
+    if ((rc = launch_combine<double>(c, din, a0, nr, dout + a0 * nb, true, c->lean, i + 1 == n))) return rc;
     SBDX_CUDA(c, cudaEventRecord(ev[n + i], c->stream));
   }
   for (size_t i = 0; i < n; ++i) {  // each chunk out as soon as it is ready

@@ -212,10 +212,10 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
       } else {
         uint32_t t[kB];
 #pragma unroll
-        for (int u = 0; u < kB; ++u) t[u] = P * u < cnt ? __ldg(ix + G * m + 32 * u) : 0u;
+        for (int u = 0; u < kB; ++u) t[u] = P * u < cnt ? __ldg(ix + G * m + 32 * u) : kNoRow;
 #pragma unroll
         for (int u = 0; u < kB; ++u)
-          if (P * u < cnt) acc = fma(cur[u], r[t[u]], acc);
+          if (t[u] != kNoRow) acc = fma(cur[u], r[t[u]], acc);
       }
 #pragma unroll
       for (int u = 0; u < kB; ++u) cur[u] = nxt[u];
@@ -310,14 +310,14 @@ int build_stored(Ctx* c) {
     total = G * (ca.total * ns + na * (uint64_t)psd[ns] + sa * ps[ns]);
     if (G == 1 || total <= nnz + nnz / 4) break;
   }
-  std::vector<uint32_t> idx(std::max<size_t>(1, G * psd[ns]), 0);
+  std::vector<uint32_t> idx(std::max<size_t>(1, G * psd[ns]), kNoRow);
   for (size_t t = 0; t < nb; ++t) {
     const size_t s = t / G, ls = ps[s + 1] - ps[s];
     const uint32_t b = perm[t];
     uint32_t* o = idx.data() + G * psd[s] + t % G;
-    // padding reads the row's own column, which its elements touch anyway, so an
-    // infinity elsewhere stays where the matrix puts it
-    for (uint32_t m = 0; m < psd[s + 1] - psd[s]; ++m) o[G * m] = (uint32_t)t;
+    // the kernel skips the padding, so that an infinity stays where the matrix
+    // puts it (zero times it is NaN)
+    for (uint32_t m = 0; m < psd[s + 1] - psd[s]; ++m) o[G * m] = kNoRow;
     for (uint32_t m = 0; m < bs[b] + bd[b]; ++m)
       o[G * (m < bs[b] ? (size_t)m : ls + m - bs[b])] = pos[bket[boff[b] + m]];
   }

@@ -215,23 +215,26 @@ constexpr int kAbPacks = 5;
 constexpr size_t kAbStaticSmem = 512;
 
 // Stored Hamiltonian (the reference's method 1): off-diagonal elements with the
-// basis phases folded in, in blocks of G determinants (ia; a slice of G beta
-// strings in the order `perm`, most single excitations first). Per block,
-// G values (one per string of the slice) for every alpha same-spin entry of
-// ia, then for every beta single and double of the slice's longest lists, then
-// for every alpha single of ia x every beta single of the slice (stored.cu).
+// basis phases folded in, in blocks of G determinants: a string r of one spin
+// ("rows") and a slice of G strings of the spin with more strings ("slices") in
+// the order `perm`, most single excitations first. Per block, G values (one per
+// string of the slice) for every same-spin entry of r, then for every single
+// and double of the slice's longest lists, then for every single of r x every
+// single of the slice (stored.cu).
 struct StoredH {
   double* val = nullptr;
-  uint64_t* rowbase = nullptr;  // [na] first value of the blocks of ia
-  uint32_t* perm = nullptr;     // [nb + 32] beta string of each position (kNoRow beyond nb)
+  uint64_t* rowbase = nullptr;  // [rows] first value of the blocks of r
+  uint32_t* perm = nullptr;     // [slice strings + 32] string of each position (kNoRow beyond them)
   uint32_t* idx = nullptr;      // [G * psd[nslice]] position of each lane's m-th excited string
   uint32_t *psd = nullptr, *ps = nullptr;  // [nslice + 1] prefix sums of singles + doubles, of singles, per slice
-  uint4* item = nullptr;        // [nitem] {ia, group of slices, alpha singles first | end << 16, 1 + slot or 0}
+  uint4* item = nullptr;        // [nitem] {r, group of slices, row singles first | end << 16, 1 + slot or 0}
   uint2* split = nullptr;       // per split item {first slot, slots}
   uint32_t *slot_split = nullptr, *done = nullptr;
   double* part = nullptr;       // partial rows, 256 per slot
   uint32_t nitem = 0;
   int width = 32, nslice = 0, warps = 8;  // G, slices, slices per CTA
+  int rows = 0;                 // spin of the rows (0 alpha, 1 beta)
+  bool direct = false;          // idx counts strings, not positions: the product reads the vector itself
   uint64_t nnz = 0;             // off-diagonal elements, padding not counted
 };
 

@@ -4,32 +4,39 @@
 // multiplies with them (mult, chemistry/tpb/mult.h:13-123): Wb[ih] += hij *
 // T[jh] after Wb += hii * T. Here the elements lie in blocks that share their
 // column lists:
-//   - a block is one alpha string ia and a slice of G = 32 beta strings ib, the
-//     strings with the most single excitations first so that the lists of a
-//     slice have like lengths; lane l of a warp owns row (ia, ib_l). Where the
-//     padding would be more than a quarter of the elements (few beta strings,
-//     lists of very different lengths) G is the largest power of two below that,
-//     and a warp takes 32 / G entries of the block at a time (at G = 1 nothing is
-//     padded);
-//   - its values, G per entry and one per row: the alpha same-spin entries of
-//     ia (columns (ja, ib_l): consecutive in the permuted vector), the beta
-//     singles and doubles of the slice (columns (ia, jb)), and the pairs of an
-//     alpha single of ia and a beta single (columns (ja, jb)), the same elements
-//     the on-the-fly sigma evaluates; shorter lists are padded with zeros;
-//   - the column lists are per slice (jb) and per alpha string (ja), so an
-//     element costs its 8 bytes;
+//   - a block is one string r of the spin with fewer strings and a slice of G =
+//     32 strings of the other, the strings with the most single excitations
+//     first so that the lists of a slice have like lengths; lane l of a warp owns
+//     row (r, s_l). Where the padding would be more than a tenth of the elements
+//     (few strings, lists of very different lengths) G is the largest power of
+//     two below that, and a warp takes 32 / G entries of the block at a time (at
+//     G = 1 nothing is padded). A quarter instead of a tenth is slower on nearly
+//     every shape: 150 x 1000 strings, 7 electrons in 58 orbitals, 231 us against
+//     181, 600 x 1000, 6 in 32, 646 against 572, 1000 x 1000, 5 in 24, 1077
+//     against 1054 (300 x 300, 7 in 58, 138 against 144); a twenty-fifth 191, 768
+//     and 1126. Only the smallest problems, short of warps for narrow slices' long
+//     chains, keep a quarter (150 x 150, 5 in 24: 24.7 us against 27.0);
+//   - its values, G per entry and one per row: the same-spin entries of r
+//     (columns (r', s_l): consecutive in the permuted vector), the singles and
+//     doubles of the slice (columns (r, s')), and the pairs of a single of r and
+//     one of the slice (columns (r', s')), the same elements the on-the-fly sigma
+//     evaluates; shorter lists are padded with zeros, which the product skips;
+//   - the column lists are per slice (s') and per row string (r'), so an element
+//     costs its 8 bytes;
 //   - the values carry the determinant phases, H_IJ = phi_I phi_J H'_IJ with
 //     H' the alpha-first-basis matrix of the sigma kernels; the diagonal stays
 //     in the context's hii vector.
-// The product permutes the vector's columns, then a CTA per alpha string and
-// group of slices streams the values, with the vector row that the current
-// entries gather from in shared memory. Deterministic (a lane sums its row in
-// one order). Bound: HBM, 8 bytes per element, and the latency of a warp's
-// stream. 1000 x 1000 strings, 575 M elements: 1.12 ms (4.1 TB/s); as CSR, 12 bytes
-// per element, a warp per row and 32 gather wavefronts per 32 elements, 1.62 ms.
-// Tighter register bounds spill (1.7 to 2.8 ms at 4 values in flight), 16 values
-// in flight took 1.24 ms, several slices per warp 2.0 ms: the warp with the
-// longest lists holds up the others at every staged row.
+// The product permutes the vector (the slices' spin innermost), then a CTA per
+// row string and group of slices streams the values, with the vector row that
+// the current entries gather from in shared memory. Deterministic (a lane sums
+// its row in one order). Bound: HBM, 8 bytes per element, and the latency of a
+// warp's stream. 1000 x 1000 strings, 575 M elements: 0.99 ms (4.6 TB/s); as CSR,
+// 12 bytes per element, a warp per row and 32 gather wavefronts per 32 elements,
+// 1.62 ms. 1000 x 150 strings: 130 us, with the slices over the spin with fewer
+// strings 205, as CSR 163. 150 x 150, where two launches and short streams are all,
+// 24.7 us, as CSR 22.2. Tighter register bounds spill (1.7 to 2.8 ms at 4
+// values in flight), 16 values in flight took 1.24 ms, several slices per warp
+// 2.0 ms: the warp with the longest lists holds up the others at every staged row.
 #include "sbdx.h"
 #include "sbdx_internal.cuh"
 
@@ -42,6 +49,7 @@ namespace {
 
 constexpr int kStoredThreads = 256;  // 8 warps
 constexpr int kStoredBatch = 8;      // values a lane has in flight
+constexpr size_t kDirectDets = size_t(1) << 15;  // up to here the product reads the vector itself
 
 // Same-spin element of entry e (first `ns` entries of the row are singles):
 // sign * (value + opposite-spin Coulomb term of a single, table row pq).
@@ -51,70 +59,78 @@ __device__ __forceinline__ double same_element(uint32_t inf, double v, bool sing
   return (inf >> 31) ? -v : v;
 }
 
-// First value of block (ia, s), in entries of G values from rowbase: the blocks
-// of ia follow each other, the entries of ia (ne of them, nas singles) per slice
+// First value of block (r, s), in entries of G values from rowbase: the blocks
+// of r follow each other, the entries of r (ne of them, ns singles) per slice
 // plus the slices' own lists.
-__device__ __forceinline__ uint64_t block_entry(uint64_t ne, uint64_t nas, int s, const uint32_t* __restrict__ psd,
+__device__ __forceinline__ uint64_t block_entry(uint64_t ne, uint64_t ns, int s, const uint32_t* __restrict__ psd,
                                                 const uint32_t* __restrict__ ps) {
-  return ne * s + psd[s] + nas * ps[s];
+  return ne * s + psd[s] + ns * ps[s];
 }
+
+// The phase of the determinant of a row and a slice string.
+__device__ __forceinline__ uint32_t block_phase(int rows, uint64_t r, uint64_t s) {
+  return rows == 0 ? basis_phase(prefix_parity(r), s) : basis_phase(prefix_parity(s), r);
+}
+
+// The lists of one spin, and its singles' Coulomb terms with each string of the
+// other one.
+struct SpinLists {
+  const uint64_t* str;
+  const uint64_t* off;
+  const uint32_t *ns, *ket, *info;
+  const double *val, *Dt;
+  size_t dstride;
+};
 
 // A warp per block.
 __global__ void __launch_bounds__(kStoredThreads)
-stored_fill_kernel(const uint64_t* __restrict__ astr, const uint64_t* __restrict__ bstr,
-                   const uint64_t* __restrict__ a_off, const uint32_t* __restrict__ a_ns,
-                   const uint32_t* __restrict__ a_ket, const double* __restrict__ a_val,
-                   const uint32_t* __restrict__ a_info, const uint64_t* __restrict__ b_off,
-                   const uint32_t* __restrict__ b_ns, const uint32_t* __restrict__ b_ket,
-                   const double* __restrict__ b_val, const uint32_t* __restrict__ b_info,
-                   const double* __restrict__ Da, size_t da_stride, const double* __restrict__ Db, size_t db_stride,
-                   const double* __restrict__ V, size_t vstride, const uint64_t* __restrict__ rowbase,
-                   const uint32_t* __restrict__ perm, const uint32_t* __restrict__ psd,
-                   const uint32_t* __restrict__ ps, int nslice, int G, double* __restrict__ val) {
+stored_fill_kernel(const SpinLists R, const SpinLists S, int rows, const double* __restrict__ V, size_t vstride,
+                   const uint64_t* __restrict__ rowbase, const uint32_t* __restrict__ perm,
+                   const uint32_t* __restrict__ psd, const uint32_t* __restrict__ ps, int nslice, int G,
+                   double* __restrict__ val) {
   const uint32_t lane = threadIdx.x & 31, col = lane & (G - 1), sub = lane / G, step = 32 / G;
-  const size_t ia = blockIdx.x;
-  const uint64_t a0 = a_off[ia], ne = a_off[ia + 1] - a0, nas = a_ns[ia];
-  const uint64_t ppa = prefix_parity(astr[ia]);
+  const size_t r = blockIdx.x;
+  const uint64_t a0 = R.off[r], ne = R.off[r + 1] - a0, nas = R.ns[r], rI = R.str[r];
   for (int s = blockIdx.y * (kStoredThreads / 32) + (threadIdx.x >> 5); s < nslice;
        s += gridDim.y * (kStoredThreads / 32)) {
-    double* out = val + rowbase[ia] + G * block_entry(ne, nas, s, psd, ps) + col;
-    const uint32_t ib = perm[G * s + col];
-    const bool in = ib != kNoRow;
-    const uint64_t bI = in ? bstr[ib] : 0ull;
-    const uint32_t phI = basis_phase(ppa, bI);
-    // alpha same-spin: (ja, ib)
+    double* out = val + rowbase[r] + G * block_entry(ne, nas, s, psd, ps) + col;
+    const uint32_t is = perm[G * s + col];
+    const bool in = is != kNoRow;
+    const uint64_t sI = in ? S.str[is] : 0ull;
+    const uint32_t phI = block_phase(rows, rI, sI);
+    // same-spin entries of r: (r', s)
     for (uint64_t k = sub; k < ne; k += step) {
       const uint64_t e = a0 + k;
-      double v = in ? same_element(a_info[e], a_val[e], k < nas, Db, db_stride, ib) : 0.0;
-      if (phI ^ basis_phase(prefix_parity(astr[a_ket[e]]), bI)) v = -v;
+      double v = in ? same_element(R.info[e], R.val[e], k < nas, R.Dt, R.dstride, is) : 0.0;
+      if (phI ^ block_phase(rows, R.str[R.ket[e]], sI)) v = -v;
       out[G * k] = v;
     }
     out += G * ne;
-    // beta same-spin: (ia, jb), singles then doubles, each padded to the slice's longest list
-    const uint64_t b0 = in ? b_off[ib] : 0, nbs = in ? b_ns[ib] : 0, nbd = in ? b_off[ib + 1] - b0 - nbs : 0;
+    // those of the slice: (r, s'), singles then doubles, each padded to the slice's longest list
+    const uint64_t b0 = in ? S.off[is] : 0, nbs = in ? S.ns[is] : 0, nbd = in ? S.off[is + 1] - b0 - nbs : 0;
     const uint32_t ls = ps[s + 1] - ps[s], ld = psd[s + 1] - psd[s] - ls;
     for (uint32_t m = sub; m < ls + ld; m += step) {
       const bool single = m < ls, has = single ? m < nbs : m - ls < nbd;
       double v = 0.0;
       if (has) {
         const uint64_t e = b0 + (single ? m : nbs + m - ls);
-        v = same_element(b_info[e], b_val[e], single, Da, da_stride, ia);
-        if (phI ^ basis_phase(ppa, bstr[b_ket[e]])) v = -v;
+        v = same_element(S.info[e], S.val[e], single, S.Dt, S.dstride, r);
+        if (phI ^ block_phase(rows, rI, S.str[S.ket[e]])) v = -v;
       }
       out[G * (size_t)m] = v;
     }
     out += G * (size_t)(ls + ld);
-    // alpha single x beta single: (ja, jb), s_a s_b (a i|b j)
+    // single of r x single of the slice: (r', s'), the two signs times (pair|pair)
     for (uint64_t ka = 0; ka < nas; ++ka, out += G * (size_t)ls) {
-      const uint32_t inf = a_info[a0 + ka];
+      const uint32_t inf = R.info[a0 + ka];
       const double* row = V + (size_t)((inf >> 12) & 0xfffu) * vstride;
-      const uint64_t ppj = prefix_parity(astr[a_ket[a0 + ka]]);
+      const uint64_t rJ = R.str[R.ket[a0 + ka]];
       for (uint32_t m = sub; m < ls; m += step) {
         double v = 0.0;
         if (m < nbs) {
-          const uint32_t ib_inf = b_info[b0 + m];
-          v = row[(ib_inf >> 12) & 0xfffu];
-          if ((inf >> 31) ^ (ib_inf >> 31) ^ phI ^ basis_phase(ppj, bstr[b_ket[b0 + m]])) v = -v;
+          const uint32_t s_inf = S.info[b0 + m];
+          v = row[(s_inf >> 12) & 0xfffu];
+          if ((inf >> 31) ^ (s_inf >> 31) ^ phI ^ block_phase(rows, rJ, S.str[S.ket[b0 + m]])) v = -v;
         }
         out[G * (size_t)m] = v;
       }
@@ -130,17 +146,37 @@ __global__ void permute_columns_kernel(const double* __restrict__ X, size_t nb, 
   Xq[blockIdx.y * xs + t] = t < nb ? X[blockIdx.y * nb + perm[t]] : 0.0;
 }
 
-// S = hii o X + H_offdiag X: CTA = work item (alpha string, up to 8 slices, one per
-// warp; or a range of the alpha singles of that, the partial rows added in item
-// order by the last of them to finish), longest first. Xq: X
-// with permuted columns. A block's values are one stream that the warp reads in
+// The same with the alpha strings in the slices: Xq[ib, t] = X[perm[t], ib], one
+// 32 x 32 tile per CTA.
+__global__ void __launch_bounds__(256)
+permute_rows_kernel(const double* __restrict__ X, size_t na, size_t nb, const uint32_t* __restrict__ perm, size_t xs,
+                    double* __restrict__ Xq) {
+  __shared__ double tile[32][33];
+  const size_t t0 = (size_t)blockIdx.x * 32, b0 = (size_t)blockIdx.y * 32;
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    const size_t t = t0 + k, ib = b0 + threadIdx.x;
+    tile[k][threadIdx.x] = t < na && ib < nb ? X[(size_t)perm[t] * nb + ib] : 0.0;
+  }
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
+    const size_t ib = b0 + k, t = t0 + threadIdx.x;
+    if (ib < nb && t < xs) Xq[ib * xs + t] = tile[threadIdx.x][k];
+  }
+}
+
+// S = hii o X + H_offdiag X: CTA = work item (row string, up to 8 slices, one per
+// warp; or a range of the singles of that, the partial rows added in item
+// order by the last of them to finish), longest first. Xq: the permuted vector.
+// A block's values are one stream that the warp reads in
 // batches, the next batch (of the next section too) loaded before the current
 // one is used. The vector row that the entries gather from is staged with
 // cp.async while the row before it is in use (kStaged), two buffers of xs
-// doubles; without room it is read from global memory.
-template <bool kStaged, int G>
+// doubles; without room it is read from global memory. kDirect: Xq is X itself,
+// rows of nb doubles (8-byte copies, and a gather for the entries of r: a launch
+// less for small problems).
+template <bool kStaged, bool kDirect, int G>
 __global__ void __launch_bounds__(kStoredThreads, 3)
-stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, const uint32_t* __restrict__ a_ns,
+stored_product_kernel(int row_spin, size_t nb, size_t nsl, size_t xs, const uint64_t* __restrict__ a_off, const uint32_t* __restrict__ a_ns,
                       const uint32_t* __restrict__ a_ket, const uint64_t* __restrict__ rowbase,
                       const uint32_t* __restrict__ perm, const uint32_t* __restrict__ idx,
                       const uint32_t* __restrict__ psd, const uint32_t* __restrict__ ps, int nslice,
@@ -151,17 +187,22 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
   extern __shared__ __align__(16) double rows[];  // [2][xs] when staged
   constexpr int kB = kStoredBatch, P = 32 / G;  // P entries per warp and load
   const int lane = threadIdx.x & 31, col = lane & (G - 1), sub = lane / G;
-  const uint4 item = items[blockIdx.x];  // ia, slice group, alpha singles [z & 0xffff, z >> 16), slot
+  const uint4 item = items[blockIdx.x];  // row string, slice group, its singles [z & 0xffff, z >> 16), slot
   const size_t ia = item.x;
   const int j0 = (int)(item.z & 0xffffu), j1 = (int)(item.z >> 16);
   const bool first = j0 == 0;  // the item with the same-spin entries
   const uint64_t a0 = a_off[ia];
   const int ne = (int)(a_off[ia + 1] - a0), nas = (int)a_ns[ia];
+  const size_t stride = kDirect ? nb : xs;
   auto stage = [&](int buf, size_t row) {
     if constexpr (kStaged) {
-      for (size_t t = 2 * threadIdx.x; t < xs; t += 2 * blockDim.x) {
+      constexpr int kStep = kDirect ? 1 : 2;
+      for (size_t t = kStep * threadIdx.x; t < (kDirect ? nb : xs); t += kStep * blockDim.x) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(rows + buf * xs + t);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(Xq + row * xs + t) : "memory");
+        if constexpr (kDirect)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(Xq + row * stride + t) : "memory");
+        else
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(Xq + row * stride + t) : "memory");
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
@@ -172,11 +213,12 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
   const bool active = s < nslice;
   const int lb = active ? (int)(psd[s + 1] - psd[s]) : 0, ls = active ? (int)(ps[s + 1] - ps[s]) : 0;
   const int na_e = active ? ne : 0;
-  // sections: -2 alpha same-spin entries, -1 beta same-spin, j >= 0 alpha single j with the beta singles
+  // sections: -2 same-spin entries of the row, -1 of the slice, j >= 0 single j with the slice's singles
   auto size = [&](int j) { return j == -2 ? na_e : j == -1 ? lb : j < j1 ? ls : 0; };
   const double* p = active ? val + rowbase[ia] + G * block_entry((uint64_t)ne, (uint64_t)nas, s, psd, ps) + lane : val;
   const uint32_t* ix = idx + (active ? (uint64_t)G * psd[s] : 0ull) + lane;
-  const double* xcol = Xq + min((size_t)G * (active ? s : 0) + col, xs - 1);  // values beyond nb are zero
+  const size_t at = (size_t)G * (active ? s : 0) + col;  // values beyond the strings are zero
+  const double* xcol = Xq + (kDirect ? (size_t)perm[min(at, nsl - 1)] : min(at, xs - 1));
   if (!first) p += G * ((int64_t)ne + lb + (int64_t)j0 * ls);
   double cur[kB], acc = 0.0;
   auto load = [&](double (&o)[kB], int n) {
@@ -184,7 +226,7 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
     for (int u = 0; u < kB; ++u) o[u] = P * u + sub < n ? __ldcs(p + 32 * u) : 0.0;
     p += G * (int64_t)n;
   };
-  load(cur, min(kB * P, !first ? ls : na_e > 0 ? na_e : lb));  // without beta entries there are no pairs either
+  load(cur, min(kB * P, !first ? ls : na_e > 0 ? na_e : lb));  // without slice entries there are no pairs either
   for (int j = first ? -2 : j0; j < j1; ++j) {
     const double* r = nullptr;
     if (j >= -1) {
@@ -195,7 +237,7 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
         if (j + 1 < j1) stage(buf ^ 1, a_ket[a0 + j + 1]);
         r = rows + buf * xs;
       } else {
-        r = Xq + (j < 0 ? ia : (size_t)a_ket[a0 + j]) * xs;
+        r = Xq + (j < 0 ? ia : (size_t)a_ket[a0 + j]) * stride;
       }
     }
     const int n = size(j);
@@ -206,7 +248,7 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
       if (j == -2) {
         double x[kB];
 #pragma unroll
-        for (int u = 0; u < kB; ++u) x[u] = P * u < cnt ? __ldg(xcol + (size_t)__ldg(a_ket + a0 + m + sub + P * u) * xs) : 0.0;
+        for (int u = 0; u < kB; ++u) x[u] = P * u < cnt ? __ldg(xcol + (size_t)__ldg(a_ket + a0 + m + sub + P * u) * stride) : 0.0;
 #pragma unroll
         for (int u = 0; u < kB; ++u) acc = fma(cur[u], x[u], acc);
       } else {
@@ -242,7 +284,7 @@ stored_product_kernel(size_t nb, size_t xs, const uint64_t* __restrict__ a_off, 
     for (uint32_t k = 0; k < sp.y; ++k) acc += __ldcg(part + (size_t)(sp.x + k) * kStoredThreads + threadIdx.x);
   }
   if (ib == kNoRow) return;
-  const size_t I = ia * nb + ib;
+  const size_t I = row_spin == 0 ? ia * nb + ib : ib * nb + ia;
   S[I] = fma(hii[I], X[I], acc);
 }
 
@@ -261,14 +303,17 @@ int build_stored(Ctx* c) {
   if (!c->have_hii) { int rc = diag_terms(c); if (rc) return rc; }
   if (int rc = ensure_coulomb_a(c)) return rc;
   release_stored(c);
-  const size_t na = c->na, nb = c->nb, D = na * nb;
+  const size_t D = c->na * c->nb;
   if (D > (size_t)UINT32_MAX) {  // a limit that callers can rely on, whatever the layout
     c->err = "build_hamiltonian: " + std::to_string(D) +
              " determinants exceed the stored matrix's 4294967295";
     return SBDX_ERR_ARG;
   }
-  const Conn& ca = c->conn[0];
-  const Conn& cb = c->conn[1];
+  // the slices run over the spin with more strings (below: b), the rows over the other (a)
+  const int rows = c->na > c->nb ? 1 : 0;
+  const Conn& ca = c->conn[rows];
+  const Conn& cb = c->conn[1 - rows];
+  const size_t na = ca.n, nb = cb.n;
   std::vector<uint32_t> as(na), bs(nb), bd(nb), bket(std::max<size_t>(1, cb.total));
   std::vector<uint64_t> aoff(na + 1), boff(nb + 1);
   auto down = [&](void* h, const void* d, size_t bytes) {
@@ -281,7 +326,8 @@ int build_stored(Ctx* c) {
   SBDX_CUDA(c, down(boff.data(), cb.off, sizeof(uint64_t) * (nb + 1)));
   if (cb.total) SBDX_CUDA(c, down(bket.data(), cb.ket, sizeof(uint32_t) * cb.total));
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
-  // beta strings with the most singles, then doubles, first
+  const bool direct = rows == 0 && D <= kDirectDets && 2 * sizeof(double) * pad8(nb) <= kAbSmemBudget;
+  // slice strings with the most singles, then doubles, first
   uint64_t sa = 0, sb = 0;
   for (uint32_t x : as) sa += x;
   for (uint32_t x : bs) sb += x;
@@ -308,7 +354,7 @@ int build_stored(Ctx* c) {
       psd[s + 1] = psd[s] + ls + ld;
     }
     total = G * (ca.total * ns + na * (uint64_t)psd[ns] + sa * ps[ns]);
-    if (G == 1 || total <= nnz + nnz / 4) break;
+    if (G == 1 || total <= nnz + nnz / (D <= kDirectDets ? 4 : 10)) break;
   }
   std::vector<uint32_t> idx(std::max<size_t>(1, G * psd[ns]), kNoRow);
   for (size_t t = 0; t < nb; ++t) {
@@ -319,7 +365,7 @@ int build_stored(Ctx* c) {
     // puts it (zero times it is NaN)
     for (uint32_t m = 0; m < psd[s + 1] - psd[s]; ++m) o[G * m] = kNoRow;
     for (uint32_t m = 0; m < bs[b] + bd[b]; ++m)
-      o[G * (m < bs[b] ? (size_t)m : ls + m - bs[b])] = pos[bket[boff[b] + m]];
+      o[G * (m < bs[b] ? (size_t)m : ls + m - bs[b])] = direct ? bket[boff[b] + m] : pos[bket[boff[b] + m]];
   }
   std::vector<uint64_t> rowbase(na);
   uint64_t base = 0;
@@ -328,9 +374,10 @@ int build_stored(Ctx* c) {
     base += G * ((aoff[a + 1] - aoff[a]) * ns + psd[ns] + (uint64_t)as[a] * ps[ns]);
   }
   // work items: a CTA walks its entries batch by batch, so the strings with the
-  // most excitations would be a serial chain much longer than the rest (1000 x 150
-  // strings, L = 24: 417 us without the split, 204 with it); items above a quarter of an SM slot's share are
-  // split over their alpha singles
+  // most excitations would be a serial chain much longer than the rest; items
+  // above a quarter of an SM slot's share are split over their row's singles,
+  // down to 48 batches (24 and 96: 150 x 200 strings 30.5 us against 34.9 and
+  // 41.3)
   constexpr size_t kMinCap = 48, kMaxWarps = kStoredThreads / 32;  // cap in batches
   const size_t ng = (ns + kMaxWarps - 1) / kMaxWarps, warps = (ns + ng - 1) / ng;  // few idle warps
   const auto batches = [&](uint64_t n) { return (n * G + 32 * kStoredBatch - 1) / (32 * kStoredBatch); };
@@ -385,6 +432,8 @@ int build_stored(Ctx* c) {
     return e != cudaSuccess ? e : cudaMemcpyAsync(*d, h.data(), bytes, cudaMemcpyHostToDevice, c->stream);
   };
   H.nslice = (int)ns;
+  H.rows = rows;
+  H.direct = direct;
   H.width = (int)G;
   H.warps = (int)warps;
   H.nitem = (uint32_t)item.size();
@@ -402,9 +451,13 @@ int build_stored(Ctx* c) {
     return SBDX_ERR_NOMEM;
   }
   const dim3 grid((unsigned)na, (unsigned)std::min<size_t>((ns + 7) / 8, 65535));
-  stored_fill_kernel<<<grid, kStoredThreads, 0, c->stream>>>(
-      c->d_a, c->d_b, ca.off, ca.nsing, ca.ket, ca.val, ca.info, cb.off, cb.nsing, cb.ket, cb.val, cb.info, c->d_Da,
-      c->da_stride, c->d_Db, c->db_stride, c->d_V, c->vstride, H.rowbase, H.perm, H.psd, H.ps, (int)ns, (int)G, H.val);
+  auto lists = [&](int spin) {
+    const Conn& cn = c->conn[spin];
+    return SpinLists{spin == 0 ? c->d_a : c->d_b, cn.off, cn.nsing, cn.ket, cn.info, cn.val, spin == 0 ? c->d_Db : c->d_Da,
+                     spin == 0 ? c->db_stride : c->da_stride};
+  };
+  stored_fill_kernel<<<grid, kStoredThreads, 0, c->stream>>>(lists(rows), lists(1 - rows), rows, c->d_V, c->vstride,
+                                                             H.rowbase, H.perm, H.psd, H.ps, (int)ns, (int)G, H.val);
   SBDX_LAUNCHED(c);
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));  // host vectors die at return
   H.nnz = nnz;
@@ -412,37 +465,47 @@ int build_stored(Ctx* c) {
   return 0;
 }
 
-// The permuted vector lies in the sigma's scratch (d_xp, row stride xsa).
+// The permuted vector lies in the sigma's scratch (d_xp, row stride xsa or,
+// with the alpha strings in the slices, xsb).
 int stored_sigma(Ctx* c, const double* X, double* S) {
   const StoredH& H = c->stored;
-  const size_t xs = c->xsa, smem = 2 * sizeof(double) * xs;
+  const size_t nrow = H.rows == 0 ? c->na : c->nb, nsl = H.rows == 0 ? c->nb : c->na;
+  const size_t xs = H.rows == 0 ? c->xsa : c->xsb, smem = 2 * sizeof(double) * xs;
   double* Xq = reinterpret_cast<double*>(c->d_xp);
-  // alpha rows in launches of at most 65535 (the y extent of a grid)
-  for (size_t a = 0; a < c->na; a += 65535) {
-    const dim3 grid((unsigned)((xs + 255) / 256), (unsigned)std::min<size_t>(65535, c->na - a));
-    permute_columns_kernel<<<grid, 256, 0, c->stream>>>(X + a * c->nb, c->nb, H.perm, xs, Xq + a * xs);
+  // rows in launches of at most 65535 blocks (the y extent of a grid)
+  if (H.rows == 1) {
+    const dim3 grid((unsigned)((xs + 31) / 32), (unsigned)((c->nb + 31) / 32));  // at most 65,536 beta strings here
+    permute_rows_kernel<<<grid, dim3(32, 8), 0, c->stream>>>(X, c->na, c->nb, H.perm, xs, Xq);
     SBDX_LAUNCHED(c);
+  } else if (!H.direct) {
+    for (size_t a = 0; a < c->na; a += 65535) {
+      const dim3 grid((unsigned)((xs + 255) / 256), (unsigned)std::min<size_t>(65535, c->na - a));
+      permute_columns_kernel<<<grid, 256, 0, c->stream>>>(X + a * c->nb, c->nb, H.perm, xs, Xq + a * xs);
+      SBDX_LAUNCHED(c);
+    }
   }
-  const Conn& ca = c->conn[0];
+  const Conn& cr = c->conn[H.rows];
   auto launch = [&](auto kernel, size_t bytes) -> int {
     SBDX_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAbSmemBudget));
-    kernel<<<H.nitem, 32 * H.warps, bytes, c->stream>>>(c->nb, xs, ca.off, ca.nsing, ca.ket, H.rowbase, H.perm, H.idx,
-                                                       H.psd, H.ps, H.nslice, H.val, c->d_hii, X, Xq, S, H.item,
-                                                       H.split, H.slot_split, H.done, H.part);
+    kernel<<<H.nitem, 32 * H.warps, bytes, c->stream>>>(H.rows, c->nb, nsl, xs, cr.off, cr.nsing, cr.ket, H.rowbase, H.perm,
+                                                       H.idx, H.psd, H.ps, H.nslice, H.val, c->d_hii, X,
+                                                       H.direct ? X : Xq, S, H.item, H.split, H.slot_split, H.done, H.part);
     SBDX_LAUNCHED(c);
     return 0;
   };
   // a CTA's rows gather from the staged one about as many elements as it has,
   // or more; narrow slices of many strings use too little of it
-  const bool staged = smem <= kAbSmemBudget && (H.width == 32 || c->nb <= 64 * (size_t)H.width);
-  auto pick = [&](auto st, auto unst) -> int { return staged ? launch(st, smem) : launch(unst, 0); };
+  const bool staged = H.direct || (smem <= kAbSmemBudget && (H.width == 32 || nsl <= 64 * (size_t)H.width));
+  auto pick = [&](auto st, auto unst, auto dir) -> int {
+    return H.direct ? launch(dir, smem) : staged ? launch(st, smem) : launch(unst, 0);
+  };
   switch (H.width) {
-    case 32: return pick(stored_product_kernel<true, 32>, stored_product_kernel<false, 32>);
-    case 16: return pick(stored_product_kernel<true, 16>, stored_product_kernel<false, 16>);
-    case 8: return pick(stored_product_kernel<true, 8>, stored_product_kernel<false, 8>);
-    case 4: return pick(stored_product_kernel<true, 4>, stored_product_kernel<false, 4>);
-    case 2: return pick(stored_product_kernel<true, 2>, stored_product_kernel<false, 2>);
-    default: return pick(stored_product_kernel<true, 1>, stored_product_kernel<false, 1>);
+    case 32: return pick(stored_product_kernel<true, false, 32>, stored_product_kernel<false, false, 32>, stored_product_kernel<true, true, 32>);
+    case 16: return pick(stored_product_kernel<true, false, 16>, stored_product_kernel<false, false, 16>, stored_product_kernel<true, true, 16>);
+    case 8: return pick(stored_product_kernel<true, false, 8>, stored_product_kernel<false, false, 8>, stored_product_kernel<true, true, 8>);
+    case 4: return pick(stored_product_kernel<true, false, 4>, stored_product_kernel<false, false, 4>, stored_product_kernel<true, true, 4>);
+    case 2: return pick(stored_product_kernel<true, false, 2>, stored_product_kernel<false, false, 2>, stored_product_kernel<true, true, 2>);
+    default: return pick(stored_product_kernel<true, false, 1>, stored_product_kernel<false, false, 1>, stored_product_kernel<true, true, 1>);
   }
 }
 

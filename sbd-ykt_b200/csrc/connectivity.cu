@@ -774,11 +774,11 @@ void free_row_range(Ctx* c) {
 }
 
 // Work items of the alpha rows [a0, a1) only, for a sigma that writes those
-// output rows (one shard of the alpha strings, or one chunk of a pipelined
-// product): the same-spin and alpha-beta items of build_same_items /
-// build_ab_items over that range, their caps derived from the range's own
-// work.
-int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r) {
+// output rows: the same-spin and alpha-beta items over that range, their caps
+// derived from the range's own work (one shard of the alpha strings), or the
+// FP64 same-spin items alone (one chunk of a pipelined product, which evaluates
+// the alpha-beta product of all rows in one launch).
+int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r, bool chunk) {
   free_range_items(c, r);
   const Conn& ca = c->conn[0];
   const size_t n = a1 - a0;
@@ -792,14 +792,14 @@ int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r) {
   hd.resize(n);
   int rc = build_same_items(c, r, hs, hd, c->nb, a0);
   if (rc) return rc;
-  for (int q = 0; q < 2; ++q)
+  for (int q = 0; q < (chunk ? 1 : 2); ++q)
     if ((rc = build_same_blocks(c, ca, c->h_a, a0, n, c->nb, q == 0 ? kBlkRows64 : kBlkRows32, r.blk[q]))) return rc;
-  return build_ab_items(c, r.ab, hs, c->nb, a0);
+  return chunk ? 0 : build_ab_items(c, r.ab, hs, c->nb, a0);
 }
 
 int build_row_range(Ctx* c, size_t a0, size_t a1) {
   free_row_range(c);
-  const int rc = build_range_items(c, a0, a1, c->range_conn);
+  const int rc = build_range_items(c, a0, a1, c->range_conn, false);
   if (rc) return rc;
   c->range_a0 = a0;
   c->range_a1 = a1;

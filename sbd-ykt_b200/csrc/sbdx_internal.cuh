@@ -245,6 +245,13 @@ struct Tune {
   bool by_size = false;  // same_code is the default: a product with few columns takes its own
 };
 
+// Alpha-row chunks of a host-buffer sigma.
+struct IoChunks {
+  std::vector<size_t> bounds;        // multiples of 8
+  std::vector<Conn> items;           // FP64 same-spin work items of each chunk's output rows
+  std::vector<cudaEvent_t> events;   // per chunk: input copied, output ready; then start, end
+};
+
 struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -329,10 +336,8 @@ struct Ctx {
   // copies run on io_copy beside the chunks' kernels on the context stream
   // (io_chunks_req: 0 automatic, 1 no pipeline, K >= 2 that many chunks)
   int io_chunks_req = 0;
-  std::vector<size_t> io_bounds;  // chunk boundaries, multiples of 8
-  std::vector<Conn> io_items;     // work items of each chunk's output rows
+  IoChunks io[2];  // for pageable buffers, for page-locked ones
   cudaStream_t io_copy = nullptr;
-  std::vector<cudaEvent_t> io_events;  // per chunk: input copied, output ready; then one for the last copy
   void* d_io_out = nullptr;
   // the wavefunction of the last Davidson solve, resident on the device:
   // wf_roots vectors of D FP64 (root r at d_wf + r*D), kept until the next
@@ -491,8 +496,9 @@ void free_connectivity(Ctx* c);
 // Work items of the output rows [a0, a1) (Ctx::range_conn) and their release.
 int build_row_range(Ctx* c, size_t a0, size_t a1);
 void free_row_range(Ctx* c);
-// The work items of rows [a0, a1) into r, and their release.
-int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r);
+// The work items of rows [a0, a1) into r, and their release. chunk: the FP64
+// same-spin ones only.
+int build_range_items(Ctx* c, size_t a0, size_t a1, Conn& r, bool chunk);
 void free_range_items(Ctx* c, Conn& r);
 void free_blocks(Ctx* c, SameBlocks& b);
 // The host-buffer sigma's chunks (their work items, copy stream, events).

@@ -2941,10 +2941,9 @@ int sigma_device(Ctx* c, int precision, const void* X, void* S) {
 // transpose (which read that chunk only). Once every chunk is in, the context
 // stream runs the alpha-beta product of all rows (it reads any ket row), then
 // per chunk the alpha same-spin work items of its rows and the combine of its
-// rows; the copy stream takes each
-// finished chunk out while the next one computes. Exposed: the first chunk's
-// copy in, the last chunk's beta same-spin product and the last chunk's copy
-// out.
+// rows; the copy stream takes each finished chunk out while the next one
+// computes. Exposed: the first chunk's copy in, the last chunk's beta same-spin
+// product and the last chunk's copy out.
 
 namespace {
 
@@ -2993,30 +2992,32 @@ std::vector<size_t> io_bounds_for(const Ctx* c, int K) {
   return b;
 }
 
-int build_io_chunks(Ctx* c, const std::vector<size_t>& bounds) {
-  free_io_chunks(c);
+void free_chunks(Ctx* c, IoChunks& io) {
+  for (auto& r : io.items) free_range_items(c, r);
+  for (auto e : io.events)
+    if (e) cudaEventDestroy(e);
+  io = IoChunks{};
+}
+
+int build_io_chunks(Ctx* c, IoChunks& io, const std::vector<size_t>& bounds) {
+  free_chunks(c, io);
   const size_t n = bounds.size() - 1;
-  c->io_items.resize(n);
+  io.items.resize(n);
   for (size_t i = 0; i < n; ++i) {
-    const int rc = build_range_items(c, bounds[i], bounds[i + 1], c->io_items[i]);
+    const int rc = build_range_items(c, bounds[i], bounds[i + 1], io.items[i], true);
     if (rc) return rc;
   }
-  SBDX_CUDA(c, cudaStreamCreateWithFlags(&c->io_copy, cudaStreamNonBlocking));
-  c->io_events.assign(2 * n + 2, nullptr);
-  for (auto& e : c->io_events) SBDX_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  c->io_bounds = bounds;  // last: a build that failed part way leaves no bounds, so the next call rebuilds
+  if (!c->io_copy) SBDX_CUDA(c, cudaStreamCreateWithFlags(&c->io_copy, cudaStreamNonBlocking));
+  io.events.assign(2 * n + 2, nullptr);
+  for (auto& e : io.events) SBDX_CUDA(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  io.bounds = bounds;  // last: a build that failed part way leaves no bounds, so the next call rebuilds
   return 0;
 }
 
 }  // namespace
 
 void free_io_chunks(Ctx* c) {
-  for (auto& r : c->io_items) free_range_items(c, r);
-  c->io_items.clear();
-  c->io_bounds.clear();
-  for (auto e : c->io_events)
-    if (e) cudaEventDestroy(e);
-  c->io_events.clear();
+  for (IoChunks& io : c->io) free_chunks(c, io);
   if (c->io_copy) cudaStreamDestroy(c->io_copy);
   c->io_copy = nullptr;
 }
@@ -3030,7 +3031,8 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
   double* din = static_cast<double*>(c->d_io_in);
   double* dout = static_cast<double*>(c->d_io_out);
   const Tune t = effective_tune(c, true);
-  const int K = io_chunk_count(c, page_locked(hC) && page_locked(hS));
+  const bool locked = page_locked(hC) && page_locked(hS);
+  const int K = io_chunk_count(c, locked);
   const bool pipe = K >= 2 && c->stored.val == nullptr && is_v6(t) && t.ab_code == 71 && !c->profiling;
   if (!pipe) {  // one copy in, the sigma, one copy out
     SBDX_CUDA(c, cudaMemcpyAsync(din, hC, sizeof(double) * D, cudaMemcpyHostToDevice, c->stream));
@@ -3039,12 +3041,13 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
     return 0;
   }
   const std::vector<size_t> want = io_bounds_for(c, K);
-  if (want != c->io_bounds) {
-    if ((rc = build_io_chunks(c, want))) return rc;
+  IoChunks& io = c->io[locked ? 1 : 0];  // a caller may use both kinds of buffers in turn
+  if (want != io.bounds) {
+    if ((rc = build_io_chunks(c, io, want))) return rc;
   }
-  const size_t n = c->io_bounds.size() - 1;
-  const std::vector<size_t>& b = c->io_bounds;
-  cudaEvent_t* ev = c->io_events.data();  // [0, n): chunk in; [n, 2n): chunk out ready; 2n: start; 2n + 1: end
+  const std::vector<size_t>& b = io.bounds;
+  const size_t n = b.size() - 1;
+  cudaEvent_t* ev = io.events.data();  // [0, n): chunk in; [n, 2n): chunk out ready; 2n: start; 2n + 1: end
   const Conn& ca = c->conn[0];
   const Conn& cb = c->conn[1];
   double* xp = static_cast<double*>(c->d_xp);
@@ -3077,7 +3080,7 @@ int sigma_host(Ctx* c, const double* hC, double* hS) {
   if (rc) return rc;
   for (size_t i = 0; i < n; ++i) {
     const size_t a0 = b[i], nr = b[i + 1] - b[i];
-    const Conn& it = c->io_items[i];
+    const Conn& it = io.items[i];
     Conn ra = ca;
     for (int q = 0; q < 2; ++q) ra.blk[q] = it.blk[q];
     ra.same_item = it.same_item;

@@ -133,3 +133,39 @@ def test_sigma_with_few_alpha_strings(size, port):
     assert np.array_equal(S, again)
     assert np.abs(rows.cpu().numpy() - ref.reshape(prob.na, prob.nb)[a0:]).max() <= 1e-12 * top
     assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top
+
+
+@pytest.mark.parametrize("size", [(58, 7, 14000, 41), (64, 8, 14000, 23)])
+def test_sigma_with_two_panels_of_bra_strings(size, port):
+    """More beta strings than y slots fit in shared memory beside the integrals of
+    many orbitals: the alpha-beta kernel runs once per panel. The alpha strings
+    are a sample's, with lists of very different lengths, so that some are split
+    into several items; whole products in both storage types and a row range."""
+    torch = pytest.importorskip("torch")
+    L, n, nb, na = size
+    I0, h, eri = synth.make_integrals(L, 16, 51)
+    prob = synth.Problem(L=L, nelec=2 * n, I0=I0, h=h, eri=eri, alpha=synth.sample_strings(L, n, na, 52),
+                         beta=synth.sample_strings(L, n, nb, 53), name="panels")
+    C = np.random.default_rng(54).standard_normal(prob.D)
+    x = torch.from_numpy(C).cuda()
+    s = torch.empty_like(x)
+    x32, s32 = x.float(), torch.empty(prob.D, dtype=torch.float32, device="cuda")
+    ref = port.sigma(prob, C)
+    top = np.abs(ref).max()
+    with sbdx.Context(0) as ctx:
+        ctx.load(prob)
+        ctx.set_tuning(22, 71)
+        ctx.sigma_device(sbdx.SBDX_FP64, x.data_ptr(), s.data_ptr())
+        before = ctx.launches
+        again = torch.empty_like(s)
+        ctx.sigma_device(sbdx.SBDX_FP64, x.data_ptr(), again.data_ptr())
+        assert ctx.launches - before >= 6  # split, two same-spin, combine and a launch per panel
+        ctx.sigma_device(sbdx.SBDX_FP32, x32.data_ptr(), s32.data_ptr())
+        a0 = na // 2 // 8 * 8
+        rows = torch.empty((na - a0, nb), dtype=torch.float64, device="cuda")
+        ctx.sigma_rows_device(sbdx.SBDX_FP64, x.data_ptr(), rows.data_ptr(), a0, na)
+        torch.cuda.synchronize()
+    assert np.abs(s.cpu().numpy() - ref).max() <= 1e-12 * top
+    assert torch.equal(s, again)
+    assert np.abs(rows.cpu().numpy() - ref.reshape(na, nb)[a0:]).max() <= 1e-12 * top
+    assert np.abs(s32.cpu().numpy() - ref).max() <= 2e-6 * top

@@ -338,8 +338,8 @@ __global__ void finalize_kernel(const double* __restrict__ partial, int nblk, do
 // The end of a reduction kernel with at most a few sums: the last CTA to arrive
 // adds the CTA partials of every row in the order of finalize_kernel (one
 // launch less per sum: a step of a small solve is bound by its launches; a
-// full solve at 400 x 400: 9.9 -> 9.4 ms, five roots: 30.5 -> 28.5 ms). ctr
-// is zero between launches; with out null the partials are left as they are.
+// full solve at 400 x 400: 9.9 -> 9.0 ms, two roots at 613 x 1187: 30.5 -> 28.5
+// ms). ctr is zero between launches; with out null the partials are left as they are.
 __device__ __forceinline__ void finish_sums(const double* partial, int rows, double* out, uint32_t* ctr, double* sh) {
   if (out == nullptr) return;
   __shared__ int s_last;

@@ -8,7 +8,10 @@
 // with every matrix element recomputed from the strings, as Hij does
 // (chemistry/basic/determinants.h:467-526).
 //
-// B200 form (one sigma = 5 launches):
+// B200 form: the alpha-first kernels (below, "the alpha-first sigma"), which
+// evaluate the product in the alpha-before-beta determinant ordering. The
+// kernels of the interleaved ordering (launch codes 1 to 49) are kept for
+// comparison; one such sigma is 5 launches:
 //   1. same-spin kernel over alpha rows of C: a CTA owns one bra alpha row ia
 //      and a strip of beta columns; it walks the connectivity list of ia
 //      (staged in shared memory) and streams the ket rows C[ja, strip]
@@ -29,6 +32,7 @@
 
 #include <cstdint>
 #include <type_traits>
+#include <vector>
 
 namespace sbdx {
 
@@ -1021,7 +1025,8 @@ int run_ab(Ctx* c, const T* X) {
 //   1. alpha same-spin on Xp -> Y                     (sigma_same_*_kernel)
 //   2. beta same-spin on Xpt -> Yt                    (sigma_same_*_kernel)
 //   3. alpha x beta on Xk -> Yab                      (sigma_ab_kernel)
-//   (steps 1 to 3 side by side where the context's streams allow it)
+//   (steps 1 to 3 side by side; in the lean form of large problems, Ctx::lean, one
+//   after another, step 3 on lanes written after step 2 and added to Y)
 //   4. S = phi o (Y + Yab + Yt^T) + hii o X           (combine_phase_kernel)
 // Step 1 includes the Coulomb terms of the alpha singles with the beta string,
 // step 3 those of the beta singles with the alpha string (one more integral
@@ -1548,7 +1553,7 @@ sigma_same_nonfinite_kernel(const int* __restrict__ nonfinite, const T* __restri
 // 1} in one 16-byte load per i, the operands of an even and an odd tile; it ends
 // with string l >> 2, columns 16 i + 4 (l & 3) .. + 3. Rows in shared memory are
 // 32 bytes longer than the strip, so the four kets that a quarter-warp reads
-// lie in different banks. Bound: the FP64 tensor pipe (67% busy at 4800 x 4800);
+// lie in different banks. Bound: the FP64 tensor pipe (72% busy at 4800 x 4800);
 // padding of the unions counts as work there. 8000 x 8000: 5.1 ms for the beta
 // side, where CUDA-core products of four strings per block took 7.5 ms and of
 // eight 6.0 ms (issue slots, 60% of the FP64 pipe); with the B operands loaded
@@ -2769,7 +2774,9 @@ int autotune(Ctx* c) {
   if (!c->ev[0])
     for (auto& e : c->ev) SBDX_CUDA(c, cudaEventCreate(&e));
   c->profiling = true;
-  const int same_cand[] = {32, 34, 38, 24, 28, 22};
+  // one code per kernel and launch shape: the blocked FP64 kernel has one, and
+  // the FP32 one takes at most 4 columns per thread
+  const std::vector<int> same_cand[2] = {{34, 24, 28, 22}, {34, 32, 24, 28, 22}};
   const int ab_cand[] = {71, 62, 61, 63, 64};
   for (int prec = 0; prec < 2 && rc == 0; ++prec) {
     const Tune saved = c->tune[prec];
@@ -2790,7 +2797,7 @@ int autotune(Ctx* c) {
     };
     int best_same = 0, best_ab = 0;
     double t_same = 1e300, t_ab = 1e300;
-    for (int sc : same_cand) {
+    for (int sc : same_cand[prec]) {
       double sm = 0, ab = 0;
       if ((rc = measure(sc, ab_cand[0], &sm, &ab))) break;
       if (sm < t_same) { t_same = sm; best_same = sc; }

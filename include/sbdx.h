@@ -49,7 +49,9 @@ typedef struct sbdx_ctx sbdx_ctx;
 int sbdx_ctx_create(sbdx_ctx** ctx, int device);
 int sbdx_ctx_destroy(sbdx_ctx* ctx);
 const char* sbdx_last_error(const sbdx_ctx* ctx);
-/* Stream used by all subsequent work (a cudaStream_t; NULL = legacy stream). */
+/* Stream used by all subsequent work (a cudaStream_t; NULL = legacy stream). That
+ * work follows what the context has queued on the stream before, which has to
+ * exist still: destroy a stream after the context has left it. */
 int sbdx_set_stream(sbdx_ctx* ctx, void* cuda_stream);
 /* Kernels launched by this context since creation (instrumentation). */
 unsigned long long sbdx_launch_count(const sbdx_ctx* ctx);
@@ -63,8 +65,9 @@ int sbdx_set_profiling(sbdx_ctx* ctx, int on);
 long long sbdx_phase_times(sbdx_ctx* ctx, double* ms, int n);
 /* Launch shapes of the sigma kernels (no reference counterpart), applied to
  * both precisions; 0 selects the built-in default (alpha-first kernels; the
- * blocked same-spin kernel from 2 M determinants in FP64 and 1 M with FP32
- * storage, the one-string-per-CTA kernel below).
+ * blocked same-spin kernel from 2 M determinants in FP64, for products of 448
+ * columns or more, and from 1 M with FP32 storage, the one-string-per-CTA kernel
+ * below).
  * Alpha-first kernels (the sigma evaluated in the alpha-before-beta
  * determinant ordering, conjugated by the +-1 basis phase):
  *   same_code: 21/22/24/28 = 1/2/4/8 columns per thread, one bra string per
@@ -116,8 +119,8 @@ int sbdx_get_connectivity(sbdx_ctx* ctx, int spin, uint64_t* slen, uint64_t* dle
  * makeQCham, chemistry/tpb/qcham.h:10-312, then the stored-element mult,
  * chemistry/tpb/mult.h:13-123). Builds every off-diagonal H_IJ on the device
  * (FP64 values with the determinant phases, 8 bytes per element, in blocks of one
- * alpha string and up to 32 beta strings that share their column lists; lists shorter
- * than the block's longest are padded) after the connectivity and the diagonal;
+ * string of one spin and up to 32 of the other that share their column lists; lists
+ * shorter than the block's longest are padded) after the connectivity and the diagonal;
  * from then on every FP64 sigma of this context (sbdx_sigma, sbdx_sigma_device
  * with SBDX_FP64, the Davidson solvers' FP64 products) is its sparse product,
  * and FP32 sigmas stay on the fly. *nnz (may be NULL) receives the number of

@@ -148,13 +148,13 @@ __global__ void diag_finalize_kernel(int L, const double* __restrict__ Pa, const
 }
 
 // G = A A^T of the n rows of A (K columns, row stride lda), lower tiles only,
-// from tile row bi0 on (G's first row is row 64 bi0): CTA = one 64 x 64 tile,
-// four warps of 32 x 32, m8n8k4 on the FP64
-// tensor pipe. The operands pass through shared memory in two stages of 16
-// columns (cp.async, zero beyond n and K); a lane reads two consecutive
-// columns per 16-byte load and uses them as the k-slots of two steps, the same
-// ones in A and B. Rows are padded to 24 doubles, so that the 8 lanes of a
-// quarter-warp (two rows) read 128 different bytes.
+// from tile t0 on, row r at G + r n (the caller's panel starts there: an offset
+// taken off at the stores costs 40 registers and a CTA per SM): CTA = one 64 x 64
+// tile, four warps of 32 x 32, m8n8k4 on the FP64 tensor pipe. The operands pass
+// through shared memory in two stages of 16 columns (cp.async, zero beyond n and
+// K); a lane reads two consecutive columns per 16-byte load and uses them as the
+// k-slots of two steps, the same ones in A and B. Rows are padded to 24 doubles, so
+// that the 8 lanes of a quarter-warp (two rows) read 128 different bytes.
 constexpr int kGramTile = 64, kGramK = 16, kGramPad = 24;
 __device__ __forceinline__ void dmma_m8n8k4(double (&d)[2], double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
@@ -162,10 +162,10 @@ __device__ __forceinline__ void dmma_m8n8k4(double (&d)[2], double a, double b) 
       : "d"(a), "d"(b));
 }
 __global__ void __launch_bounds__(128)
-gram_kernel(const double* __restrict__ A, size_t n, size_t K, size_t lda, double* __restrict__ G, size_t bi0) {
+gram_kernel(const double* __restrict__ A, size_t n, size_t K, size_t lda, double* __restrict__ G, size_t t0) {
   __shared__ __align__(16) double sm[2][2][kGramTile][kGramPad];  // [stage][operand]
   // tile t -> (bi, bj), bj <= bi
-  const size_t t = blockIdx.x + bi0 * (bi0 + 1) / 2;
+  const size_t t = blockIdx.x + t0;
   size_t bi = (size_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
   while (bi * (bi + 1) / 2 > t) --bi;
   while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
@@ -225,9 +225,8 @@ gram_kernel(const double* __restrict__ A, size_t n, size_t K, size_t lda, double
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const size_t c = bj * kGramTile + wc + 8 * j + 2 * q;
-      double* o = G + (r - kGramTile * bi0) * n + c;
-      if (c < n) o[0] = acc[i][j][0];
-      if (c + 1 < n) o[1] = acc[i][j][1];
+      if (c < n) G[r * n + c] = acc[i][j][0];
+      if (c + 1 < n) G[r * n + c + 1] = acc[i][j][1];
     }
   }
 }
@@ -715,18 +714,25 @@ __global__ void backward_eri_kernel(int L, const double* __restrict__ two, doubl
   g[t] = sum;
 }
 
-// Device scratch of one call, released on the context's stream.
+// Device scratch of one call, released on the context's stream; after more than
+// kTrimBytes of it the pool gives back what it does not keep.
 struct Scratch {
+  static constexpr size_t kTrimBytes = size_t(128) << 20;
   Ctx* c;
   std::vector<void*> p;
+  size_t bytes = 0;
   explicit Scratch(Ctx* ctx) : c(ctx) {}
   ~Scratch() {
     for (void* q : p) dev_free(c, q);
+    if (bytes > kTrimBytes) pool_trim(c);
   }
   template <typename T>
   cudaError_t get(T** d, size_t n) {
     const cudaError_t e = temp_alloc(c, d, sizeof(T) * std::max<size_t>(1, n));
-    if (e == cudaSuccess) p.push_back(*d);
+    if (e == cudaSuccess) {
+      p.push_back(*d);
+      bytes += sizeof(T) * n;
+    }
     return e;
   }
   // a copy of a host array; the array must stay until the stream has run
@@ -736,12 +742,6 @@ struct Scratch {
     if (e != cudaSuccess || h.empty()) return e;
     return cudaMemcpyAsync(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, c->stream);
   }
-};
-
-// At the end of a call, after its scratch: the pool keeps kPoolKeep bytes.
-struct Trim {
-  Ctx* c;
-  ~Trim() { pool_trim(c); }
 };
 
 constexpr size_t kMaxPartials = size_t(256) << 20;  // bytes of chunk partials at a time
@@ -833,7 +833,8 @@ static int rdm_same(Ctx* c, Scratch& sc, int spin, const double* Wm, size_t ldw,
     const size_t r1 = G ? std::min(n, r0 + prow) : n;
     if (G) {
       const size_t b0 = r0 / kGramTile, b1 = (r1 + kGramTile - 1) / kGramTile;
-      gram_kernel<<<(unsigned)((b1 * (b1 + 1) - b0 * (b0 + 1)) / 2), 128, 0, c->stream>>>(Wm, n, cols, ldw, G, b0);
+      gram_kernel<<<(unsigned)((b1 * (b1 + 1) - b0 * (b0 + 1)) / 2), 128, 0, c->stream>>>(Wm, n, cols, ldw, G - r0 * n,
+                                                                                         b0 * (b0 + 1) / 2);
       SBDX_LAUNCHED(c);
     }
     auto entries = [&](auto kernel) {
@@ -1039,7 +1040,6 @@ int rdm_device(Ctx* c, const double* dW, double* d_one, double* d_two) {
   const size_t na = c->na, nb = c->nb, L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
   SingleGroups S[2];
   std::vector<uint64_t> keep[2];  // host sources of copies, alive until the last synchronisation
-  const Trim trim{c};
   Scratch sc(c);
   double* wa = nullptr;
   SBDX_CUDA(c, sc.get(&wa, na + nb + 3 * L2));
@@ -1081,7 +1081,6 @@ int occupation_device(Ctx* c, const double* dW, double* d_density) {
   int rc = ensure_sigma_scratch(c);
   if (rc) return rc;
   const size_t na = c->na, nb = c->nb, L = (size_t)c->L, L2 = L * L;
-  const Trim trim{c};
   Scratch sc(c);
   double* wa = nullptr;
   SBDX_CUDA(c, sc.get(&wa, na + nb + 2 * L2));
@@ -1102,7 +1101,6 @@ int occupation_device(Ctx* c, const double* dW, double* d_density) {
 }
 
 int alpha_weights_device(Ctx* c, const double* dW, double* d_w) {
-  const Trim trim{c};
   const int rc = weights(c, dW, c->nb, d_w, nullptr, nullptr, nullptr, nullptr, nullptr, 0);
   if (rc) return rc;
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1116,7 +1114,6 @@ int backward_device(Ctx* c, const double* dW, double* dE_dh, double* dE_deri) {
   int rc = build_connectivity(c, false);
   if (rc) return rc;
   const size_t L = (size_t)c->L, L2 = L * L, L4 = L2 * L2;
-  const Trim trim{c};
   Scratch sc(c);
   double* one = nullptr;
   SBDX_CUDA(c, sc.get(&one, 2 * L2 + 4 * L4 + c->neri));

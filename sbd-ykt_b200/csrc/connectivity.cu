@@ -182,9 +182,12 @@ conn_fill_kernel(int spin, const uint64_t* __restrict__ s, size_t n, const uint6
   }
 }
 
-void free_ab_items(Ctx* c, AbItems& a) {
-  dev_free(c, a.item); dev_free(c, a.split); dev_free(c, a.slot); dev_free(c, a.done); dev_free(c, a.ypart);
-  a = AbItems{};
+void free_ab_items(Ctx* c, AbItems (&ab)[2]) {
+  dev_free(c, ab[0].ypart);  // both precisions'
+  for (AbItems& a : ab) {
+    dev_free(c, a.item); dev_free(c, a.split); dev_free(c, a.slot); dev_free(c, a.done);
+    a = AbItems{};
+  }
 }
 
 void free_conn(Ctx* c, Conn& cn) {
@@ -195,7 +198,7 @@ void free_conn(Ctx* c, Conn& cn) {
   SellPanel& p = cn.bal;
   dev_free(c, p.sell); dev_free(c, p.soff); dev_free(c, p.slen); dev_free(c, p.vrow); dev_free(c, p.vslot);
   dev_free(c, p.split_row); dev_free(c, p.split_slot);
-  for (AbItems& a : cn.ab) free_ab_items(c, a);
+  free_ab_items(c, cn.ab);
   dev_free(c, cn.same_item); dev_free(c, cn.same_split); dev_free(c, cn.same_slot); dev_free(c, cn.same_done); dev_free(c, cn.same_ypart);
   for (SameBlocks& b : cn.blk) free_blocks(c, b);
   cn = Conn{};
@@ -236,7 +239,7 @@ int upload_items(Ctx* c, const std::vector<uint4>& items, const std::vector<uint
   if (!split.empty()) {
     SBDX_CUDA(c, cudaMemcpyAsync(*d_split, split.data(), sizeof(uint4) * split.size(), cudaMemcpyHostToDevice,
                                  c->stream));
-    SBDX_CUDA(c, dev_alloc(c, d_part, sizeof(double) * (size_t)nslot * std::max<size_t>(8, pad8(ncol))));
+    if (d_part) SBDX_CUDA(c, dev_alloc(c, d_part, sizeof(double) * (size_t)nslot * std::max<size_t>(8, pad8(ncol))));
   }
   SBDX_CUDA(c, cudaStreamSynchronize(c->stream));  // host vectors die at return
   return 0;
@@ -516,7 +519,11 @@ int build_ab_items(Ctx* c, AbItems (&out)[2], std::vector<uint32_t> hs, size_t n
     A.n_split = (int)split.size();
     A.n_part = slot;
     int rc = upload_slots(c, split, slot, 1, &A.slot, &A.done);
-    if (rc || (rc = upload_items(c, items, split, slot, nb, &A.item, &A.split, &A.ypart))) return rc;
+    if (rc || (rc = upload_items(c, items, split, slot, nb, &A.item, &A.split, nullptr))) return rc;
+  }
+  if (const int most = std::max(out[0].n_part, out[1].n_part)) {  // one product runs at a time
+    SBDX_CUDA(c, dev_alloc(c, &out[0].ypart, sizeof(double) * (size_t)most * std::max<size_t>(8, pad8(nb))));
+    out[1].ypart = out[0].ypart;
   }
   return 0;
 }
@@ -760,7 +767,7 @@ void free_range_items(Ctx* c, Conn& r) {
   for (SameBlocks& b : r.blk) free_blocks(c, b);
   dev_free(c, r.same_item); dev_free(c, r.same_split); dev_free(c, r.same_slot); dev_free(c, r.same_done); dev_free(c, r.same_ypart);
   r.same_slot = r.same_done = nullptr;
-  for (AbItems& a : r.ab) free_ab_items(c, a);
+  free_ab_items(c, r.ab);
   r.same_item = r.same_split = nullptr;
   r.same_ypart = nullptr;
   r.n_same_item = 0;

@@ -148,7 +148,7 @@ struct AbItems {
   uint32_t* slot = nullptr;  // [n_part]: entry of split
   uint32_t* done = nullptr;  // [n_split]: items finished (zero between launches)
   int n_split = 0, n_part = 0;
-  double* ypart = nullptr;   // [n_part * pad8(nb)]
+  double* ypart = nullptr;   // [n_part * pad8(nb)], the larger of both precisions'
 };
 
 struct Conn {
